@@ -1330,81 +1330,144 @@ __global__ void __launch_bounds__(256)
   lo[c] = l;
 }
 
-// Column moments of an f32 density: one warp per (i,j) column, Kahan-compensated
-// FP32 sums along k, FP64 across columns (the reference's column scheme,
-// multigrid.py:192-221, finished in FP64). Block partials of the ten raw moments.
-__global__ void __launch_bounds__(256)
-    k_moments_rho(const float *__restrict__ rho, int G, double dx, double *__restrict__ parts, unsigned *status) {
-  const int lane = threadIdx.x & 31;
-  const long long col = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
-  double v[10];
+// Moments of an f32 density and, with b0, its h^2-scaled right-hand side
+// b0 = h^2 * f32(f32(4 pi G) * rho) with ||b0||^2, in one pass. A warp takes
+// eight neighbouring columns (i, j .. j+7) at a time, persistent over those
+// units: Kahan-compensated FP32 sums of rho, rho k and rho k^2 along k (the
+// reference's column scheme, multigrid.py:192-221), finished in FP64.
+//
+// Bound by HBM (read rho, write b0) once FP64 is kept out of the way: an FP64
+// warp instruction, conversions included, takes 16 clocks of the SM on this part.
+// So the lanes' column sums, unevaluated pairs s - c as they are, meet as FP32 pairs
+// in a reduce-scatter (9 pair additions per sum for eight columns) and only the
+// eight column totals become FP64; the block's sums are added by ten lanes, and
+// the last block finishes the grid's. Measured at 256^3: 405 us for the moments
+// (10 values reduced by FP64 shuffles in each of 8192 blocks) and 29 us for the
+// right-hand side before, 50 us for both now (99 us with the reduce-scatter in FP64);
+// at 64^3 33 + 3 us before, 12 now.
+#define MOM_COLS 8
+// (rh, rl) = (ah + al) + (bh + bl) as a pair
+__device__ __forceinline__ void pair_add(float ah, float al, float bh, float bl, float &rh, float &rl) {
+  float h, e;
+  df_two_sum(ah, bh, h, e);
+  df_fast_two_sum(h, __fadd_rn(e, __fadd_rn(al, bl)), rh, rl);
+}
+
+__global__ void __launch_bounds__(256, 2)
+    k_rhs_moments(const float *__restrict__ rho, float *__restrict__ b0, int G, double dx, float fpg, float h2,
+                  double *__restrict__ parts, unsigned *__restrict__ ticket, double *__restrict__ mom,
+                  double *__restrict__ bnorm2, unsigned *__restrict__ status) {
+  __shared__ double wsum[8 * MOM_COLS][11];
+  __shared__ double bsum[1];
+  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+  const int upr = (G + MOM_COLS - 1) / MOM_COLS;  // units per i
+  const long long nunits = (long long)G * upr;
+  // a row of sums per (warp, column): kept in shared memory, only its lane touches it
+  for (int t = threadIdx.x; t < 8 * MOM_COLS * 11; t += 256) (&wsum[0][0])[t] = 0.0;
+  __syncthreads();
+  float acc = 0.0f;
+  bool bad = false;
+  // the column of the unit whose sums this lane ends up with (bits 4, 3, 2 of the lane)
+  const int mine = lane >> 2;
+  for (long long u = (long long)blockIdx.x * 8 + wid; u < nunits; u += (long long)gridDim.x * 8) {
+    const int i = (int)(u / upr), j0 = (int)(u - (long long)i * upr) * MOM_COLS;
+    const int nc = G - j0 < MOM_COLS ? G - j0 : MOM_COLS;
+    const size_t at = ((size_t)i * G + j0) * G;
+    float s[3][MOM_COLS], c[3][MOM_COLS];
 #pragma unroll
-  for (int q = 0; q < 10; ++q) v[q] = 0.0;
-  if (col < (long long)G * G) {
-    const int i = (int)(col / G), j = (int)(col % G);
-    const float *p = rho + (size_t)col * G;
-    float s0 = 0.f, c0 = 0.f, s1 = 0.f, c1 = 0.f, s2 = 0.f, c2 = 0.f;
-    bool bad = false;
+    for (int t = 0; t < MOM_COLS; ++t)
+#pragma unroll
+      for (int q = 0; q < 3; ++q) s[q][t] = c[q][t] = 0.0f;
+    // the next 32 nodes of the columns are loaded while these are summed
+    float r[MOM_COLS], rn[MOM_COLS];
+    const float *src = rho + at + lane;
+#pragma unroll
+    for (int t = 0; t < MOM_COLS; ++t) rn[t] = t < nc && lane < G ? src[(size_t)t * G] : 0.0f;
     for (int k = lane; k < G; k += 32) {
-      const float r = p[k];
-      if (!isfinite(r)) { bad = true; continue; }
       const float fk = (float)k;
-      float y, t;
-      y = r - c0; t = s0 + y; c0 = (t - s0) - y; s0 = t;
-      const float r1 = r * fk;
-      y = r1 - c1; t = s1 + y; c1 = (t - s1) - y; s1 = t;
-      const float r2 = r1 * fk;
-      y = r2 - c2; t = s2 + y; c2 = (t - s2) - y; s2 = t;
+#pragma unroll
+      for (int t = 0; t < MOM_COLS; ++t) r[t] = rn[t];
+      src += 32;
+#pragma unroll
+      for (int t = 0; t < MOM_COLS; ++t) rn[t] = t < nc && k + 32 < G ? src[(size_t)t * G] : 0.0f;
+      if (b0) {
+#pragma unroll
+        for (int t = 0; t < MOM_COLS; ++t) {
+          const float bv = __fmul_rn(__fmul_rn(fpg, r[t]), h2);
+          if (t < nc) b0[at + (size_t)t * G + k] = bv;
+          acc += bv * bv;
+        }
+      }
+#pragma unroll
+      for (int t = 0; t < MOM_COLS; ++t) {
+        const bool fin = fabsf(r[t]) <= 3.402823466e38f;
+        bad |= !fin;
+        float x = fin ? r[t] : 0.0f;
+#pragma unroll
+        for (int q = 0; q < 3; ++q) {
+          const float y = __fsub_rn(x, c[q][t]), z = __fadd_rn(s[q][t], y);
+          c[q][t] = __fsub_rn(__fsub_rn(z, s[q][t]), y);
+          s[q][t] = z;
+          x = __fmul_rn(x, fk);
+        }
+      }
     }
-    if (bad) atomicOr(status, GC_FLAG_NONFINITE_RHO);
-    double S0 = (double)s0 - (double)c0, S1 = (double)s1 - (double)c1, S2 = (double)s2 - (double)c2;
-    for (int o = 16; o > 0; o >>= 1) {
-      S0 += __shfl_down_sync(0xffffffffu, S0, o);
-      S1 += __shfl_down_sync(0xffffffffu, S1, o);
-      S2 += __shfl_down_sync(0xffffffffu, S2, o);
+    double S[3];
+#pragma unroll
+    for (int q = 0; q < 3; ++q) {
+      // the lanes' pairs (s, -c) summed as pairs: lane bits 4, 3, 2 pick the column
+#pragma unroll
+      for (int t = 0; t < MOM_COLS; ++t) c[q][t] = -c[q][t];
+#pragma unroll
+      for (int w = MOM_COLS / 2, o = 16; w >= 1; w >>= 1, o >>= 1) {
+        const bool up = (lane & o) != 0;  // keeps the upper half of the columns
+#pragma unroll
+        for (int t = 0; t < MOM_COLS / 2; ++t) {
+          if (t >= w) break;
+          const float gh = __shfl_xor_sync(0xffffffffu, up ? s[q][t] : s[q][t + w], o);
+          const float gl = __shfl_xor_sync(0xffffffffu, up ? c[q][t] : c[q][t + w], o);
+          pair_add(up ? s[q][t + w] : s[q][t], up ? c[q][t + w] : c[q][t], gh, gl, s[q][t], c[q][t]);
+        }
+      }
+#pragma unroll
+      for (int o = 2; o >= 1; o >>= 1) {
+        const float gh = __shfl_xor_sync(0xffffffffu, s[q][0], o), gl = __shfl_xor_sync(0xffffffffu, c[q][0], o);
+        pair_add(s[q][0], c[q][0], gh, gl, s[q][0], c[q][0]);
+      }
+      S[q] = (double)s[q][0] + (double)c[q][0];
     }
-    if (lane == 0) {
-      const double vol = dx * dx * dx;
-      const double x = i * dx, y = j * dx;
-      const double m0 = S0 * vol, m1 = S1 * vol * dx, m2 = S2 * vol * dx * dx;
-      v[0] = m0; v[1] = m0 * x; v[2] = m0 * y; v[3] = m1;
-      v[4] = m0 * x * x; v[5] = m0 * y * y; v[6] = m2;
-      v[7] = m0 * x * y; v[8] = m1 * x; v[9] = m1 * y;
+    if ((lane & 3) == 0) {  // raw moments in node units; the spacing is applied at the end
+      const double x = (double)i, y = (double)(j0 + mine);
+      const double S0x = S[0] * x, S0y = S[0] * y;
+      double *v = wsum[wid * MOM_COLS + mine];
+      v[0] += S[0]; v[1] += S0x; v[2] += S0y; v[3] += S[1];
+      v[4] += S0x * x; v[5] += S0y * y; v[6] += S[2];
+      v[7] += S0x * y; v[8] += S[1] * x; v[9] += S[1] * y;
     }
   }
-  block_partials<10>(v, parts + (size_t)blockIdx.x * 10);
-}
-
-// b0 = h^2 * f32(f32(4 pi G) * rho); partial sums of b0^2 over all nodes.
-__global__ void __launch_bounds__(256)
-    k_rhs_from_rho(const float *__restrict__ rho, float *__restrict__ b0, size_t n, float fpg, float h2,
-                   double *__restrict__ parts) {
-  float acc = 0.0f;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x) {
-    const float rhs = __fmul_rn(fpg, rho[t]);
-    const float bv = __fmul_rn(rhs, h2);
-    b0[t] = bv;
-    acc += bv * bv;
+  if (bad) atomicOr(status, GC_FLAG_NONFINITE_RHO);
+  block_sum_f32(acc, bsum);  // (its barrier also orders wsum)
+  __syncthreads();
+  if (threadIdx.x < 10) {
+    const int q = threadIdx.x;
+    const double vol = dx * dx * dx;
+    const double sc = q == 0 ? vol : q <= 3 ? vol * dx : vol * dx * dx;
+    double a = 0.0;
+    for (int r = 0; r < 8 * MOM_COLS; ++r) a += wsum[r][q];
+    wsum[0][q] = a * sc;
   }
-  block_sum_f32(acc, parts + blockIdx.x);
-}
-
-__global__ void __launch_bounds__(256) k_sumsq(const float *__restrict__ a, size_t n, double *__restrict__ parts) {
-  float acc = 0.0f;
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
-    acc += a[t] * a[t];
-  block_sum_f32(acc, parts + blockIdx.x);
+  __syncthreads();
+  if (threadIdx.x == 0) {  // one writer: the last-block reduction fences its stores
+    for (int q = 0; q < 10; ++q) parts[(size_t)blockIdx.x * 11 + q] = wsum[0][q];
+    parts[(size_t)blockIdx.x * 11 + 10] = bsum[0];
+  }
+  if (grid_finish_sum<11>(parts, gridDim.x, ticket, mom) && threadIdx.x == 0 && b0) *bnorm2 = mom[10];
 }
 
 // Zero the interior nodes 1 .. G-2 of a G^3 array (node_grid launch shape).
 __global__ void __launch_bounds__(256) k_zero_interior(float *__restrict__ a, int G) {
   const int k = blockIdx.x * 32 + threadIdx.x + 1, j = blockIdx.y * 8 + threadIdx.y + 1, i = blockIdx.z + 1;
   if (k <= G - 2 && j <= G - 2) a[((size_t)i * G + j) * G + k] = 0.0f;
-}
-
-__global__ void k_copy_hi_to(const float *__restrict__ hi, float *__restrict__ out, size_t n) {
-  for (size_t t = blockIdx.x * (size_t)blockDim.x + threadIdx.x; t < n; t += (size_t)gridDim.x * blockDim.x)
-    out[t] = hi[t];
 }
 
 // ------------------------------------------------------------------------------
@@ -1753,17 +1816,6 @@ static int read_small(gc_ctx *ctx, int slot, int count) {
   return GC_OK;
 }
 
-// ||b0||^2 into dsmall[GC_S_BNORM2] (async).
-int gc_norm_b(gc_ctx *ctx) {
-  const size_t g3 = (size_t)ctx->G * ctx->G * ctx->G;
-  const int nb = 2048;
-  int st = gc_ensure_red(ctx, nb);
-  if (st) return st;
-  gc_launch(ctx, GK_REDUCE, k_sumsq, dim3(nb), dim3(256), 0, ctx->b0, g3, ctx->red);
-  GC_LAUNCH_CHECK(ctx, "sumsq");
-  return finalize_to(ctx, nb, 1, GC_S_BNORM2);
-}
-
 int gc_faces_from_moments(gc_ctx *ctx) {
   const long long tot = 6LL * ctx->G * ctx->G;
   gc_launch(ctx, GK_FACES, k_faces, dim3(gc_blocks(tot, 256)), dim3(256), 0, ctx->hi, ctx->lo, ctx->G, ctx->dx, ctx->grav, ctx->dmom);
@@ -1901,23 +1953,27 @@ int gc_mg_check_params(gc_ctx *ctx, const gc_mg_params *p) {
   return GC_OK;
 }
 
-// Moments of an f32 density into ctx->dmom (async). Raises GC_FLAG_NONFINITE_RHO.
-static int moments_rho_async(gc_ctx *ctx, const float *rho) {
-  const long long cols = (long long)ctx->G * ctx->G;
-  const unsigned nb = gc_blocks(cols, 8);
-  int s = gc_ensure_red(ctx, (size_t)nb * 10);
+// Moments of an f32 density into ctx->dmom and, when b0 is given, the right-hand
+// side and dsmall[GC_S_BNORM2] (async). Raises GC_FLAG_NONFINITE_RHO.
+static int rhs_moments_async(gc_ctx *ctx, const float *rho, float *b0) {
+  const long long units = (long long)ctx->G * ((ctx->G + MOM_COLS - 1) / MOM_COLS);
+  unsigned nb = gc_blocks(units, 8);
+  if (nb > gc_sms() * 2u) nb = gc_sms() * 2u;  // persistent: two CTAs per SM (registers)
+  int s = gc_ensure_red(ctx, (size_t)nb * 11);
   if (s) return s;
-  gc_launch(ctx, GK_MOMENTS, k_moments_rho, dim3(nb), dim3(256), 0, rho, ctx->G, ctx->dx, ctx->red, ctx->dstatus);
+  // b0 = h^2 * 4 pi G rho (multigrid.py:463)
+  gc_launch(ctx, b0 ? GK_RHS : GK_MOMENTS, k_rhs_moments, dim3(nb), dim3(256), 0, rho, b0, ctx->G, ctx->dx,
+            (float)(4.0 * M_PI * ctx->grav), (float)(ctx->dx * ctx->dx), ctx->red,
+            reinterpret_cast<unsigned *>(ctx->dsmall + GC_S_TICKET), ctx->dmom, ctx->dsmall + GC_S_BNORM2,
+            ctx->dstatus);
   GC_LAUNCH_CHECK(ctx, "moments");
-  if ((s = gc_finalize(ctx, ctx->red, (int)nb, 10, ctx->dmom))) return s;
-  GC_LAUNCH_CHECK(ctx, "moments finalize");
   return GC_OK;
 }
 
 extern "C" int gc_moments(gc_ctx *ctx, const float *rho, double out[10]) {
   if (!ctx) return GC_ERR_ARG;
   GC_REQUIRE(ctx, rho && out, "gc_moments: NULL pointer");
-  int s = moments_rho_async(ctx, rho);
+  int s = rhs_moments_async(ctx, rho, nullptr);
   if (s) return s;
   GC_CUDA(ctx, cudaMemcpyAsync(out, ctx->dmom, 10 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
   GC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
@@ -1936,18 +1992,8 @@ extern "C" int gc_mg_solve(gc_ctx *ctx, const float *rho, float *phi, int warm_s
   int s = gc_mg_check_params(ctx, &p);
   if (s) return s;
   const size_t g3 = (size_t)ctx->G * ctx->G * ctx->G;
-  // moments (multigrid.py:364-389), on the device, no host round trip
-  if ((s = moments_rho_async(ctx, rho))) return s;
-  // b0 = h^2 * 4 pi G rho (multigrid.py:463) and ||b0||^2 (multigrid.py:477)
-  {
-    const int nb = 2048;
-    if ((s = gc_ensure_red(ctx, nb))) return s;
-    const float fpg = (float)(4.0 * M_PI * ctx->grav);
-    const float h2 = (float)(ctx->dx * ctx->dx);
-    gc_launch(ctx, GK_RHS, k_rhs_from_rho, dim3(nb), dim3(256), 0, rho, ctx->b0, g3, fpg, h2, ctx->red);
-    GC_LAUNCH_CHECK(ctx, "rhs");
-    if ((s = finalize_to(ctx, nb, 1, GC_S_BNORM2))) return s;
-  }
+  // moments (multigrid.py:364-389), b0 and ||b0||^2 (multigrid.py:477), on the device
+  if ((s = rhs_moments_async(ctx, rho, ctx->b0))) return s;
   // initial guess (multigrid.py:464-467): previous phi or zero; the lo part starts at zero
   if (p.flags & GC_MG_FACES_GIVEN) {  // faces (and the guess) from phi
     GC_CUDA(ctx, cudaMemcpyAsync(ctx->hi, phi, g3 * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
@@ -1964,8 +2010,7 @@ extern "C" int gc_mg_solve(gc_ctx *ctx, const float *rho, float *phi, int warm_s
   if (!(p.flags & GC_MG_FACES_GIVEN) && (s = gc_faces_from_moments(ctx))) return s;
   if ((s = gc_mg_run(ctx, &p, stats))) return s;
   // phi = f32(hi + lo) == hi (the pair is normalised)
-  gc_launch(ctx, GK_COPY, k_copy_hi_to, dim3(1024), dim3(256), 0, ctx->hi, phi, g3);
-  GC_LAUNCH_CHECK(ctx, "copy phi");
+  GC_CUDA(ctx, cudaMemcpyAsync(phi, ctx->hi, g3 * sizeof(float), cudaMemcpyDeviceToDevice, ctx->stream));
   uint32_t flags = 0;
   if ((s = gc_status(ctx, &flags, 0))) return s;
   if (flags & GC_FLAG_NONFINITE_RHO) {
