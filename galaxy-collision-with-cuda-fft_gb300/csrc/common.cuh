@@ -417,7 +417,8 @@ int gc_finalize(gc_ctx *ctx, const double *parts, int nparts, int nv, double *ds
 int gc_fixed_point_setup(gc_ctx *ctx, const float *m, int64_t n, int bits, int mass_slot, int exp_slot);
 // int64 fixed-point CIC deposit into ctx->q (which must be zero on entry). Any
 // particle order; runs of equal cells (cell-sorted input) are summed in registers.
-int gc_deposit_q(gc_ctx *ctx, const float *x, const float *y, const float *z, const float *m, int64_t n,
+// `bits` is the fixed-point resolution *qexp was set up with (it only picks the pass).
+int gc_deposit_q(gc_ctx *ctx, const float *x, const float *y, const float *z, const float *m, int64_t n, int bits,
                  const double *qexp);
 // Read ctx->q, write rho (may be NULL) and b = f32(q 2^E 4 pi G h^2) (may be NULL),
 // zero q, and reduce the ten moments into ctx->dmom and ||b||^2 into dsmall[GC_S_BNORM2].

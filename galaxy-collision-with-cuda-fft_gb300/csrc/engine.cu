@@ -26,7 +26,8 @@ static int pm_solve(gc_ctx *ctx, const gc_particles *p, const gc_step_params *sp
   // the previous particle pass may have deposited these positions already
   const bool have_q = ctx->q_next_ready && sp->mode != GC_STEP_PRIME && (sp->flags & GC_STEP_DEPOSIT_NEXT);
   ctx->q_next_ready = 0;
-  if (!have_q && (s = gc_deposit_q(ctx, p->x, p->y, p->z, p->m, p->n, ctx->dsmall + GC_S_QEXP_PM))) return s;
+  if (!have_q && (s = gc_deposit_q(ctx, p->x, p->y, p->z, p->m, p->n, sp->fixed_point_bits,
+                                     ctx->dsmall + GC_S_QEXP_PM))) return s;
   // 2. b0, moments, ||b0||
   if ((s = gc_convert_q(ctx, ctx->dsmall + GC_S_QEXP_PM, nullptr, ctx->b0))) return s;
   // 3. initial guess and faces, then V-cycles

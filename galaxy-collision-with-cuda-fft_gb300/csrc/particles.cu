@@ -229,31 +229,43 @@ __global__ void __launch_bounds__(256)
 //
 // Into the shared-memory box (below) the warp keeps a run cell (dep_warp_runs):
 // lanes in it add their corners in registers, and the run is reduced across the
-// warp with one redux.sync per corner when the warp leaves the cell. Directly
-// into the grid (dep_warp_pass) the cells of lane 0 and lane 31 are the warp's
-// "main" cells, each reduced with one full-warp redux.sync per corner. In both,
-// lanes in any other cell (drifted particles, or sparse regions where every
-// particle has its own cell) add their own corners. A redux.sync over the full
+// warp with one redux.sync per corner when the warp leaves the cell. Lanes in any
+// other cell (drifted particles) add their own corners. A redux.sync over the full
 // warp costs the same whatever the keys, unlike one per group of equal keys,
-// which serialises over the groups.
+// which serialises over the groups. (dep_warp_pass, of the particle pass that
+// deposits too, reduces the cells of lane 0 and lane 31 instead.)
 //
 // Each warp owns an int32 box of nodes in shared memory (no block-wide
 // barriers: warps never wait for each other). Corners go to it when the cells
-// of the warp's 256 particles fit DEP_WBOX nodes (the box is the cell range of
+// of the warp's 256 particles fit the box (it is the cell range of
 // their coordinate range: x/dx is monotone) and their total quanta bound every
 // node below 2^31; the box is added to the int64 grid with one atomic per
-// nonzero node when the warp moves on. Otherwise corners go to the grid
-// directly. Particles whose contribution reaches 2^22 quanta (point masses) are
+// nonzero node when the warp moves on. Otherwise every lane's corners go to the
+// grid directly (dep_warp_direct). Particles whose contribution reaches 2^22 quanta (point masses) are
 // deposited out of line at the end of the tile with the general int64
 // rounding. Correct for any particle order;
 // the sort makes it fast.
+//
+// WIDE is the same pass for fine quanta, where ordinary particles reach 2^22 of
+// them (2^52 quanta in all, the default, below 2^30 particles): a corner value
+// up to 2^41 quanta is split as h 2^20 + l with |l| <= 2^19 by two fused
+// multiply-adds (dep_corners_wide), and h and l are summed separately in
+// int32, each with its own half of the box. One particle per thread went to the
+// grid with eight int64 atomics before. Measured, 1.5M particles sorted on a
+// 100^3 grid at 2^-52 of the mass: 327 us before, 21 us now.
 #define DEP_NONE 0xffffffffu
 #define DEP_PER 8
-#define DEP_TILE (256 * DEP_PER)
-#define DEP_BOX 8192
-#define DEP_WBOX (DEP_BOX / 8)  // nodes of one warp's box
-static_assert(DEP_WBOX <= 1024, "the box flush's reciprocal quotients are exact below 2^10 nodes");
+#define DEP_WTILE (32 * DEP_PER)  // particles of one warp
+template <bool WIDE>
+struct DepW {
+  static constexpr int box = WIDE ? 768 : 1024;         // nodes of one warp's box
+  static constexpr float limit = WIDE ? 2199023255552.0f : 4194304.0f;  // 2^41, 2^22: largest quanta in the pass
+  static constexpr int words = WIDE ? 2 * box : box;    // shared memory of a warp (int32)
+};
+static_assert(DepW<false>::box <= 1024 && DepW<true>::box <= 1024,
+              "the box flush's reciprocal quotients are exact below 2^10 nodes");
 #define DEP_BIAS 0x4B400000u
+#define DEP_BIAS_H 0x55400000u  // the bits of 1.5 * 2^43
 
 // Packed f32x2 arithmetic (two lanes of a 64-bit register, IEEE round to
 // nearest per lane).
@@ -291,6 +303,34 @@ __device__ __forceinline__ void dep_corners(float s, float wx0, float fx, float 
   r[2] = __float_as_uint(r23.x); r[3] = __float_as_uint(r23.y);
   r[4] = __float_as_uint(r45.x); r[5] = __float_as_uint(r45.y);
   r[6] = __float_as_uint(r67.x); r[7] = __float_as_uint(r67.y);
+}
+
+// The same corner values for |s| < 2^41 quanta, as h 2^20 + l: F = b * wz + 1.5 * 2^43
+// has spacing 2^20, so h = (F - 1.5 * 2^43) / 2^20 is the product rounded to a
+// multiple of 2^20; 1.5 * 2^23 - h 2^20 = (1.5 * 2^43 + 1.5 * 2^23) - F is exact (a
+// multiple of 2^20 below 2^44), and b * wz plus it is one fused multiply-add
+// of spacing 1 around 1.5 * 2^23: l is the exact remainder rounded to the nearest
+// integer (ties to even, as of the whole product: h 2^20 is even). So h 2^20 + l is
+// the exact product rounded once.
+__device__ __forceinline__ void dep_corners_wide(float s, float wx0, float fx, float wy0, float fy, float wz0,
+                                                 float fz, int (&h)[8], int (&l)[8]) {
+  const float2 a = f2_mul(make_float2(s, s), make_float2(wx0, fx));
+  const float2 wy = make_float2(wy0, fy), wz = make_float2(wz0, fz);
+  const float2 b[2] = {f2_mul(make_float2(a.x, a.x), wy), f2_mul(make_float2(a.y, a.y), wy)};
+  const float2 M = make_float2(13194139533312.0f, 13194139533312.0f);  // 1.5 * 2^43
+  const float2 K = make_float2(13194152116224.0f, 13194152116224.0f);  // ... + 1.5 * 2^23
+  const float2 neg = make_float2(-1.0f, -1.0f);
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const float bv = (p & 1) ? b[p >> 1].y : b[p >> 1].x;
+    const float2 bb = make_float2(bv, bv);
+    const float2 F = f2_fma(bb, wz, M);
+    const float2 L = f2_fma(bb, wz, f2_fma(F, neg, K));
+    h[2 * p] = (int)(__float_as_uint(F.x) - DEP_BIAS_H);
+    h[2 * p + 1] = (int)(__float_as_uint(F.y) - DEP_BIAS_H);
+    l[2 * p] = (int)(__float_as_uint(L.x) - DEP_BIAS);
+    l[2 * p + 1] = (int)(__float_as_uint(L.y) - DEP_BIAS);
+  }
 }
 
 // Corner contributions of a particle whose mass exceeds 2^22 quanta.
@@ -516,44 +556,149 @@ __device__ __forceinline__ void dep_warp_runs(const float (&px)[NJ], const float
   }
 }
 
+// The same for fine quanta, the two halves of the corner values side by side.
+__device__ __forceinline__ void dep_box_add_wide(int *bp, const DepBox &bx, const int (&l)[8], const int (&h)[8]) {
+  const int nz = bx.nz, nyz = bx.nyz;
+#pragma unroll
+  for (int c = 0; c < 8; ++c) {
+    int *q = bp + (c >> 2) * nyz + ((c >> 1) & 1) * nz + (c & 1);
+    atomicAdd(q, l[c]);
+    atomicAdd(q + DepW<true>::box, h[c]);
+  }
+}
+
+template <bool POW2, int NJ = DEP_PER>
+__device__ __forceinline__ void dep_warp_runs_wide(const float (&px)[NJ], const float (&py)[NJ], const float (&pz)[NJ],
+                                              const float (&pm)[NJ], long long nrem, const DepCtx &d, float inv_dx,
+                                              float qscale, const DepBox &bx, unsigned *__restrict__ status, int lane,
+                                              unsigned &large) {
+  const int G1 = d.G + 1;
+  const float hi = (float)d.G;
+  unsigned K = DEP_NONE;  // the run's cell (warp-uniform) ...
+  int Kbo = 0;            // ... and its node in the box
+  int acc[8], acch[8];
+#pragma unroll
+  for (int c = 0; c < 8; ++c) acc[c] = acch[c] = 0;
+  // one lane's sums of the warp, into the box
+  auto reduce_put = [&](bool mine, int bo, bool in, const int (&l)[8], const int (&h)[8]) {
+    int t[8], th[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      t[c] = __reduce_add_sync(0xffffffffu, in ? l[c] : 0);
+      th[c] = __reduce_add_sync(0xffffffffu, in ? h[c] : 0);
+    }
+    if (mine) dep_box_add_wide(bx.b + bo, bx, t, th);
+  };
+#pragma unroll
+  for (int j = 0; j < NJ; ++j) {
+    float gx, gy, gz;
+    if (POW2) {  // x / dx == x * (1/dx) exactly when dx is a power of two
+      gx = __fmul_rn(px[j], inv_dx); gy = __fmul_rn(py[j], inv_dx); gz = __fmul_rn(pz[j], inv_dx);
+    } else {
+      gx = __fdiv_rn(px[j], d.dx); gy = __fdiv_rn(py[j], d.dx); gz = __fdiv_rn(pz[j], d.dx);
+    }
+    const bool inr = gx >= -1.0f && gx < hi && gy >= -1.0f && gy < hi && gz >= -1.0f && gz < hi;
+    const int ix = __float2int_rd(gx), iy = __float2int_rd(gy), iz = __float2int_rd(gz);
+    const float fx = __fsub_rn(gx, __int2float_rn(ix)), fy = __fsub_rn(gy, __int2float_rn(iy)),
+                fz = __fsub_rn(gz, __int2float_rn(iz));
+    const float mmq = __fmul_rn(__fmul_rn(pm[j], d.inv_vol), qscale);
+    const bool small = fabsf(mmq) < DepW<true>::limit;
+    if (!inr && 32 * j < nrem && !gc_finite3(px[j], py[j], pz[j])) atomicOr(status, GC_FLAG_NONFINITE_POS);
+    if (inr && !small) large |= 1u << j;
+    const bool ok = inr && small;
+    const float s = ok ? mmq : 0.0f;
+    const float wx0 = __fsub_rn(1.0f, fx), wy0 = __fsub_rn(1.0f, fy), wz0 = __fsub_rn(1.0f, fz);
+    int v[8], vh[8];
+    dep_corners_wide(s, wx0, fx, wy0, fy, wz0, fz, vh, v);
+    const unsigned key = ok ? (unsigned)(((ix + 1) * G1 + (iy + 1)) * G1 + (iz + 1)) : DEP_NONE;
+    // the lane's node in the box (unsigned: a lane without a key may hold any cell)
+    const int bo = (int)((((unsigned)ix - (unsigned)bx.x0) * (unsigned)bx.ny + ((unsigned)iy - (unsigned)bx.y0)) *
+                             (unsigned)bx.nz +
+                         ((unsigned)iz - (unsigned)bx.z0));
+    if (!__any_sync(0xffffffffu, K != DEP_NONE && key == K)) {  // the run has ended (warp-uniform)
+      if (K != DEP_NONE) reduce_put(lane == 0, Kbo, true, acc, acch);
+      const unsigned have = __ballot_sync(0xffffffffu, key != DEP_NONE);
+      const int src = have ? __ffs(have) - 1 : 0;
+      K = have ? __shfl_sync(0xffffffffu, key, src) : DEP_NONE;
+      Kbo = __shfl_sync(0xffffffffu, bo, src);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) acc[c] = acch[c] = 0;
+    }
+    const bool inK = K != DEP_NONE && key == K;
+    if (inK) {
+#pragma unroll
+      for (int c = 0; c < 8; ++c) {
+        acc[c] += v[c];
+        acch[c] += vh[c];
+      }
+    }
+    const unsigned kB = __shfl_sync(0xffffffffu, key, 31);
+    const bool bnext = kB != K && kB != DEP_NONE;  // lane 31 already in another cell (warp-uniform)
+    const bool inB = bnext && key == kB;
+    if (bnext) reduce_put(lane == 31, bo, inB, v, vh);
+    if (key != DEP_NONE && !inK && !inB) dep_box_add_wide(bx.b + bo, bx, v, vh);
+  }
+  if (K != DEP_NONE) reduce_put(lane == 0, Kbo, true, acc, acch);
+}
+
 // The warp's particles straight into the grid (a tile whose cells do not fit the
-// box): out of line, reloading the particles, so that the registers of the box
-// path are not shaped by this rare one. Returns the `large` bits.
+// box: sparse regions, where hardly two lanes share a cell): every lane adds its
+// own corners, up to 2^41 quanta. Out of line, reloading the particles, so that
+// the registers of the box path are not shaped by this rare one. Returns the
+// `large` bits. (Reducing the cells of lanes 0 and 31 across the warp first, as
+// dep_warp_pass does, cost more than it merged: the deposit of 1.9M particles on
+// 128^3 took 33 us with it, 19 without; of 10M on 256^3 75 and 64 us.)
 template <bool POW2>
 __device__ __noinline__ unsigned dep_warp_direct(const float *__restrict__ x, const float *__restrict__ y,
-                                                 const float *__restrict__ z, const float *__restrict__ m, long long wb,
-                                                 long long nrem, const DepCtx d, float inv_dx, float qscale,
-                                                 long long *__restrict__ qg, unsigned *__restrict__ status, int lane) {
-  float px[DEP_PER], py[DEP_PER], pz[DEP_PER], pm[DEP_PER];
-#pragma unroll
-  for (int j = 0; j < DEP_PER; ++j) {
-    if (32 * j < nrem) {
-      px[j] = __ldg(x + wb + 32 * j); py[j] = __ldg(y + wb + 32 * j); pz[j] = __ldg(z + wb + 32 * j);
-      pm[j] = __ldg(m + wb + 32 * j);
-    } else {
-      px[j] = py[j] = pz[j] = __int_as_float(0x7fc00000);
-      pm[j] = 0.0f;
-    }
-  }
-  DepBox bx = {};
+                                                      const float *__restrict__ z, const float *__restrict__ m,
+                                                      long long wb, long long nrem, const DepCtx d, float inv_dx,
+                                                      float qscale, long long *__restrict__ qg,
+                                                      unsigned *__restrict__ status) {
   unsigned large = 0;
-  dep_warp_pass<POW2, false>(px, py, pz, pm, nrem, d, inv_dx, qscale, bx, qg, status, lane, large);
+#pragma unroll 2
+  for (int j = 0; j < DEP_PER; ++j) {
+    if (32 * j >= nrem) break;
+    const float px = __ldg(x + wb + 32 * j), py = __ldg(y + wb + 32 * j), pz = __ldg(z + wb + 32 * j);
+    const float mmq = __fmul_rn(__fmul_rn(__ldg(m + wb + 32 * j), d.inv_vol), qscale);
+    const float gx = POW2 ? __fmul_rn(px, inv_dx) : __fdiv_rn(px, d.dx);
+    const float gy = POW2 ? __fmul_rn(py, inv_dx) : __fdiv_rn(py, d.dx);
+    const float gz = POW2 ? __fmul_rn(pz, inv_dx) : __fdiv_rn(pz, d.dx);
+    const float hi = (float)d.G;
+    if (!(gx >= -1.0f && gx < hi && gy >= -1.0f && gy < hi && gz >= -1.0f && gz < hi)) {
+      if (!gc_finite3(px, py, pz)) atomicOr(status, GC_FLAG_NONFINITE_POS);
+      continue;
+    }
+    if (!(fabsf(mmq) < DepW<true>::limit)) {
+      large |= 1u << j;
+      continue;
+    }
+    const int ix = __float2int_rd(gx), iy = __float2int_rd(gy), iz = __float2int_rd(gz);
+    const float fx = __fsub_rn(gx, __int2float_rn(ix)), fy = __fsub_rn(gy, __int2float_rn(iy)),
+                fz = __fsub_rn(gz, __int2float_rn(iz));
+    int h[8], l[8];
+    dep_corners_wide(mmq, __fsub_rn(1.0f, fx), fx, __fsub_rn(1.0f, fy), fy, __fsub_rn(1.0f, fz), fz, h, l);
+    long long q[8];
+#pragma unroll
+    for (int c = 0; c < 8; ++c) q[c] = (long long)h[c] * 1048576LL + l[c];
+    corners_to_grid(qg, d.G, ix, iy, iz, q);
+  }
   return large;
 }
 
-template <bool POW2>
-__global__ void __launch_bounds__(256, 4)
+template <bool POW2, bool WIDE, int WARPS>
+__global__ void __launch_bounds__(32 * WARPS, (WIDE ? 3 : 4) * (8 / WARPS))
     k_deposit_sorted(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
                      const float *__restrict__ m, long long n, DepCtx d, float inv_dx,
                      const double *__restrict__ qexp, long long *__restrict__ qg, unsigned *__restrict__ status) {
-  __shared__ int box[DEP_BOX];
+  __shared__ int dep_box[WARPS * DepW<WIDE>::words];
   const float qscale = ldexpf(1.0f, -(int)(*qexp));
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  int *wbox = box + warp * DEP_WBOX;  // each warp owns a box: no block-wide barriers
-  for (int i = lane; i < DEP_WBOX; i += 32) wbox[i] = 0;  // every flush zeroes what it read
+  constexpr int tile = WARPS * DEP_WTILE;
+  int *wbox = dep_box + warp * DepW<WIDE>::words;  // each warp owns a box: no block-wide barriers
+  for (int i = lane; i < DepW<WIDE>::words; i += 32) wbox[i] = 0;  // every flush zeroes what it read
   __syncwarp();
-  for (long long t0 = (long long)blockIdx.x * DEP_TILE; t0 < n; t0 += (long long)gridDim.x * DEP_TILE) {
-    const long long wb = t0 + warp * (32 * DEP_PER) + lane;
+  for (long long t0 = (long long)blockIdx.x * tile; t0 < n; t0 += (long long)gridDim.x * tile) {
+    const long long wb = t0 + warp * DEP_WTILE + lane;
     const long long nrem = n - wb;  // particle j of this lane exists when 32 j < nrem
     if (nrem + lane <= 0) continue;  // this warp's part of the last tile is empty (warp-uniform)
     float px[DEP_PER], py[DEP_PER], pz[DEP_PER], pm[DEP_PER];
@@ -602,16 +747,18 @@ __global__ void __launch_bounds__(256, 4)
       bx.ny = hi[1] - lo[1] + 2;
       bx.nz = hi[2] - lo[2] + 2;
       bx.nyz = bx.ny * bx.nz;
-      // every small corner is at most min(largest |m| in quanta, 2^22) + 1/2
+      // every small corner is at most min(largest |m| in quanta, 2^22) + 1/2; a wide
+      // one's halves are at most 2^21 and 2^19, so 256 of them stay below 2^30
       const float mq = __fmul_rn(__fmul_rn(__uint_as_float(mb), d.inv_vol), qscale);
-      use_box = hi[0] >= lo[0] && (long long)nx * bx.nyz <= DEP_WBOX &&
-                __fmul_rn(fminf(mq, 4194304.0f) + 1.0f, (float)(32 * DEP_PER)) < 1073741824.0f;
+      use_box = hi[0] >= lo[0] && (long long)nx * bx.nyz <= DepW<WIDE>::box &&
+                (WIDE || __fmul_rn(fminf(mq, 4194304.0f) + 1.0f, (float)DEP_WTILE) < 1073741824.0f);
     }
     unsigned large = 0;
     if (use_box)
-      dep_warp_runs<POW2>(px, py, pz, pm, nrem, d, inv_dx, qscale, bx, status, lane, large);
+      WIDE ? dep_warp_runs_wide<POW2>(px, py, pz, pm, nrem, d, inv_dx, qscale, bx, status, lane, large)
+           : dep_warp_runs<POW2>(px, py, pz, pm, nrem, d, inv_dx, qscale, bx, status, lane, large);
     else
-      large = dep_warp_direct<POW2>(x, y, z, m, wb, nrem, d, inv_dx, qscale, qg, status, lane);
+      large = dep_warp_direct<POW2>(x, y, z, m, wb, nrem, d, inv_dx, qscale, qg, status);
     while (large) {  // rare: point masses
       const int j = __ffs(large) - 1;
       large &= large - 1;
@@ -632,38 +779,52 @@ __global__ void __launch_bounds__(256, 4)
       const int vol = nx * bx.nyz;
       const float inv_nyz = __frcp_rn((float)bx.nyz), inv_nz = __frcp_rn((float)bx.nz);
       for (int i = lane; i < vol; i += 32) {
-        const int v = wbox[i];
-        if (v == 0) continue;
+        const int v = wbox[i], vh = WIDE ? wbox[DepW<WIDE>::box + i] : 0;
+        if ((v | vh) == 0) continue;
         wbox[i] = 0;
+        if (WIDE) wbox[DepW<WIDE>::box + i] = 0;
         const int rx = (int)(((float)i + 0.5f) * inv_nyz), rem = i - rx * bx.nyz;
         const int ry = (int)(((float)rem + 0.5f) * inv_nz), rz = rem - ry * bx.nz;
         const int jx = bx.x0 + rx, jy = bx.y0 + ry, jz = bx.z0 + rz;
         if ((unsigned)jx < (unsigned)d.G && (unsigned)jy < (unsigned)d.G && (unsigned)jz < (unsigned)d.G)
-          atomicAdd((unsigned long long *)(qg + ((size_t)jx * d.G + jy) * d.G + jz), (unsigned long long)(long long)v);
+          atomicAdd((unsigned long long *)(qg + ((size_t)jx * d.G + jy) * d.G + jz), (unsigned long long)((long long)vh * 1048576LL + v));
       }
       __syncwarp();
     }
   }
 }
 
-int gc_deposit_q(gc_ctx *ctx, const float *x, const float *y, const float *z, const float *m, int64_t n,
+int gc_deposit_q(gc_ctx *ctx, const float *x, const float *y, const float *z, const float *m, int64_t n, int bits,
                  const double *qexp) {
   if (n <= 0) return GC_OK;
   DepCtx d;
   d.dx = (float)ctx->dx;
   d.inv_vol = 1.0f / ((d.dx * d.dx) * d.dx);
   d.G = ctx->G;
-  const long long ntiles = (n + DEP_TILE - 1) / DEP_TILE;
-  const unsigned nb = (unsigned)(ntiles < (long long)gc_sms() * 4 ? ntiles : (long long)gc_sms() * 4);  // 4 CTAs per SM, persistent
   int fe = 0;
   const bool pow2 = std::frexp(d.dx, &fe) == 0.5f;
   const float inv_dx = pow2 ? std::ldexp(1.0f, 1 - fe) : 0.0f;
-  if (pow2)
-    gc_launch(ctx, GK_DEPOSIT_RUNS, k_deposit_sorted<true>, dim3(nb), dim3(256), 0, x, y, z, m, (long long)n, d,
-              inv_dx, qexp, ctx->q, ctx->dstatus);
-  else
-    gc_launch(ctx, GK_DEPOSIT_RUNS, k_deposit_sorted<false>, dim3(nb), dim3(256), 0, x, y, z, m, (long long)n, d,
-              inv_dx, qexp, ctx->q, ctx->dstatus);
+  // The narrow pass takes particles below 2^22 quanta, the wide one below 2^41;
+  // both leave the rest to the out-of-line rounding, so the choice changes only
+  // speed. The mean particle has at least 2^(bits - 1) / n quanta: wide from 2^20
+  // on, where particles of a few times the mean leave the narrow range (1.5M sorted
+  // particles at 2^-52: 327 us narrow, 21 wide; where both fit, the narrow pass has
+  // half the sums: 10M sorted particles at 2^-44 take 64 us narrow, 105 wide).
+  const bool wide = std::ldexp(1.0, bits - 1) / (double)n >= 1048576.0;
+  // CTAs of eight warps; of two while eight would leave SMs without one (131072
+  // particles: 20.4 us with eight, 18.5 with two)
+  const bool few = n < (int64_t)gc_sms() * 8 * DEP_WTILE;
+  auto k = few ? (wide ? (pow2 ? k_deposit_sorted<true, true, 2> : k_deposit_sorted<false, true, 2>)
+                       : (pow2 ? k_deposit_sorted<true, false, 2> : k_deposit_sorted<false, false, 2>))
+               : (wide ? (pow2 ? k_deposit_sorted<true, true, 8> : k_deposit_sorted<false, true, 8>)
+                       : (pow2 ? k_deposit_sorted<true, false, 8> : k_deposit_sorted<false, false, 8>));
+  const int warps = few ? 2 : 8;
+  const long long tile = (long long)warps * DEP_WTILE;
+  const long long ntiles = (n + tile - 1) / tile;
+  const long long most = (long long)gc_sms() * (wide ? 3 : 4) * (8 / warps);  // resident CTAs: persistent
+  const unsigned nb = (unsigned)(ntiles < most ? ntiles : most);
+  gc_launch(ctx, GK_DEPOSIT_RUNS, k, dim3(nb), dim3(32 * warps), 0, x, y, z, m, (long long)n, d, inv_dx, qexp, ctx->q,
+            ctx->dstatus);
   GC_LAUNCH_CHECK(ctx, "deposit");
   return GC_OK;
 }
@@ -801,7 +962,7 @@ extern "C" int gc_deposit_cic(gc_ctx *ctx, const float *x, const float *y, const
   int s;
   if (n > 0) {
     if ((s = gc_fixed_point_setup(ctx, m, n, fixed_point_bits, GC_S_MASS, GC_S_QEXP))) return s;
-    if ((s = gc_deposit_q(ctx, x, y, z, m, n, ctx->dsmall + GC_S_QEXP))) return s;
+    if ((s = gc_deposit_q(ctx, x, y, z, m, n, fixed_point_bits, ctx->dsmall + GC_S_QEXP))) return s;
   }
   return gc_convert_q(ctx, ctx->dsmall + GC_S_QEXP, rho, nullptr);
 }
