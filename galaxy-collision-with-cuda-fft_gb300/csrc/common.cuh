@@ -121,6 +121,7 @@ struct gc_ctx {
   double mass_sum_cache; // sum of masses for the engine's fixed-point quantum
   int last_step_valid;
   int q_next_ready;     // q holds the deposit of the current positions (made by the last particle pass)
+  int tail_smem_set;    // the tail kernel's dynamic shared-memory limit has been raised
   int gt_smem_set;      // the TMA particle-pass kernels' dynamic shared-memory limit has been raised
   const uint32_t *import_perm;  // gc_pm_import_order's permutation (in the sort scratch) ...
   int64_t import_n;             // ... for this many particles (0: none pending)
