@@ -37,7 +37,6 @@ enum {
   GC_S_CYCLES = 2,   // V-cycles of the last device-decided (graph-captured) solve
   GC_S_CONVERGED = 3,// 1 if that solve met its tolerance
   GC_S_MIRROR = 4,   // slots [0, 4) are copied to the pinned mirror by captured solves
-  GC_S_GRIDBAR = 10, // [10, 12): grid-barrier words of the persistent coarse launches
   GC_S_MASS = 12,    // total deposited density-mass used for the fixed-point quantum
   GC_S_QEXP = 13,    // quantum exponent E: quantum = 2^E (density units)
   GC_S_SOLVES = 14,  // device-decided solves since the counters were reset ...
@@ -77,7 +76,6 @@ struct gc_ctx {
   cudaStream_t stream;
   int device;
 
-  int coarse_blocks;    // CTAs of the persistent coarse-level launches (0: not sized yet)
   int capturing;        // a gc_pm_graph_create capture is in progress (no host reads, no events)
   cudaStream_t side;    // stream the V-cycle body of a captured solve is recorded on
   cudaStream_t fork;    // second stream of the engine step (the faces beside the warm-start passes)
@@ -97,8 +95,10 @@ struct gc_ctx {
   size_t half0;
   int H0;
   // coarse levels (index >= 1): correction e and h^2-scaled right-hand side b
+  // (ed: the correction the way down hands to the way up)
   float *e[GC_MAX_LEVELS];
   float *b[GC_MAX_LEVELS];
+  float *ed[GC_MAX_LEVELS];
   float *rc;            // residual scratch for coarse levels (sized for level 1)
 
   long long *q;         // int64 fixed-point mass grid (G^3)

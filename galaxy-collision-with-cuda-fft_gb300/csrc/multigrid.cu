@@ -95,6 +95,10 @@ int gc_mg_alloc(gc_ctx *ctx) {
     GC_CUDA(ctx, cudaMalloc(&ctx->b[l], n3 * sizeof(float)));
     GC_CUDA(ctx, cudaMemset(ctx->e[l], 0, n3 * sizeof(float)));
     GC_CUDA(ctx, cudaMemset(ctx->b[l], 0, n3 * sizeof(float)));
+    if (l < ctx->tail) {  // the black nodes of the way down
+      GC_CUDA(ctx, cudaMalloc(&ctx->ed[l], n3 * sizeof(float)));
+      GC_CUDA(ctx, cudaMemset(ctx->ed[l], 0, n3 * sizeof(float)));
+    }
     if (l < ctx->tail && n3 > rc_n) rc_n = n3;
   }
   if (rc_n) {
@@ -121,8 +125,8 @@ void gc_mg_free(gc_ctx *ctx) {
   cudaFree(ctx->b0); cudaFree(ctx->r0);
   cudaFree(ctx->e0s); cudaFree(ctx->r0s); cudaFree(ctx->e0n); cudaFree(ctx->r0n);
   for (int l = 1; l < GC_MAX_LEVELS; ++l) {
-    cudaFree(ctx->e[l]); cudaFree(ctx->b[l]);
-    ctx->e[l] = ctx->b[l] = nullptr;
+    cudaFree(ctx->e[l]); cudaFree(ctx->b[l]); cudaFree(ctx->ed[l]);
+    ctx->e[l] = ctx->b[l] = ctx->ed[l] = nullptr;
   }
   cudaFree(ctx->rc);
   ctx->hi = ctx->lo = ctx->b0 = ctx->r0 = ctx->rc = nullptr;
@@ -367,26 +371,34 @@ __device__ __forceinline__ int prolong_w(int i, const LevelGeom &f, const LevelG
   return 1;
 }
 
-__device__ __forceinline__ float prolong_value(const float *__restrict__ ec, int i, int j, int k,
-                                               const LevelGeom &f, const LevelGeom &cg) {
+// P(e_c) at fine node (i, j, k); coarse node (I, J, K) at ec[I si + J sj + K].
+__device__ __forceinline__ float prolong_at(const float *__restrict__ ec, int si, int sj, int i, int j, int k,
+                                            const LevelGeom &f, const LevelGeom &cg) {
   int ci, cj, ck;
   float wi0, wi1, wj0, wj1, wk0, wk1;
   const int ni = prolong_w(i, f, cg, ci, wi0, wi1);
   const int nj = prolong_w(j, f, cg, cj, wj0, wj1);
   const int nk = prolong_w(k, f, cg, ck, wk0, wk1);
-  const size_t m = cg.n;
   float val = 0.0f;
-  for (int a = 0; a < ni; ++a) {
+#pragma unroll
+  for (int a = 0; a < 2; ++a) {
     const float wa = a ? wi1 : wi0;
-    for (int bb = 0; bb < nj; ++bb) {
+#pragma unroll
+    for (int bb = 0; bb < 2; ++bb) {
+      if (a >= ni || bb >= nj) continue;
       const float wb = bb ? wj1 : wj0;
-      const size_t row = ((size_t)(ci + a) * m + (cj + bb)) * m + ck;
+      const float *row = ec + (ci + a) * si + (cj + bb) * sj + ck;
       const float wab = wa * wb;
-      val += wab * wk0 * ec[row];
-      if (nk == 2) val += wab * wk1 * ec[row + 1];
+      val += wab * wk0 * row[0];
+      if (nk == 2) val += wab * wk1 * row[1];
     }
   }
   return val;
+}
+
+__device__ __forceinline__ float prolong_value(const float *__restrict__ ec, int i, int j, int k,
+                                               const LevelGeom &f, const LevelGeom &cg) {
+  return prolong_at(ec, cg.n * cg.n, cg.n, i, j, k, f, cg);  // coarse levels have < 2^31 nodes
 }
 
 __global__ void __launch_bounds__(256)
@@ -397,240 +409,6 @@ __global__ void __launch_bounds__(256)
   if (k > f.J || j > f.J) return;
   const size_t n = f.n;
   ef[((size_t)i * n + j) * n + k] += prolong_value(ec, i, j, k, f, cg);
-}
-
-// ------------------------------------------------------------------------------
-// coarse levels in two persistent launches
-// ------------------------------------------------------------------------------
-// Levels 1 .. tail-1 are relaxed grid-wide by one cooperative launch on the way
-// down (pre-smoothing, residual, restriction per level) and one on the way up
-// (prolongation, post-smoothing), with a grid barrier between phases instead of
-// a kernel boundary. The arithmetic per node is that of k_smooth / k_resid /
-// k_restrict / k_prolong, so the result equals the per-phase launches bit for
-// bit. The first half-sweep of a level starts from a zero correction and reads
-// no neighbour, so the level needs no clearing.
-struct GridBar {
-  unsigned count;  // arrivals since the start of the solve (grows by the grid size per barrier)
-  unsigned pad0;
-  unsigned abort;  // set by a CTA that gave up waiting
-  unsigned pad1;
-};
-
-struct CoarseDesc {
-  int l0, l1;  // levels l0 .. l1-1
-  int pre, post;
-  long long budget;  // SM clocks a CTA waits at one barrier before it gives up
-  GridBar *bar;
-  unsigned *status;
-  float *rc;
-  LevelGeom g[GC_MAX_LEVELS];
-  float *e[GC_MAX_LEVELS];
-  float *b[GC_MAX_LEVELS];
-};
-
-__device__ __forceinline__ unsigned ld_acquire_u32(const unsigned *p) {
-  unsigned v;
-  asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
-  return v;
-}
-
-// Grid-wide barrier of a cooperative launch on a monotonic arrival count: thread
-// 0 of each CTA adds one arrival (a release reduction, no return value) and
-// waits with acquire loads until the count reaches its target, a multiple of
-// the grid size. The count is cleared before every solve and only grows within
-// it; a launch starts from the count rounded down to a multiple of the grid
-// size (every barrier of earlier launches has completed, and a CTA that reads
-// it late can see at most the other CTAs' first arrivals). The wait is bounded
-// by `budget` clocks: a CTA that gives up raises GC_FLAG_TIMEOUT and the abort
-// word (so the others stop waiting too) and the kernel returns.
-__device__ __forceinline__ unsigned grid_barrier_base(GridBar *gb) {
-  return (ld_acquire_u32(&gb->count) / gridDim.x) * gridDim.x;
-}
-
-__device__ __forceinline__ bool grid_barrier(GridBar *gb, unsigned &target, unsigned *status, long long budget) {
-  __shared__ int ok_s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    target += gridDim.x;
-    __threadfence();
-    asm volatile("red.release.gpu.global.add.u32 [%0], %1;" ::"l"(&gb->count), "r"(1u) : "memory");
-    const long long t0 = clock64();
-    unsigned spins = 0;
-    while ((int)(ld_acquire_u32(&gb->count) - target) < 0) {
-      if ((++spins & 63u) == 0 && (ld_acquire_u32(&gb->abort) || clock64() - t0 > budget)) {
-        ok = 0;
-        atomicOr(status, GC_FLAG_TIMEOUT);
-        atomicExch(&gb->abort, 1u);
-        break;
-      }
-    }
-    ok_s = ok;
-  }
-  __syncthreads();
-  return ok_s != 0;
-}
-
-// A phase deals the rows (i, j), 1 <= i, j <= J, of its level to the grid's
-// warps round robin, PR rows per warp per round, and the lanes of a warp take
-// the nodes k of a row (SK per lane per group of 32 * SK): one division per
-// row instead of per node, coalesced row accesses, and up to PR * SK nodes per
-// lane whose loads are all issued before any result is stored, so that a lane
-// has several independent L2 round trips in flight. Within a phase no node
-// reads a value that the phase writes (a half-sweep reads only the other
-// colour; the residual, restriction and prolongation write other arrays or
-// only the node itself), so deferring the stores changes nothing.
-#define PR 1  // (2 and 4 rows per round measured slower: more registers, fewer warps)
-#define SK 2
-__device__ __forceinline__ unsigned p_warp() { return (blockIdx.x * blockDim.x + threadIdx.x) >> 5; }
-__device__ __forceinline__ unsigned p_nwarps() { return (gridDim.x * blockDim.x) >> 5; }
-
-// One red-black half-sweep of level g (k_smooth's slots and arithmetic): row
-// (i, j) holds the nodes k = 2 kk + ((color + i + j) & 1), kk = 0 .. J/2.
-__device__ void p_smooth(float *__restrict__ e, const float *__restrict__ b, const LevelGeom &g, int color,
-                         bool first) {
-  const int J = g.J, n = g.n, nkk = J / 2 + 1;
-  const unsigned rows = (unsigned)J * (unsigned)J, NW = p_nwarps(), lane = threadIdx.x & 31u;
-  for (unsigned r0 = p_warp(); r0 < rows; r0 += PR * NW) {
-    for (int kk0 = 0; kk0 < nkk; kk0 += 32 * SK) {
-      float val[PR][SK];
-      unsigned at[PR][SK];  // coarse levels have < 2^32 nodes
-      bool ok[PR][SK];
-#pragma unroll
-      for (int u = 0; u < PR; ++u) {
-        const unsigned r = r0 + u * NW;
-        const int i = (int)(r / (unsigned)J) + 1, j = (int)(r % (unsigned)J) + 1;
-        const int par = (color + i + j) & 1;
-#pragma unroll
-        for (int q = 0; q < SK; ++q) {
-          const int k = 2 * (kk0 + (int)lane + 32 * q) + par;
-          ok[u][q] = r < rows && k >= 1 && k <= J;
-          if (!ok[u][q]) continue;
-          const size_t c = ((size_t)i * n + j) * n + k;
-          float sum, diag;
-          if (first) {  // zero neighbours: the diagonal alone
-            sum = 0.0f;
-            diag = ((i == J ? g.dB : 2.0f) + (j == J ? g.dB : 2.0f)) + (k == J ? g.dB : 2.0f);
-          } else {
-            sw_stencil(e, c, i, j, k, g, sum, diag);
-          }
-          val[u][q] = gs_value(sum, b[c], diag);
-          at[u][q] = (unsigned)c;
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < PR; ++u)
-#pragma unroll
-        for (int q = 0; q < SK; ++q)
-          if (ok[u][q]) e[at[u][q]] = val[u][q];
-    }
-  }
-}
-
-__device__ void p_zero(float *__restrict__ e, const LevelGeom &g) {
-  const size_t tot = (size_t)g.n * g.n * g.n, T = (size_t)gridDim.x * blockDim.x;
-  for (size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x; t < tot; t += T) e[t] = 0.0f;
-}
-
-// The nodes k = k0 + lane + 32 q (1 <= k <= J) of RR rows per round, for the
-// residual and the prolongation: node(i, j, k, v) returns the node's index in
-// `out` and sets its new value v; all of a lane's values are stored after all
-// of its nodes are computed.
-template <int RR, typename F>
-__device__ __forceinline__ void p_node_rows(int J, float *__restrict__ out, F node) {
-  const unsigned rows = (unsigned)J * (unsigned)J, NW = p_nwarps(), lane = threadIdx.x & 31u;
-  for (unsigned r0 = p_warp(); r0 < rows; r0 += RR * NW) {
-    for (int k0 = 1; k0 <= J; k0 += 32 * SK) {
-      float val[RR][SK];
-      unsigned at[RR][SK];  // coarse levels have < 2^32 nodes
-      bool ok[RR][SK];
-#pragma unroll
-      for (int u = 0; u < RR; ++u) {
-        const unsigned r = r0 + u * NW;
-        const int i = (int)(r / (unsigned)J) + 1, j = (int)(r % (unsigned)J) + 1;
-#pragma unroll
-        for (int q = 0; q < SK; ++q) {
-          const int k = k0 + (int)lane + 32 * q;
-          ok[u][q] = r < rows && k <= J;
-          if (ok[u][q]) at[u][q] = node(i, j, k, val[u][q]);
-        }
-      }
-#pragma unroll
-      for (int u = 0; u < RR; ++u)
-#pragma unroll
-        for (int q = 0; q < SK; ++q)
-          if (ok[u][q]) out[at[u][q]] = val[u][q];
-    }
-  }
-}
-
-__device__ void p_resid(const float *__restrict__ e, const float *__restrict__ b, float *__restrict__ r_out,
-                        const LevelGeom &g) {
-  const size_t n = (size_t)g.n;
-  p_node_rows<1>(g.J, r_out, [&](int i, int j, int k, float &v) {
-    const size_t c = ((size_t)i * n + j) * n + k;
-    float sum, diag;
-    sw_stencil(e, c, i, j, k, g, sum, diag);
-    v = b[c] - (sum - diag * e[c]);
-    return (unsigned)c;
-  });
-}
-
-__device__ void p_restrict(const float *__restrict__ rf, const LevelGeom &f, float *__restrict__ bc,
-                           const LevelGeom &cg) {
-  const int J = cg.J;
-  const unsigned rows = (unsigned)J * (unsigned)J, NW = p_nwarps(), lane = threadIdx.x & 31u;
-  for (unsigned r = p_warp(); r < rows; r += NW) {
-    const int I = (int)(r / (unsigned)J) + 1, Jj = (int)(r % (unsigned)J) + 1;
-    for (int K = 1 + (int)lane; K <= J; K += 32) restrict_node(rf, f, bc, cg, I, Jj, K);
-  }
-}
-
-__device__ void p_prolong(const float *__restrict__ ec, const LevelGeom &cg, float *__restrict__ ef,
-                          const LevelGeom &f) {
-  const size_t n = (size_t)f.n;
-  // one row per round: the prolongation's weights take the registers
-  p_node_rows<1>(f.J, ef, [&](int i, int j, int k, float &v) {
-    const size_t c = ((size_t)i * n + j) * n + k;
-    v = ef[c] + prolong_value(ec, i, j, k, f, cg);
-    return (unsigned)c;
-  });
-}
-
-#define COARSE_THREADS 512
-
-// Down: for each level, pre-smoothing, residual, restriction into b[l+1].
-__global__ void __launch_bounds__(COARSE_THREADS, 2) k_coarse_down(CoarseDesc d) {
-  unsigned tgt = threadIdx.x == 0 ? grid_barrier_base(d.bar) : 0u;
-  for (int l = d.l0; l < d.l1; ++l) {
-    const LevelGeom &g = d.g[l];
-    if (d.pre == 0) {
-      p_zero(d.e[l], g);
-      if (!grid_barrier(d.bar, tgt, d.status, d.budget)) return;
-    }
-    for (int h = 0; h < 2 * d.pre; ++h) {
-      p_smooth(d.e[l], d.b[l], g, h & 1, h == 0);
-      if (!grid_barrier(d.bar, tgt, d.status, d.budget)) return;
-    }
-    p_resid(d.e[l], d.b[l], d.rc, g);
-    if (!grid_barrier(d.bar, tgt, d.status, d.budget)) return;
-    p_restrict(d.rc, g, d.b[l + 1], d.g[l + 1]);
-    if (l + 1 < d.l1 && !grid_barrier(d.bar, tgt, d.status, d.budget)) return;
-  }
-}
-
-// Up: for each level from l1-1 down to l0, prolongation of e[l+1], post-smoothing.
-__global__ void __launch_bounds__(COARSE_THREADS, 2) k_coarse_up(CoarseDesc d) {
-  unsigned tgt = threadIdx.x == 0 ? grid_barrier_base(d.bar) : 0u;
-  for (int l = d.l1 - 1; l >= d.l0; --l) {
-    const LevelGeom &g = d.g[l];
-    p_prolong(d.e[l + 1], d.g[l + 1], d.e[l], g);
-    for (int h = 0; h < 2 * d.post; ++h) {
-      if (!grid_barrier(d.bar, tgt, d.status, d.budget)) return;
-      p_smooth(d.e[l], d.b[l], g, h & 1, false);
-    }
-    if (l > d.l0 && !grid_barrier(d.bar, tgt, d.status, d.budget)) return;
-  }
 }
 
 // ------------------------------------------------------------------------------
@@ -682,19 +460,25 @@ __global__ void __launch_bounds__(256)
   own[s] = __fmul_rn(sum - rv, GC_SIXTH);
 }
 
-// phi += e at natural node c: double-float add (or a plain f32 add).
+// (h, l) += ev: double-float add (or a plain f32 add).
+template <bool PLAIN>
+__device__ __forceinline__ void phi_sum(float &h, float &l, float ev) {
+  if (PLAIN) {
+    h = __fadd_rn(h, ev);
+  } else {
+    float s1, e1;
+    df_two_sum(h, ev, s1, e1);
+    df_fast_two_sum(s1, __fadd_rn(l, e1), h, l);
+  }
+}
+
+// phi += e at natural node c.
 template <bool PLAIN>
 __device__ __forceinline__ void phi_add(float *__restrict__ hi, float *__restrict__ lo, size_t c, float ev) {
-  if (PLAIN) {
-    hi[c] = __fadd_rn(hi[c], ev);
-  } else {
-    float s1, e1, h, l;
-    df_two_sum(hi[c], ev, s1, e1);
-    const float ln = __fadd_rn(lo[c], e1);
-    df_fast_two_sum(s1, ln, h, l);
-    hi[c] = h;
-    lo[c] = l;
-  }
+  float h = hi[c], l = PLAIN ? 0.0f : lo[c];
+  phi_sum<PLAIN>(h, l, ev);
+  hi[c] = h;
+  if (!PLAIN) lo[c] = l;
 }
 
 // The last half-sweep (black) fused with the update phi += e: thread kk of row
@@ -913,7 +697,7 @@ __global__ void __launch_bounds__(256)
 }
 
 // Residual of the potential on four consecutive nodes 4t .. 4t+3 (see k_resid0).
-template <bool PLAIN>
+template <bool PLAIN, bool SPLIT>
 __global__ void __launch_bounds__(256)
     k_resid0x4(const float *__restrict__ hi, const float *__restrict__ lo, const float *__restrict__ b,
                float *__restrict__ rout, float *__restrict__ e_first, double *__restrict__ parts, Split0 d) {
@@ -953,14 +737,18 @@ __global__ void __launch_bounds__(256)
       const int k = 4 * t + q;
       if (k < 1 || k > G - 2) rv[q] = 0.0f;  // faces: no residual, zero correction
     }
-    // nodes 4t, 4t+2 share a colour (slots 2t, 2t+1), as do 4t+1, 4t+3
-    const int c0col = (i + j) & 1;  // colour of node 4t
-    const size_t sl = ((size_t)i * G + j) * d.H + 2 * t;
-    st2(rout + (size_t)c0col * d.half + sl, rv[0], rv[2]);
-    st2(rout + (size_t)(c0col ^ 1) * d.half + sl, rv[1], rv[3]);
-    if (e_first) {  // red = colour 0
-      if (c0col == 0) st2(e_first + sl, __fmul_rn(0.0f - rv[0], GC_SIXTH), __fmul_rn(0.0f - rv[2], GC_SIXTH));
-      else st2(e_first + sl, __fmul_rn(0.0f - rv[1], GC_SIXTH), __fmul_rn(0.0f - rv[3], GC_SIXTH));
+    if (SPLIT) {
+      // nodes 4t, 4t+2 share a colour (slots 2t, 2t+1), as do 4t+1, 4t+3
+      const int c0col = (i + j) & 1;  // colour of node 4t
+      const size_t sl = ((size_t)i * G + j) * d.H + 2 * t;
+      st2(rout + (size_t)c0col * d.half + sl, rv[0], rv[2]);
+      st2(rout + (size_t)(c0col ^ 1) * d.half + sl, rv[1], rv[3]);
+      if (e_first) {  // red = colour 0
+        if (c0col == 0) st2(e_first + sl, __fmul_rn(0.0f - rv[0], GC_SIXTH), __fmul_rn(0.0f - rv[2], GC_SIXTH));
+        else st2(e_first + sl, __fmul_rn(0.0f - rv[1], GC_SIXTH), __fmul_rn(0.0f - rv[3], GC_SIXTH));
+      }
+    } else {
+      st4(rout + c0, make_float4(rv[0], rv[1], rv[2], rv[3]));
     }
     acc = ((rv[0] * rv[0] + rv[1] * rv[1]) + rv[2] * rv[2]) + rv[3] * rv[3];
   }
@@ -1039,6 +827,336 @@ __global__ void __launch_bounds__(256)
   float *blk = e + d.half + ((size_t)i * d.G + j) * d.H + kk0;
   const float2 old = ld2(blk);
   st2(blk, old.x + v0, old.y + v1);
+}
+
+// ------------------------------------------------------------------------------
+// a level's way down and way up in one launch each, block by block
+// ------------------------------------------------------------------------------
+// k_block_down: the pre-smoothing from a zero correction, the residual and its
+// restriction. k_block_up: the prolongation and the post-smoothing (on the finest
+// level with phi += e). A CTA takes a block of nodes and relaxes a region around it
+// in shared memory that shrinks by one node a side with every half-sweep, so that
+// its block is exact when it gets there: no grid-wide barrier or launch between
+// the phases, at the price of relaxing the halo in several CTAs (about four times
+// the nodes; the data comes from L2). The arithmetic of every node is that of
+// k_smooth / k_resid / k_restrict / k_prolong, so the results equal theirs bit for bit.
+//
+// A warp is a row j of the region, its lanes the 32 nodes k of the row, and a thread
+// walks its column along i: the nodes of one colour lie on every other plane, odd
+// and even lanes on alternating ones, so all lanes work at each step and their
+// shared-memory words are in 32 different banks. Bound by shared-memory accesses:
+// six a node and half-sweep (the i neighbours are carried along the column, the
+// right-hand sides stay in registers: reading them from L1 in every half-sweep
+// took twice as long).
+//
+// Only the black nodes pass from the way down to the way up: the first half-sweep of
+// the way up overwrites the red ones without reading them. They go through an
+// array of their own (neighbouring blocks still read it while a block writes its
+// result).
+//
+// Measured (us per V-cycle, levels 129^3, 65^3 and 33^3 under a 256^3 grid): 124 now
+// (down 30.6 + 7.6 + 7.6, up 37.5 + 10 + 10, one launch each) against 156 for two
+// cooperative launches with a grid barrier between the phases; one level of 33^3
+// under 64^3: 17 against 26.
+template <int NS>
+struct BlkD {  // way down, NS sweeps: coarse nodes per block along j and k, region
+  static constexpr int H = 2 * NS - 1;            // extra halo of the first half-sweep
+  static constexpr int CJ = 8, CK = (32 - 3 - 2 * H) / 2;
+  static constexpr int LJ = 2 * CJ + 3 + 2 * H;   // rows (warps)
+};
+template <int NS>
+struct BlkU {  // way up: nodes per block along j and k, region
+  static constexpr int H = 2 * NS;
+  static constexpr int TJ = 16, TK = 32 - 2 * H;
+  static constexpr int LJ = TJ + 2 * H;
+};
+
+// A thread's column in shared memory and registers: node (i0 + t, j, k) at col + t SI,
+// t < LI; its nodes of one colour are t = 2 m + o, and their right-hand sides bv[m].
+template <int LI, int LJ>
+struct BlkCol {
+  static constexpr int SI = LJ * 32, M = (LI + 1) / 2;
+  float *col;
+  int i0, J, o[2];   // o[c]: first plane of colour c
+  float bv[2][M];
+  float a, d0, d1, r0, r1;  // far-face weight; diagonal and its reciprocal below and at i = J
+  bool lj, lk, in_jk;
+
+  __device__ __forceinline__ void init(float *c, const float *__restrict__ b, const LevelGeom &g, int i0_, int j, int k) {
+    col = c;
+    i0 = i0_;
+    J = g.J;
+    in_jk = j >= 1 && j <= J && k >= 1 && k <= J;
+    o[0] = (i0 + j + k) & 1;
+    o[1] = o[0] ^ 1;
+    lj = j == J;
+    lk = k == J;
+    a = g.a;
+    const float dj = lj ? g.dB : 2.0f, dk = lk ? g.dB : 2.0f;
+    d0 = (2.0f + dj) + dk;
+    d1 = (g.dB + dj) + dk;
+    r0 = d0 == 6.0f ? GC_SIXTH : __frcp_rn(d0);
+    r1 = d1 == 6.0f ? GC_SIXTH : __frcp_rn(d1);
+    const long long n = g.n, nn = n * n;
+    const float *bp = b + (long long)i0 * nn + (long long)j * n + k;
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+#pragma unroll
+      for (int c2 = 0; c2 < 2; ++c2) {  // all in flight together
+        const int t = 2 * m + o[c2];
+        bv[c2][m] = in_jk && t < LI && i0 + t >= 1 && i0 + t <= J ? __ldg(bp + t * nn) : 0.0f;
+      }
+  }
+  // x / diagonal as gs_value does it: times 1/6 where the diagonal is 6, else the
+  // correctly rounded quotient from the reciprocal and the exact remainder
+  // (Markstein, IBM J. Res. Dev. 34, 1990)
+  __device__ __forceinline__ float over(float x, bool li) const {
+    const float d = li ? d1 : d0, r = li ? r1 : r0, q = __fmul_rn(x, r);
+    return d == 6.0f ? q : __fmaf_rn(__fmaf_rn(-q, d, x), r, q);
+  }
+  __device__ __forceinline__ float sum_at(const float *p, float below, float above, bool li) const {
+    const float sx = li ? __fmul_rn(a, below) : __fadd_rn(above, below);
+    const float sy = lj ? __fmul_rn(a, p[-32]) : __fadd_rn(p[32], p[-32]);
+    const float sz = lk ? __fmul_rn(a, p[-1]) : __fadd_rn(p[1], p[-1]);
+    return __fadd_rn(__fadd_rn(sx, sy), sz);
+  }
+  // One half-sweep of colour C over the planes [s, LI - 1 - s]; `far` (uniform in the
+  // warp): the block holds far-face nodes.
+  template <int C>
+  __device__ __forceinline__ void sweep(int s, bool far) {
+    const int tl = s > 1 - i0 ? s : 1 - i0, th = LI - 1 - s < J - i0 ? LI - 1 - s : J - i0;
+    float *p = col + o[C] * SI;
+    float below = o[C] ? col[0] : 0.0f;
+    if (far) {
+#pragma unroll
+      for (int m = 0; m < M; ++m, p += 2 * SI) {
+        const int t = 2 * m + o[C];
+        const float above = t + 1 < LI ? p[SI] : 0.0f;
+        if (t >= tl && t <= th) {
+          const bool li = i0 + t == J;
+          *p = over(__fsub_rn(sum_at(p, below, above, li), bv[C][m]), li);
+        }
+        below = above;
+      }
+    } else {
+#pragma unroll
+      for (int m = 0; m < M; ++m, p += 2 * SI) {
+        const int t = 2 * m + o[C];
+        const float above = t + 1 < LI ? p[SI] : 0.0f;
+        if (t >= tl && t <= th) {
+          const float sum = __fadd_rn(__fadd_rn(__fadd_rn(above, below), __fadd_rn(p[32], p[-32])),
+                                      __fadd_rn(p[1], p[-1]));
+          *p = __fmul_rn(__fsub_rn(sum, bv[C][m]), GC_SIXTH);
+        }
+        below = above;
+      }
+    }
+  }
+};
+
+// The separable full weighting of restrict_node on a residual in shared memory (zero
+// on the faces); p points at fine node (2 I - 1, 2 J - 1, 2 K - 1).
+__device__ __forceinline__ float blk_restrict(const float *p, int SI, const float (&wi)[3], const float (&wj)[3],
+                                              const float (&wk)[3]) {
+  float acc = 0.0f;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+    float ta = 0.0f;
+#pragma unroll
+    for (int bb = 0; bb < 3; ++bb) {
+      const float *row = p + a * SI + bb * 32;
+      float sab = wk[1] * row[1];
+      sab += wk[0] * row[0];
+      sab += wk[2] * row[2];
+      ta += wj[bb] * sab;
+    }
+    acc += wi[a] * ta;
+  }
+  return 4.0f * acc;
+}
+
+template <int NS, int CI>
+__global__ void __launch_bounds__(32 * BlkD<NS>::LJ, 1)
+    k_block_down(float *__restrict__ e, const float *__restrict__ b, LevelGeom g, float *__restrict__ bc, LevelGeom cg) {
+  using B = BlkD<NS>;
+  constexpr int H = B::H, LJ = B::LJ, LI = 2 * CI + 3 + 2 * H;
+  using Col = BlkCol<LI, LJ>;
+  constexpr int SI = Col::SI, M = Col::M;
+  extern __shared__ float blk_sm[];
+  float *E = blk_sm;
+  float *R = E + LI * SI;                 // residual on planes and rows [H + 1, L - 2 - H] of E
+  constexpr int RJ = 2 * B::CJ + 1, RSI = RJ * 32;
+  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+  const int I0 = 1 + blockIdx.z * CI, J0 = 1 + blockIdx.y * B::CJ, K0 = 1 + blockIdx.x * B::CK;
+  const int i0 = 2 * I0 - 2 - H, j = 2 * J0 - 2 - H + row, k0 = 2 * K0 - 2 - H, k = k0 + lane;
+  const bool far = i0 + LI > g.J || j == g.J || k0 + 31 >= g.J;
+  Col c;
+  c.init(E + row * 32 + lane, b, g, i0, j, k);
+  // red half-sweep from zero; black nodes and everything outside the interior are zero
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    const int tr = 2 * m + c.o[0], tb = 2 * m + c.o[1];
+    if (tr < LI) c.col[tr * SI] = c.over(0.0f - c.bv[0][m], i0 + tr == g.J);
+    if (tb < LI) c.col[tb * SI] = 0.0f;
+  }
+  __syncthreads();
+#pragma unroll
+  for (int s = 1; s < 2 * NS; ++s) {
+    if (c.in_jk && row >= s && row < LJ - s && lane >= s && lane < 32 - s) {
+      if (s & 1) c.template sweep<1>(s, far);
+      else c.template sweep<0>(s, far);
+    }
+    __syncthreads();
+  }
+  // residual around the block's coarse nodes, zero off the interior
+  if (row >= H + 1 && row < H + 1 + RJ) {
+    const bool mine = c.in_jk && lane >= H + 1 && lane < 32 - H - 1;
+    float *rp = R + (row - H - 1) * 32 + lane;
+#pragma unroll
+    for (int m = 0; m < M; ++m)
+#pragma unroll
+      for (int q = 0; q < 2; ++q) {
+        const int t = 2 * m + c.o[q], i = i0 + t;
+        if (t < H + 1 || t > LI - 2 - H) continue;
+        float v = 0.0f;
+        if (mine && i >= 1 && i <= g.J) {
+          const float *p = c.col + t * SI;
+          const bool li = i == g.J;
+          const float sum = c.sum_at(p, p[-SI], p[SI], li), diag = li ? c.d1 : c.d0;
+          v = c.bv[q][m] - (sum - diag * p[0]);
+        }
+        rp[(t - H - 1) * RSI] = v;
+      }
+  }
+  // the block's black nodes (fine nodes 2 I - 1 and 2 I of its coarse nodes I, and the
+  // one past the last coarse node) for the way up
+  {
+    const size_t n = g.n, nn = n * n;
+    const int ie = I0 + CI > cg.J ? g.J : 2 * (I0 + CI) - 2, je = J0 + B::CJ > cg.J ? g.J : 2 * (J0 + B::CJ) - 2,
+              ke = K0 + B::CK > cg.J ? g.J : 2 * (K0 + B::CK) - 2;
+    if (j >= 2 * J0 - 1 && j <= je && k >= 2 * K0 - 1 && k <= ke) {
+#pragma unroll 4
+      for (int i = 2 * I0 - 1 + ((j + k) & 1); i <= ie; i += 2)
+        e[(size_t)i * nn + (size_t)j * n + k] = c.col[(i - i0) * SI];
+    }
+  }
+  __syncthreads();
+  constexpr int NC = CI * B::CJ * B::CK;
+  for (int q = threadIdx.x; q < NC; q += 32 * LJ) {
+    const int dk = q % B::CK, r = q / B::CK, dj = r % B::CJ, di = r / B::CJ;
+    const int I = I0 + di, Jc = J0 + dj, K = K0 + dk;
+    if (I > cg.J || Jc > cg.J || K > cg.J) continue;
+    float wi[3], wj[3], wk[3];
+#pragma unroll
+    for (int o = -1; o <= 1; ++o) {
+      wi[o + 1] = restrict_w(I, o, g, cg);
+      wj[o + 1] = restrict_w(Jc, o, g, cg);
+      wk[o + 1] = restrict_w(K, o, g, cg);
+    }
+    bc[((size_t)I * cg.n + Jc) * cg.n + K] =
+        blk_restrict(R + 2 * di * RSI + 2 * dj * 32 + (H + 1 + 2 * dk), RSI, wi, wj, wk);
+  }
+}
+
+// PHI: 0 coarse level (e_out), 1 finest level in double-float, 2 in plain f32 (phi += e).
+template <int NS, int TI, int PHI>
+__global__ void __launch_bounds__(32 * BlkU<NS>::LJ, 1)
+    k_block_up(const float *__restrict__ ec, LevelGeom cg, const float *__restrict__ e, const float *__restrict__ b,
+               LevelGeom g, float *__restrict__ e_out, float *__restrict__ hi, float *__restrict__ lo) {
+  using B = BlkU<NS>;
+  constexpr int H = B::H, LJ = B::LJ, LI = TI + 2 * H;
+  using Col = BlkCol<LI, LJ>;
+  constexpr int SI = Col::SI, M = Col::M;
+  constexpr int PJ = LJ / 2 + 2, PI = LI / 2 + 2, PK = 18;  // the coarse nodes the region interpolates from
+  extern __shared__ float blk_sm[];
+  float *E = blk_sm, *C = E + LI * SI;
+  const int lane = threadIdx.x & 31, row = threadIdx.x >> 5;
+  const int i0 = 1 + blockIdx.z * TI - H, j0 = 1 + blockIdx.y * B::TJ - H, k0 = 1 + blockIdx.x * B::TK - H;
+  const int j = j0 + row, k = k0 + lane;
+  const int ci = i0 >> 1, cj = j0 >> 1, ck = k0 >> 1;  // (floor, also below zero)
+  const bool far = i0 + LI > g.J || j == g.J || k0 + 31 >= g.J;
+  const long long n = g.n, nn = n * n;
+  Col c;
+  c.init(E + row * 32 + lane, b, g, i0, j, k);
+  // black nodes: the correction of the way down ...
+  float ev[M];
+  {
+    const float *ep = e + (long long)i0 * nn + (long long)j * n + k;
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const int t = 2 * m + c.o[1];
+      ev[m] = c.in_jk && t < LI && i0 + t >= 1 && i0 + t <= g.J ? __ldg(ep + t * nn) : 0.0f;
+    }
+  }
+  for (int q = threadIdx.x; q < PI * PJ * PK; q += 32 * LJ) {
+    const int dk = q % PK, r = q / PK, dj = r % PJ, di = r / PJ;
+    const int I = ci + di, Jc = cj + dj, K = ck + dk;
+    const bool in = I >= 0 && I < cg.n && Jc >= 0 && Jc < cg.n && K >= 0 && K < cg.n;
+    C[q] = in ? __ldg(ec + ((size_t)I * cg.n + Jc) * cg.n + K) : 0.0f;
+  }
+  __syncthreads();
+  // ... plus the prolonged coarse one; the rest starts at zero (red nodes are
+  // overwritten unread)
+  {
+    // (prolong_value's terms in its order; the j and k weights are the column's)
+    int c0, cj0, ck0;
+    float wi0, wi1, wj[2], wk[2];
+    const int nj = prolong_w(j, g, cg, cj0, wj[0], wj[1]), nk = prolong_w(k, g, cg, ck0, wk[0], wk[1]);
+    const float *cs = C + (cj0 - cj) * PK + (ck0 - ck);
+#pragma unroll
+    for (int m = 0; m < M; ++m) {
+      const int tb = 2 * m + c.o[1], tr = 2 * m + c.o[0], i = i0 + tb;
+      float v = 0.0f;
+      if (c.in_jk && i >= 1 && i <= g.J) {
+        const int ni = prolong_w(i, g, cg, c0, wi0, wi1);
+#pragma unroll
+        for (int a = 0; a < 2; ++a)
+#pragma unroll
+          for (int bb = 0; bb < 2; ++bb) {
+            if (a >= ni || bb >= nj) continue;
+            const float *q = cs + (c0 - ci + a) * (PJ * PK) + bb * PK;
+            const float wab = (a ? wi1 : wi0) * wj[bb];
+            v += wab * wk[0] * q[0];
+            if (nk == 2) v += wab * wk[1] * q[1];
+          }
+        v = ev[m] + v;
+      }
+      if (tb < LI) c.col[tb * SI] = v;
+      if (tr < LI) c.col[tr * SI] = 0.0f;
+    }
+  }
+  __syncthreads();
+#pragma unroll
+  for (int s = 0; s < 2 * NS; ++s) {
+    if (c.in_jk && row > s && row < LJ - 1 - s && lane > s && lane < 31 - s) {
+      if (s & 1) c.template sweep<1>(s + 1, far);
+      else c.template sweep<0>(s + 1, far);
+    }
+    __syncthreads();
+  }
+  if (!(c.in_jk && row >= H && row < LJ - H && lane >= H && lane < 32 - H)) return;
+  const size_t q0 = (size_t)(i0 + H) * nn + (size_t)j * n + k;
+  const int nt = g.J - (i0 + H) + 1;  // planes of the block inside the interior
+  if (PHI == 0) {
+#pragma unroll
+    for (int t = 0; t < TI; ++t)
+      if (t < nt) e_out[q0 + t * nn] = c.col[(H + t) * SI];
+  } else {
+    float h[TI], l[TI];
+#pragma unroll
+    for (int t = 0; t < TI; ++t) {
+      h[t] = t < nt ? hi[q0 + t * nn] : 0.0f;
+      l[t] = PHI == 1 && t < nt ? lo[q0 + t * nn] : 0.0f;
+    }
+#pragma unroll
+    for (int t = 0; t < TI; ++t) {
+      phi_sum<PHI == 2>(h[t], l[t], c.col[(H + t) * SI]);
+      if (t < nt) {
+        hi[q0 + t * nn] = h[t];
+        if (PHI == 1) lo[q0 + t * nn] = l[t];
+      }
+    }
+  }
 }
 
 // ------------------------------------------------------------------------------
@@ -1643,74 +1761,96 @@ static dim3 quad_grid(const gc_ctx *ctx) {
 }
 static bool vec4(const gc_ctx *ctx) { return ctx->G % 4 == 0; }
 
-// CTAs of the persistent coarse launches: as many as fit at once (a cooperative
-// launch needs them all resident), at most two per SM (fewer arrivals per grid
-// barrier), and no more than the largest phase has work for.
-static int coarse_grid(gc_ctx *ctx) {
-  if (ctx->coarse_blocks > 0) return GC_OK;
-  int occ_d = 0, occ_u = 0;
-  GC_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_d, k_coarse_down, COARSE_THREADS, 0));
-  GC_CUDA(ctx, cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_u, k_coarse_up, COARSE_THREADS, 0));
-  int per_sm = occ_d < occ_u ? occ_d : occ_u;
-  if (per_sm > 2) per_sm = 2;
-  if (per_sm < 1) {
-    gc_set_error(ctx, "coarse levels: the persistent kernel does not fit on an SM");
-    return GC_ERR_CUDA;
-  }
-  const LevelGeom &g1 = ctx->lev[1];
-  const long long rows = (long long)g1.J * g1.J;  // the largest phase: level 1's rows
-  long long nb = (long long)gc_sms() * per_sm;
-  const long long per_block = (long long)PR * (COARSE_THREADS / 32);
-  const long long need = (rows + per_block - 1) / per_block;
-  if (nb > need) nb = need;
-  ctx->coarse_blocks = (int)(nb < 1 ? 1 : nb);
-  return GC_OK;
+template <int NS, int CI>
+static size_t blk_down_smem() {
+  using B = BlkD<NS>;
+  return sizeof(float) * 32 * ((size_t)(2 * CI + 3 + 2 * B::H) * B::LJ + (size_t)(2 * CI + 1) * (2 * B::CJ + 1));
+}
+template <int NS, int TI>
+static size_t blk_up_smem() {
+  using B = BlkU<NS>;
+  const size_t LI = TI + 2 * B::H;
+  return sizeof(float) * (32 * LI * B::LJ + (LI / 2 + 2) * (B::LJ / 2 + 2) * 18);
 }
 
-static int launch_coarse(gc_ctx *ctx, const gc_mg_params *p, bool up) {
-  CoarseDesc d;
-  memset(&d, 0, sizeof(d));
-  d.l0 = 1;
-  d.l1 = ctx->tail;
-  d.pre = coarse_pre(p);
-  d.post = coarse_post(p);
-  d.budget = 100000000LL;  // ~50 ms of SM clocks; a barrier normally takes microseconds
-  d.bar = reinterpret_cast<GridBar *>(ctx->dsmall + GC_S_GRIDBAR);
-  d.status = ctx->dstatus;
-  d.rc = ctx->rc;
-  for (int l = 1; l < ctx->nlev; ++l) {
-    d.g[l] = ctx->lev[l];
-    d.e[l] = ctx->e[l];
-    d.b[l] = ctx->b[l];
-  }
-  int st = coarse_grid(ctx);
-  if (st) return st;
-  void *args[] = {&d};
-  const void *fn = up ? (const void *)k_coarse_up : (const void *)k_coarse_down;
-  ctx->prof.launches[GK_COARSE]++;
-  const int slot = ctx->prof.enabled && !ctx->capturing ? gc_prof_slot(ctx, GK_COARSE) : -1;
-  if (slot >= 0) cudaEventRecord(ctx->prof.ev[2 * slot], ctx->stream);
-  GC_CUDA(ctx, cudaLaunchCooperativeKernel(fn, dim3(ctx->coarse_blocks), dim3(COARSE_THREADS), args, 0, ctx->stream));
-  if (slot >= 0) cudaEventRecord(ctx->prof.ev[2 * slot + 1], ctx->stream);
+// Blocks are 8 coarse planes (way down) or 16 planes (way up) long; half as long
+// where that leaves SMs without a block (63^3 nodes: 48 long blocks, 96 short ones).
+template <int NS, int CI>
+static int blk_down(gc_ctx *ctx, int kid, float *e, const float *b, const LevelGeom &g, float *bc,
+                    const LevelGeom &cg) {
+  using B = BlkD<NS>;
+  const dim3 grid(gc_blocks(cg.J, B::CK), gc_blocks(cg.J, B::CJ), gc_blocks(cg.J, CI));
+  if (CI > 4 && (unsigned long long)grid.x * grid.y * grid.z < gc_sms())
+    return blk_down<NS, 4>(ctx, kid, e, b, g, bc, cg);
+  const size_t smem = blk_down_smem<NS, CI>();
+  if (smem > 48 * 1024)
+    GC_CUDA(ctx, cudaFuncSetAttribute(k_block_down<NS, CI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  gc_launch(ctx, kid, k_block_down<NS, CI>, grid, dim3(32 * B::LJ), smem, e, b, g, bc, cg);
+  GC_LAUNCH_CHECK(ctx, "block down");
   return GC_OK;
 }
+static int block_down(gc_ctx *ctx, int kid, int sweeps, float *e, const float *b, const LevelGeom &g, float *bc,
+                      const LevelGeom &cg) {
+  return sweeps == 1 ? blk_down<1, 8>(ctx, kid, e, b, g, bc, cg) : blk_down<2, 8>(ctx, kid, e, b, g, bc, cg);
+}
 
-// Levels 1 .. nlev-1 of a V-cycle: b[1] in, e[1] out. Default: two persistent
-// launches around the single-CTA tail; the validation path (natural layout)
-// keeps one launch per phase.
+template <int NS, int PHI, int TI>
+static int blk_up(gc_ctx *ctx, int kid, const float *ec, const LevelGeom &cg, const float *e, const float *b,
+                  const LevelGeom &g, float *e_out) {
+  using B = BlkU<NS>;
+  const dim3 grid(gc_blocks(g.J, B::TK), gc_blocks(g.J, B::TJ), gc_blocks(g.J, TI));
+  if (TI > 8 && (unsigned long long)grid.x * grid.y * grid.z < gc_sms())
+    return blk_up<NS, PHI, 8>(ctx, kid, ec, cg, e, b, g, e_out);
+  const size_t smem = blk_up_smem<NS, TI>();
+  if (smem > 48 * 1024)
+    GC_CUDA(ctx,
+            cudaFuncSetAttribute(k_block_up<NS, TI, PHI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  gc_launch(ctx, kid, k_block_up<NS, TI, PHI>, grid, dim3(32 * B::LJ), smem, ec, cg, e, b, g, e_out, ctx->hi, ctx->lo);
+  GC_LAUNCH_CHECK(ctx, "block up");
+  return GC_OK;
+}
+template <int PHI>
+static int block_up(gc_ctx *ctx, int kid, int sweeps, const float *ec, const LevelGeom &cg, const float *e,
+                    const float *b, const LevelGeom &g, float *e_out) {
+  return sweeps == 1 ? blk_up<1, PHI, 16>(ctx, kid, ec, cg, e, b, g, e_out)
+                     : blk_up<2, PHI, 16>(ctx, kid, ec, cg, e, b, g, e_out);
+}
+
+// Sweep counts the block kernels are built for.
+static bool block_sweeps(int pre, int post) { return pre >= 1 && pre <= 2 && post >= 1 && post <= 2; }
+
+// The finest level block by block on a natural-layout correction: for grids whose
+// eleven colour-split passes are too short to fill the GPU. Measured, kernel us per
+// V-cycle in blocks and in passes: 64^3 66 and 73, 80^3 93 and 91, 100^3 120 and 105;
+// without the vectorised passes (G not a multiple of 4) 97^3 111 and 116, 129^3 157
+// and 162. Nine launches fewer decide where the two are even.
+static bool finest_blocks(const gc_ctx *ctx, const gc_mg_params *p) {
+  return ctx->nlev > 1 && ctx->G <= (ctx->G % 4 == 0 ? 80 : 129) && !(p->flags & GC_MG_NATURAL_LAYOUT) &&
+         block_sweeps(p->pre_sweeps, p->post_sweeps);
+}
+
+// Levels 1 .. nlev-1 of a V-cycle: b[1] in, e[1] out: one launch per level each way
+// around the single-CTA tail. Sweep counts the block kernels do not have, and the
+// validation path (natural layout), take one launch per phase.
 static int coarse_levels(gc_ctx *ctx, const gc_mg_params *p) {
-  const int L = ctx->nlev;
+  const int L = ctx->nlev, pre = coarse_pre(p), post = coarse_post(p);
   int st;
-  if (!(p->flags & (GC_MG_NATURAL_LAYOUT | GC_MG_PHASE_LAUNCHES)) && ctx->tail > 1) {
-    if ((st = launch_coarse(ctx, p, false))) return st;
+  if (!(p->flags & GC_MG_NATURAL_LAYOUT) && block_sweeps(pre, post)) {
+    for (int l = 1; l < ctx->tail; ++l)
+      if ((st = block_down(ctx, GK_COARSE, pre, ctx->ed[l], ctx->b[l], ctx->lev[l], ctx->b[l + 1], ctx->lev[l + 1])))
+        return st;
     if (ctx->tail < L && (st = launch_tail(ctx, p))) return st;
-    return launch_coarse(ctx, p, true);
+    for (int l = ctx->tail - 1; l >= 1; --l)
+      if ((st = block_up<0>(ctx, GK_COARSE, post, ctx->e[l + 1], ctx->lev[l + 1], ctx->ed[l], ctx->b[l], ctx->lev[l],
+                            ctx->e[l])))
+        return st;
+    return GC_OK;
   }
   for (int l = 1; l < ctx->tail; ++l) {
     const LevelGeom &g = ctx->lev[l];
     const size_t n3 = (size_t)g.n * g.n * g.n;
     GC_CUDA(ctx, cudaMemsetAsync(ctx->e[l], 0, n3 * sizeof(float), ctx->stream));
-    if ((st = launch_smooth(ctx, l, coarse_pre(p)))) return st;
+    if ((st = launch_smooth(ctx, l, pre))) return st;
     gc_launch(ctx, GK_RESID, k_resid, dim3(node_grid(g)), dim3(dim3(32, 8)), 0, ctx->e[l], ctx->b[l], ctx->rc, g);
     gc_launch(ctx, GK_RESTRICT, k_restrict, dim3(node_grid(ctx->lev[l + 1])), dim3(dim3(32, 8)), 0, ctx->rc, g,
               ctx->b[l + 1], ctx->lev[l + 1]);
@@ -1723,7 +1863,7 @@ static int coarse_levels(gc_ctx *ctx, const gc_mg_params *p) {
     gc_launch(ctx, GK_PROLONG, k_prolong, dim3(node_grid(ctx->lev[l])), dim3(dim3(32, 8)), 0, ctx->e[l + 1],
               ctx->lev[l + 1], ctx->e[l], ctx->lev[l]);
     GC_LAUNCH_CHECK(ctx, "prolong");
-    if ((st = launch_smooth(ctx, l, coarse_post(p)))) return st;
+    if ((st = launch_smooth(ctx, l, post))) return st;
   }
   return GC_OK;
 }
@@ -1739,40 +1879,25 @@ static int residual0(gc_ctx *ctx, const gc_mg_params *p) {
   if (st) return st;
   const bool plain = (p->flags & GC_MG_PLAIN_F32) != 0;
   const Split0 d = split0(ctx);
-  if (p->flags & GC_MG_NATURAL_LAYOUT) {
-    if ((st = mg_alloc_natural(ctx))) return st;
-    if (plain)
-      gc_launch(ctx, GK_RESID0, k_resid0<true, false>, grid, dim3(32, 8), 0, ctx->hi, ctx->lo, ctx->b0, ctx->r0n,
-                nullptr, ctx->red, d);
-    else
-      gc_launch(ctx, GK_RESID0, k_resid0<false, false>, grid, dim3(32, 8), 0, ctx->hi, ctx->lo, ctx->b0, ctx->r0n,
-                nullptr, ctx->red, d);
-  } else if (vec4(ctx)) {
-    const int pre = ctx->nlev == 1 ? p->coarse_sweeps : p->pre_sweeps;
-    float *ef = pre >= 1 ? ctx->e0s : nullptr;
+  const bool natural = (p->flags & GC_MG_NATURAL_LAYOUT) != 0 || finest_blocks(ctx, p);
+  if (natural && (st = mg_alloc_natural(ctx))) return st;
+  const int pre = ctx->nlev == 1 ? p->coarse_sweeps : p->pre_sweeps;
+  float *ef = pre >= 1 && !natural ? ctx->e0s : nullptr, *r = natural ? ctx->r0n : ctx->r0s;
+  if (vec4(ctx) && !(p->flags & GC_MG_NATURAL_LAYOUT)) {
     const dim3 qg = quad_grid(ctx);
     const size_t nq = (size_t)qg.x * qg.y * qg.z;
     if ((st = gc_ensure_red(ctx, nq))) return st;
-    if (plain)
-      gc_launch(ctx, GK_RESID0, k_resid0x4<true>, qg, dim3(32, 8), 0, ctx->hi, ctx->lo, ctx->b0, ctx->r0s, ef,
-                ctx->red, d);
-    else
-      gc_launch(ctx, GK_RESID0, k_resid0x4<false>, qg, dim3(32, 8), 0, ctx->hi, ctx->lo, ctx->b0, ctx->r0s, ef,
-                ctx->red, d);
+    auto k = natural ? (plain ? k_resid0x4<true, false> : k_resid0x4<false, false>)
+                     : (plain ? k_resid0x4<true, true> : k_resid0x4<false, true>);
+    gc_launch(ctx, GK_RESID0, k, qg, dim3(32, 8), 0, ctx->hi, ctx->lo, ctx->b0, r, ef, ctx->red, d);
     GC_LAUNCH_CHECK(ctx, "resid0");
     // (a last-block sum of the 16k block partials in this kernel was slower: the
     // blocks' tickets serialise on one counter)
     return finalize_to(ctx, (int)nq, 1, GC_S_RNORM2);
-  } else {
-    const int pre = ctx->nlev == 1 ? p->coarse_sweeps : p->pre_sweeps;
-    float *ef = pre >= 1 ? ctx->e0s : nullptr;
-    if (plain)
-      gc_launch(ctx, GK_RESID0, k_resid0<true, true>, grid, dim3(32, 8), 0, ctx->hi, ctx->lo, ctx->b0, ctx->r0s, ef,
-                ctx->red, d);
-    else
-      gc_launch(ctx, GK_RESID0, k_resid0<false, true>, grid, dim3(32, 8), 0, ctx->hi, ctx->lo, ctx->b0, ctx->r0s, ef,
-                ctx->red, d);
   }
+  auto k = natural ? (plain ? k_resid0<true, false> : k_resid0<false, false>)
+                   : (plain ? k_resid0<true, true> : k_resid0<false, true>);
+  gc_launch(ctx, GK_RESID0, k, grid, dim3(32, 8), 0, ctx->hi, ctx->lo, ctx->b0, r, ef, ctx->red, d);
   GC_LAUNCH_CHECK(ctx, "resid0");
   return finalize_to(ctx, (int)nb, 1, GC_S_RNORM2);
 }
@@ -1814,6 +1939,13 @@ static int vcycle(gc_ctx *ctx, const gc_mg_params *p) {
                 ctx->hi, ctx->lo, d);
     GC_LAUNCH_CHECK(ctx, "natural cycle");
     return residual0(ctx, p);
+  }
+  if (finest_blocks(ctx, p)) {
+    if ((st = block_down(ctx, GK_SMOOTH0, pre, ctx->e0n, ctx->r0n, g0, ctx->b[1], ctx->lev[1]))) return st;
+    if ((st = coarse_levels(ctx, p))) return st;
+    st = plain ? block_up<2>(ctx, GK_UPDATE0, post, ctx->e[1], ctx->lev[1], ctx->e0n, ctx->r0n, g0, nullptr)
+               : block_up<1>(ctx, GK_UPDATE0, post, ctx->e[1], ctx->lev[1], ctx->e0n, ctx->r0n, g0, nullptr);
+    return st ? st : residual0(ctx, p);
   }
   const dim3 sg = split_grid(ctx), sg2 = split_grid2(ctx), qg = quad_grid(ctx);
   const bool v4 = vec4(ctx);
@@ -1961,8 +2093,6 @@ int gc_mg_run(gc_ctx *ctx, const gc_mg_params *p, gc_mg_stats *stats) {
   gc_mg_stats st;
   memset(&st, 0, sizeof(st));
   int s;
-  // the persistent coarse launches' grid barrier starts every solve clean
-  GC_CUDA(ctx, cudaMemsetAsync(ctx->dsmall + GC_S_GRIDBAR, 0, 2 * sizeof(double), ctx->stream));
   if (ctx->capturing && !(p->flags & GC_MG_FIXED_CYCLES)) {
     if ((s = mg_run_captured(ctx, p))) return s;
     st.cycles = -1;  // decided on the device: read them with gc_pm_graph_stats

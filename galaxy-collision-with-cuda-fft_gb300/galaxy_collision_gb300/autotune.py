@@ -1,12 +1,10 @@
 """Measured engine settings per (device, grid, particle-count bucket), cached in JSON.
 
 Some of the engine's choices change its speed and nothing else (the states are
-bit-identical, or every solve still meets the same tolerance): the coarse
-multigrid levels by the two persistent cooperative kernels or one launch per
-phase (``phase_launches``), and the cell-sort period (``sort_every``, with the
-look-ahead at half the period). Which is faster depends on the grid and the
-particle count: per-phase launches win at 64^3 and 128^3, the persistent
-kernels at 256^3. ``tune`` times every candidate on a short run of a given
+bit-identical, or every solve still meets the same tolerance): the cell-sort
+period (``sort_every``, with the look-ahead at half the period), and
+``phase_launches``, which no longer changes anything and stays so that older
+cache files keep their meaning. ``tune`` times every candidate on a short run of a given
 state (CUDA events around whole-step graph replays) and caches the fastest
 under the key ``<device>/G<grid>/N2^<k>`` (k = floor(log2 particle count)) in
 a JSON file: ``$GC_AUTOTUNE_CACHE`` or ``~/.cache/galaxy_collision_gb300/

@@ -58,7 +58,7 @@ class PMEngine:
         self.mg.tol = float(tol)
         if plain_f32:  # the all-FP32 method: stalls at the FP32 floor, runs to max_cycles
             self.mg.flags |= _native.GC_MG_PLAIN_F32
-        if phase_launches:  # coarse levels launched phase by phase (ensembles of small runs)
+        if phase_launches:  # accepted and without effect
             self.mg.flags |= _native.GC_MG_PHASE_LAUNCHES
         # sweeps each way below the finest level: None (the default) for pre/post_sweeps
         # on every level, as the reference; 1 for fewer latency-bound coarse phases at

@@ -16,9 +16,8 @@ Workload (the batched-ensemble configuration): 64 two-disk collisions with
 particle counts log-uniform in [0.25M, 4M], 64^3 grids below 1M particles and
 128^3 otherwise, geometry randomised as in the training set. The comparison is
 the same runs advanced one after the other, each through its own step graph.
-The runs' coarse multigrid levels are launched phase by phase
-(GC_MG_PHASE_LAUNCHES): at 64^3 and 128^3 that is faster than the persistent
-cooperative kernels, alone and side by side.
+The runs' coarse multigrid levels are ordinary launches, one per level each
+way, so those of different runs interleave.
 
 Command line::
 
@@ -187,7 +186,7 @@ def main(argv=None):
     ap.add_argument("--one-by-one-steps", type=int, default=None)
     ap.add_argument("--seed", type=int, default=5)
     ap.add_argument("--persistent-coarse", action="store_true",
-                    help="coarse multigrid levels by the persistent kernels instead of one launch per phase")
+                    help="(without effect: kept for older command lines)")
     ap.add_argument("--autotune", action="store_true",
                     help="per (grid, particle-count bucket) settings from the autotuner's JSON cache (tuned on "
                          "first use)")

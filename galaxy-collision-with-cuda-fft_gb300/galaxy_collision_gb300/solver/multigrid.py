@@ -70,8 +70,7 @@ class MultigridPoissonSolver(PoissonSolver):
         # natural_layout: validation path, the finest correction in natural
         # layout through the generic level kernels (identical potentials)
         self.natural_layout = bool(natural_layout)
-        # phase_launches: the coarse levels by one launch per phase instead of
-        # the persistent kernels (identical potentials)
+        # phase_launches: accepted and without effect (GC_MG_PHASE_LAUNCHES)
         self.phase_launches = bool(phase_launches)
         # coarse_level_sweeps=1: one sweep each way below the finest level (the
         # engine's default); None keeps pre/post sweeps on every level, as the reference

@@ -72,14 +72,14 @@ enum gc_status_code {
  * warm_start, else zero. With faces from a free-space (lattice Green's function)
  * evaluation this is the isolated-boundary solve of James's method. */
 #define GC_MG_FACES_GIVEN 0x10
-/* gc_mg_params.flags: the coarse levels by one launch per phase instead of the
- * two persistent cooperative launches: slower for one solve alone, but the
- * launches of many small solves running at once on one GPU (an ensemble of
- * runs on separate streams) can interleave. Same potentials bit for bit. */
+/* gc_mg_params.flags: accepted and without effect. It replaced cooperative
+ * coarse-level launches, which could not run side by side, by one launch per
+ * phase; the levels now take one ordinary launch each way, which interleave
+ * with those of other solves. */
 #define GC_MG_PHASE_LAUNCHES 0x20
 /* gc_mg_params.flags: every level below the finest relaxes with one red-black
  * sweep before restriction and one after prolongation; the finest keeps
- * pre_sweeps / post_sweeps. Fewer barrier-separated phases on the latency-bound
+ * pre_sweeps / post_sweeps. Fewer dependent phases on the latency-bound
  * coarse levels for a slightly weaker V-cycle; the stopping rule is unchanged. */
 #define GC_MG_COARSE_ONE_SWEEP 0x40
 
