@@ -830,6 +830,497 @@ __global__ void __launch_bounds__(256)
 }
 
 // ------------------------------------------------------------------------------
+// finest level: the way down and the way up as one pass each over the planes
+// ------------------------------------------------------------------------------
+// k_fine_down: three half-sweeps, the residual of the correction and its restriction
+// (the first red half-sweep, from zero, included). k_fine_up: the prolongation, four
+// half-sweeps and phi += e. Instead of one pass over memory per half-sweep, a CTA takes
+// all k of a strip of rows and marches along i: at plane p it relaxes the newest plane
+// for the first time, plane p-1 for the second time, and so on, so that a plane
+// leaves the pipeline four planes later and is read and written once. Rows at the
+// strip's edges (four each side) and the planes at the ends of its march are relaxed
+// by its neighbours too. The arithmetic of every node is that of k_rb0x2,
+// k_resid0ex4, k_restrict, k_prolong0bx2 and k_rb0_lastx4: identical potentials.
+//
+// A thread owns four nodes along k (two slots of each colour) of FL_RJ neighbouring
+// rows and keeps, for each stage, the other colour's values at its nodes on the last
+// two planes (z: plane q, x: plane q - 1) in registers; plane q + 1 is what the stage
+// before has just produced. So the i neighbours, and the j neighbours inside its rows,
+// cost nothing; the others come from shared memory, where every stage publishes its
+// plane for the next step. One barrier per plane. With rows starting on odd j the
+// k parity of the active nodes is the same in every stage of a step and alternates
+// with the row and the plane: compile-time constants in a loop over plane pairs.
+//
+// The next step's right-hand sides are loaded at the end of a step, all together: loads
+// issued among the stages held up every later wait (a warp has few scoreboards) and
+// took a quarter longer. Bound by instruction issue and latency (12 warps an SM: 168
+// registers each; issue slots 51 % and LSU 53 % busy, DRAM 14 to 46 %), with 24 rows of
+// which 14 (down) or 16 (up) are a strip's own. Measured at 256^3: 95 us down and 99 us
+// up, against 126 us for three half-sweeps, the residual and the restriction and 146 us
+// for the prolongation, three half-sweeps and the last one with the update; the
+// residual kernel also no longer writes the first half-sweep (69 -> 65 us).
+#define FL_RJ 4
+#define FL_THREADS 384
+struct FL {
+  static constexpr int W = 2;                         // warps along k: 128 nodes each
+  static constexpr int NG = FL_THREADS / 32 / W, ROWS = FL_RJ * NG, PH = 64 * W + 4;
+  static constexpr int plane = ROWS * PH;             // floats of one published half plane
+  static constexpr int NJ = (ROWS - 10) / 2;          // coarse rows of a strip on the way down
+  static constexpr int NR = ROWS - 8;                 // rows of a strip on the way up
+  static constexpr int CR = ROWS / 2 + 2;             // coarse rows under a strip on the way up
+  // a margin row, two sets of four published planes, then the pass's own
+  static constexpr int pub = PH + 8 * plane;
+  static constexpr size_t smem_down = sizeof(float) * (pub + 2 * ROWS * 32 * W + 2 * NG * 64 * W);
+  static constexpr size_t smem_up = sizeof(float) * (pub + 2 * CR * PH + 16 * FL_RJ * FL_THREADS);
+};
+
+struct FlThread {
+  int t, g, j0;        // quad, row group, first row
+  bool first, last;    // quad 0, the quad of k = G - 1
+  int at[FL_RJ];       // (j H + 2 t) of the row, rows and quads clamped to the grid's
+  float six[FL_RJ];    // 1/6 on interior rows, else 0: results off the interior are zero
+};
+
+// The neighbour sums of the active nodes; pa: their k parity.
+__device__ __forceinline__ float2 fl_sum(float2 xp, float2 xm, float2 yp, float2 ym, float2 z, float zo, int pa) {
+  const float az0 = pa ? __fadd_rn(z.y, z.x) : __fadd_rn(z.x, zo);
+  const float az1 = pa ? __fadd_rn(zo, z.y) : __fadd_rn(z.y, z.x);
+  return make_float2(__fadd_rn(__fadd_rn(__fadd_rn(xp.x, xm.x), __fadd_rn(yp.x, ym.x)), az0),
+                     __fadd_rn(__fadd_rn(__fadd_rn(xp.y, xm.y), __fadd_rn(yp.y, ym.y)), az1));
+}
+// (sum - r) / 6, zero on the faces k = 0 and k = G - 1 (six: 1/6, or 0 off the
+// interior rows and planes)
+__device__ __forceinline__ float2 fl_relax(float2 s, float2 r, float six, const FlThread &T, int pa) {
+  float2 v = make_float2(__fmul_rn(__fsub_rn(s.x, r.x), six), __fmul_rn(__fsub_rn(s.y, r.y), six));
+  if (pa == 0) v.x = T.first ? 0.0f : v.x;
+  else v.y = T.last ? 0.0f : v.y;
+  return v;
+}
+
+// One stage on all rows of the thread: the neighbour sums of its active nodes from
+// xp (plane q + 1), z and x (planes q and q - 1) and, outside its rows, the plane q
+// that the stage before published (buf: this thread's first slot in row 0 of the
+// strip). The strip's outermost rows read whatever lies beside them: their results
+// are not used.
+template <int PH>
+__device__ __forceinline__ void fl_sums(const float2 (&xp)[FL_RJ], const float2 (&x)[FL_RJ], const float2 (&z)[FL_RJ],
+                                        const float *buf, const FlThread &T, int par, float2 (&sum)[FL_RJ]) {
+  const float2 below = ld2(buf - PH), above = ld2(buf + FL_RJ * PH);
+#pragma unroll
+  for (int a = 0; a < FL_RJ; ++a) {
+    const int pa = (par + a) & 1;
+    const float zo = buf[a * PH + (pa ? 2 : -1)];
+    const float2 yp = a + 1 < FL_RJ ? z[a + 1 < FL_RJ ? a + 1 : a] : above;
+    const float2 ym = a > 0 ? z[a > 0 ? a - 1 : a] : below;
+    sum[a] = fl_sum(xp[a], x[a], yp, ym, z[a], zo, pa);
+  }
+}
+
+template <int PH>
+__device__ __forceinline__ void fl_publish(float *buf, const float2 (&v)[FL_RJ]) {
+#pragma unroll
+  for (int a = 0; a < FL_RJ; ++a) st2(buf + a * PH, v[a].x, v[a].y);
+}
+
+__device__ __forceinline__ void fl_shift(float2 (&x)[FL_RJ], float2 (&z)[FL_RJ], const float2 (&v)[FL_RJ]) {
+#pragma unroll
+  for (int a = 0; a < FL_RJ; ++a) {
+    x[a] = z[a];
+    z[a] = v[a];
+  }
+}
+
+__device__ __forceinline__ FlThread fl_thread(int jb, const Split0 &d) {
+  FlThread T;
+  const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+  T.t = 32 * (w % FL::W) + lane;
+  T.g = w / FL::W;
+  T.j0 = jb + FL_RJ * T.g;
+  T.first = T.t == 0;
+  T.last = 4 * T.t + 4 == d.G;
+  const int tc = min(T.t, d.G / 4 - 1);
+#pragma unroll
+  for (int a = 0; a < FL_RJ; ++a) {
+    const int j = T.j0 + a;
+    T.six[a] = 4 * T.t < d.G && j >= 1 && j <= d.G - 2 ? GC_SIXTH : 0.0f;
+    T.at[a] = min(max(j, 0), d.G - 1) * d.H + 2 * tc;
+  }
+  return T;
+}
+
+// Two slots of row a on plane q (clamped) of a colour half.
+__device__ __forceinline__ float2 fl_load(const float *__restrict__ half, int q, const Split0 &d, const FlThread &T,
+                                          int a) {
+  const float *plane = half + (size_t)min(max(q, 0), d.G - 1) * (size_t)(d.G * d.H);
+  return __ldg(reinterpret_cast<const float2 *>(plane + T.at[a]));
+}
+
+struct FlDown {
+  float2 x1[FL_RJ], z1[FL_RJ], x2[FL_RJ], z2[FL_RJ], x3[FL_RJ], z3[FL_RJ], x4[FL_RJ], z4[FL_RJ];
+  float2 n0[FL_RJ], n1[FL_RJ], n2[FL_RJ], n3[FL_RJ], n4[FL_RJ];  // each stage's r, loaded a step ahead
+  float2 rb[FL_RJ];                         // residual of the black nodes one plane ahead of the red ones'
+  float r0[FL_RJ], r1[FL_RJ], sB[FL_RJ];    // plane p - 4: residuals at k = 4t, 4t + 1; k sum of K = 2t + 1
+  float tA[FL_RJ], tB[FL_RJ];               // plane p - 5: k sums of K = 2t and 2t + 1
+  float accA[FL_RJ / 2], accB[FL_RJ / 2];   // restricted sums under way
+
+  // PP: parity of plane p. Restriction weights are 1/4, 1/2, 1/4, but 0 for a face
+  // (wB, wj: 1/4 or 0): with G a multiple of 4 no node lies beyond the last coarse one.
+  template <int PP>
+  __device__ __forceinline__ void step(int p, int c, float *fs, const FlThread &T, const float *__restrict__ r,
+                                       float *__restrict__ eb, float *__restrict__ bc, const Split0 &d, int m, int Jm,
+                                       int I0, int I1, int je, float wB, const float (&wj)[FL_RJ / 2], unsigned own) {
+    using L = FL;
+    constexpr int W = L::W;
+    constexpr int PH = L::PH, par = PP + 1;  // k parity of the active nodes of row 0
+    const int G = d.G;
+    float *base = fs + PH + FL_RJ * T.g * PH + 2 + 2 * T.t;
+    float *wr = base + c * 4 * L::plane, *rd = base + (c ^ 1) * 4 * L::plane;
+    float *edge = fs + L::pub + FL_RJ * T.g * 32 * W + T.t, *rows = fs + L::pub + 2 * L::ROWS * 32 * W;
+    const float *red = r, *blk = r + d.half;
+    // restriction, plane p - 6: row and plane sums
+    {
+      const float2 next = ld2(rows + 2 * (((c ^ 1) * L::NG + min(T.g + 1, L::NG - 1)) * 32 * W + T.t));
+      const int i = p - 6, I = (i - 1) >> 1;  // (i has the parity of p)
+#pragma unroll
+      for (int h = 0; h < FL_RJ / 2; ++h) {
+        const int a = 2 * h + 1;  // the centre row
+        const float sA2 = a + 1 < FL_RJ ? tA[a + 1 < FL_RJ ? a + 1 : a] : next.x;
+        const float sB2 = a + 1 < FL_RJ ? tB[a + 1 < FL_RJ ? a + 1 : a] : next.y;
+        float uA = 0.25f * tA[a - 1], uB = 0.25f * tB[a - 1];
+        uA += 0.5f * tA[a]; uB += 0.5f * tB[a];
+        uA += wj[h] * sA2; uB += wj[h] * sB2;
+        if (PP == 0) {  // even plane: the centre one of I
+          accA[h] += 0.5f * uA;
+          accB[h] += 0.5f * uB;
+        } else {        // odd plane: the last one of I, the first one of I + 1
+          const float wi = i <= G - 2 ? 0.25f : 0.0f;
+          accA[h] += wi * uA;
+          accB[h] += wi * uB;
+          if (I >= I0 && I <= I1 && ((own >> (8 + h)) & 1u)) {
+            float *o = bc + ((size_t)I * m + ((T.j0 + a) >> 1)) * m + 2 * T.t;
+            if (!T.first) o[0] = 4.0f * accA[h];
+            o[1] = 4.0f * accB[h];
+          }
+          accA[h] = 0.25f * uA;
+          accB[h] = 0.25f * uB;
+        }
+      }
+    }
+    // restriction, plane p - 5: the k sums (K = 2t needs the quad before)
+    {
+      const float *er = edge + (c ^ 1) * L::ROWS * 32 * W;
+#pragma unroll
+      for (int a = 0; a < FL_RJ; ++a) {
+        float s = 0.5f * r0[a];
+        s += 0.25f * er[a * 32 * W - 1];
+        s += 0.25f * r1[a];
+        tA[a] = s;
+        tB[a] = sB[a];
+      }
+      st2(rows + 2 * ((c * L::NG + T.g) * 32 * W + T.t), tA[0], tB[0]);
+    }
+    float2 v0[FL_RJ], v1[FL_RJ], v2[FL_RJ], v3[FL_RJ], s[FL_RJ];
+    // plane p: red from zero (r is zero on the face planes)
+#pragma unroll
+    for (int a = 0; a < FL_RJ; ++a) {
+      v0[a] = make_float2(__fmul_rn(0.0f - n0[a].x, T.six[a]), __fmul_rn(0.0f - n0[a].y, T.six[a]));
+    }
+    fl_publish<PH>(wr, v0);
+    // plane p - 1: black
+    fl_sums<PH>(v0, x1, z1, rd, T, par, s);
+    const bool ok1 = p - 1 >= 1 && p - 1 <= G - 2;
+#pragma unroll
+    for (int a = 0; a < FL_RJ; ++a) {
+      v1[a] = fl_relax(s[a], n1[a], ok1 ? T.six[a] : 0.0f, T, (par + a) & 1);
+    }
+    fl_shift(x1, z1, v0);
+    fl_publish<PH>(wr + L::plane, v1);
+    // plane p - 2: red
+    fl_sums<PH>(v1, x2, z2, rd + L::plane, T, par, s);
+    const bool ok2 = p - 2 >= 1 && p - 2 <= G - 2;
+#pragma unroll
+    for (int a = 0; a < FL_RJ; ++a) {
+      v2[a] = fl_relax(s[a], n2[a], ok2 ? T.six[a] : 0.0f, T, (par + a) & 1);
+    }
+    fl_shift(x2, z2, v1);
+    fl_publish<PH>(wr + 2 * L::plane, v2);
+    // plane p - 3: black, and its residual
+    fl_sums<PH>(v2, x3, z3, rd + 2 * L::plane, T, par, s);
+    const bool ok3 = p - 3 >= 1 && p - 3 <= G - 2;
+    const float diag = 6.0f;
+    float2 rbn[FL_RJ];
+#pragma unroll
+    for (int a = 0; a < FL_RJ; ++a) {
+      v3[a] = fl_relax(s[a], n3[a], ok3 ? T.six[a] : 0.0f, T, (par + a) & 1);
+      rbn[a] = make_float2(n3[a].x - (s[a].x - diag * v3[a].x), n3[a].y - (s[a].y - diag * v3[a].y));
+    }
+    if (p - 3 >= 2 * I0 - 1 && p - 3 <= je) {  // the black correction for the way up
+      float *o = eb + (size_t)(p - 3) * (size_t)(G * d.H);
+#pragma unroll
+      for (int a = 0; a < FL_RJ; ++a)
+        if ((own >> a) & 1u) st2(o + T.at[a], v3[a].x, v3[a].y);
+    }
+    fl_publish<PH>(wr + 3 * L::plane, v3);
+    // plane p - 4: residual of the red nodes (their values are x3), both colours in order
+    fl_sums<PH>(v3, x4, z4, rd + 3 * L::plane, T, par, s);
+#pragma unroll
+    for (int a = 0; a < FL_RJ; ++a) {
+      const float2 rr = make_float2(n4[a].x - (s[a].x - diag * x3[a].x), n4[a].y - (s[a].y - diag * x3[a].y));
+      const bool even = ((par + a) & 1) == 0;
+      const float q2 = even ? rr.y : rb[a].y, q3 = even ? rb[a].y : rr.y;
+      r0[a] = even ? rr.x : rb[a].x;
+      r1[a] = even ? rb[a].x : rr.x;
+      edge[c * L::ROWS * 32 * W + a * 32 * W] = q3;
+      float k = 0.5f * q2;  // K = 2t + 1
+      k += 0.25f * r1[a];
+      k += wB * q3;
+      sB[a] = k;
+      rb[a] = rbn[a];
+    }
+    fl_shift(x3, z3, v2);
+    fl_shift(x4, z4, v3);
+    // the next step's r, all at once (a load issued among the stages would be waited for
+    // with the next one's: a warp has few scoreboards)
+#pragma unroll
+    for (int a = 0; a < FL_RJ; ++a) {
+      n0[a] = fl_load(red, p + 1, d, T, a);
+      n1[a] = fl_load(blk, p, d, T, a);
+      n2[a] = fl_load(red, p - 1, d, T, a);
+      n3[a] = fl_load(blk, p - 2, d, T, a);
+      n4[a] = fl_load(red, p - 3, d, T, a);
+    }
+    __syncthreads();
+  }
+};
+
+__global__ void __launch_bounds__(FL_THREADS, 1)
+    k_fine_down(const float *__restrict__ r, float *__restrict__ eb, float *__restrict__ bc, Split0 d, int m, int Jm,
+                int per) {
+  using L = FL;
+  extern __shared__ __align__(16) float fs[];
+  for (int i = threadIdx.x; i < (int)(L::smem_down / sizeof(float)); i += FL_THREADS) fs[i] = 0.0f;
+  const int J0 = 1 + blockIdx.x * L::NJ, I0 = 1 + blockIdx.y * per, I1 = min(I0 + per - 1, Jm);
+  const FlThread T = fl_thread(2 * J0 - 5, d);
+  const bool in = 4 * T.t < d.G;
+  // rows (bits 0 .. 3) and coarse rows (bits 8, 9) this thread writes
+  const int re = J0 + L::NJ > Jm ? d.G - 2 : 2 * (J0 + L::NJ - 1);
+  unsigned own = 0;
+  float wj[FL_RJ / 2];
+#pragma unroll
+  for (int a = 0; a < FL_RJ; ++a) {
+    const int j = T.j0 + a, lr = FL_RJ * T.g + a;
+    if (in && j >= 2 * J0 - 1 && j <= re) own |= 1u << a;
+    if (a & 1) {
+      wj[a >> 1] = j + 1 <= d.G - 2 ? 0.25f : 0.0f;
+      if (in && lr >= 5 && lr < 5 + 2 * L::NJ && j >= 2 && j <= 2 * Jm) own |= 1u << (8 + (a >> 1));
+    }
+  }
+  const float wB = T.last ? 0.0f : 0.25f;
+  const int je = I1 == Jm ? d.G - 2 : 2 * I1;
+  FlDown S = {};
+  {  // the first step's loads
+    const int p = 2 * I0 - 5;
+#pragma unroll
+    for (int a = 0; a < FL_RJ; ++a) {
+      S.n0[a] = fl_load(r, p, d, T, a);
+      S.n1[a] = fl_load(r + d.half, p - 1, d, T, a);
+    }
+  }
+  __syncthreads();
+  for (int p = 2 * I0 - 5; p <= 2 * I1 + 7; p += 2) {
+    S.step<1>(p, 0, fs, T, r, eb, bc, d, m, Jm, I0, I1, je, wB, wj, own);
+    S.step<0>(p + 1, 1, fs, T, r, eb, bc, d, m, Jm, I0, I1, je, wB, wj, own);
+  }
+}
+
+__device__ __forceinline__ void fl_cp4(float *dst, const float *src, bool in) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src),
+               "r"(in ? 4u : 0u)
+               : "memory");
+}
+__device__ __forceinline__ void fl_cp16(float *dst, const float *src) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+               : "memory");
+}
+__device__ __forceinline__ void fl_cp_wait() { asm volatile("cp.async.wait_all;" ::: "memory"); }
+
+template <bool PLAIN>
+struct FlUp {
+  float2 x1[FL_RJ], z1[FL_RJ], x2[FL_RJ], z2[FL_RJ], x3[FL_RJ], z3[FL_RJ], x4[FL_RJ], z4[FL_RJ];
+  float2 ne[FL_RJ], n1[FL_RJ], n2[FL_RJ], n3[FL_RJ], n4[FL_RJ];  // the next step's correction and r
+
+  // coarse plane I under the strip (rows from c0) into its slot of the ring of two
+  static __device__ __forceinline__ void coarse(float *ring, const float *__restrict__ ec, int I, int c0, int m) {
+    using L = FL;
+    const int lane = threadIdx.x & 31;
+    for (int rr = threadIdx.x >> 5; rr < L::CR; rr += FL_THREADS / 32) {
+      const int J = c0 + rr;
+      const bool in = I >= 0 && I < m && J >= 0 && J < m;
+      const float *src = ec + (in ? ((size_t)I * m + J) * m : 0);
+      float *dst = ring + ((I & 1) * L::CR + rr) * L::PH;
+#pragma unroll
+      for (int K = 0; K < L::PH; K += 32)
+        if (K + lane < L::PH) fl_cp4(dst + K + lane, in && K + lane < m ? src + K + lane : ec, in && K + lane < m);
+    }
+  }
+  // hi and lo of plane q (the strip's own rows), into the thread's own slots
+  static __device__ __forceinline__ void phi(float *slot, const float *hi, const float *lo, int q, int i1, int i2,
+                                             int G, const FlThread &T, unsigned own) {
+    if (q < i1 || q > i2) return;
+#pragma unroll
+    for (int a = 0; a < FL_RJ; ++a) {
+      if (!((own >> a) & 1u)) continue;
+      const size_t c0 = ((size_t)q * G + T.j0 + a) * G + 4 * T.t;
+      fl_cp16(slot + (2 * a) * 4 * FL_THREADS, hi + c0);
+      if (!PLAIN) fl_cp16(slot + (2 * a + 1) * 4 * FL_THREADS, lo + c0);
+    }
+  }
+
+  template <int PP>
+  __device__ __forceinline__ void step(int p, int c, float *fs, const FlThread &T, const float *__restrict__ ec,
+                                       const float *__restrict__ eb, const float *__restrict__ r, float *hi, float *lo,
+                                       const Split0 &d, int m, int i1, int i2, int cr0, unsigned own) {
+    using L = FL;
+    constexpr int PH = L::PH, par = PP;  // k parity of the active nodes of row 0
+    const int G = d.G;
+    float *base = fs + PH + FL_RJ * T.g * PH + 2 + 2 * T.t;
+    float *wr = base + c * 4 * L::plane, *rd = base + (c ^ 1) * 4 * L::plane;
+    float *ring = fs + L::pub, *slot = ring + 2 * L::CR * PH + 4 * threadIdx.x;
+    const float *red = r, *blk = r + d.half;
+    // the next step's potential, and the next coarse plane before an odd plane needs it
+    phi(slot + (c ^ 1) * 8 * FL_RJ * FL_THREADS, hi, lo, p - 3, i1, i2, G, T, own);
+    if (PP == 0) coarse(ring, ec, (p >> 1) + 1, cr0, m);
+    float2 v0[FL_RJ], v1[FL_RJ], v2[FL_RJ], v3[FL_RJ], s[FL_RJ];
+    // plane p: black, the correction of the way down plus the prolonged coarse one:
+    // weight 1 on even coordinates, 1/2 and 1/2 on odd ones (with G a multiple of 4 no
+    // interior node lies beyond the last coarse one), in k_prolong0bx2's order
+    const float okp = p >= 1 && p <= G - 2 ? 1.0f : 0.0f;
+#pragma unroll
+    for (int a = 0; a < FL_RJ; ++a) {
+      // row j0 + a is odd for even a; its coarse row and the one after it
+      constexpr int ni = PP ? 2 : 1;
+      const int pa = (par + a) & 1, nj = a & 1 ? 1 : 2;
+      const float *q = ring + (((T.j0 + a) >> 1) - cr0) * PH + 2 * T.t;
+      const float w = (ni == 2 ? 0.5f : 1.0f) * (nj == 2 ? 0.5f : 1.0f) * (pa ? 0.5f : 1.0f);
+      float2 v = make_float2(0.0f, 0.0f);
+#pragma unroll
+      for (int u = 0; u < ni; ++u)
+#pragma unroll
+        for (int h = 0; h < nj; ++h) {
+          const float *row = q + ((((p >> 1) + u) & 1) * L::CR + h) * PH;
+          const float2 e01 = ld2(row);
+          v.x += w * e01.x;
+          if (pa) v.x += w * e01.y;
+          v.y += w * e01.y;
+          if (pa) v.y += w * row[2];
+        }
+      const float on = T.six[a] != 0.0f ? okp : 0.0f;
+      v = make_float2(__fmul_rn(__fadd_rn(ne[a].x, v.x), on), __fmul_rn(__fadd_rn(ne[a].y, v.y), on));
+      if (pa == 0) v.x = T.first ? 0.0f : v.x;
+      else v.y = T.last ? 0.0f : v.y;
+      v0[a] = v;
+    }
+    fl_publish<PH>(wr, v0);
+    // planes p - 1 (red), p - 2 (black), p - 3 (red)
+    fl_sums<PH>(v0, x1, z1, rd, T, par, s);
+    const bool ok1 = p - 1 >= 1 && p - 1 <= G - 2;
+#pragma unroll
+    for (int a = 0; a < FL_RJ; ++a) {
+      v1[a] = fl_relax(s[a], n1[a], ok1 ? T.six[a] : 0.0f, T, (par + a) & 1);
+    }
+    fl_shift(x1, z1, v0);
+    fl_publish<PH>(wr + L::plane, v1);
+    fl_sums<PH>(v1, x2, z2, rd + L::plane, T, par, s);
+    const bool ok2 = p - 2 >= 1 && p - 2 <= G - 2;
+#pragma unroll
+    for (int a = 0; a < FL_RJ; ++a) {
+      v2[a] = fl_relax(s[a], n2[a], ok2 ? T.six[a] : 0.0f, T, (par + a) & 1);
+    }
+    fl_shift(x2, z2, v1);
+    fl_publish<PH>(wr + 2 * L::plane, v2);
+    fl_sums<PH>(v2, x3, z3, rd + 2 * L::plane, T, par, s);
+    const bool ok3 = p - 3 >= 1 && p - 3 <= G - 2;
+#pragma unroll
+    for (int a = 0; a < FL_RJ; ++a) {
+      v3[a] = fl_relax(s[a], n3[a], ok3 ? T.six[a] : 0.0f, T, (par + a) & 1);
+    }
+    fl_shift(x3, z3, v2);
+    fl_publish<PH>(wr + 3 * L::plane, v3);
+    // plane p - 4: black, then phi += e for the quad (the red nodes are z4)
+    fl_sums<PH>(v3, x4, z4, rd + 3 * L::plane, T, par, s);
+    const int q = p - 4;
+    const bool mine = q >= i1 && q <= i2;
+    const float *pv = slot + c * 8 * FL_RJ * FL_THREADS;
+#pragma unroll
+    for (int a = 0; a < FL_RJ; ++a) {
+      const float2 rv = n4[a];
+      if (!mine || !((own >> a) & 1u)) continue;
+      const float2 e = make_float2(__fmul_rn(s[a].x - rv.x, GC_SIXTH), __fmul_rn(s[a].y - rv.y, GC_SIXTH));
+      const bool even = ((par + a) & 1) == 0;  // the black nodes are k = 4t, 4t + 2
+      const float ev[4] = {even ? e.x : z4[a].x, even ? z4[a].x : e.x, even ? e.y : z4[a].y, even ? z4[a].y : e.y};
+      const size_t c0 = ((size_t)q * G + T.j0 + a) * G + 4 * T.t;
+      float4 h = ld4(pv + (2 * a) * 4 * FL_THREADS);
+      float4 l = PLAIN ? make_float4(0.f, 0.f, 0.f, 0.f) : ld4(pv + (2 * a + 1) * 4 * FL_THREADS);
+      const float hx = h.x, lx = l.x, hw = h.w, lw = l.w;
+      phi_sum<PLAIN>(h.x, l.x, ev[0]);
+      phi_sum<PLAIN>(h.y, l.y, ev[1]);
+      phi_sum<PLAIN>(h.z, l.z, ev[2]);
+      phi_sum<PLAIN>(h.w, l.w, ev[3]);
+      if (T.first) { h.x = hx; l.x = lx; }
+      if (T.last) { h.w = hw; l.w = lw; }
+      st4(hi + c0, h);
+      if (!PLAIN) st4(lo + c0, l);
+    }
+    fl_shift(x4, z4, v3);
+    fl_cp_wait();
+#pragma unroll
+    for (int a = 0; a < FL_RJ; ++a) {
+      ne[a] = fl_load(eb, p + 1, d, T, a);
+      n1[a] = fl_load(red, p, d, T, a);
+      n2[a] = fl_load(blk, p - 1, d, T, a);
+      n3[a] = fl_load(red, p - 2, d, T, a);
+      n4[a] = fl_load(blk, p - 3, d, T, a);
+    }
+    __syncthreads();
+  }
+};
+
+template <bool PLAIN>
+__global__ void __launch_bounds__(FL_THREADS, 1)
+    k_fine_up(const float *__restrict__ ec, int m, const float *__restrict__ eb, const float *__restrict__ r, float *hi,
+              float *lo, Split0 d, int per) {
+  using L = FL;
+  extern __shared__ __align__(16) float fs[];
+  for (int i = threadIdx.x; i < (int)(L::smem_up / sizeof(float)); i += FL_THREADS) fs[i] = 0.0f;
+  const int j1 = 1 + blockIdx.x * L::NR, i1 = 1 + blockIdx.y * per, i2 = min(i1 + per - 1, d.G - 2);
+  const FlThread T = fl_thread(j1 - 4, d);
+  const int cr0 = (j1 - 4) >> 1;
+  unsigned own = 0;  // rows whose potential this thread updates
+#pragma unroll
+  for (int a = 0; a < FL_RJ; ++a)
+    if (T.six[a] != 0.0f && T.j0 + a >= j1 && T.j0 + a < j1 + L::NR) own |= 1u << a;
+  FlUp<PLAIN> S = {};
+  __syncthreads();
+  {  // the first step's coarse planes and loads
+    const int p = i1 - 4;
+    float *ring = fs + L::pub;
+    FlUp<PLAIN>::coarse(ring, ec, p >> 1, cr0, m);
+    FlUp<PLAIN>::coarse(ring, ec, (p >> 1) + 1, cr0, m);
+#pragma unroll
+    for (int a = 0; a < FL_RJ; ++a) {
+      S.ne[a] = fl_load(eb, p, d, T, a);
+      S.n1[a] = fl_load(r, p - 1, d, T, a);
+    }
+    fl_cp_wait();
+  }
+  __syncthreads();
+  for (int p = i1 - 4; p <= i2 + 4; p += 2) {
+    S.template step<1>(p, 0, fs, T, ec, eb, r, hi, lo, d, m, i1, i2, cr0, own);
+    S.template step<0>(p + 1, 1, fs, T, ec, eb, r, hi, lo, d, m, i1, i2, cr0, own);
+  }
+}
+
+// ------------------------------------------------------------------------------
 // a level's way down and way up in one launch each, block by block
 // ------------------------------------------------------------------------------
 // k_block_down: the pre-smoothing from a zero correction, the residual and its
@@ -1829,6 +2320,43 @@ static bool finest_blocks(const gc_ctx *ctx, const gc_mg_params *p) {
          block_sweeps(p->pre_sweeps, p->post_sweeps);
 }
 
+// The finest level as two passes over its planes (two sweeps each way): rows of at most
+// 64 quads, and grids large enough that the passes' halos weigh less than the traffic
+// they save. Measured, kernel us per V-cycle in plane passes and in half-sweeps: 128^3
+// 140 and 126, 144^3 177 and 181, 192^3 254 and 277, 256^3 405 and 488.
+static bool finest_planes(const gc_ctx *ctx, const gc_mg_params *p) {
+  return ctx->nlev > 1 && ctx->G % 4 == 0 && ctx->G >= 144 && ctx->G <= 256 && !(p->flags & GC_MG_NATURAL_LAYOUT) &&
+         p->pre_sweeps == 2 && p->post_sweeps == 2 && !finest_blocks(ctx, p);
+}
+
+// Strips of rows along x; along y as many stretches of planes as the remaining SMs
+// allow (one CTA per SM).
+static int fine_down(gc_ctx *ctx) {
+  using L = FL;
+  const LevelGeom &cg = ctx->lev[1];
+  const unsigned strips = gc_blocks(cg.J, L::NJ);
+  const unsigned parts = gc_sms() > strips ? gc_sms() / strips : 1;
+  const int per = (int)gc_blocks(cg.J, (int)parts);
+  GC_CUDA(ctx, cudaFuncSetAttribute(k_fine_down, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::smem_down));
+  gc_launch(ctx, GK_SMOOTH0, k_fine_down, dim3(strips, gc_blocks(cg.J, per)), dim3(FL_THREADS), L::smem_down,
+            ctx->r0s, ctx->e0s + ctx->half0, ctx->b[1], split0(ctx), cg.n, cg.J, per);
+  GC_LAUNCH_CHECK(ctx, "fine down");
+  return GC_OK;
+}
+template <bool PLAIN>
+static int fine_up(gc_ctx *ctx) {
+  using L = FL;
+  const LevelGeom &g0 = ctx->lev[0], &cg = ctx->lev[1];
+  const unsigned strips = gc_blocks(g0.J, L::NR);
+  const unsigned parts = gc_sms() > strips ? gc_sms() / strips : 1;
+  const int per = ((int)gc_blocks(g0.J, (int)parts) + 1) & ~1;  // even: a stretch starts on an odd plane
+  GC_CUDA(ctx, cudaFuncSetAttribute(k_fine_up<PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::smem_up));
+  gc_launch(ctx, GK_UPDATE0, k_fine_up<PLAIN>, dim3(strips, gc_blocks(g0.J, per)), dim3(FL_THREADS), L::smem_up,
+            ctx->e[1], cg.n, ctx->e0s + ctx->half0, ctx->r0s, ctx->hi, ctx->lo, split0(ctx), per);
+  GC_LAUNCH_CHECK(ctx, "fine up");
+  return GC_OK;
+}
+
 // Levels 1 .. nlev-1 of a V-cycle: b[1] in, e[1] out: one launch per level each way
 // around the single-CTA tail. Sweep counts the block kernels do not have, and the
 // validation path (natural layout), take one launch per phase.
@@ -1882,7 +2410,7 @@ static int residual0(gc_ctx *ctx, const gc_mg_params *p) {
   const bool natural = (p->flags & GC_MG_NATURAL_LAYOUT) != 0 || finest_blocks(ctx, p);
   if (natural && (st = mg_alloc_natural(ctx))) return st;
   const int pre = ctx->nlev == 1 ? p->coarse_sweeps : p->pre_sweeps;
-  float *ef = pre >= 1 && !natural ? ctx->e0s : nullptr, *r = natural ? ctx->r0n : ctx->r0s;
+  float *ef = pre >= 1 && !natural && !finest_planes(ctx, p) ? ctx->e0s : nullptr, *r = natural ? ctx->r0n : ctx->r0s;
   if (vec4(ctx) && !(p->flags & GC_MG_NATURAL_LAYOUT)) {
     const dim3 qg = quad_grid(ctx);
     const size_t nq = (size_t)qg.x * qg.y * qg.z;
@@ -1945,6 +2473,12 @@ static int vcycle(gc_ctx *ctx, const gc_mg_params *p) {
     if ((st = coarse_levels(ctx, p))) return st;
     st = plain ? block_up<2>(ctx, GK_UPDATE0, post, ctx->e[1], ctx->lev[1], ctx->e0n, ctx->r0n, g0, nullptr)
                : block_up<1>(ctx, GK_UPDATE0, post, ctx->e[1], ctx->lev[1], ctx->e0n, ctx->r0n, g0, nullptr);
+    return st ? st : residual0(ctx, p);
+  }
+  if (finest_planes(ctx, p)) {
+    if ((st = fine_down(ctx))) return st;
+    if ((st = coarse_levels(ctx, p))) return st;
+    st = plain ? fine_up<true>(ctx) : fine_up<false>(ctx);
     return st ? st : residual0(ctx, p);
   }
   const dim3 sg = split_grid(ctx), sg2 = split_grid2(ctx), qg = quad_grid(ctx);
