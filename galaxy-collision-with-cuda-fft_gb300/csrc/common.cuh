@@ -81,6 +81,16 @@ struct gc_ctx {
   cudaStream_t fork;    // second stream of the engine step (the faces beside the warm-start passes)
   cudaEvent_t ev_fork, ev_join;  // its fork and join (no timing)
   long long cap_body_launches;  // kernel launches in that body (one V-cycle)
+  int cap_body[GK_COUNT];       // ... by kernel id
+  // the eager solve's adaptive loop as a graph (see mg_loop_build): the parameters and
+  // reduction scratch it was built with, its launches by kernel id, the last solve's
+  // parameters
+  cudaGraphExec_t loop_exec;
+  cudaStream_t cap;             // the context's own stream: it is captured here
+  gc_mg_params loop_params, loop_last;
+  const double *loop_red;
+  int loop_fixed[GK_COUNT], loop_body[GK_COUNT];
+  int loop_seen, loop_off;
   int nlev;             // multigrid levels (0 = finest)
   int tail;             // first level handled by the single-CTA tail kernel (== nlev if none)
   LevelGeom lev[GC_MAX_LEVELS];
@@ -89,13 +99,14 @@ struct gc_ctx {
   // natural-layout scratch r0 (residual of the correction, the restriction's
   // input); colour-split correction e0s and potential residual r0s (two halves
   // of half0 = G*G*H0 nodes, H0 = (G+1)/2); natural-layout correction and
-  // residual e0n, r0n of the validation path (GC_MG_NATURAL_LAYOUT, lazily)
+  // residual e0n, r0n (small grids and GC_MG_NATURAL_LAYOUT); see mg_alloc_finest
   float *hi, *lo, *b0, *r0;
   float *e0s, *r0s, *e0n, *r0n;
   size_t half0;
   int H0;
   // coarse levels (index >= 1): correction e and h^2-scaled right-hand side b
-  // (ed: the correction the way down hands to the way up)
+  // (ed: the correction the way down hands to the way up), all in one block
+  float *coarse;
   float *e[GC_MAX_LEVELS];
   float *b[GC_MAX_LEVELS];
   float *ed[GC_MAX_LEVELS];
@@ -410,6 +421,7 @@ __device__ bool grid_finish_sum(const double *parts, unsigned nparts, unsigned *
 int gc_mg_build_levels(gc_ctx *ctx);
 int gc_mg_alloc(gc_ctx *ctx);
 void gc_mg_free(gc_ctx *ctx);
+void gc_mg_loop_free(gc_ctx *ctx);
 int gc_mg_run(gc_ctx *ctx, const gc_mg_params *p, gc_mg_stats *st);
 int gc_faces_from_moments(gc_ctx *ctx);
 int gc_finalize(gc_ctx *ctx, const double *parts, int nparts, int nv, double *dst);

@@ -206,6 +206,7 @@ extern "C" int gc_ctx_create(gc_ctx **out, int grid_size, double dx, double grav
 extern "C" int gc_ctx_destroy(gc_ctx *ctx) {
   if (!ctx) return GC_OK;
   cudaStreamSynchronize(ctx->stream);
+  gc_mg_loop_free(ctx);
   gc_mg_free(ctx);
   cudaFree(ctx->q);
   cudaFree(ctx->g4);

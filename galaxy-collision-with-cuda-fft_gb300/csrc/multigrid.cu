@@ -70,6 +70,43 @@ int gc_mg_build_levels(gc_ctx *ctx) {
   return GC_OK;
 }
 
+static bool finest_blocks(const gc_ctx *ctx, const gc_mg_params *p);
+static bool finest_planes(const gc_ctx *ctx, const gc_mg_params *p);
+
+// (cleared on the context's own stream and waited for: the caller's stream may be under
+// capture, and need not be ordered after the default one)
+static int alloc_zero(gc_ctx *ctx, float **a, size_t n) {
+  if (*a) return GC_OK;
+  if (!ctx->cap) GC_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->cap, cudaStreamNonBlocking));
+  float *p = nullptr;
+  GC_CUDA(ctx, cudaMalloc(&p, n * sizeof(float)));
+  cudaError_t e = cudaMemsetAsync(p, 0, n * sizeof(float), ctx->cap);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(ctx->cap);
+  if (e != cudaSuccess) {
+    cudaFree(p);
+    GC_CUDA(ctx, e);
+  }
+  *a = p;
+  return GC_OK;
+}
+
+// The finest level's correction and residual as the solve with these parameters keeps
+// them (allocated on first use; faces stay zero): natural layout (in blocks, or
+// GC_MG_NATURAL_LAYOUT) or colour-split, and the scratch of the paths that store the
+// correction's residual.
+static int mg_alloc_finest(gc_ctx *ctx, const gc_mg_params *p) {
+  if (ctx->nlev == 0) return GC_OK;
+  const size_t g3 = (size_t)ctx->G * ctx->G * ctx->G;
+  const bool blocks = finest_blocks(ctx, p);
+  int s;
+  if (blocks || (p->flags & GC_MG_NATURAL_LAYOUT)) {
+    if ((s = alloc_zero(ctx, &ctx->e0n, g3)) || (s = alloc_zero(ctx, &ctx->r0n, g3))) return s;
+  } else {
+    if ((s = alloc_zero(ctx, &ctx->e0s, 2 * ctx->half0)) || (s = alloc_zero(ctx, &ctx->r0s, 2 * ctx->half0))) return s;
+  }
+  return ctx->nlev > 1 && !blocks && !finest_planes(ctx, p) ? alloc_zero(ctx, &ctx->r0, g3) : GC_OK;
+}
+
 int gc_mg_alloc(gc_ctx *ctx) {
   const size_t G = ctx->G;
   const size_t g3 = G * G * G;
@@ -78,57 +115,46 @@ int gc_mg_alloc(gc_ctx *ctx) {
   GC_CUDA(ctx, cudaMalloc(&ctx->hi, g3 * sizeof(float)));
   GC_CUDA(ctx, cudaMalloc(&ctx->lo, g3 * sizeof(float)));
   GC_CUDA(ctx, cudaMalloc(&ctx->b0, g3 * sizeof(float)));
-  GC_CUDA(ctx, cudaMalloc(&ctx->r0, g3 * sizeof(float)));
   GC_CUDA(ctx, cudaMemset(ctx->hi, 0, g3 * sizeof(float)));
   GC_CUDA(ctx, cudaMemset(ctx->lo, 0, g3 * sizeof(float)));
   GC_CUDA(ctx, cudaMemset(ctx->b0, 0, g3 * sizeof(float)));
-  GC_CUDA(ctx, cudaMemset(ctx->r0, 0, g3 * sizeof(float)));
-  // colour-split correction and residual of the finest level (faces stay zero)
-  GC_CUDA(ctx, cudaMalloc(&ctx->e0s, 2 * ctx->half0 * sizeof(float)));
-  GC_CUDA(ctx, cudaMalloc(&ctx->r0s, 2 * ctx->half0 * sizeof(float)));
-  GC_CUDA(ctx, cudaMemset(ctx->e0s, 0, 2 * ctx->half0 * sizeof(float)));
-  GC_CUDA(ctx, cudaMemset(ctx->r0s, 0, 2 * ctx->half0 * sizeof(float)));
-  size_t rc_n = 0;
-  for (int l = 1; l < ctx->nlev; ++l) {
-    size_t n3 = (size_t)ctx->lev[l].n * ctx->lev[l].n * ctx->lev[l].n;
-    GC_CUDA(ctx, cudaMalloc(&ctx->e[l], n3 * sizeof(float)));
-    GC_CUDA(ctx, cudaMalloc(&ctx->b[l], n3 * sizeof(float)));
-    GC_CUDA(ctx, cudaMemset(ctx->e[l], 0, n3 * sizeof(float)));
-    GC_CUDA(ctx, cudaMemset(ctx->b[l], 0, n3 * sizeof(float)));
-    if (l < ctx->tail) {  // the black nodes of the way down
-      GC_CUDA(ctx, cudaMalloc(&ctx->ed[l], n3 * sizeof(float)));
-      GC_CUDA(ctx, cudaMemset(ctx->ed[l], 0, n3 * sizeof(float)));
+  // the coarse levels' arrays in one block (each on a 256-byte boundary): e and b, the
+  // black nodes of the way down (ed) above the tail, and a residual scratch
+  size_t need = 0, rc_n = 0;
+  auto take = [&](float **p, size_t n) {
+    if (p) *p = ctx->coarse + need;
+    need += (n + 63) & ~(size_t)63;
+  };
+  for (int pass = 0; pass < 2; ++pass) {
+    need = 0;
+    for (int l = 1; l < ctx->nlev; ++l) {
+      const size_t n3 = (size_t)ctx->lev[l].n * ctx->lev[l].n * ctx->lev[l].n;
+      take(pass ? &ctx->e[l] : nullptr, n3);
+      take(pass ? &ctx->b[l] : nullptr, n3);
+      if (l < ctx->tail) {
+        take(pass ? &ctx->ed[l] : nullptr, n3);
+        if (n3 > rc_n) rc_n = n3;
+      }
     }
-    if (l < ctx->tail && n3 > rc_n) rc_n = n3;
+    if (rc_n) take(pass ? &ctx->rc : nullptr, rc_n);
+    if (!pass && need) {
+      GC_CUDA(ctx, cudaMalloc(&ctx->coarse, need * sizeof(float)));
+      GC_CUDA(ctx, cudaMemset(ctx->coarse, 0, need * sizeof(float)));
+    }
   }
-  if (rc_n) {
-    GC_CUDA(ctx, cudaMalloc(&ctx->rc, rc_n * sizeof(float)));
-    GC_CUDA(ctx, cudaMemset(ctx->rc, 0, rc_n * sizeof(float)));
-  }
-  return GC_OK;
-}
-
-// Natural-layout correction and residual of the finest level, for
-// GC_MG_NATURAL_LAYOUT (allocated on first use).
-static int mg_alloc_natural(gc_ctx *ctx) {
-  if (ctx->e0n) return GC_OK;
-  const size_t g3 = (size_t)ctx->G * ctx->G * ctx->G;
-  GC_CUDA(ctx, cudaMalloc(&ctx->e0n, g3 * sizeof(float)));
-  GC_CUDA(ctx, cudaMalloc(&ctx->r0n, g3 * sizeof(float)));
-  GC_CUDA(ctx, cudaMemset(ctx->e0n, 0, g3 * sizeof(float)));
-  GC_CUDA(ctx, cudaMemset(ctx->r0n, 0, g3 * sizeof(float)));
-  return GC_OK;
+  // the finest level's arrays of the default parameters' path
+  gc_mg_params p;
+  gc_mg_default_params(&p);
+  return mg_alloc_finest(ctx, &p);
 }
 
 void gc_mg_free(gc_ctx *ctx) {
   cudaFree(ctx->hi); cudaFree(ctx->lo);
   cudaFree(ctx->b0); cudaFree(ctx->r0);
   cudaFree(ctx->e0s); cudaFree(ctx->r0s); cudaFree(ctx->e0n); cudaFree(ctx->r0n);
-  for (int l = 1; l < GC_MAX_LEVELS; ++l) {
-    cudaFree(ctx->e[l]); cudaFree(ctx->b[l]); cudaFree(ctx->ed[l]);
-    ctx->e[l] = ctx->b[l] = ctx->ed[l] = nullptr;
-  }
-  cudaFree(ctx->rc);
+  for (int l = 1; l < GC_MAX_LEVELS; ++l) ctx->e[l] = ctx->b[l] = ctx->ed[l] = nullptr;
+  cudaFree(ctx->coarse);
+  ctx->coarse = nullptr;
   ctx->hi = ctx->lo = ctx->b0 = ctx->r0 = ctx->rc = nullptr;
   ctx->e0s = ctx->r0s = ctx->e0n = ctx->r0n = nullptr;
 }
@@ -2169,7 +2195,7 @@ __global__ void __launch_bounds__(256) k_zero_interior(float *__restrict__ a, in
 // ||r|| < tol ||b|| with ||b|| > 0). The verdict goes to the conditional node
 // that repeats the V-cycle body, the converged flag to dsmall[GC_S_CONVERGED].
 __global__ void k_mg_decide(cudaGraphConditionalHandle h, double *__restrict__ small, double tol, int min_c,
-                            int max_c, int first) {
+                            int max_c, int first, int count) {
   if (threadIdx.x != 0) return;
   const int c = first ? 0 : (int)small[GC_S_CYCLES] + 1;
   small[GC_S_CYCLES] = (double)c;
@@ -2178,7 +2204,7 @@ __global__ void k_mg_decide(cudaGraphConditionalHandle h, double *__restrict__ s
   const bool conv = c >= minc && b2 > 0.0 && sqrt(r2) < tol * sqrt(b2);
   small[GC_S_CONVERGED] = conv ? 1.0 : 0.0;
   const bool more = !conv && c < max_c;
-  if (!more) {  // the solve ends here: count it
+  if (!more && count) {  // the solve ends here: count it
     small[GC_S_SOLVES] += 1.0;
     small[GC_S_CYC_TOTAL] += (double)c;
     const double rel2 = b2 > 0.0 ? r2 / b2 : 0.0;
@@ -2408,7 +2434,7 @@ static int residual0(gc_ctx *ctx, const gc_mg_params *p) {
   const bool plain = (p->flags & GC_MG_PLAIN_F32) != 0;
   const Split0 d = split0(ctx);
   const bool natural = (p->flags & GC_MG_NATURAL_LAYOUT) != 0 || finest_blocks(ctx, p);
-  if (natural && (st = mg_alloc_natural(ctx))) return st;
+  if ((st = mg_alloc_finest(ctx, p))) return st;
   const int pre = ctx->nlev == 1 ? p->coarse_sweeps : p->pre_sweeps;
   float *ef = pre >= 1 && !natural && !finest_planes(ctx, p) ? ctx->e0s : nullptr, *r = natural ? ctx->r0n : ctx->r0s;
   if (vec4(ctx) && !(p->flags & GC_MG_NATURAL_LAYOUT)) {
@@ -2574,7 +2600,7 @@ int gc_faces_from_moments(gc_ctx *ctx) {
 // Same kernels in the same order as the host loop, so the same potential. The
 // cycle count, the converged flag and both norms are left in dsmall and copied
 // to the pinned host mirror at the end.
-static int mg_run_captured(gc_ctx *ctx, const gc_mg_params *p) {
+static int mg_run_captured(gc_ctx *ctx, const gc_mg_params *p, int count) {
   int s;
   if (ctx->nlev == 0) return GC_OK;
   if ((s = residual0(ctx, p))) return s;
@@ -2586,7 +2612,8 @@ static int mg_run_captured(gc_ctx *ctx, const gc_mg_params *p) {
   GC_REQUIRE(ctx, cs == cudaStreamCaptureStatusActive, "captured solve outside a stream capture");
   cudaGraphConditionalHandle h;
   GC_CUDA(ctx, cudaGraphConditionalHandleCreate(&h, graph, 0, 0));
-  gc_launch(ctx, GK_REDUCE, k_mg_decide, dim3(1), dim3(32), 0, h, ctx->dsmall, p->tol, p->min_cycles, p->max_cycles, 1);
+  gc_launch(ctx, GK_REDUCE, k_mg_decide, dim3(1), dim3(32), 0, h, ctx->dsmall, p->tol, p->min_cycles, p->max_cycles, 1,
+            count);
   GC_LAUNCH_CHECK(ctx, "decide");
   GC_CUDA(ctx, cudaStreamGetCaptureInfo(ctx->stream, &cs, nullptr, &graph, &deps, nullptr, &nd));
   cudaGraphNodeParams np = {};
@@ -2601,13 +2628,16 @@ static int mg_run_captured(gc_ctx *ctx, const gc_mg_params *p) {
   GC_CUDA(ctx, cudaStreamBeginCaptureToGraph(ctx->side, body, nullptr, nullptr, 0, cudaStreamCaptureModeRelaxed));
   ctx->stream = ctx->side;
   const long long before = gc_launch_total(ctx);
+  long long at[GK_COUNT];
+  memcpy(at, ctx->prof.launches, sizeof(at));
   s = vcycle(ctx, p);
   if (!s) {
     gc_launch(ctx, GK_REDUCE, k_mg_decide, dim3(1), dim3(32), 0, h, ctx->dsmall, p->tol, p->min_cycles,
-              p->max_cycles, 0);
+              p->max_cycles, 0, count);
     s = gc_check_launch(ctx, "decide");
   }
   ctx->cap_body_launches = gc_launch_total(ctx) - before;
+  for (int k = 0; k < GK_COUNT; ++k) ctx->cap_body[k] = (int)(ctx->prof.launches[k] - at[k]);
   cudaGraph_t got = nullptr;
   const cudaError_t e = cudaStreamEndCapture(ctx->side, &got);
   ctx->stream = main;
@@ -2616,6 +2646,75 @@ static int mg_run_captured(gc_ctx *ctx, const gc_mg_params *p) {
   GC_CUDA(ctx, cudaStreamUpdateCaptureDependencies(main, &cond, nullptr, 1, cudaStreamSetCaptureDependencies));
   GC_CUDA(ctx, cudaMemcpyAsync(ctx->hsmall, ctx->dsmall, GC_S_MIRROR * sizeof(double), cudaMemcpyDeviceToHost, main));
   return GC_OK;
+}
+
+// The adaptive loop of an eager solve as a graph of its own: the residual of the guess,
+// then the conditional V-cycle loop, then the counts and norms to the pinned mirror: one
+// launch and one host wait per solve instead of ten launches and a host read per cycle
+// (about 40 us of an idle GPU per cycle: a 64^3 step of 2.2 cycles 356 -> 240 us, a 97^3
+// cold solve of 6 cycles 951 -> 776 us). Everything it touches belongs to the context (faces,
+// guess and right-hand side are in place before it), so it stays valid while the
+// parameters and the reduction scratch stay the same. It is built when the same
+// parameters come a second time: a single solve does not pay for it.
+static void mg_loop_drop(gc_ctx *ctx) {
+  if (ctx->loop_exec) cudaGraphExecDestroy(ctx->loop_exec);
+  ctx->loop_exec = nullptr;
+}
+
+static bool same_params(const gc_mg_params &a, const gc_mg_params &b) {
+  return a.pre_sweeps == b.pre_sweeps && a.post_sweeps == b.post_sweeps && a.coarse_sweeps == b.coarse_sweeps &&
+         a.max_cycles == b.max_cycles && a.min_cycles == b.min_cycles && a.flags == b.flags && a.tol == b.tol;
+}
+
+static int mg_loop_build(gc_ctx *ctx, const gc_mg_params *p) {
+  mg_loop_drop(ctx);
+  if (!ctx->side) GC_CUDA(ctx, cudaStreamCreateWithFlags(&ctx->side, cudaStreamNonBlocking));
+  GC_CUDA(ctx, cudaStreamBeginCapture(ctx->cap, cudaStreamCaptureModeRelaxed));
+  cudaStream_t main = ctx->stream;  // (it may be the default stream, which cannot be captured)
+  long long at[GK_COUNT];
+  memcpy(at, ctx->prof.launches, sizeof(at));
+  ctx->stream = ctx->cap;
+  ctx->capturing = 1;
+  const int s = mg_run_captured(ctx, p, 0);
+  ctx->capturing = 0;
+  ctx->stream = main;
+  for (int k = 0; k < GK_COUNT; ++k) {
+    ctx->loop_body[k] = ctx->cap_body[k];
+    ctx->loop_fixed[k] = (int)(ctx->prof.launches[k] - at[k]) - ctx->cap_body[k];
+  }
+  memcpy(ctx->prof.launches, at, sizeof(at));  // nothing ran
+  cudaGraph_t g = nullptr;
+  const cudaError_t e = cudaStreamEndCapture(ctx->cap, &g);
+  cudaError_t ei = cudaErrorUnknown;
+  if (!s && e == cudaSuccess) ei = cudaGraphInstantiate(&ctx->loop_exec, g, 0);
+  if (g) cudaGraphDestroy(g);
+  if (s || e != cudaSuccess || ei != cudaSuccess) {
+    ctx->loop_exec = nullptr;
+    cudaGetLastError();
+    return s ? s : GC_ERR_CUDA;
+  }
+  ctx->loop_params = *p;
+  ctx->loop_red = ctx->red;
+  return GC_OK;
+}
+
+// Whether this solve's loop runs as the context's graph (built here when due).
+static bool mg_loop_ready(gc_ctx *ctx, const gc_mg_params *p) {
+  if (ctx->nlev == 0 || ctx->prof.enabled || ctx->loop_off) return false;
+  const bool repeated = ctx->loop_seen && same_params(ctx->loop_last, *p);
+  ctx->loop_seen = 1;
+  ctx->loop_last = *p;
+  if (ctx->loop_exec && ctx->loop_red == ctx->red && same_params(ctx->loop_params, *p)) return true;
+  if (!repeated) return false;
+  if (mg_loop_build(ctx, p) == GC_OK) return true;
+  ctx->loop_off = 1;  // keep the host loop
+  return false;
+}
+
+void gc_mg_loop_free(gc_ctx *ctx) {
+  mg_loop_drop(ctx);
+  if (ctx->cap) cudaStreamDestroy(ctx->cap);
+  ctx->cap = nullptr;
 }
 
 // Adaptive V-cycling (multigrid.py:473-485): at least one cycle, then stop once
@@ -2628,10 +2727,24 @@ int gc_mg_run(gc_ctx *ctx, const gc_mg_params *p, gc_mg_stats *stats) {
   memset(&st, 0, sizeof(st));
   int s;
   if (ctx->capturing && !(p->flags & GC_MG_FIXED_CYCLES)) {
-    if ((s = mg_run_captured(ctx, p))) return s;
+    if ((s = mg_run_captured(ctx, p, 1))) return s;
     st.cycles = -1;  // decided on the device: read them with gc_pm_graph_stats
     st.converged = -1;
     st.rhs_norm = st.res_norm = NAN;
+    ctx->last_stats = st;
+    ctx->solved_once = 1;
+    if (stats) *stats = st;
+    return GC_OK;
+  }
+  if (!(p->flags & GC_MG_FIXED_CYCLES) && mg_loop_ready(ctx, p)) {
+    GC_CUDA(ctx, cudaGraphLaunch(ctx->loop_exec, ctx->stream));
+    GC_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
+    st.cycles = (int)ctx->hsmall[GC_S_CYCLES];
+    st.converged = ctx->hsmall[GC_S_CONVERGED] != 0.0;
+    st.rhs_norm = sqrt(ctx->hsmall[GC_S_BNORM2]) / (ctx->dx * ctx->dx);
+    st.res_norm = sqrt(ctx->hsmall[GC_S_RNORM2]) / (ctx->dx * ctx->dx);
+    for (int k = 0; k < GK_COUNT; ++k)
+      ctx->prof.launches[k] += ctx->loop_fixed[k] + (long long)st.cycles * ctx->loop_body[k];
     ctx->last_stats = st;
     ctx->solved_once = 1;
     if (stats) *stats = st;
