@@ -251,15 +251,20 @@ __global__ void __launch_bounds__(256) k_conv_fwd(ConvFwd a) {
       const int t0 = g * a.tpg, t1 = min(27, t0 + a.tpg);
       // descriptors differ only in the start address (bits 0..13, address / 16)
       const uint64_t ad0 = umma::sdesc(tile_u32, a_lbo, 128u), bd0 = umma::sdesc(ring_u32, b_lbo, 128u);
+      // One thread feeds the tensor core an instruction every few tens of clocks, so
+      // the loop carries the descriptors by additions only. With the address
+      // arithmetic in the inner loop an issue took 59 clk of an SM at 128 x 16 x 16
+      // (16 -> 16 channels, R = 128), so 40: the operand rows are 32 clk to read.
+      const uint32_t kstep_a = (2u * a_lbo) >> 4, kstep_b = (2u * b_lbo) >> 4;
+      const int nks = kci / 2;
       for (int t = t0; t < t1; ++t) {
-        const int off = tap_offset(t, P, W2);
-        const uint32_t boff = ((uint32_t)s * slot_bytes + (uint32_t)(t - t0) * tap_bytes) >> 4;
-        for (int mt = warp; mt < a.n_mt; mt += WS_ISSUERS) {
-          const uint32_t aoff = ((uint32_t)(L0 + 128 * mt + off) * 16u) >> 4;
-          for (int ks = 0; ks < kci / 2; ++ks) {
-            umma::mma_bf16(tmem + (uint32_t)(mt * a.Cout), ad0 + aoff + ((2u * ks * a_lbo) >> 4),
-                           bd0 + boff + ((2u * ks * b_lbo) >> 4), idesc, (t > 0 || ks > 0) ? 1u : 0u);
-          }
+        const uint64_t bd = bd0 + (((uint32_t)s * slot_bytes + (uint32_t)(t - t0) * tap_bytes) >> 4);
+        uint64_t ad = ad0 + (uint32_t)(L0 + 128 * warp + tap_offset(t, P, W2));
+        uint32_t td = tmem + (uint32_t)(warp * a.Cout);
+#pragma unroll 4
+        for (int mt = warp; mt < a.n_mt; mt += WS_ISSUERS, ad += 128u * WS_ISSUERS, td += (uint32_t)(WS_ISSUERS * a.Cout)) {
+          umma::mma_bf16(td, ad, bd, idesc, t > 0 ? 1u : 0u);
+          for (int ks = 1; ks < nks; ++ks) umma::mma_bf16(td, ad + ks * kstep_a, bd + ks * kstep_b, idesc, 1u);
         }
       }
       umma::mma_commit(&bars[s]);
