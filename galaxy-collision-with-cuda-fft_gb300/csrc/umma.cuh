@@ -39,6 +39,10 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, long l
   return true;
 }
 
+__device__ __forceinline__ void mbar_arrive(uint64_t *bar) {
+  asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(bar)) : "memory");
+}
+
 // ---- bulk (TMA engine) copies of contiguous bytes ----------------------------------
 // Addresses 16-byte aligned, sizes multiples of 16. Global -> shared completes its
 // bytes on an mbarrier that one thread armed with the expected byte count;
@@ -53,6 +57,16 @@ __device__ __forceinline__ void bulk_g2s(void *smem, const void *gmem, uint32_t 
                    smem_u32(smem)),
                "l"(gmem), "r"(bytes), "r"(smem_u32(bar))
                : "memory");
+}
+// One box of a four-dimensional tensor map (tensor-core operand tiles, zeros outside
+// the tensor), completing its bytes on `bar`. c0 counts elements of the innermost
+// dimension and must land on a 16-byte boundary.
+__device__ __forceinline__ void tma_load_4d(void *smem, const void *map, int c0, int c1, int c2, int c3, uint64_t *bar) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4, %5}], "
+      "[%6];" ::"r"(smem_u32(smem)),
+      "l"(map), "r"(c0), "r"(c1), "r"(c2), "r"(c3), "r"(smem_u32(bar))
+      : "memory");
 }
 __device__ __forceinline__ void bulk_s2g(void *gmem, const void *smem, uint32_t bytes) {
   asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(gmem), "r"(smem_u32(smem)),
@@ -154,6 +168,30 @@ __device__ __forceinline__ void mma_bf16(uint32_t d_tmem, uint64_t adesc, uint64
       "setp.ne.b32 p, %4, 0;\n\t"
       "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
       ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+// 1 in one lane of a converged warp, 0 in the others.
+__device__ __forceinline__ uint32_t elect_one() {
+  uint32_t e;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(e));
+  return e;
+}
+
+// The same MMA from a warp that runs it as a whole with uniform operands: the lane
+// with a nonzero `lead` issues.
+__device__ __forceinline__ void mma_bf16_if(uint32_t lead, uint32_t d_tmem, uint64_t adesc, uint64_t bdesc,
+                                            uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "setp.ne.b32 q, %5, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate), "r"(lead)
       : "memory");
 }
 

@@ -3,6 +3,8 @@
 // This file holds the tensor-core kernels of the warm-start network (implicit-GEMM
 // convolution forward / data-gradient / weight-gradient) and a single-tile GEMM
 // used to check the shared-memory descriptor conventions on the device.
+#include <cuda.h>
+#include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -116,10 +118,8 @@ __device__ __forceinline__ float bf_lo(uint32_t w) { return __uint_as_float(w <<
 __device__ __forceinline__ float bf_hi(uint32_t w) { return __uint_as_float(w & 0xffff0000u); }
 __device__ __forceinline__ uint32_t bf_pack(float a, float b) {
   // round to nearest even, NaN kept quiet
-  uint32_t ua = __float_as_uint(a), ub = __float_as_uint(b);
-  ua = (ua & 0x7fffffffu) > 0x7f800000u ? 0x7fc00000u : ua + 0x7fffu + ((ua >> 16) & 1u);
-  ub = (ub & 0x7fffffffu) > 0x7f800000u ? 0x7fc00000u : ub + 0x7fffu + ((ub >> 16) & 1u);
-  return (ua >> 16) | (ub & 0xffff0000u);
+  const __nv_bfloat162 p = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t *>(&p);
 }
 __device__ __forceinline__ void unpack8(const uint4 &v, float (&f)[8]) {
   f[0] = bf_lo(v.x); f[1] = bf_hi(v.x); f[2] = bf_lo(v.y); f[3] = bf_hi(v.y);
@@ -142,10 +142,12 @@ __device__ __forceinline__ uint4 pack8(const float (&f)[N]) {
 // at padded index s is simply the descriptor at row s + off_t: no im2col copy.
 // Output rows are the padded linear range [L0, L1] cut into 128-row M tiles;
 // rows that fall on halo voxels are computed and discarded. Accumulators live
-// in Tensor Memory (M tile mt in columns mt*Cout ..). Weights stream through a
-// two-slot ring of tap groups; one thread issues the MMAs, completion is
-// tracked by tcgen05.commit on one mbarrier per slot.
+// in Tensor Memory (M tile mt in columns mt*Cn ..). Weights stream through a
+// two-slot ring of tap groups; completion of the MMAs is tracked by
+// tcgen05.commit on one mbarrier per slot.
 struct ConvFwd {
+  CUtensorMap map;     // input: 8-channel rows of x, y, z, chunk; box one tile
+  int use_map;         // the tile's lines fit a box (R <= 126)
   const uint4 *in;
   const uint4 *w;
   const float *bias;   // [Cout] or null
@@ -155,6 +157,7 @@ struct ConvFwd {
   float *out_f32;      // channel 0 as f32 [R^3] or null
   unsigned *status;
   int R, Cin, Cout, BZ, BY;
+  int Cn;              // output channels of a CTA (blockIdx.y is the slice)
   int relu;
   int tpg;             // taps per weight group
   int n_mt;
@@ -173,19 +176,73 @@ __device__ __forceinline__ int tap_offset(int t, int P, int W2) {
   return (t / 9 - 1) * P + ((t / 3) % 3 - 1) * W2 + (t % 3 - 1);
 }
 
-// Copy the weights of tap group g (taps g*tpg .. min(27, (g+1)*tpg)) to dst.
-__device__ __forceinline__ void load_taps(const uint4 *__restrict__ w, int g, int tpg, uint32_t tap_bytes, uint8_t *dst,
-                                          int tid) {
+// Copy the weights of tap group g (taps g*tpg .. min(27, (g+1)*tpg)), output channels
+// c0 .. c0 + Cn, to dst.
+__device__ __forceinline__ void load_taps(const uint4 *__restrict__ w, int g, int tpg, int kci, int Cout, int Cn, int c0,
+                                          uint8_t *dst, int tid, int nthreads) {
   const int t0 = g * tpg, t1 = min(27, t0 + tpg);
-  const uint4 *src = w + (size_t)t0 * (tap_bytes / 16u);
+  const uint4 *src = w + (size_t)t0 * kci * Cout + c0;
   uint4 *d = reinterpret_cast<uint4 *>(dst);
-  const int n16 = (t1 - t0) * (int)(tap_bytes / 16u);
-  for (int i = tid; i < n16; i += blockDim.x) umma::cp_async16(d + i, src + i, true);
+  const int n16 = (t1 - t0) * kci * Cn, sh = 31 - __clz(Cn);  // Cn is a power of two
+  for (int i = tid; i < n16; i += nthreads)
+    umma::cp_async16(d + i, src + (size_t)(i >> sh) * Cout + (i & (Cn - 1)), true);
 }
 
-__global__ void __launch_bounds__(256) k_conv_fwd(ConvFwd a) {
+// Mask rows (16 channels from c) of one voxel, read ahead of the accumulators.
+template <class A>
+__device__ __forceinline__ void conv_mask16(const A &a, int c, size_t vox, size_t R3, uint4 (&m)[2]) {
+  if (a.mask) {
+    m[0] = __ldg(a.mask + (size_t)(c >> 3) * R3 + vox);
+    m[1] = __ldg(a.mask + (size_t)((c >> 3) + 1) * R3 + vox);
+  }
+}
+
+// Bias, skip, activation, mask and stores of 16 channels (c ..) of one voxel; the bias
+// is in shared memory (zeros where there is none).
+template <class A>
+__device__ __forceinline__ void conv_store16(const A &a, const uint32_t (&r)[16], const float *bias, const uint4 (&m)[2],
+                                             int c, size_t vox, size_t R3) {
+  float v[16];
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    const float4 b4 = *reinterpret_cast<const float4 *>(bias + c + 4 * q);
+    v[4 * q] = __uint_as_float(r[4 * q]) + b4.x;
+    v[4 * q + 1] = __uint_as_float(r[4 * q + 1]) + b4.y;
+    v[4 * q + 2] = __uint_as_float(r[4 * q + 2]) + b4.z;
+    v[4 * q + 3] = __uint_as_float(r[4 * q + 3]) + b4.w;
+  }
+  if (a.skip) {
+    float s0[8], s1[8];
+    unpack8(__ldg(a.skip + (size_t)(c >> 3) * R3 + vox), s0);
+    unpack8(__ldg(a.skip + (size_t)((c >> 3) + 1) * R3 + vox), s1);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) { v[j] += s0[j]; v[8 + j] += s1[j]; }
+  }
+  if (a.relu) {
+#pragma unroll
+    for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j], 0.0f);
+  }
+  if (a.mask) {
+    float m0[8], m1[8];
+    unpack8(m[0], m0);
+    unpack8(m[1], m1);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) {
+      v[j] = m0[j] > 0.0f ? v[j] : 0.0f;
+      v[8 + j] = m1[j] > 0.0f ? v[8 + j] : 0.0f;
+    }
+  }
+  if (a.out) {
+    a.out[(size_t)(c >> 3) * R3 + vox] = pack8<0>(v);
+    a.out[(size_t)((c >> 3) + 1) * R3 + vox] = pack8<8>(v);
+  }
+  if (a.out_f32 && c == 0) a.out_f32[vox] = v[0];
+}
+
+__global__ void __launch_bounds__(256) k_conv_fwd(const __grid_constant__ ConvFwd a) {
   extern __shared__ __align__(1024) uint8_t sm[];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
   const int R = a.R;
   int W2, P, V, L0, L1;
   conv_geom(R, a.BZ, a.BY, W2, P, V, L0, L1);
@@ -194,12 +251,15 @@ __global__ void __launch_bounds__(256) k_conv_fwd(ConvFwd a) {
   const int nby = R / a.BY;
   const int z0 = (blockIdx.x / nby) * a.BZ, y0 = (blockIdx.x % nby) * a.BY;
   const uint32_t tile_bytes = (uint32_t)(kci * V + 128) * 16u;
-  const uint32_t tap_bytes = (uint32_t)a.Cin * a.Cout * 2u;
+  const int Cn = a.Cn, c0 = blockIdx.y * Cn;
+  const uint32_t tap_bytes = (uint32_t)a.Cin * Cn * 2u;
   const uint32_t slot_bytes = (uint32_t)a.tpg * tap_bytes;
   uint8_t *tile = sm;
   uint8_t *ring = sm + ((tile_bytes + 1023u) & ~1023u);
   uint64_t *bars = reinterpret_cast<uint64_t *>(ring + 2u * slot_bytes);
-  uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 2);
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 3);
+  float *bias = reinterpret_cast<float *>(bars + 8);
+  if (tid < Cn) bias[tid] = a.bias ? a.bias[c0 + tid] : 0.0f;
   const int ngroups = (27 + a.tpg - 1) / a.tpg;
 
   if (warp == 0) {
@@ -209,12 +269,19 @@ __global__ void __launch_bounds__(256) k_conv_fwd(ConvFwd a) {
   if (tid == 0) {  // one arrival per issuing warp (WS_ISSUERS commits per phase)
     umma::mbar_init(&bars[0], WS_ISSUERS);
     umma::mbar_init(&bars[1], WS_ISSUERS);
+    umma::mbar_init(&bars[2], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    if (a.use_map) {
+      umma::fence_async_smem();
+      umma::mbar_arrive_expect_tx(&bars[2], (uint32_t)(kci * V) * 16u);
+      umma::tma_load_4d(sm, &a.map, -2, y0 - 1, z0 - 1, 0, &bars[2]);
+    }
   }
-  // input tile, zero outside the grid, plus a zero margin read by the last M tile;
-  // one warp per padded line, lanes along x
+  // input tile, zero outside the grid, plus a zero margin read by the last M tile: one
+  // box of the tensor map (1.2k clk for 23 KB), or one warp per padded line with lanes
+  // along x (10k clk) where a line is longer than a box may be
   uint4 *trow = reinterpret_cast<uint4 *>(tile);
-  {
+  if (!a.use_map) {
     const int nzy = (a.BZ + 2) * (a.BY + 2), nrows = kci * nzy, nwarps = blockDim.x >> 5;
     for (int row = warp; row < nrows; row += nwarps) {
       const int kc = row / nzy, rr = row - kc * nzy;
@@ -231,43 +298,46 @@ __global__ void __launch_bounds__(256) k_conv_fwd(ConvFwd a) {
     }
   }
   for (int i = tid; i < 128; i += blockDim.x) trow[kci * V + i] = make_uint4(0u, 0u, 0u, 0u);
-  load_taps(a.w, 0, a.tpg, tap_bytes, ring, tid);
+  load_taps(a.w, 0, a.tpg, kci, a.Cout, Cn, c0, ring, tid, blockDim.x);
   umma::cp_async_wait_all();
   umma::fence_async_smem();
   umma::tc_fence_before();
   __syncthreads();
   umma::tc_fence_after();
   const uint32_t tmem = *tslot;
-  const uint32_t idesc = umma::idesc_bf16(128, a.Cout, 0, 0);
-  const uint32_t a_lbo = (uint32_t)V * 16u, b_lbo = (uint32_t)a.Cout * 16u;
+  const uint32_t idesc = umma::idesc_bf16(128, Cn, 0, 0);
+  const uint32_t a_lbo = (uint32_t)V * 16u, b_lbo = (uint32_t)Cn * 16u;
   const uint32_t tile_u32 = umma::smem_u32(tile), ring_u32 = umma::smem_u32(ring);
   uint32_t ph0 = 0u, ph1 = 0u;  // next completion parity of each slot's barrier
   int last = 0;                  // slot of the last commit
-  bool fail = false;
+  bool fail = a.use_map && !umma::mbar_wait(&bars[2], 0, WS_WAIT_BUDGET);
   for (int g = 0; g < ngroups; ++g) {
     const int s = g & 1;
-    if (lane == 0 && warp < WS_ISSUERS) {  // issuer w owns the M tiles mt = w (mod WS_ISSUERS)
+    if (warp < WS_ISSUERS) {  // issuer w owns the M tiles mt = w (mod WS_ISSUERS)
       umma::tc_fence_after();
+      const uint32_t lead = umma::elect_one();
       const int t0 = g * a.tpg, t1 = min(27, t0 + a.tpg);
       // descriptors differ only in the start address (bits 0..13, address / 16)
       const uint64_t ad0 = umma::sdesc(tile_u32, a_lbo, 128u), bd0 = umma::sdesc(ring_u32, b_lbo, 128u);
-      // One thread feeds the tensor core an instruction every few tens of clocks, so
-      // the loop carries the descriptors by additions only. With the address
-      // arithmetic in the inner loop an issue took 59 clk of an SM at 128 x 16 x 16
+      // A warp feeds the tensor core an instruction every few tens of clocks: the whole
+      // warp runs the loop on uniform values, the descriptors carried by additions only,
+      // and one elected lane issues. With the address arithmetic in the inner loop of one
+      // thread, the four issuers together took 59 clk an instruction at 128 x 16 x 16
       // (16 -> 16 channels, R = 128), so 40: the operand rows are 32 clk to read.
       const uint32_t kstep_a = (2u * a_lbo) >> 4, kstep_b = (2u * b_lbo) >> 4;
       const int nks = kci / 2;
       for (int t = t0; t < t1; ++t) {
         const uint64_t bd = bd0 + (((uint32_t)s * slot_bytes + (uint32_t)(t - t0) * tap_bytes) >> 4);
         uint64_t ad = ad0 + (uint32_t)(L0 + 128 * warp + tap_offset(t, P, W2));
-        uint32_t td = tmem + (uint32_t)(warp * a.Cout);
+        uint32_t td = tmem + (uint32_t)(warp * Cn);
 #pragma unroll 4
-        for (int mt = warp; mt < a.n_mt; mt += WS_ISSUERS, ad += 128u * WS_ISSUERS, td += (uint32_t)(WS_ISSUERS * a.Cout)) {
-          umma::mma_bf16(td, ad, bd, idesc, t > 0 ? 1u : 0u);
-          for (int ks = 1; ks < nks; ++ks) umma::mma_bf16(td, ad + ks * kstep_a, bd + ks * kstep_b, idesc, 1u);
+        for (int mt = warp; mt < a.n_mt; mt += WS_ISSUERS, ad += 128u * WS_ISSUERS, td += (uint32_t)(WS_ISSUERS * Cn)) {
+          umma::mma_bf16_if(lead, td, ad, bd, idesc, t > 0 ? 1u : 0u);
+          for (int ks = 1; ks < nks; ++ks) umma::mma_bf16_if(lead, td, ad + ks * kstep_a, bd + ks * kstep_b, idesc, 1u);
         }
       }
-      umma::mma_commit(&bars[s]);
+      if (lead) umma::mma_commit(&bars[s]);
+      __syncwarp();
     }
     last = s;
     if (g + 1 < ngroups) {
@@ -277,7 +347,7 @@ __global__ void __launch_bounds__(256) k_conv_fwd(ConvFwd a) {
         if (s1) ph1 ^= 1u; else ph0 ^= 1u;
       }
       if (__syncthreads_or(fail)) { fail = true; break; }
-      load_taps(a.w, g + 1, a.tpg, tap_bytes, ring + (uint32_t)s1 * slot_bytes, tid);
+      load_taps(a.w, g + 1, a.tpg, kci, a.Cout, Cn, c0, ring + (uint32_t)s1 * slot_bytes, tid, blockDim.x);
       umma::cp_async_wait_all();
       umma::fence_async_smem();
       __syncthreads();
@@ -296,43 +366,240 @@ __global__ void __launch_bounds__(256) k_conv_fwd(ConvFwd a) {
       const int tz = L / P, rem = L - tz * P, ty = rem / W2, tx = rem - ty * W2;
       const bool valid = L <= L1 && tz >= 1 && tz <= a.BZ && ty >= 1 && ty <= a.BY && tx >= 1 && tx <= R;
       const size_t vox = ((size_t)(z0 + tz - 1) * R + (y0 + ty - 1)) * R + (tx - 1);
-      for (int c = 0; c < a.Cout; c += 16) {
+      for (int c = 0; c < Cn; c += 16) {
         uint32_t r[16];
-        umma::tmem_ld16(tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)(mt * a.Cout + c), r);
+        uint4 m[2] = {};
+        umma::tmem_ld16(tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)(mt * Cn + c), r);
+        if (valid) conv_mask16(a, c0 + c, vox, R3, m);
         umma::tmem_wait_ld();
         if (!valid) continue;
-        float v[16];
-#pragma unroll
-        for (int j = 0; j < 16; ++j) v[j] = __uint_as_float(r[j]) + (a.bias ? __ldg(a.bias + c + j) : 0.0f);
-        if (a.skip) {
-          float s0[8], s1[8];
-          unpack8(__ldg(a.skip + (size_t)(c >> 3) * R3 + vox), s0);
-          unpack8(__ldg(a.skip + (size_t)((c >> 3) + 1) * R3 + vox), s1);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) { v[j] += s0[j]; v[8 + j] += s1[j]; }
-        }
-        if (a.relu) {
-#pragma unroll
-          for (int j = 0; j < 16; ++j) v[j] = fmaxf(v[j], 0.0f);
-        }
-        if (a.mask) {
-          float m0[8], m1[8];
-          unpack8(__ldg(a.mask + (size_t)(c >> 3) * R3 + vox), m0);
-          unpack8(__ldg(a.mask + (size_t)((c >> 3) + 1) * R3 + vox), m1);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) {
-            v[j] = m0[j] > 0.0f ? v[j] : 0.0f;
-            v[8 + j] = m1[j] > 0.0f ? v[8 + j] : 0.0f;
-          }
-        }
-        if (a.out) {
-          a.out[(size_t)(c >> 3) * R3 + vox] = pack8<0>(v);
-          a.out[(size_t)((c >> 3) + 1) * R3 + vox] = pack8<8>(v);
-        }
-        if (a.out_f32 && c == 0) a.out_f32[vox] = v[0];
+        conv_store16(a, r, bias - c0, m, c0 + c, vox, R3);
       }
     }
   }
+  umma::tc_fence_before();
+  __syncthreads();
+  if (warp == 0) umma::tmem_dealloc(tmem, a.tmem_cols);
+}
+
+// ------------------------------------------------------------------------------
+// the same convolution marching along z
+// ------------------------------------------------------------------------------
+// A CTA walks the planes of a strip of MA_LINES lines x BX voxels: a ring of input
+// planes (with their one-voxel halo) is filled ahead by the TMA engine, the MMAs of a
+// plane go to one half of Tensor Memory while the other half is read out, and all 27
+// taps of the weights stay in shared memory. Loads, MMAs and epilogue therefore run
+// beside each other; in k_conv_fwd they follow one another within a CTA, and its large
+// input tile leaves room for one CTA on an SM (16 -> 16 channels, R = 128: 9.0k clk of
+// loads, 20.6k of MMAs, 12.0k of epilogue for 2048 voxels). An M tile is 8 voxels of
+// each of 16 lines: the 8-row groups of the operand lie one line apart (row order
+// [line][chunk][x]), so every row is an output voxel and no halo row is computed
+// (19 x 128 rows for 2048 voxels there). The accumulation order of an output is that
+// of k_conv_fwd, taps outermost: results are the same bits.
+// Measured (16 -> 16 channels): R = 128 155 -> 70 us, R = 64 18.5 -> 13.9. What is left
+// is the MMAs: 9.1k clk a unit of 16 x 64 voxels against 216 x 40; each reads its 128
+// operand rows from shared memory again (32 clk), and taps cannot share a read without
+// another order of accumulation. A plane is one box of a tensor map: 0.8k clk for 36 KB
+// with several in flight, where one bulk copy per line and chunk took 70 clk a copy
+// (3.3k) and 16-byte asynchronous copies by a warp 13k.
+// The units of work, (strip, plane) with the plane fastest, are dealt to the CTAs in
+// equal contiguous runs; a run that enters a new strip reloads its first two planes.
+struct ConvMarch {
+  CUtensorMap map;  // input: 8-channel rows of x, chunk, y, z; box one slot
+  const uint4 *w;
+  const float *bias;  // as in ConvFwd, down to out_f32
+  const uint4 *skip;
+  const uint4 *mask;
+  uint4 *out;
+  float *out_f32;
+  unsigned *status;
+  int R, Cin, Cout, BX;
+  int Cn;     // output channels of a CTA (blockIdx.y is the slice)
+  int relu;
+  int ns;     // ring slots (planes)
+  int units;  // (R / BX) * (R / MA_LINES) * R
+  uint32_t tmem_cols;
+};
+
+#define MA_LINES 16
+#define MA_EPI 8  // epilogue warps, then WS_ISSUERS issuing warps, then one loading warp
+#define MA_THREADS (32 * (MA_EPI + WS_ISSUERS + 1))
+#define MA_MAX_SLOTS 6
+
+static __host__ __device__ inline uint32_t march_slot_bytes(int Cin, int BX) {
+  return ((uint32_t)((MA_LINES + 2) * (Cin >> 3) * (BX + 2)) * 16u + 127u) & ~127u;
+}
+
+__global__ void __launch_bounds__(MA_THREADS) k_conv_march(const __grid_constant__ ConvMarch a) {
+  extern __shared__ __align__(1024) uint8_t sm[];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int R = a.R, kci = a.Cin >> 3, W2 = a.BX + 2, ns = a.ns, n_mt = a.BX >> 3;
+  const uint32_t slot_bytes = march_slot_bytes(a.Cin, a.BX);
+  const int Cn = a.Cn, c0 = blockIdx.y * Cn;
+  const uint32_t tap_bytes = (uint32_t)a.Cin * Cn * 2u, w_bytes = 27u * tap_bytes;
+  uint8_t *wsm = sm + (uint32_t)ns * slot_bytes;
+  uint64_t *full = reinterpret_cast<uint64_t *>(wsm + w_bytes);  // [ns] a plane has arrived
+  uint64_t *empty = full + MA_MAX_SLOTS;                         // [ns] its last reader is done
+  uint64_t *tfull = empty + MA_MAX_SLOTS;                        // [2] accumulators complete
+  uint64_t *tempty = tfull + 2;                                  // [2] accumulators read out
+  uint64_t *wbar = tempty + 2;                                   // weights have arrived
+  uint64_t *done = wbar + 1;                                     // every MMA of the CTA is complete
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(done + 1);
+  float *bias = reinterpret_cast<float *>(full + 2 * MA_MAX_SLOTS + 8);
+  if (tid < Cn) bias[tid] = a.bias ? a.bias[c0 + tid] : 0.0f;
+  if (warp == 0) {
+    umma::tmem_alloc(tslot, a.tmem_cols);
+    umma::tmem_relinquish();
+  }
+  if (tid == 32) {
+    for (int s = 0; s < ns; ++s) {
+      umma::mbar_init(&full[s], 1);
+      umma::mbar_init(&empty[s], WS_ISSUERS);
+    }
+    for (int b = 0; b < 2; ++b) {
+      umma::mbar_init(&tfull[b], WS_ISSUERS);
+      umma::mbar_init(&tempty[b], MA_EPI);
+    }
+    umma::mbar_init(wbar, 32 * MA_EPI);
+    umma::mbar_init(done, WS_ISSUERS);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  umma::tc_fence_before();
+  __syncthreads();
+  umma::tc_fence_after();
+  const uint32_t tmem = *tslot;
+  const int nbx = R / a.BX;
+  const int u0 = (int)((long long)a.units * blockIdx.x / gridDim.x);
+  const int u1 = (int)((long long)a.units * (blockIdx.x + 1) / gridDim.x);
+  bool ok = true;
+
+  if (warp < MA_EPI) {
+    // ---- epilogue: warp w reads lane quarter w % 4 of the M tiles w / 4, w / 4 + 2, ..
+    const int quad = warp & 3, line = 4 * quad + (lane >> 3);
+    const size_t R3 = (size_t)R * R * R;
+    const int nc = Cn >> 4, nit = ((n_mt - (warp >> 2) + 1) >> 1) * nc;  // 16-channel pieces of this warp
+    load_taps(a.w, 0, 27, kci, a.Cout, Cn, c0, wsm, tid, 32 * MA_EPI);
+    umma::cp_async_wait_all();
+    umma::fence_async_smem();
+    umma::mbar_arrive(wbar);
+    int n = 0;
+    uint4 m[2] = {};  // mask rows of the next piece
+    for (int u = u0; u < u1; ++u, ++n) {
+      const int strip = u / R, z = u - strip * R, sy = strip / nbx;
+      const int b = n & 1;
+      const size_t vox0 = ((size_t)z * R + (MA_LINES * sy + line)) * R + (strip - sy * nbx) * a.BX + (lane & 7);
+      int mt = warp >> 2, c = 0;
+      if (nit) conv_mask16(a, c0, vox0 + 8 * mt, R3, m);
+      ok = __all_sync(0xffffffffu, umma::mbar_wait(&tfull[b], (n >> 1) & 1, WS_WAIT_BUDGET));
+      if (!ok) break;
+      umma::tc_fence_after();
+      for (int it = 0; it < nit; ++it) {
+        uint32_t r[16];
+        umma::tmem_ld16(tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)((b * n_mt + mt) * Cn + c), r);
+        const int mt0 = mt, cc = c;
+        const uint4 mc[2] = {m[0], m[1]};
+        c += 16;
+        if (c == Cn) { c = 0; mt += MA_EPI / 4; }
+        if (it + 1 < nit) conv_mask16(a, c0 + c, vox0 + 8 * mt, R3, m);
+        umma::tmem_wait_ld();
+        conv_store16(a, r, bias - c0, mc, c0 + cc, vox0 + 8 * mt0, R3);
+      }
+      umma::tc_fence_before();
+      __syncwarp();
+      if (lane == 0) umma::mbar_arrive(&tempty[b]);
+    }
+  } else if (warp < MA_EPI + WS_ISSUERS) {
+    // ---- issue: warp w owns the M tiles w, w + WS_ISSUERS, ..; its whole warp runs the
+    // loop on uniform values and one elected lane issues
+    const int w = warp - MA_EPI;
+    const uint32_t lead = umma::elect_one();
+    const uint32_t idesc = umma::idesc_bf16(128, Cn, 0, 0);
+    const uint64_t ad0 = umma::sdesc(umma::smem_u32(sm), (uint32_t)W2 * 16u, (uint32_t)(kci * W2) * 16u);
+    const uint64_t bd0 = umma::sdesc(umma::smem_u32(wsm), (uint32_t)Cn * 16u, 128u);
+    const uint32_t kstep_a = 2u * (uint32_t)W2, kstep_b = 2u * (uint32_t)Cn;
+    const int nks = kci / 2;
+    ok = __all_sync(0xffffffffu, umma::mbar_wait(wbar, 0, WS_WAIT_BUDGET));
+    int n = 0;
+    int fs = 0;           // slot and phase of the first plane that the next unit reads
+    uint32_t fph = 0u;
+    for (int u = u0; u < u1 && ok;) {
+      const int len = min(R - u % R, u1 - u);
+      for (int i = 0; i < len && ok; ++i, ++n) {
+        int sl[3];
+        sl[0] = fs;
+#pragma unroll
+        for (int d = 0; d < 3; ++d) {
+          if (d) sl[d] = sl[d - 1] + 1 < ns ? sl[d - 1] + 1 : 0;
+        }
+        const int b = n & 1;
+        if (n >= 2) ok = ok && umma::mbar_wait(&tempty[b], ((n >> 1) - 1) & 1, WS_WAIT_BUDGET);
+        ok = __all_sync(0xffffffffu, ok);
+        if (!ok) break;
+        umma::tc_fence_after();
+        uint64_t bd = bd0;
+        const uint32_t td0 = tmem + (uint32_t)((b * n_mt + w) * Cn);
+#pragma unroll
+        for (int dz = 0; dz < 3; ++dz) {
+          if (dz == 2 || i == 0) {  // the planes of a strip are waited for one by one
+            ok = __all_sync(0xffffffffu, ok && umma::mbar_wait(&full[sl[dz]], fph ^ (sl[dz] < fs ? 1u : 0u), WS_WAIT_BUDGET));
+            if (!ok) break;
+          }
+          for (int dy = 0; dy < 3; ++dy) {
+            uint64_t al = ad0 + (uint32_t)(((uint32_t)sl[dz] * slot_bytes) >> 4) + (uint32_t)(dy * kci * W2 + 8 * w);
+            for (int dx = 0; dx < 3; ++dx, ++al, bd += tap_bytes >> 4) {
+              uint64_t ad = al;
+              uint32_t td = td0;
+              const uint32_t acc = (dz | dy | dx) ? 1u : 0u;
+              for (int mt = w; mt < n_mt; mt += WS_ISSUERS, ad += 8u * WS_ISSUERS, td += (uint32_t)(WS_ISSUERS * Cn)) {
+                umma::mma_bf16_if(lead, td, ad, bd, idesc, acc);
+                for (int ks = 1; ks < nks; ++ks)
+                  umma::mma_bf16_if(lead, td, ad + ks * kstep_a, bd + ks * kstep_b, idesc, 1u);
+              }
+            }
+          }
+        }
+        if (lead) {
+          umma::mma_commit(&tfull[b]);
+          umma::mma_commit(&empty[sl[0]]);
+          if (i == len - 1) {
+            umma::mma_commit(&empty[sl[1]]);
+            umma::mma_commit(&empty[sl[2]]);
+          }
+        }
+        __syncwarp();
+        const int adv = i == len - 1 ? 3 : 1;
+        fs += adv;
+        if (fs >= ns) { fs -= ns; fph ^= 1u; }
+      }
+      u += len;
+    }
+    if (lead) umma::mma_commit(done);
+  } else {
+    // ---- load: one box per plane
+    if (lane == 0) {
+      const uint32_t bytes = (uint32_t)((MA_LINES + 2) * kci * W2) * 16u;
+      int s = 0;
+      uint32_t ph = 1u;  // the first round finds the slots empty
+      for (int u = u0; u < u1 && ok;) {
+        const int strip = u / R, z = u - strip * R, len = min(R - z, u1 - u), sy = strip / nbx;
+        for (int p = z - 1; p <= z + len; ++p) {
+          ok = umma::mbar_wait(&empty[s], ph, WS_WAIT_BUDGET);
+          if (!ok) break;
+          umma::mbar_arrive_expect_tx(&full[s], bytes);
+          umma::tma_load_4d(sm + (uint32_t)s * slot_bytes, &a.map, 2 * ((strip - sy * nbx) * a.BX - 1), 0,
+                            MA_LINES * sy - 1, p, &full[s]);
+          if (++s == ns) { s = 0; ph ^= 1u; }
+        }
+        u += len;
+      }
+      if (!ok) {  // after a timeout: let the copies in flight land before the CTA ends
+        for (int i = 0; i < ns; ++i) umma::mbar_wait(&full[i], i < s ? ph ^ 1u : ph, WS_WAIT_BUDGET);
+      }
+    }
+  }
+  if (!ok && lane == 0) atomicOr(a.status, 1u);
+  if (warp == 0 && !umma::mbar_wait(done, 0, WS_WAIT_BUDGET) && lane == 0) atomicOr(a.status, 1u);
   umma::tc_fence_before();
   __syncthreads();
   if (warp == 0) umma::tmem_dealloc(tmem, a.tmem_cols);
@@ -723,7 +990,10 @@ static const int kWsLayer[WS_NL][4] = {  // cin, cout, level, relu
     {64, 32, 2, 0}, {32, 32, 1, 1}, {32, 16, 1, 0}, {16, 16, 0, 1}, {16, 16, 0, 0}};
 
 struct FwdPlan {
+  int BX;  // 0: blocks of whole lines (k_conv_fwd); else strips of BX voxels (k_conv_march)
   int BZ, BY, tpg, n_mt, grid;
+  int ns;
+  int Cn;  // output channels of a CTA
   uint32_t cols;
   size_t smem;
 };
@@ -786,46 +1056,83 @@ static size_t smem_for_residency(size_t smem, int k) {
 }
 
 static const size_t WS_SMEM_MAX = 232448;
+static const size_t WS_BARS = 64 + 512;  // barriers and the bias of k_conv_fwd
 
-// Tile plans of the forward kernel. Every feasible (BZ, BY) is enumerated; the
-// default pick minimises a cycle estimate per SM -- staging the input tile (L2 ->
-// shared, ~64 B/clk), the MMAs (one 128 x Cout x 16 step every max(8,
-// 128*Cout*16/4096) clocks, issued by four threads) and the epilogue, with at
-// most `occ` CTAs overlapping on an SM -- and gc_ws_autotune replaces it by the
-// fastest measured candidate.
+// Tile plans of the convolution. Every feasible block (BZ, BY) and marching strip (BX)
+// is enumerated, each for every split of the output channels over CTAs; the default pick
+// minimises an estimate in clocks, from clocks taken inside the kernels: staging moves
+// 40 bytes a clock and SM, an MMA takes 40 clk (32 to read its 128 operand rows), or Cn / 2
+// where that is more, or 57 from a single issuing warp, the epilogue 1000 clk per 16
+// channels and pair of M tiles. In a block these follow one another and co-resident CTAs
+// share the busiest of them; in a strip they overlap. gc_ws_autotune replaces the pick by
+// the fastest measured candidate.
+// Where the families meet, forward pass, strips against blocks: 16 -> 16 channels R = 128
+// 70 / 155 us, R = 64 13.9 / 18.5; 64 -> 32 R = 16 7.8 / 14.8. Strips want R to be a
+// multiple of MA_LINES and all taps in shared memory; splitting the channels makes room
+// for the weights of the deep levels (128 -> 64, R = 8: 17.4 us, 25.4 unsplit).
 static std::vector<FwdPlan> enum_fwd(int R, int Cin, int Cout, int sm_count, std::vector<double> *costs) {
   std::vector<FwdPlan> out;
   const int bys[] = {32, 16, 8, 4, 2, 1};
   const int bzs[] = {1, 2, 4, 8};
-  for (int BY : bys) {
-    if (BY > R || R % BY) continue;
-    for (int BZ : bzs) {
-      if (BZ > R || R % BZ) continue;
-      int W2, P, V, L0, L1;
-      conv_geom(R, BZ, BY, W2, P, V, L0, L1);
-      const int n_mt = (L1 - L0 + 128) / 128;
-      if (n_mt * Cout > 512) continue;
-      const size_t tile = (((size_t)(Cin / 8) * V + 128) * 16 + 1023) & ~(size_t)1023;
-      const size_t tap = (size_t)Cin * Cout * 2;
-      if (tile + 2 * tap + 64 > WS_SMEM_MAX) continue;
-      const int tpg = (int)std::min<size_t>(27, (WS_SMEM_MAX - tile - 64) / (2 * tap));
-      const int ngroups = (27 + tpg - 1) / tpg;
-      const int tpg_even = (27 + ngroups - 1) / ngroups;
-      const size_t smem = tile + 2 * (size_t)tpg_even * tap + 64;
-      FwdPlan p;
-      p.BZ = BZ; p.BY = BY; p.tpg = tpg_even; p.n_mt = n_mt; p.grid = (R / BZ) * (R / BY);
-      p.cols = pow2_cols(n_mt * Cout);
-      p.smem = smem_for_residency(smem, (int)(512 / p.cols));
+  for (int Cn = Cout; Cn >= 16; Cn >>= 1) {
+    const size_t tap = (size_t)Cin * Cn * 2;
+    const double mma1 = std::max(40.0, 0.5 * Cn);
+    for (int BY : bys) {
+      if (BY > R || R % BY) continue;
+      for (int BZ : bzs) {
+        if (BZ > R || R % BZ) continue;
+        int W2, P, V, L0, L1;
+        conv_geom(R, BZ, BY, W2, P, V, L0, L1);
+        const int n_mt = (L1 - L0 + 128) / 128;
+        if (n_mt * Cn > 512) continue;
+        const size_t tile = (((size_t)(Cin / 8) * V + 128) * 16 + 1023) & ~(size_t)1023;
+        if (tile + 2 * tap + WS_BARS > WS_SMEM_MAX) continue;
+        const int tpg = (int)std::min<size_t>(27, (WS_SMEM_MAX - tile - WS_BARS) / (2 * tap));
+        const int ngroups = (27 + tpg - 1) / tpg;
+        const int tpg_even = (27 + ngroups - 1) / ngroups;
+        const size_t smem = tile + 2 * (size_t)tpg_even * tap + WS_BARS;
+        FwdPlan p = {};
+        p.BZ = BZ; p.BY = BY; p.tpg = tpg_even; p.n_mt = n_mt; p.grid = (R / BZ) * (R / BY);
+        p.Cn = Cn;
+        p.cols = pow2_cols(n_mt * Cn);
+        p.smem = smem_for_residency(smem, (int)(512 / p.cols));
+        out.push_back(p);
+        if (costs) {
+          const int occ = std::max(1, std::min(8, (int)(233472 / (p.smem + 1024))));
+          const double load = ((double)(Cin / 8) * V * 16 + 27.0 * tap) / 40.0;
+          const double mma = 27.0 * n_mt * (Cin / 16) * (n_mt == 1 ? std::max(57.0, mma1) : mma1) + 1200.0 * ngroups;
+          const double epi = 1000.0 * ((n_mt + 1) / 2) * (Cn / 16);
+          const double per_cta = load + mma + epi + 2000.0;
+          const double busiest = std::max(load, std::max(mma, epi));
+          const double ctas = (double)p.grid * (Cout / Cn);
+          const double together = std::min<double>(occ, std::ceil(ctas / sm_count));
+          costs->push_back(std::ceil(ctas / (sm_count * together)) * (per_cta + (together - 1.0) * busiest));
+        }
+      }
+    }
+    // marching strips: MA_LINES lines x BX voxels, all weights in shared memory
+    const int bxs[] = {64, 32, 16, 8};  // a line of a box is at most 128 rows
+    for (int BX : bxs) {
+      if (R % MA_LINES || BX > R || R % BX) continue;
+      const int n_mt = BX / 8;
+      if (2 * n_mt * Cn > 512) continue;
+      const size_t slot = march_slot_bytes(Cin, BX), fixed = 27 * tap + (2 * MA_MAX_SLOTS + 8) * 8 + 512;
+      if (fixed + 3 * slot > WS_SMEM_MAX) continue;
+      const int units = (R / BX) * (R / MA_LINES) * R, split = Cout / Cn;
+      FwdPlan p = {};
+      p.BX = BX; p.BZ = 1; p.BY = MA_LINES; p.tpg = 27; p.n_mt = n_mt;
+      p.Cn = Cn;
+      p.ns = (int)std::min<size_t>(MA_MAX_SLOTS, (WS_SMEM_MAX - fixed) / slot);
+      p.cols = pow2_cols(2 * n_mt * Cn);
+      p.smem = smem_for_residency(fixed + p.ns * slot, 1);
+      p.grid = std::min(units, std::max(1, sm_count / split));
       out.push_back(p);
       if (costs) {
-        const int occ = std::max(1, std::min(8, (int)(233472 / (p.smem + 1024))));
-        const double load = (double)(Cin / 8) * V * 16 / 64.0 + (double)27 * tap / 64.0;
-        const double mma = 27.0 * n_mt * (Cin / 16) * std::max(8.0, 128.0 * Cout * 16 / 4096.0) / 4.0 + 300.0;
-        const double epi = (double)n_mt * 128 * Cout * 2 / 64.0;
-        const double per_cta = load + mma + epi + 2000.0;
-        const double busiest = std::max(load, std::max(mma, epi));
-        const double waves = std::ceil((double)p.grid / (sm_count * occ));
-        costs->push_back(waves * std::max(per_cta, occ * busiest));
+        const int per = (units + p.grid - 1) / p.grid;
+        const double load = (double)slot / 40.0;
+        const double mma = 27.0 * n_mt * (Cin / 16) * (n_mt == 1 ? std::max(57.0, mma1) : mma1);
+        const double epi = 500.0 * ((n_mt + 1) / 2) * (Cn / 16);
+        costs->push_back(3000.0 + 27.0 * tap / 40.0 + load + per * std::max(mma + 600.0, std::max(load, epi)) + epi);
       }
     }
   }
@@ -894,14 +1201,64 @@ static unsigned ew_blocks(size_t n, int sm_count) {
   return (unsigned)std::max<size_t>(1, b);
 }
 
+// Tensor map over a channel-chunk planar activation (kci chunks of R^3 16-byte rows).
+// A row is two 8-byte elements, so a box spans up to 128 voxels along x and x
+// coordinates are even, 16-byte aligned. chunk_dim: position of the chunk among the
+// outer three dimensions (0: x, chunk, y, z; 2: x, y, z, chunk). The encoder is reached
+// through the runtime: the library does not link the driver. `base` belongs to the
+// network object; maps are made for each launch (below a microsecond) and not kept.
+static int ws_tmap(gc_ws *ws, CUtensorMap *map, const uint4 *base, int R, int kci, int chunk_dim, int bx, int b1, int b2,
+                   int b3) {
+  typedef CUresult (*encode_t)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
+                               const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
+                               CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
+  static const encode_t encode = [] {
+    void *fn = nullptr;
+    cudaDriverEntryPointQueryResult q;
+    if (cudaGetDriverEntryPointByVersion("cuTensorMapEncodeTiled", &fn, 12000, cudaEnableDefault, &q) != cudaSuccess ||
+        q != cudaDriverEntryPointSuccess)
+      fn = nullptr;
+    return (encode_t)fn;
+  }();
+  if (!encode) return ws_fail(ws, GC_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
+  const cuuint64_t n = (cuuint64_t)R, line = n * 16, plane = n * line, vol = n * plane;
+  const cuuint64_t dims0[4] = {2 * n, (cuuint64_t)kci, n, n}, dims2[4] = {2 * n, n, n, (cuuint64_t)kci};
+  const cuuint64_t str0[3] = {vol, line, plane}, str2[3] = {line, plane, vol};
+  const cuuint32_t box[4] = {2u * (cuuint32_t)bx, (cuuint32_t)b1, (cuuint32_t)b2, (cuuint32_t)b3};
+  const cuuint32_t one[4] = {1, 1, 1, 1};
+  if (encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<uint4 *>(base), chunk_dim == 0 ? dims0 : dims2,
+             chunk_dim == 0 ? str0 : str2, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
+             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+    return ws_fail(ws, GC_ERR_CUDA, "cuTensorMapEncodeTiled failed (R = %d, %d chunks)", R, kci);
+  return GC_OK;
+}
+
 static int ws_conv(gc_ws *ws, const FwdPlan &p, int R, int Cin, int Cout, const uint4 *in, const uint16_t *w,
                    const float *bias, const uint4 *skip, const uint4 *mask, uint4 *out, float *out_f32, int relu) {
-  ConvFwd a;
+  if (p.BX) {
+    ConvMarch m = {};
+    const int st = ws_tmap(ws, &m.map, in, R, Cin / 8, 0, p.BX + 2, Cin / 8, MA_LINES + 2, 1);
+    if (st) return st;
+    m.w = reinterpret_cast<const uint4 *>(w); m.bias = bias; m.skip = skip; m.mask = mask;
+    m.out = out; m.out_f32 = out_f32; m.status = ws->status;
+    m.R = R; m.Cin = Cin; m.Cout = Cout; m.BX = p.BX; m.Cn = p.Cn; m.relu = relu; m.ns = p.ns;
+    m.units = (R / p.BX) * (R / MA_LINES) * R;
+    m.tmem_cols = p.cols;
+    k_conv_march<<<dim3(p.grid, Cout / p.Cn), MA_THREADS, p.smem, ws->stream>>>(m);
+    WS_CUDA(ws, cudaGetLastError());
+    return GC_OK;
+  }
+  ConvFwd a = {};
+  a.use_map = R <= 126;
+  if (a.use_map) {
+    const int st = ws_tmap(ws, &a.map, in, R, Cin / 8, 2, R + 2, p.BY + 2, p.BZ + 2, Cin / 8);
+    if (st) return st;
+  }
   a.in = in; a.w = reinterpret_cast<const uint4 *>(w); a.bias = bias; a.skip = skip; a.mask = mask;
   a.out = out; a.out_f32 = out_f32; a.status = ws->status;
-  a.R = R; a.Cin = Cin; a.Cout = Cout; a.BZ = p.BZ; a.BY = p.BY; a.relu = relu; a.tpg = p.tpg; a.n_mt = p.n_mt;
+  a.R = R; a.Cin = Cin; a.Cout = Cout; a.BZ = p.BZ; a.BY = p.BY; a.Cn = p.Cn; a.relu = relu; a.tpg = p.tpg; a.n_mt = p.n_mt;
   a.tmem_cols = p.cols;
-  k_conv_fwd<<<p.grid, 256, p.smem, ws->stream>>>(a);
+  k_conv_fwd<<<dim3(p.grid, Cout / p.Cn), 256, p.smem, ws->stream>>>(a);
   WS_CUDA(ws, cudaGetLastError());
   return GC_OK;
 }
@@ -1047,7 +1404,9 @@ extern "C" int gc_ws_create(gc_ws **out, int R) {
     cudaMemset(ws->status, 0, sizeof(unsigned));
   }
   if (rc == GC_OK) {
-    if (cudaFuncSetAttribute(k_conv_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM_MAX) != cudaSuccess ||
+    if (cudaFuncSetAttribute(k_conv_march, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM_MAX) !=
+            cudaSuccess ||
+        cudaFuncSetAttribute(k_conv_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM_MAX) != cudaSuccess ||
         cudaFuncSetAttribute(k_conv_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM_MAX) !=
             cudaSuccess)
       fail("shared memory attribute");
@@ -1300,6 +1659,8 @@ extern "C" int gc_ws_autotune(gc_ws *ws, int iters, float *ms_out) {
   return rc;
 }
 
+static int ws_cout(int l, int kind) { return kWsLayer[l][kind == 0 ? 1 : 0]; }
+
 // The plan in use: out[0..4] = BZ, BY, taps per group (or per pass), CTAs, M tiles
 // (0 for the weight gradient). kind 0 forward, 1 data gradient, 2 weight gradient.
 extern "C" int gc_ws_plan_info(const gc_ws *ws, int layer, int kind, int *out) {
@@ -1309,7 +1670,26 @@ extern "C" int gc_ws_plan_info(const gc_ws *ws, int layer, int kind, int *out) {
     out[0] = p.BZ; out[1] = p.BY; out[2] = p.tpp; out[3] = p.grid; out[4] = 0;
   } else {
     const FwdPlan &p = kind == 0 ? ws->pf[layer] : ws->pb[layer];
-    out[0] = p.BZ; out[1] = p.BY; out[2] = p.tpg; out[3] = p.grid; out[4] = p.n_mt;
+    out[0] = p.BZ; out[1] = p.BY; out[2] = p.tpg; out[3] = p.grid * ws_cout(layer, kind) / p.Cn; out[4] = p.n_mt;
+  }
+  return GC_OK;
+}
+
+// Take candidate `index` of the plans of (layer, kind); *count receives how many there
+// are. A negative index only counts.
+extern "C" int gc_ws_set_plan(gc_ws *ws, int layer, int kind, int index, int *count) {
+  if (!ws || layer < 0 || layer >= WS_NL || kind < 0 || kind > 2) return GC_ERR_ARG;
+  const int Cin = kWsLayer[layer][0], Cout = kWsLayer[layer][1], R = ws->R >> kWsLayer[layer][2];
+  if (kind == 2) {
+    const std::vector<WgPlan> c = enum_wgrad(R, Cin, Cout, ws->sm_count, nullptr);
+    if (count) *count = (int)c.size();
+    if (index >= (int)c.size()) return GC_ERR_ARG;
+    if (index >= 0) ws->pw[layer] = c[index];
+  } else {
+    const std::vector<FwdPlan> c = enum_fwd(R, kind ? Cout : Cin, kind ? Cin : Cout, ws->sm_count, nullptr);
+    if (count) *count = (int)c.size();
+    if (index >= (int)c.size()) return GC_ERR_ARG;
+    if (index >= 0) (kind ? ws->pb[layer] : ws->pf[layer]) = c[index];
   }
   return GC_OK;
 }

@@ -182,6 +182,7 @@ _PROTOS = {
     "gc_ws_status": (C.c_int, [_vp, C.POINTER(C.c_uint32), C.c_int]),
     "gc_ws_autotune": (C.c_int, [_vp, C.c_int, _vp]),
     "gc_ws_plan_info": (C.c_int, [_vp, C.c_int, C.c_int, _vp]),
+    "gc_ws_set_plan": (C.c_int, [_vp, C.c_int, C.c_int, C.c_int, _vp]),
     "gc_pm_graph_create": (C.c_int, [_ctxp, C.POINTER(Particles), C.POINTER(StepParams), C.POINTER(_vp)]),
     "gc_pm_graph_launch": (C.c_int, [_vp]),
     "gc_pm_graph_destroy": (C.c_int, [_vp]),

@@ -523,8 +523,8 @@ int gc_ws_backward(gc_ws *ws, const void *target, float *loss_out);
 int gc_ws_adam(gc_ws *ws, float lr, float beta1, float beta2, float eps, int step);
 /* Device status bits (bit 0: a tensor-core completion wait timed out); clear resets them. */
 int gc_ws_status(gc_ws *ws, unsigned *flags, int clear);
-/* Autotuner: time every feasible tile plan (block of output planes x lines,
- * taps per weight group) of each layer's forward, data-gradient and weight-
+/* Autotuner: time every feasible tile plan (block of output planes x lines, or a
+ * strip marching along z; taps per weight group; split of the output channels) of each layer's forward, data-gradient and weight-
  * gradient kernels with CUDA events over `iters` launches and keep the fastest.
  * Overwrites activations. ms_out (host, nullable, 33 floats): best milliseconds
  * per [layer][pass]. Synchronises the stream. */
@@ -532,6 +532,10 @@ int gc_ws_autotune(gc_ws *ws, int iters, float *ms_out);
 /* Plan in use for (layer, pass 0/1/2): out[5] = {planes, lines, taps per group or
  * pass, CTAs, M tiles per CTA (0 for the weight gradient)}. */
 int gc_ws_plan_info(const gc_ws *ws, int layer, int kind, int *out);
+/* Take candidate `index` among the plans of (layer, pass) that the autotuner would
+ * time; *count (nullable) = how many there are, index < 0 only counts. Convolution
+ * results are the same bits under every plan. */
+int gc_ws_set_plan(gc_ws *ws, int layer, int kind, int index, int *count);
 
 /* Initial guess of the engine's solve (gc_pm_step with warm_start != 0):
  *   GC_WS_PLAIN       phi(n-1), the previous potential (the reference's warm start);
