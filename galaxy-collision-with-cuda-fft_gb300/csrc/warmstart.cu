@@ -615,9 +615,10 @@ __global__ void __launch_bounds__(MA_THREADS) k_conv_march(const __grid_constant
 // (8 output channels) placed in 2 KB groups of 8 voxels so that every one of the
 // 128 M rows addresses shared memory of the stage (rows >= Cout are never read
 // back). Voxels outside the CTA's block are zero in gy. Taps are split into
-// passes so that a pass's accumulators (tpp x Cin columns) fit Tensor Memory;
-// persistent CTAs accumulate over all their blocks and write one partial per
-// CTA, summed in a fixed order afterwards.
+// passes so that a pass's accumulators (tpp x Cin columns) fit Tensor Memory, one
+// CTA row of the grid per pass; persistent CTAs accumulate over all their blocks and
+// write one partial per CTA, summed in a fixed order afterwards. This form takes lines
+// of any length (levels whose size is not a multiple of 8).
 struct ConvW {
   const uint4 *x;    // layer input, Cin channels
   const uint4 *gy;   // gradient of the pre-activation output, Cout channels
@@ -668,7 +669,7 @@ __global__ void __launch_bounds__(256) k_conv_wgrad(ConvW a) {
   long long gs = 0;  // stages issued by this CTA
   uint4 *trow = reinterpret_cast<uint4 *>(tile);
   const int npass = (27 + a.tpp - 1) / a.tpp;
-  for (int pass = 0; pass < npass && !fail; ++pass) {
+  for (int pass = blockIdx.y; pass < npass && !fail; pass += gridDim.y) {
     const int t0 = pass * a.tpp, t1 = min(27, t0 + a.tpp);
     bool first = true;
     for (int b = blockIdx.x; b < a.nblocks && !fail; b += gridDim.x) {
@@ -767,6 +768,224 @@ __global__ void __launch_bounds__(256) k_conv_wgrad(ConvW a) {
   if (warp == 0) umma::tmem_dealloc(tmem, a.tmem_cols);
 }
 
+// ------------------------------------------------------------------------------
+// the same weight gradient with taps in the rows and columns of one product
+// ------------------------------------------------------------------------------
+// Both operands lie in shared memory as rows of 8 channels, so a group of 8 M (or N)
+// indices is named by an address and the next group by a constant distance. With x
+// stored [line][chunk][x], groups one line-and-chunk row apart run over (dy, chunk): one
+// MMA gives the three dy taps at once (N = 3 Cin). With gy of three planes stored
+// [line][plane][chunk][x], its groups run over (dz, chunk) (M = 3 Cout, where that is at
+// most 128 rows). The 27 taps are then 3 MMAs per 16 voxels, one per dx, instead of 27,
+// each with Cout of 128 rows in use. K runs over the voxels of the strip alone, so no
+// halo row is multiplied. Cases, by channels:
+//   mz = 3 (Cout <= 40): rows (dz, co), gy planes z - 1 .. z + 1 beside x plane z;
+//   mz = 1: rows co, one gy plane z - dz, dz by CTA group;
+//   ndx = 3 where 3 accumulators of 3 Cin columns fit Tensor Memory, else dx by CTA
+//   group; 3 Cin > 256 columns (Cin = 128): one MMA per dy.
+// A CTA (split, group) goes over its share of the units (strip, plane) with a ring of
+// stages, one box each of x and gy, and writes one partial. The bias gradient is summed
+// from the staged gy by the warps that read the accumulators out at the end.
+// An MMA of 64 x 48 x 16 takes 29 clk here, of 128 x 96 x 16 57, of 128 x 192 x 16 97.
+struct ConvWS {
+  CUtensorMap mx;  // x: rows of x, chunk, y, z
+  CUtensorMap mg;  // gy: rows of x, chunk, z, y
+  float *part;     // [gridDim.x][27 Cout Cin weights, Cout biases]
+  unsigned *status;
+  int R, Cin, Cout, BX, LN;
+  int mz, ndx;
+  int ns;    // stages
+  int units; // (R / BX) * (R / LN) * R
+  uint32_t tmem_cols;
+};
+
+#define WW_READ 4  // warps: readers (bias sums, accumulators out), issuers, loader
+#define WW_ISS 3
+#define WW_THREADS (32 * (WW_READ + WW_ISS + 1))
+#define WW_MAX_STAGES 4
+
+static __host__ __device__ inline uint32_t wgs_gy_bytes(int Cout, int BX, int LN, int mz) {
+  return ((uint32_t)(LN * mz * (Cout >> 3) * BX) * 16u + 127u) & ~127u;
+}
+static __host__ __device__ inline uint32_t wgs_x_bytes(int Cin, int BX, int LN) {
+  return ((uint32_t)((LN + 2) * (Cin >> 3) * (BX + 2)) * 16u + 127u) & ~127u;
+}
+
+__global__ void __launch_bounds__(WW_THREADS) k_wgrad_strip(const __grid_constant__ ConvWS a) {
+  extern __shared__ __align__(1024) uint8_t sm[];
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int R = a.R, kci = a.Cin >> 3, kco = a.Cout >> 3, BX = a.BX, LN = a.LN, W2 = BX + 2, ns = a.ns;
+  const uint32_t gbytes = wgs_gy_bytes(a.Cout, BX, LN, a.mz), sbytes = gbytes + wgs_x_bytes(a.Cin, BX, LN);
+  uint64_t *full = reinterpret_cast<uint64_t *>(sm + (uint32_t)ns * sbytes);  // [ns] x and gy have arrived
+  uint64_t *empty = full + WW_MAX_STAGES;                                     // [ns] their readers are done
+  uint64_t *done = empty + WW_MAX_STAGES;                                     // the accumulators are complete
+  uint32_t *tslot = reinterpret_cast<uint32_t *>(done + 1);
+  float *red = reinterpret_cast<float *>(done + 2);  // [4 warps][4 chunks][8]
+  // this group's taps and accumulators
+  const int ngx = a.ndx == 3 ? 1 : 3;
+  const int gdz = blockIdx.y / ngx, gdx = blockIdx.y - gdz * ngx;  // dz (mz = 1) and dx (ndx = 1) of the group
+  const int ndy = 3 * a.Cin <= 256 ? 3 : 1;                        // dy taps in the columns of one MMA
+  const int nacc = a.ndx == 3 || ndy == 1 ? 3 : 1, N = ndy * a.Cin;
+  const int M = 8 * a.mz * kco <= 64 ? 64 : 128;
+  const bool bias = a.mz == 3 ? gdx == 0 : (gdz == 1 && gdx == 0);
+  if (warp == 0) {
+    umma::tmem_alloc(tslot, a.tmem_cols);
+    umma::tmem_relinquish();
+  }
+  if (tid == 32) {
+    for (int s = 0; s < ns; ++s) {
+      umma::mbar_init(&full[s], 1);
+      umma::mbar_init(&empty[s], nacc + (bias ? WW_READ : 0));
+    }
+    umma::mbar_init(done, nacc);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  umma::tc_fence_before();
+  __syncthreads();
+  umma::tc_fence_after();
+  const uint32_t tmem = *tslot;
+  const int nbx = R / BX;
+  const int u0 = (int)((long long)a.units * blockIdx.x / gridDim.x);
+  const int u1 = (int)((long long)a.units * (blockIdx.x + 1) / gridDim.x);
+  bool ok = true;
+
+  if (warp < WW_READ) {
+    float *part = a.part + (size_t)blockIdx.x * (27 * a.Cin + 1) * a.Cout;
+    if (bias) {
+      // ---- channel sums of plane z: warp w takes the (line, chunk) rows w, w + 4, ..
+      float acc[4][8] = {};
+      const int nch = kco > WW_READ ? kco / WW_READ : 1;  // chunks of this warp
+      const int c0 = warp & (kco - 1), lstep = kco < WW_READ ? WW_READ / kco : 1, l0 = kco < WW_READ ? warp / kco : 0;
+      int s = 0;
+      uint32_t ph = 0u;
+      for (int u = u0; u < u1; ++u) {
+        ok = __all_sync(0xffffffffu, umma::mbar_wait(&full[s], ph, WS_WAIT_BUDGET));
+        if (!ok) break;
+        const uint4 *g = reinterpret_cast<const uint4 *>(sm + (uint32_t)s * sbytes) + (size_t)(a.mz >> 1) * kco * BX;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (j >= nch) continue;
+          const uint4 *gc = g + (size_t)(c0 + WW_READ * j) * BX;
+          for (int l = l0; l < LN; l += lstep)
+            for (int x = lane; x < BX; x += 32) {
+              float f[8];
+              unpack8(gc[(size_t)l * a.mz * kco * BX + x], f);
+#pragma unroll
+              for (int k = 0; k < 8; ++k) acc[j][k] += f[k];
+            }
+        }
+        __syncwarp();
+        if (lane == 0) umma::mbar_arrive(&empty[s]);
+        if (++s == ns) { s = 0; ph ^= 1u; }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          float v = acc[j][k];
+#pragma unroll
+          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+          if (lane == 0) red[(warp * 4 + j) * 8 + k] = v;
+        }
+      asm volatile("bar.sync 1, 128;" ::: "memory");
+      if (tid < a.Cout && ok) {
+        const int c = tid >> 3, k = tid & 7;
+        float v;
+        if (kco >= WW_READ) {
+          v = red[((c & 3) * 4 + (c >> 2)) * 8 + k];
+        } else {
+          v = 0.0f;
+          for (int w = c; w < WW_READ; w += kco) v += red[w * 32 + k];
+        }
+        part[(size_t)27 * a.Cout * a.Cin + tid] = v;
+      }
+    }
+    // ---- accumulators out: row (dz, co) of column (dx or dy, .., ci)
+    ok = __all_sync(0xffffffffu, ok && umma::mbar_wait(done, 0, WS_WAIT_BUDGET));
+    umma::tc_fence_after();
+    if (ok) {
+      const int row = M == 64 ? 16 * warp + lane : 32 * warp + lane;
+      const int m = row / a.Cout, co = row - m * a.Cout;
+      const bool valid = m < a.mz && (M == 128 || lane < 16);
+      const int dz = a.mz == 3 ? 2 - m : gdz;  // gy plane z - 1 + m meets x plane z: dz = 1 - m
+      for (int q = 0; q < nacc; ++q)
+        for (int c = 0; c < N; c += 16) {
+          uint32_t r[16];
+          umma::tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(q * N + c), r);
+          umma::tmem_wait_ld();
+          const int dyc = c / a.Cin, ci = c - dyc * a.Cin;
+          const int dy = ndy == 3 ? dyc : q, dx = a.ndx == 3 ? q : gdx;
+          if (valid) {
+            float4 *dst = reinterpret_cast<float4 *>(part + ((size_t)(9 * dz + 3 * dy + dx) * a.Cout + co) * a.Cin + ci);
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              dst[j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
+                                   __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+          }
+        }
+    }
+  } else if (warp < WW_READ + WW_ISS) {
+    // ---- issue: warp q feeds accumulator q
+    const int q = warp - WW_READ;
+    if (q < nacc) {
+      const uint32_t lead = umma::elect_one();
+      const uint32_t idesc = umma::idesc_bf16(M, N, 1, 1);
+      const uint32_t gl = (uint32_t)(a.mz * kco * BX), xl = (uint32_t)(kci * W2);  // rows of a line
+      const bool pair = BX < 16;  // 16 voxels of K: along x, or 8 of two lines
+      const uint64_t ad0 = umma::sdesc_mn(umma::smem_u32(sm), pair ? gl * 16u : 128u, (uint32_t)BX * 16u);
+      const uint64_t bd0 = umma::sdesc_mn(umma::smem_u32(sm) + gbytes, pair ? xl * 16u : 128u, (uint32_t)W2 * 16u) +
+                           (uint32_t)(a.ndx == 3 ? q : gdx) + (ndy == 1 ? (uint32_t)q * xl : 0u);
+      const uint32_t td = tmem + (uint32_t)(q * N);
+      const int lines = pair ? LN / 2 : LN, nxb = pair ? 1 : BX / 16;
+      const uint32_t glp = pair ? 2 * gl : gl, xlp = pair ? 2 * xl : xl;
+      uint32_t accum = 0u;
+      int s = 0;
+      uint32_t ph = 0u;
+      for (int u = u0; u < u1; ++u) {
+        ok = __all_sync(0xffffffffu, umma::mbar_wait(&full[s], ph, WS_WAIT_BUDGET));
+        if (!ok) break;
+        umma::tc_fence_after();
+        uint64_t al = ad0 + (((uint32_t)s * sbytes) >> 4), bl = bd0 + (((uint32_t)s * sbytes) >> 4);
+        for (int l = 0; l < lines; ++l, al += glp, bl += xlp) {
+#pragma unroll 4
+          for (int xb = 0; xb < nxb; ++xb) {
+            umma::mma_bf16_if(lead, td, al + 16u * xb, bl + 16u * xb, idesc, accum);
+            accum = 1u;
+          }
+        }
+        if (lead) umma::mma_commit(&empty[s]);
+        __syncwarp();
+        if (++s == ns) { s = 0; ph ^= 1u; }
+      }
+      if (lead) umma::mma_commit(done);
+    }
+  } else if (lane == 0) {
+    // ---- load: a box of x and one of gy per unit
+    const uint32_t bytes = (uint32_t)(LN * a.mz * kco * BX + (LN + 2) * kci * W2) * 16u;
+    int s = 0;
+    uint32_t ph = 1u;  // the first round finds the stages empty
+    for (int u = u0; u < u1; ++u) {
+      const int strip = u / R, z = u - strip * R, sy = strip / nbx, x0 = (strip - sy * nbx) * BX, y0 = sy * LN;
+      ok = umma::mbar_wait(&empty[s], ph, WS_WAIT_BUDGET);
+      if (!ok) break;
+      uint8_t *st = sm + (uint32_t)s * sbytes;
+      umma::mbar_arrive_expect_tx(&full[s], bytes);
+      umma::tma_load_4d(st, &a.mg, 2 * x0, 0, a.mz == 3 ? z - 1 : z + 1 - gdz, y0, &full[s]);
+      umma::tma_load_4d(st + gbytes, &a.mx, 2 * (x0 - 1), 0, y0 - 1, z, &full[s]);
+      if (++s == ns) { s = 0; ph ^= 1u; }
+    }
+    if (!ok) {  // after a timeout: let the copies in flight land before the CTA ends
+      for (int i = 0; i < ns; ++i) umma::mbar_wait(&full[i], i < s ? ph ^ 1u : ph, WS_WAIT_BUDGET);
+    }
+  }
+  if (!ok && lane == 0) atomicOr(a.status, 1u);
+  if (warp == 0 && !umma::mbar_wait(done, 0, WS_WAIT_BUDGET) && lane == 0) atomicOr(a.status, 1u);
+  umma::tc_fence_before();
+  __syncthreads();
+  if (warp == 0) umma::tmem_dealloc(tmem, a.tmem_cols);
+}
+
 // out[e] = sum over c of part[c*nelem + e] for few elements and many partials:
 // one block per element, a fixed strided split and a fixed tree (deterministic).
 __global__ void __launch_bounds__(256) k_reduce_cols(const float *__restrict__ part, int nparts, int nelem,
@@ -784,14 +1003,31 @@ __global__ void __launch_bounds__(256) k_reduce_cols(const float *__restrict__ p
   if (threadIdx.x == 0) out[e] = red[0];
 }
 
-// dW[e] = sum over CTAs of the partials, in CTA order.
+// out[e] = sum over partials p of part[p][e], e < nelem (a multiple of 4): thread (x, y)
+// adds the partials y, y + 8, .. of four elements, then the eight sums are added in
+// order. One thread per element over all partials took as long as the product at 16
+// channels: 27 blocks of it, each a chain of 152 loads.
 __global__ void __launch_bounds__(256) k_wgrad_reduce(const float *__restrict__ part, int nparts, int nelem,
-                                                      float *__restrict__ dw) {
-  const int e = blockIdx.x * blockDim.x + threadIdx.x;
-  if (e >= nelem) return;
-  float s = 0.0f;
-  for (int c = 0; c < nparts; ++c) s += part[(size_t)c * nelem + e];
-  dw[e] = s;
+                                                      float *__restrict__ out) {
+  __shared__ float4 red[8][32];
+  const int x = threadIdx.x & 31, y = threadIdx.x >> 5, e = blockIdx.x * 32 + x, n4 = nelem >> 2;
+  float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+  if (e < n4) {
+#pragma unroll 4
+    for (int p = y; p < nparts; p += 8) {
+      const float4 v = __ldg(reinterpret_cast<const float4 *>(part) + (size_t)p * n4 + e);
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+  }
+  red[y][x] = s;
+  __syncthreads();
+  if (y == 0 && e < n4) {
+    for (int k = 1; k < 8; ++k) {
+      const float4 v = red[k][x];
+      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
+    }
+    reinterpret_cast<float4 *>(out)[e] = s;
+  }
 }
 
 // ------------------------------------------------------------------------------
@@ -998,7 +1234,9 @@ struct FwdPlan {
   size_t smem;
 };
 struct WgPlan {
+  int BX;  // 0: blocks of whole lines (k_conv_wgrad); else strips of BX voxels (k_wgrad_strip)
   int BZ, BY, tpp, nblocks, grid;
+  int mz, ndx, ns, groups;
   uint32_t cols;
   size_t smem;
 };
@@ -1150,12 +1388,55 @@ static bool plan_fwd(int R, int Cin, int Cout, int sm_count, FwdPlan &best) {
   return true;
 }
 
+// Weight gradient: strips wherever the lines come in multiples of 8 voxels, and only
+// where they do not, blocks of whole lines. Strips are enumerated by (BX, lines,
+// splits) with an estimate in clocks: loads at 40 bytes a clock and SM, MMAs at their
+// measured clocks, the partials written and read again at 6000 bytes a clock of the chip.
+// Strips against blocks: 16 -> 16 channels R = 128 48 / 721 us, R = 64 11.8 / 103;
+// 64 -> 64 R = 32 25 / 129, R = 16 11.2 / 94; 128 -> 64 R = 8 11.0 / 145.
 static std::vector<WgPlan> enum_wgrad(int R, int Cin, int Cout, int sm_count, std::vector<double> *scores) {
   std::vector<WgPlan> out;
+  const int lns[] = {16, 8, 4, 2};
+  const int bxs[] = {64, 32, 16, 8};
+  const int mz = 3 * Cout <= 128 ? 3 : 1, ndx = 9 * Cin <= 512 ? 3 : 1;
+  const int groups = (mz == 3 ? 1 : 3) * (ndx == 3 ? 1 : 3);
+  const int N = 3 * Cin <= 256 ? 3 * Cin : Cin, nacc = ndx == 3 || N == Cin ? 3 : 1;
+  const int M = mz * Cout <= 64 ? 64 : 128;
+  const double mma = std::max(0.5 * N, M == 64 ? 29.0 : 32.0 + 0.25 * N);
+  for (int BX : bxs) {
+    if (R % BX) continue;
+    for (int LN : lns) {
+      if (R % LN) continue;
+      const size_t gb = wgs_gy_bytes(Cout, BX, LN, mz), xb = wgs_x_bytes(Cin, BX, LN);
+      // the M groups beyond mz * Cout / 8 read on into the x box of the stage
+      if ((size_t)(M / 8 - mz * Cout / 8) * BX * 16 > xb) continue;
+      const size_t fixed = (2 * WW_MAX_STAGES + 2) * 8 + 512;
+      if (fixed + 2 * (gb + xb) > WS_SMEM_MAX) continue;
+      const int units = (R / BX) * (R / LN) * R;
+      int last = 0;
+      for (int div = 1; div <= 8; div *= 2) {
+        WgPlan p = {};
+        p.BX = BX; p.BZ = 1; p.BY = LN; p.tpp = 27 / groups; p.nblocks = units;
+        p.mz = mz; p.ndx = ndx; p.groups = groups;
+        p.ns = (int)std::min<size_t>(WW_MAX_STAGES, (WS_SMEM_MAX - fixed) / (gb + xb));
+        p.cols = pow2_cols(nacc * N);
+        p.smem = smem_for_residency(fixed + p.ns * (gb + xb), 1);
+        p.grid = std::min(units, std::max(1, sm_count / groups / div));
+        if (p.grid == last) continue;
+        last = p.grid;
+        out.push_back(p);
+        if (scores) {
+          const int per = (units + p.grid - 1) / p.grid;
+          const double load = (double)(gb + xb) / 40.0, prod = LN * BX / 16.0 * nacc * mma;
+          const double parts = (double)p.grid * 27 * Cin * Cout * 4 * 2 / 6000.0;
+          scores->push_back(-(4000.0 + load + per * std::max(load, prod + 100.0) + 60.0 * nacc * N / 16 + parts));
+        }
+      }
+    }
+  }
+  if (!out.empty()) return out;
   const int bys[] = {32, 16, 8, 4, 2, 1};
   const int bzs[] = {1, 2, 4};
-  const int tpp = std::min(27, 512 / Cin);
-  const uint32_t cols = pow2_cols(tpp * Cin);
   for (int BY : bys) {
     if (BY > R || R % BY) continue;
     for (int BZ : bzs) {
@@ -1166,8 +1447,14 @@ static std::vector<WgPlan> enum_wgrad(int R, int Cin, int Cout, int sm_count, st
       const size_t smem = tile + 2 * WG_STAGE_BYTES + 64;
       if (smem > WS_SMEM_MAX) continue;
       const int nst = (L1 - L0 + WG_STAGE_ROWS) / WG_STAGE_ROWS;
-      WgPlan p;
+      // few blocks: fewer taps a pass, more passes beside each other (64 -> 128 channels
+      // at R = 4: 2 CTAs with 4 passes each took 169 us, 54 CTAs of one tap 17)
+      int tpp = std::min(27, 512 / Cin);
+      while (tpp > 1 && (R / BZ) * (R / BY) * ((27 + tpp - 1) / tpp) * 2 < sm_count) tpp = (tpp + 1) / 2;
+      const uint32_t cols = pow2_cols(tpp * Cin);
+      WgPlan p = {};
       p.BZ = BZ; p.BY = BY; p.tpp = tpp; p.nblocks = (R / BZ) * (R / BY); p.cols = cols;
+      p.groups = (27 + tpp - 1) / tpp;
       p.smem = smem_for_residency(smem, (int)(512 / cols));
       const int per_sm = std::max(1, (int)(233472 / (p.smem + 1024)));
       p.grid = std::min(p.nblocks, sm_count * per_sm);
@@ -1203,12 +1490,13 @@ static unsigned ew_blocks(size_t n, int sm_count) {
 
 // Tensor map over a channel-chunk planar activation (kci chunks of R^3 16-byte rows).
 // A row is two 8-byte elements, so a box spans up to 128 voxels along x and x
-// coordinates are even, 16-byte aligned. chunk_dim: position of the chunk among the
-// outer three dimensions (0: x, chunk, y, z; 2: x, y, z, chunk). The encoder is reached
-// through the runtime: the library does not link the driver. `base` belongs to the
-// network object; maps are made for each launch (below a microsecond) and not kept.
-static int ws_tmap(gc_ws *ws, CUtensorMap *map, const uint4 *base, int R, int kci, int chunk_dim, int bx, int b1, int b2,
-                   int b3) {
+// coordinates are even, 16-byte aligned. `order` names the dimensions after x, nearest
+// first. The encoder is reached through the runtime: the library does not link the
+// driver. `base` belongs to the network object; maps are made for each launch (below a
+// microsecond) and not kept.
+enum WsDim { WS_Y, WS_Z, WS_C };
+static int ws_tmap(gc_ws *ws, CUtensorMap *map, const uint4 *base, int R, int kci, const WsDim (&order)[3], int bx, int b1,
+                   int b2, int b3) {
   typedef CUresult (*encode_t)(CUtensorMap *, CUtensorMapDataType, cuuint32_t, void *, const cuuint64_t *,
                                const cuuint64_t *, const cuuint32_t *, const cuuint32_t *, CUtensorMapInterleave,
                                CUtensorMapSwizzle, CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
@@ -1221,14 +1509,14 @@ static int ws_tmap(gc_ws *ws, CUtensorMap *map, const uint4 *base, int R, int kc
     return (encode_t)fn;
   }();
   if (!encode) return ws_fail(ws, GC_ERR_CUDA, "cuTensorMapEncodeTiled is not available");
-  const cuuint64_t n = (cuuint64_t)R, line = n * 16, plane = n * line, vol = n * plane;
-  const cuuint64_t dims0[4] = {2 * n, (cuuint64_t)kci, n, n}, dims2[4] = {2 * n, n, n, (cuuint64_t)kci};
-  const cuuint64_t str0[3] = {vol, line, plane}, str2[3] = {line, plane, vol};
+  const cuuint64_t n = (cuuint64_t)R, size[3] = {n, n, (cuuint64_t)kci}, stride[3] = {n * 16, n * n * 16, n * n * n * 16};
+  const cuuint64_t dims[4] = {2 * n, size[order[0]], size[order[1]], size[order[2]]};
+  const cuuint64_t strides[3] = {stride[order[0]], stride[order[1]], stride[order[2]]};
   const cuuint32_t box[4] = {2u * (cuuint32_t)bx, (cuuint32_t)b1, (cuuint32_t)b2, (cuuint32_t)b3};
   const cuuint32_t one[4] = {1, 1, 1, 1};
-  if (encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<uint4 *>(base), chunk_dim == 0 ? dims0 : dims2,
-             chunk_dim == 0 ? str0 : str2, box, one, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE,
-             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
+  if (encode(map, CU_TENSOR_MAP_DATA_TYPE_FLOAT64, 4, const_cast<uint4 *>(base), dims, strides, box, one,
+             CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
+             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) != CUDA_SUCCESS)
     return ws_fail(ws, GC_ERR_CUDA, "cuTensorMapEncodeTiled failed (R = %d, %d chunks)", R, kci);
   return GC_OK;
 }
@@ -1237,7 +1525,7 @@ static int ws_conv(gc_ws *ws, const FwdPlan &p, int R, int Cin, int Cout, const 
                    const float *bias, const uint4 *skip, const uint4 *mask, uint4 *out, float *out_f32, int relu) {
   if (p.BX) {
     ConvMarch m = {};
-    const int st = ws_tmap(ws, &m.map, in, R, Cin / 8, 0, p.BX + 2, Cin / 8, MA_LINES + 2, 1);
+    const int st = ws_tmap(ws, &m.map, in, R, Cin / 8, {WS_C, WS_Y, WS_Z}, p.BX + 2, Cin / 8, MA_LINES + 2, 1);
     if (st) return st;
     m.w = reinterpret_cast<const uint4 *>(w); m.bias = bias; m.skip = skip; m.mask = mask;
     m.out = out; m.out_f32 = out_f32; m.status = ws->status;
@@ -1251,7 +1539,7 @@ static int ws_conv(gc_ws *ws, const FwdPlan &p, int R, int Cin, int Cout, const 
   ConvFwd a = {};
   a.use_map = R <= 126;
   if (a.use_map) {
-    const int st = ws_tmap(ws, &a.map, in, R, Cin / 8, 2, R + 2, p.BY + 2, p.BZ + 2, Cin / 8);
+    const int st = ws_tmap(ws, &a.map, in, R, Cin / 8, {WS_Y, WS_Z, WS_C}, R + 2, p.BY + 2, p.BZ + 2, Cin / 8);
     if (st) return st;
   }
   a.in = in; a.w = reinterpret_cast<const uint4 *>(w); a.bias = bias; a.skip = skip; a.mask = mask;
@@ -1266,14 +1554,30 @@ static int ws_conv(gc_ws *ws, const FwdPlan &p, int R, int Cin, int Cout, const 
 static int ws_wgrad(gc_ws *ws, int l, const uint4 *x, const uint4 *gy) {
   const int Cin = kWsLayer[l][0], Cout = kWsLayer[l][1], R = ws->R >> kWsLayer[l][2];
   const WgPlan &p = ws->pw[l];
+  const int nelem = 27 * Cout * Cin;
+  if (p.BX) {
+    ConvWS a = {};
+    int st;
+    if ((st = ws_tmap(ws, &a.mx, x, R, Cin / 8, {WS_C, WS_Y, WS_Z}, p.BX + 2, Cin / 8, p.BY + 2, 1))) return st;
+    if ((st = ws_tmap(ws, &a.mg, gy, R, Cout / 8, {WS_C, WS_Z, WS_Y}, p.BX, Cout / 8, p.mz, p.BY))) return st;
+    a.part = ws->part; a.status = ws->status;
+    a.R = R; a.Cin = Cin; a.Cout = Cout; a.BX = p.BX; a.LN = p.BY; a.mz = p.mz; a.ndx = p.ndx; a.ns = p.ns;
+    a.units = p.nblocks; a.tmem_cols = p.cols;
+    k_wgrad_strip<<<dim3(p.grid, p.groups), WW_THREADS, p.smem, ws->stream>>>(a);
+    WS_CUDA(ws, cudaGetLastError());
+    // the biases follow the weights in the partials and in the gradient vector
+    const int n = nelem + Cout;
+    k_wgrad_reduce<<<(n / 4 + 31) / 32, 256, 0, ws->stream>>>(ws->part, p.grid, n, ws->grads + ws->w_off[l]);
+    WS_CUDA(ws, cudaGetLastError());
+    return GC_OK;
+  }
   ConvW a;
   a.x = x; a.gy = gy; a.part = ws->part; a.status = ws->status;
   a.R = R; a.Cin = Cin; a.Cout = Cout; a.BZ = p.BZ; a.BY = p.BY; a.tpp = p.tpp; a.nblocks = p.nblocks;
   a.tmem_cols = p.cols;
-  k_conv_wgrad<<<p.grid, 256, p.smem, ws->stream>>>(a);
+  k_conv_wgrad<<<dim3(p.grid, p.groups), 256, p.smem, ws->stream>>>(a);
   WS_CUDA(ws, cudaGetLastError());
-  const int nelem = 27 * Cout * Cin;
-  k_wgrad_reduce<<<(nelem + 255) / 256, 256, 0, ws->stream>>>(ws->part, p.grid, nelem, ws->grads + ws->w_off[l]);
+  k_wgrad_reduce<<<(nelem / 4 + 31) / 32, 256, 0, ws->stream>>>(ws->part, p.grid, nelem, ws->grads + ws->w_off[l]);
   WS_CUDA(ws, cudaGetLastError());
   // bias gradient: channel sums of gy
   const size_t R3 = (size_t)R * R * R;
@@ -1390,7 +1694,7 @@ extern "C" int gc_ws_create(gc_ws **out, int R) {
   for (int l = 0; l < WS_NL && rc == GC_OK; ++l) {
     const int Rl = R >> kWsLayer[l][2];
     for (const WgPlan &c : enum_wgrad(Rl, kWsLayer[l][0], kWsLayer[l][1], ws->sm_count, nullptr))
-      part = std::max(part, (size_t)c.grid * 27 * kWsLayer[l][0] * kWsLayer[l][1]);
+      part = std::max(part, (size_t)c.grid * (27 * kWsLayer[l][0] + 1) * kWsLayer[l][1]);
   }
   ws->part_cap = part;
   if (rc == GC_OK && cudaMalloc(&ws->part, part * sizeof(float) + (size_t)(1024 * 128 + 1024 + 16) * sizeof(float) +
@@ -1407,6 +1711,8 @@ extern "C" int gc_ws_create(gc_ws **out, int R) {
     if (cudaFuncSetAttribute(k_conv_march, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM_MAX) !=
             cudaSuccess ||
         cudaFuncSetAttribute(k_conv_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM_MAX) != cudaSuccess ||
+        cudaFuncSetAttribute(k_wgrad_strip, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM_MAX) !=
+            cudaSuccess ||
         cudaFuncSetAttribute(k_conv_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM_MAX) !=
             cudaSuccess)
       fail("shared memory attribute");
@@ -1667,7 +1973,7 @@ extern "C" int gc_ws_plan_info(const gc_ws *ws, int layer, int kind, int *out) {
   if (!ws || !out || layer < 0 || layer >= WS_NL || kind < 0 || kind > 2) return GC_ERR_ARG;
   if (kind == 2) {
     const WgPlan &p = ws->pw[layer];
-    out[0] = p.BZ; out[1] = p.BY; out[2] = p.tpp; out[3] = p.grid; out[4] = 0;
+    out[0] = p.BZ; out[1] = p.BY; out[2] = p.tpp; out[3] = p.grid * p.groups; out[4] = 0;
   } else {
     const FwdPlan &p = kind == 0 ? ws->pf[layer] : ws->pb[layer];
     out[0] = p.BZ; out[1] = p.BY; out[2] = p.tpg; out[3] = p.grid * ws_cout(layer, kind) / p.Cn; out[4] = p.n_mt;
