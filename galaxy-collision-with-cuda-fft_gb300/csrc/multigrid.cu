@@ -164,9 +164,10 @@ void gc_mg_free(gc_ctx *ctx) {
 // ------------------------------------------------------------------------------
 // Sum nparts rows of nv partials into dst[0..nv), deterministically (a fixed
 // association for given nparts and nv). FP64 runs at a small fraction of the
-// f32 rate on this GPU, so the adds are spread: warp w of one block sums value
-// w (lanes take rows lane, lane + 32, ...); a long single-value list is first
-// cut into GC_FIN_CHUNKS contiguous chunks summed by as many blocks.
+// f32 rate on this GPU (16 clk an SM for a warp's addition), so the adds are spread:
+// warp w of one block sums value w (lanes take rows lane, lane + 32, ...); a single
+// value takes one block of 256 threads, and a long list is first cut into
+// GC_FIN_CHUNKS contiguous chunks summed by as many blocks.
 #define GC_FIN_NV 32
 #define GC_FIN_CHUNKS 128
 __global__ void __launch_bounds__(1024)
@@ -174,9 +175,69 @@ __global__ void __launch_bounds__(1024)
   const int lane = threadIdx.x & 31, v = threadIdx.x >> 5;
   if (v >= nv) return;
   double s = 0.0;
+#pragma unroll 8
   for (int i = lane; i < nparts; i += 32) s += parts[(size_t)i * nv + v];
   for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
   if (lane == 0) dst[v] = s;
+}
+
+// The stopping rule of a device-decided solve (the host loop of gc_mg_run), evaluated
+// where the residual's norm is finished (on = 0: the sum alone): the cycle count lives in
+// dsmall[GC_S_CYCLES]; the loop continues while fewer than max_c cycles ran and not (at
+// least max(1, min_c) cycles ran and ||r|| < tol ||b|| with ||b|| > 0). The verdict goes
+// to the conditional node that repeats the V-cycle body, the converged flag to
+// dsmall[GC_S_CONVERGED].
+struct MgDecide {
+  cudaGraphConditionalHandle h;
+  double tol;
+  int on, min_c, max_c, first, count;
+};
+
+__device__ __forceinline__ void mg_decide(const MgDecide &d, double *__restrict__ small, double r2) {
+  const int c = d.first ? 0 : (int)small[GC_S_CYCLES] + 1;
+  const double b2 = small[GC_S_BNORM2];
+  small[GC_S_CYCLES] = (double)c;
+  const int minc = d.min_c > 1 ? d.min_c : 1;
+  const bool conv = c >= minc && b2 > 0.0 && sqrt(r2) < d.tol * sqrt(b2);
+  small[GC_S_CONVERGED] = conv ? 1.0 : 0.0;
+  const bool more = !conv && c < d.max_c;
+  if (!more && d.count) {  // the solve ends here: count it
+    small[GC_S_SOLVES] += 1.0;
+    small[GC_S_CYC_TOTAL] += (double)c;
+    const double rel2 = b2 > 0.0 ? r2 / b2 : 0.0;
+    if (rel2 > small[GC_S_MAXREL2]) small[GC_S_MAXREL2] = rel2;
+  }
+  cudaGraphSetConditional(d.h, more ? 1u : 0u);
+}
+
+// One value: 256 threads with up to 16 loads in flight each, then the stopping rule in
+// the same launch. Latency is all there is: one warp over 2048 partials took 5.3 us and
+// the rule another launch of 2.5 (64^3, one V-cycle of 90 us); together here 4.5 (97^3:
+// 9.2 + 2.7 -> 4.9). Loading the rule's operands ahead and sparing its square roots
+// changed nothing.
+__global__ void __launch_bounds__(256)
+    k_fin_one(const double *__restrict__ parts, int nparts, double *__restrict__ dst, double *__restrict__ small,
+              const __grid_constant__ MgDecide d) {
+  __shared__ double sh[8];
+  const int tid = threadIdx.x;
+  double x[4] = {0.0, 0.0, 0.0, 0.0};
+  for (int i0 = tid; i0 < nparts; i0 += 4096) {
+    double v[16];
+#pragma unroll
+    for (int u = 0; u < 16; ++u) v[u] = i0 + 256 * u < nparts ? __ldcg(parts + i0 + 256 * u) : 0.0;
+#pragma unroll
+    for (int u = 0; u < 16; ++u)
+      if (256 * u < nparts) x[u & 3] += v[u];
+  }
+  double s = (x[0] + x[1]) + (x[2] + x[3]);
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) s += __shfl_down_sync(0xffffffffu, s, o);
+  if ((tid & 31) == 0) sh[tid >> 5] = s;
+  __syncthreads();
+  if (tid != 0) return;
+  const double r = ((sh[0] + sh[1]) + (sh[2] + sh[3])) + ((sh[4] + sh[5]) + (sh[6] + sh[7]));
+  *dst = r;
+  if (d.on) mg_decide(d, small, r);
 }
 
 __global__ void __launch_bounds__(256)
@@ -2187,33 +2248,6 @@ __global__ void __launch_bounds__(256) k_zero_interior(float *__restrict__ a, in
 }
 
 // ------------------------------------------------------------------------------
-// device-side stopping rule of the adaptive loop (graph-captured solves)
-// ------------------------------------------------------------------------------
-// The host loop of gc_mg_run, evaluated on the device after every residual: the
-// cycle count lives in dsmall[GC_S_CYCLES]; the loop continues while fewer than
-// max_cycles cycles ran and not (at least max(1, min_cycles) cycles ran and
-// ||r|| < tol ||b|| with ||b|| > 0). The verdict goes to the conditional node
-// that repeats the V-cycle body, the converged flag to dsmall[GC_S_CONVERGED].
-__global__ void k_mg_decide(cudaGraphConditionalHandle h, double *__restrict__ small, double tol, int min_c,
-                            int max_c, int first, int count) {
-  if (threadIdx.x != 0) return;
-  const int c = first ? 0 : (int)small[GC_S_CYCLES] + 1;
-  small[GC_S_CYCLES] = (double)c;
-  const double b2 = small[GC_S_BNORM2], r2 = small[GC_S_RNORM2];
-  const int minc = min_c > 1 ? min_c : 1;
-  const bool conv = c >= minc && b2 > 0.0 && sqrt(r2) < tol * sqrt(b2);
-  small[GC_S_CONVERGED] = conv ? 1.0 : 0.0;
-  const bool more = !conv && c < max_c;
-  if (!more && count) {  // the solve ends here: count it
-    small[GC_S_SOLVES] += 1.0;
-    small[GC_S_CYC_TOTAL] += (double)c;
-    const double rel2 = b2 > 0.0 ? r2 / b2 : 0.0;
-    if (rel2 > small[GC_S_MAXREL2]) small[GC_S_MAXREL2] = rel2;
-  }
-  cudaGraphSetConditional(h, more ? 1u : 0u);
-}
-
-// ------------------------------------------------------------------------------
 // host orchestration
 // ------------------------------------------------------------------------------
 static dim3 rb_grid(const LevelGeom &g) {
@@ -2254,7 +2288,7 @@ static int launch_tail(gc_ctx *ctx, const gc_mg_params *p) {
   return GC_OK;
 }
 
-static int finalize_to(gc_ctx *ctx, int nparts, int nv, int slot);
+static int finalize_to(gc_ctx *ctx, int nparts, int slot, const MgDecide *dec = nullptr);
 
 static Split0 split0(const gc_ctx *ctx) {
   Split0 d;
@@ -2425,7 +2459,7 @@ static int coarse_levels(gc_ctx *ctx, const gc_mg_params *p) {
 // r = b0 - L phi on the finest interior (colour-split, or natural for the
 // validation path), with ||r||^2 into dsmall[GC_S_RNORM2] (async). The split
 // path also writes the first red half-sweep of the next pre-smoothing.
-static int residual0(gc_ctx *ctx, const gc_mg_params *p) {
+static int residual0(gc_ctx *ctx, const gc_mg_params *p, const MgDecide *dec) {
   const LevelGeom &g0 = ctx->lev[0];
   const dim3 grid = node_grid(g0);
   const size_t nb = (size_t)grid.x * grid.y * grid.z;
@@ -2447,20 +2481,20 @@ static int residual0(gc_ctx *ctx, const gc_mg_params *p) {
     GC_LAUNCH_CHECK(ctx, "resid0");
     // (a last-block sum of the 16k block partials in this kernel was slower: the
     // blocks' tickets serialise on one counter)
-    return finalize_to(ctx, (int)nq, 1, GC_S_RNORM2);
+    return finalize_to(ctx, (int)nq, GC_S_RNORM2, dec);
   }
   auto k = natural ? (plain ? k_resid0<true, false> : k_resid0<false, false>)
                    : (plain ? k_resid0<true, true> : k_resid0<false, true>);
   gc_launch(ctx, GK_RESID0, k, grid, dim3(32, 8), 0, ctx->hi, ctx->lo, ctx->b0, r, ef, ctx->red, d);
   GC_LAUNCH_CHECK(ctx, "resid0");
-  return finalize_to(ctx, (int)nb, 1, GC_S_RNORM2);
+  return finalize_to(ctx, (int)nb, GC_S_RNORM2, dec);
 }
 
 // One V-cycle of the defect correction: relax L e = r from e = 0 (FP32,
 // colour-split), restrict its residual, coarse correction, prolong, relax, then
 // phi += e and the new residual r = b0 - L phi with its norm. Expects r (and,
 // when pre-smoothing, the first red half-sweep) from the previous residual0.
-static int vcycle(gc_ctx *ctx, const gc_mg_params *p) {
+static int vcycle(gc_ctx *ctx, const gc_mg_params *p, const MgDecide *dec) {
   const int L = ctx->nlev;
   if (L == 0) return GC_OK;
   const bool plain = (p->flags & GC_MG_PLAIN_F32) != 0;
@@ -2492,20 +2526,20 @@ static int vcycle(gc_ctx *ctx, const gc_mg_params *p) {
       gc_launch(ctx, GK_UPDATE0, k_update0<false, false>, node_grid(g0), dim3(32, 8), 0, (const float *)ctx->e0n,
                 ctx->hi, ctx->lo, d);
     GC_LAUNCH_CHECK(ctx, "natural cycle");
-    return residual0(ctx, p);
+    return residual0(ctx, p, dec);
   }
   if (finest_blocks(ctx, p)) {
     if ((st = block_down(ctx, GK_SMOOTH0, pre, ctx->e0n, ctx->r0n, g0, ctx->b[1], ctx->lev[1]))) return st;
     if ((st = coarse_levels(ctx, p))) return st;
     st = plain ? block_up<2>(ctx, GK_UPDATE0, post, ctx->e[1], ctx->lev[1], ctx->e0n, ctx->r0n, g0, nullptr)
                : block_up<1>(ctx, GK_UPDATE0, post, ctx->e[1], ctx->lev[1], ctx->e0n, ctx->r0n, g0, nullptr);
-    return st ? st : residual0(ctx, p);
+    return st ? st : residual0(ctx, p, dec);
   }
   if (finest_planes(ctx, p)) {
     if ((st = fine_down(ctx))) return st;
     if ((st = coarse_levels(ctx, p))) return st;
     st = plain ? fine_up<true>(ctx) : fine_up<false>(ctx);
-    return st ? st : residual0(ctx, p);
+    return st ? st : residual0(ctx, p, dec);
   }
   const dim3 sg = split_grid(ctx), sg2 = split_grid2(ctx), qg = quad_grid(ctx);
   const bool v4 = vec4(ctx);
@@ -2560,24 +2594,34 @@ static int vcycle(gc_ctx *ctx, const gc_mg_params *p) {
                 ctx->hi, ctx->lo, d);
   }
   GC_LAUNCH_CHECK(ctx, "finest cycle");
-  return residual0(ctx, p);
+  return residual0(ctx, p, dec);
 }
 
-int gc_finalize(gc_ctx *ctx, const double *parts, int nparts, int nv, double *dst) {
-  GC_REQUIRE(ctx, nv >= 1 && nv <= GC_FIN_NV, "gc_finalize: %d values per row (at most %d)", nv, GC_FIN_NV);
-  if (nv == 1 && nparts > 32 * GC_FIN_CHUNKS) {
+// One value, with the stopping rule where `dec` asks for it.
+static int finalize_one(gc_ctx *ctx, const double *parts, int nparts, double *dst, const MgDecide *dec) {
+  MgDecide d = {};
+  if (dec) d = *dec;
+  if (nparts > 32 * GC_FIN_CHUNKS) {
     double *tmp = ctx->dsmall + GC_S_FIN_TMP;
     gc_launch(ctx, GK_REDUCE, k_fin_chunks, dim3(GC_FIN_CHUNKS), dim3(256), 0, parts, nparts, tmp);
-    gc_launch(ctx, GK_REDUCE, k_fin_warps, dim3(1), dim3(32), 0, (const double *)tmp, GC_FIN_CHUNKS, 1, dst);
-  } else {
-    gc_launch(ctx, GK_REDUCE, k_fin_warps, dim3(1), dim3(32 * nv), 0, parts, nparts, nv, dst);
+    parts = tmp;
+    nparts = GC_FIN_CHUNKS;
   }
+  gc_launch(ctx, GK_REDUCE, k_fin_one, dim3(1), dim3(256), 0, parts, nparts, dst, ctx->dsmall, d);
   GC_LAUNCH_CHECK(ctx, "finalize");
   return GC_OK;
 }
 
-static int finalize_to(gc_ctx *ctx, int nparts, int nv, int slot) {
-  return gc_finalize(ctx, ctx->red, nparts, nv, ctx->dsmall + slot);
+int gc_finalize(gc_ctx *ctx, const double *parts, int nparts, int nv, double *dst) {
+  GC_REQUIRE(ctx, nv >= 1 && nv <= GC_FIN_NV, "gc_finalize: %d values per row (at most %d)", nv, GC_FIN_NV);
+  if (nv == 1) return finalize_one(ctx, parts, nparts, dst, nullptr);
+  gc_launch(ctx, GK_REDUCE, k_fin_warps, dim3(1), dim3(32 * nv), 0, parts, nparts, nv, dst);
+  GC_LAUNCH_CHECK(ctx, "finalize");
+  return GC_OK;
+}
+
+static int finalize_to(gc_ctx *ctx, int nparts, int slot, const MgDecide *dec) {
+  return finalize_one(ctx, ctx->red, nparts, ctx->dsmall + slot, dec);
 }
 
 static int read_small(gc_ctx *ctx, int slot, int count) {
@@ -2595,15 +2639,14 @@ int gc_faces_from_moments(gc_ctx *ctx) {
 }
 
 // The adaptive loop inside a stream capture: the residual of the initial guess
-// and the first decision, then a conditional while node whose body (captured on
-// the context's side stream) is one V-cycle, its residual and the next decision.
+// with the first decision, then a conditional while node whose body (captured on
+// the context's side stream) is one V-cycle and its residual with the next decision.
 // Same kernels in the same order as the host loop, so the same potential. The
 // cycle count, the converged flag and both norms are left in dsmall and copied
 // to the pinned host mirror at the end.
 static int mg_run_captured(gc_ctx *ctx, const gc_mg_params *p, int count) {
   int s;
   if (ctx->nlev == 0) return GC_OK;
-  if ((s = residual0(ctx, p))) return s;
   cudaStreamCaptureStatus cs;
   cudaGraph_t graph = nullptr;
   const cudaGraphNode_t *deps = nullptr;
@@ -2612,9 +2655,9 @@ static int mg_run_captured(gc_ctx *ctx, const gc_mg_params *p, int count) {
   GC_REQUIRE(ctx, cs == cudaStreamCaptureStatusActive, "captured solve outside a stream capture");
   cudaGraphConditionalHandle h;
   GC_CUDA(ctx, cudaGraphConditionalHandleCreate(&h, graph, 0, 0));
-  gc_launch(ctx, GK_REDUCE, k_mg_decide, dim3(1), dim3(32), 0, h, ctx->dsmall, p->tol, p->min_cycles, p->max_cycles, 1,
-            count);
-  GC_LAUNCH_CHECK(ctx, "decide");
+  MgDecide dec = {h, p->tol, 1, p->min_cycles, p->max_cycles, 1, count};
+  if ((s = residual0(ctx, p, &dec))) return s;
+  dec.first = 0;
   GC_CUDA(ctx, cudaStreamGetCaptureInfo(ctx->stream, &cs, nullptr, &graph, &deps, nullptr, &nd));
   cudaGraphNodeParams np = {};
   np.type = cudaGraphNodeTypeConditional;
@@ -2630,12 +2673,7 @@ static int mg_run_captured(gc_ctx *ctx, const gc_mg_params *p, int count) {
   const long long before = gc_launch_total(ctx);
   long long at[GK_COUNT];
   memcpy(at, ctx->prof.launches, sizeof(at));
-  s = vcycle(ctx, p);
-  if (!s) {
-    gc_launch(ctx, GK_REDUCE, k_mg_decide, dim3(1), dim3(32), 0, h, ctx->dsmall, p->tol, p->min_cycles,
-              p->max_cycles, 0, count);
-    s = gc_check_launch(ctx, "decide");
-  }
+  s = vcycle(ctx, p, &dec);
   ctx->cap_body_launches = gc_launch_total(ctx) - before;
   for (int k = 0; k < GK_COUNT; ++k) ctx->cap_body[k] = (int)(ctx->prof.launches[k] - at[k]);
   cudaGraph_t got = nullptr;
@@ -2750,13 +2788,13 @@ int gc_mg_run(gc_ctx *ctx, const gc_mg_params *p, gc_mg_stats *stats) {
     if (stats) *stats = st;
     return GC_OK;
   }
-  if (ctx->nlev > 0 && (s = residual0(ctx, p))) return s;
+  if (ctx->nlev > 0 && (s = residual0(ctx, p, nullptr))) return s;
   if (p->flags & GC_MG_FIXED_CYCLES) {
     // exactly max_cycles V-cycles and no host read: the residual norm is left on
     // the device (gc_pm_last_residual reads it), so the solve can be captured in
     // a CUDA graph
     for (int c = 0; c < p->max_cycles && ctx->nlev > 0; ++c)
-      if ((s = vcycle(ctx, p))) return s;
+      if ((s = vcycle(ctx, p, nullptr))) return s;
     // ||b0||^2 and ||r0||^2 (slots 0 and 1) to the pinned host mirror, stream
     // ordered: after a synchronisation the caller reads them without a copy
     GC_CUDA(ctx, cudaMemcpyAsync(ctx->hsmall, ctx->dsmall, 2 * sizeof(double), cudaMemcpyDeviceToHost, ctx->stream));
@@ -2786,7 +2824,7 @@ int gc_mg_run(gc_ctx *ctx, const gc_mg_params *p, gc_mg_stats *stats) {
         break;
       }
       if (c >= p->max_cycles) break;
-      if ((s = vcycle(ctx, p))) return s;
+      if ((s = vcycle(ctx, p, nullptr))) return s;
       ++c;
       if ((s = read_small(ctx, GC_S_RNORM2, 1))) return s;
       rnorm = sqrt(ctx->hsmall[GC_S_RNORM2]);
@@ -2897,7 +2935,7 @@ extern "C" int gc_mg_residual_norm(gc_ctx *ctx, const float *phi_f32, double *ou
   else
     gc_launch(ctx, GK_RESID64, k_resid64, dim3(grid), dim3(dim3(32, 8)), 0, ctx->hi, ctx->lo, ctx->b0, ctx->red, ctx->G);
   GC_LAUNCH_CHECK(ctx, "resid64");
-  if ((s = finalize_to(ctx, (int)nb, 1, GC_S_RNORM64))) return s;
+  if ((s = finalize_to(ctx, (int)nb, GC_S_RNORM64))) return s;
   if ((s = read_small(ctx, GC_S_RNORM64, 1))) return s;
   *out = sqrt(ctx->hsmall[GC_S_RNORM64]) / (ctx->dx * ctx->dx);
   return GC_OK;
