@@ -43,6 +43,7 @@ enum {
   GC_S_CYC_TOTAL = 15, // ... their V-cycles ...
   GC_S_MAXREL2 = 16, // ... and the largest (||r|| / ||b||)^2 they ended with
   GC_S_TICKET = 17,  // block ticket of the last-block grid reductions (an unsigned, 0 between them)
+  GC_S_LIMBS = 64,   // [64, 94): integer limbs of the moments of k_convert_q (0 between calls)
   GC_S_FIN_TMP = 128, // [128, 256): chunk partials of gc_finalize
   GC_S_NSLOTS = 256
 };
@@ -375,16 +376,17 @@ __device__ __forceinline__ void block_sum_f32(float v, double *out) {
 // the nparts rows in a fixed order, writes the NV sums to dst[v] and resets
 // the ticket to 0, so the sums do not depend on which block finishes last and
 // no second launch is needed. Thread t adds value v = t mod NV of the rows
-// g, g + P, ... (g = t / NV, P = T / NV threads per value) into eight
-// accumulators; a warp per value then adds the P partials in order. Returns
-// true in the last block.
+// g, g + P, ... (g = t / NV) with 16 loads in flight; one thread per value then adds the
+// P partials. FP64 additions bound it: one takes its quarter of the SM 64 clk a warp,
+// whichever lanes take part. So four warps (P = 128 / NV), a quarter each, with their
+// lanes packed and no shuffles (the moments of a density at 97^3: 14.9 us from nine
+// warps with a warp of shuffles per value, 14.6 so). Returns true in the last block.
 template <int NV>
 __device__ bool grid_finish_sum(const double *parts, unsigned nparts, unsigned *ticket, double *dst) {
   __shared__ bool last_s;
-  __shared__ double part_s[1024];
+  __shared__ double part_s[128];
   const int tid = threadIdx.x + blockDim.x * (threadIdx.y + blockDim.y * threadIdx.z);
   const int nthr = blockDim.x * blockDim.y * blockDim.z;
-  const int lane = tid & 31, wid = tid >> 5, nw = (nthr + 31) >> 5;
   __syncthreads();
   if (tid == 0) {
     __threadfence();  // this block's partials (written by thread 0) before its ticket
@@ -393,24 +395,27 @@ __device__ bool grid_finish_sum(const double *parts, unsigned nparts, unsigned *
   __syncthreads();
   if (!last_s) return false;
   __threadfence();  // every other block's partials after the last ticket
-  const int P = nthr / NV, v = tid % NV, g = tid / NV;
-  double xs[8] = {0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0, 0.0};
+  const int P = (nthr < 128 ? nthr : 128) / NV, v = tid % NV, g = tid / NV;
   if (g < P) {
-    for (unsigned q0 = (unsigned)g; q0 < nparts; q0 += 8u * (unsigned)P) {
+    double xs[4] = {0.0, 0.0, 0.0, 0.0};
+    for (unsigned q0 = (unsigned)g; q0 < nparts; q0 += 16u * (unsigned)P) {
+      double r[16];
 #pragma unroll
-      for (int u = 0; u < 8; ++u) {
+      for (int u = 0; u < 16; ++u) {
         const unsigned q = q0 + (unsigned)u * (unsigned)P;
-        if (q < nparts) xs[u] += __ldcg(parts + (size_t)q * NV + v);
+        r[u] = q < nparts ? __ldcg(parts + (size_t)q * NV + v) : 0.0;
       }
+#pragma unroll
+      for (int u = 0; u < 16; ++u)
+        if (q0 - (unsigned)g + (unsigned)u * (unsigned)P < nparts) xs[u & 3] += r[u];
     }
+    part_s[g * NV + v] = (xs[0] + xs[1]) + (xs[2] + xs[3]);
   }
-  part_s[tid] = ((xs[0] + xs[1]) + (xs[2] + xs[3])) + ((xs[4] + xs[5]) + (xs[6] + xs[7]));
   __syncthreads();
-  for (int vv = wid; vv < NV; vv += nw) {
-    double x = 0.0;
-    for (int gg = lane; gg < P; gg += 32) x += part_s[gg * NV + vv];
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
-    if (lane == 0) dst[vv] = x;
+  if (tid < NV) {
+    double x[4] = {0.0, 0.0, 0.0, 0.0};
+    for (int gg = 0; gg < P; ++gg) x[gg & 3] += part_s[gg * NV + tid];
+    dst[tid] = (x[0] + x[1]) + (x[2] + x[3]);
   }
   if (tid == 0) *ticket = 0u;
   __syncthreads();  // dst complete for every thread of the block
@@ -424,6 +429,7 @@ void gc_mg_free(gc_ctx *ctx);
 void gc_mg_loop_free(gc_ctx *ctx);
 int gc_mg_run(gc_ctx *ctx, const gc_mg_params *p, gc_mg_stats *st);
 int gc_faces_from_moments(gc_ctx *ctx);
+int gc_convert_cpw(int G);
 int gc_finalize(gc_ctx *ctx, const double *parts, int nparts, int nv, double *dst);
 // Sum of m/dx^3 (FP64, deterministic) into dsmall[mass_slot] and the fixed-point
 // exponent E (quantum 2^E, total <= 2^bits quanta) into dsmall[exp_slot].

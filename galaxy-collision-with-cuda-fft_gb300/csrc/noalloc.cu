@@ -45,10 +45,12 @@ __global__ void __launch_bounds__(256)
     k_deposit(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
               const float *__restrict__ m, long long n, DepCtx d, const double *__restrict__ qexp,
               long long *__restrict__ qg, unsigned *__restrict__ status);
-__global__ void __launch_bounds__(256)
-    k_convert_q(long long *__restrict__ qg, int G, double dx, const double *__restrict__ qexp, float *__restrict__ rho,
-                float *__restrict__ b, double bfac, double *__restrict__ parts, unsigned *__restrict__ ticket,
-                double *__restrict__ mom, double *__restrict__ bnorm2);
+#define CQ_THREADS 352
+__global__ void __launch_bounds__(CQ_THREADS, 3)
+    k_convert_q(long long *__restrict__ qg, int G, int cpw, double dx, const double *__restrict__ qexp,
+                float *__restrict__ rho, float *__restrict__ b, double bfac, double *__restrict__ parts,
+                unsigned *__restrict__ ticket, long long *__restrict__ limbs, double *__restrict__ mom,
+                double *__restrict__ bnorm2);
 
 // Layout of the scratch array (byte offsets, each 256-byte aligned).
 #define NA_Q_BYTES ((size_t)GC_NOALLOC_MAX_GRID * GC_NOALLOC_MAX_GRID * GC_NOALLOC_MAX_GRID * 8)
@@ -157,8 +159,10 @@ extern "C" int gc_deposit_cic_noalloc(const float *x, const float *y, const floa
     k_deposit<<<nd, 256, 0, st>>>(x, y, z, m, (long long)n, d, small + 1, q, status);
   }
   // rho from q (q is cleared again by the conversion); the moments land in parts
-  const unsigned nbc = gc_blocks((long long)G * G, 8);
-  k_convert_q<<<nbc, 256, 0, st>>>(q, G, dx, small + 1, rho, nullptr, 1.0, parts, nullptr, nullptr, nullptr);
+  const int cpw = gc_convert_cpw(G);
+  const unsigned nbc = gc_blocks((long long)G * G, 8 * cpw);
+  k_convert_q<<<nbc, CQ_THREADS, 0, st>>>(q, G, cpw, dx, small + 1, rho, nullptr, 1.0, parts, nullptr, nullptr, nullptr,
+                                       nullptr);
   e = cudaGetLastError();
   if (e != cudaSuccess) {
     gc_set_error(nullptr, "gc_deposit_cic_noalloc: launch failed: %s", cudaGetErrorString(e));

@@ -832,102 +832,202 @@ int gc_deposit_q(gc_ctx *ctx, const float *x, const float *y, const float *z, co
 // ------------------------------------------------------------------------------
 // q -> rho / b, zero q, exact integer column moments, ||b||^2
 // ------------------------------------------------------------------------------
-// One warp per (i,j) column, persistent over the columns. Column sums S0 = sum q,
-// S1 = sum q k and S2 = sum q k^2 are exact in integers (S2 split at bit 32),
-// combined across columns in FP64 in a fixed order. Partials per block: 10
-// moments + ||b||^2.
-__global__ void __launch_bounds__(256)
-    k_convert_q(long long *__restrict__ qg, int G, double dx, const double *__restrict__ qexp, float *__restrict__ rho,
-                float *__restrict__ b, double bfac, double *__restrict__ parts, unsigned *__restrict__ ticket,
-                double *__restrict__ mom, double *__restrict__ bnorm2) {
-  __shared__ double wsum[8][11];
+// One warp per (i,j) column, blocks persistent over batches of 8 cpw columns. Column
+// sums S0 = sum q, S1 = sum q k and S2 = sum q k^2 are exact in integers (S2 split at
+// bit 32), and so are the grid's ten moments: each is kept as three limbs (24 bits, 32
+// for S2) that take the columns' products with 1, i, j, i^2, ij, j^2 in 64 bits and are added
+// over blocks by integer atomics; the last block puts the limbs together and rounds
+// once. Block partials of ||b||^2 (FP32 column sums, added in FP64 in a fixed order).
+//
+// FP64 is kept out because an addition takes its quarter of the SM 64 clocks a warp,
+// whichever lanes take part. With every column's terms in FP64 on lane 0 of its warp and
+// 11 x 456 partials for the last block to add, a 64^3 grid took 20 us; with the terms of
+// 32 columns in the lanes of a warp 13, of which 5k clk were the warp's and 9k the
+// last block's additions; in integers 8 (100^3: 19 -> 12; 128^3: 24 -> 14; at 256^3,
+// 47 -> 39, the grid's bytes are what is left). Three warps beside the eight that walk
+// columns take a lane per column of a batch, while the eight go on to the next.
+#define CQ_THREADS 352
+struct CqCol {
+  long long s0, s1, s2h;
+  unsigned long long s2l;
+  float bb;
+};
+
+// l0 + l1 2^r1 + l2 2^r2 of a sum of limbs, rounded once.
+__device__ __forceinline__ double limbs_to_double(long long l0, long long l1, long long l2, int r1, int r2) {
+  __int128 v = (__int128)l0 + ((__int128)l1 << r1) + ((__int128)l2 << r2);
+  const bool neg = v < 0;
+  if (neg) v = -v;
+  unsigned long long hi = (unsigned long long)(v >> 64), lo = (unsigned long long)v;
+  double d;
+  if (hi == 0) {
+    d = __ull2double_rn(lo);
+  } else {  // 64 leading bits, the rest as a sticky bit below them
+    const int z = __clzll((long long)hi);
+    unsigned long long top = z ? (hi << z) | (lo >> (64 - z)) : hi;
+    if (z ? (lo << z) != 0 : lo != 0) top |= 1ull;
+    d = ldexp(__ull2double_rn(top), 64 - z);
+  }
+  return neg ? -d : d;
+}
+
+__global__ void __launch_bounds__(CQ_THREADS, 3)
+    k_convert_q(long long *__restrict__ qg, int G, int cpw, double dx, const double *__restrict__ qexp,
+                float *__restrict__ rho, float *__restrict__ b, double bfac, double *__restrict__ parts,
+                unsigned *__restrict__ ticket, long long *__restrict__ limbs, double *__restrict__ mom,
+                double *__restrict__ bnorm2) {
+  __shared__ CqCol cols[2][32];
+  __shared__ long long red[3][12][33];
+  __shared__ double bsum[4];
+  __shared__ bool last_s;
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int E = (int)(*qexp);
   const float qinv = ldexpf(1.0f, E);
   const float bscale = (float)(ldexp(1.0, E) * bfac);
-  const double msc = ldexp(1.0, E) * dx * dx * dx;  // mass of one quantum
-  double v[11];
+  const int ncols = G * G, batch = 8 * cpw;
+  // limbs of the warp's moments (warps 8, 9, 10), a column of `red` per lane: in registers
+  // they would be live in the other warps too
+  if (wid >= 8) {
+    for (int t = 0; t < 12; ++t) red[wid - 8][t][lane] = 0;
+  }
+  double bacc = 0.0;
+  int buf = 0;
+  for (int base = blockIdx.x * batch; base < ncols; base += gridDim.x * batch, buf ^= 1) {
+    if (wid < 8) {
+      for (int c = 0; c < cpw; ++c) {
+        const int col = base + 8 * c + wid;
+        if (col >= ncols) break;
+        long long *p = qg + (size_t)col * G;
+        float *rp = rho ? rho + (size_t)col * G : nullptr;
+        float *bp = b ? b + (size_t)col * G : nullptr;
+        long long S0 = 0, S1 = 0, S2h = 0;
+        unsigned long long S2l = 0;
+        float bb = 0.0f;
+        bool some = false;
+        for (int k0 = 0; k0 < G; k0 += 32 * 8) {
+          long long qv[8];
+          bool nz = false;
 #pragma unroll
-  for (int t = 0; t < 11; ++t) v[t] = 0.0;
-  const long long ncols = (long long)G * G;
-  for (long long col = (long long)blockIdx.x * 8 + wid; col < ncols; col += (long long)gridDim.x * 8) {
-    const int i = (int)(col / G), j = (int)(col - (long long)i * G);
-    long long *p = qg + (size_t)col * G;
-    float *rp = rho ? rho + (size_t)col * G : nullptr;
-    float *bp = b ? b + (size_t)col * G : nullptr;
-    long long S0 = 0, S1 = 0, S2h = 0;
-    unsigned long long S2l = 0;
-    float bb = 0.0f;
-    for (int k0 = 0; k0 < G; k0 += 32 * 8) {
-      long long qv[8];
-      bool nz = false;
+          for (int t = 0; t < 8; ++t) {  // all loads of the lane in flight together
+            const int k = k0 + 32 * t + lane;
+            qv[t] = k < G ? p[k] : 0;
+            nz |= qv[t] != 0;
+          }
+          if (!__any_sync(0xffffffffu, nz)) {  // an empty stretch (most of a disk's box): zeros out, q stays 0
 #pragma unroll
-      for (int t = 0; t < 8; ++t) {  // all loads of the lane in flight together
-        const int k = k0 + 32 * t + lane;
-        qv[t] = k < G ? p[k] : 0;
-        nz |= qv[t] != 0;
-      }
-      if (!__any_sync(0xffffffffu, nz)) {  // an empty stretch (most of a disk's box): zeros out, q stays 0
+            for (int t = 0; t < 8; ++t) {
+              const int k = k0 + 32 * t + lane;
+              if (k >= G) continue;
+              if (rp) rp[k] = 0.0f;
+              if (bp) bp[k] = 0.0f;
+            }
+            continue;
+          }
+          some = true;
 #pragma unroll
-        for (int t = 0; t < 8; ++t) {
-          const int k = k0 + 32 * t + lane;
-          if (k >= G) continue;
-          if (rp) rp[k] = 0.0f;
-          if (bp) bp[k] = 0.0f;
+          for (int t = 0; t < 8; ++t) {
+            const int k = k0 + 32 * t + lane;
+            if (k >= G) continue;
+            if (qv[t] != 0) p[k] = 0;  // clear for the next deposit (zeros need no store)
+            const float qf = i64_to_f32_rn(qv[t]);  // one rounding, as (float)q
+            if (rp) rp[k] = __fmul_rn(qf, qinv);
+            const float bv = __fmul_rn(qf, bscale);
+            if (bp) bp[k] = bv;
+            bb += bv * bv;
+            const long long kk = k;
+            S0 += qv[t];
+            S1 += qv[t] * kk;
+            S2h += (qv[t] >> 32) * (kk * kk);
+            S2l += (unsigned long long)(qv[t] & 0xffffffffLL) * (unsigned long long)(kk * kk);
+          }
         }
-        continue;
-      }
-#pragma unroll
-      for (int t = 0; t < 8; ++t) {
-        const int k = k0 + 32 * t + lane;
-        if (k >= G) continue;
-        if (qv[t] != 0) p[k] = 0;  // clear for the next deposit (zeros need no store)
-        const float qf = i64_to_f32_rn(qv[t]);  // one rounding, as (float)q
-        if (rp) rp[k] = __fmul_rn(qf, qinv);
-        const float bv = __fmul_rn(qf, bscale);
-        if (bp) bp[k] = bv;
-        bb += bv * bv;
-        const long long kk = k;
-        S0 += qv[t];
-        S1 += qv[t] * kk;
-        S2h += (qv[t] >> 32) * (kk * kk);
-        S2l += (unsigned long long)(qv[t] & 0xffffffffLL) * (unsigned long long)(kk * kk);
+        if (some) {  // exact integer warp sums (no FP64 per lane)
+          for (int o = 16; o > 0; o >>= 1) {
+            S0 += __shfl_down_sync(0xffffffffu, S0, o);
+            S1 += __shfl_down_sync(0xffffffffu, S1, o);
+            S2h += __shfl_down_sync(0xffffffffu, S2h, o);
+            S2l += __shfl_down_sync(0xffffffffu, S2l, o);
+            bb += __shfl_down_sync(0xffffffffu, bb, o);
+          }
+        }
+        if (lane == 0) cols[buf][8 * c + wid] = {S0, S1, S2h, S2l, bb};
       }
     }
-    // exact integer warp sums (no FP64 per lane)
-    for (int o = 16; o > 0; o >>= 1) {
-      S0 += __shfl_down_sync(0xffffffffu, S0, o);
-      S1 += __shfl_down_sync(0xffffffffu, S1, o);
-      S2h += __shfl_down_sync(0xffffffffu, S2h, o);
-      S2l += __shfl_down_sync(0xffffffffu, S2l, o);
-      bb += __shfl_down_sync(0xffffffffu, bb, o);
-    }
-    if (lane == 0) v[10] += (double)bb;
-    if (lane == 0 && (S0 | S1 | S2h | (long long)S2l) != 0) {
-      const double d0 = (double)S0, d1 = (double)S1, d2 = (double)S2h * 4294967296.0 + (double)S2l;
-      const double x = i * dx, y = j * dx;
-      const double m0 = d0 * msc, m1 = d1 * msc * dx, m2 = d2 * msc * dx * dx;
-      v[0] += m0; v[1] += m0 * x; v[2] += m0 * y; v[3] += m1;
-      v[4] += m0 * x * x; v[5] += m0 * y * y; v[6] += m2;
-      v[7] += m0 * x * y; v[8] += m1 * x; v[9] += m1 * y;
+    __syncthreads();  // the other buffer is free again two batches on, behind the next barrier
+    if (wid >= 8 && ticket) {
+      const int col = base + lane;
+      if (lane < batch && col < ncols) {
+        const CqCol q = cols[buf][lane];
+        const long long i = col / G, j = col - i * G;
+        // warp 8: M, x, y; warp 9: xx, yy, xy; warp 10: z, xz, yz and zz
+        const long long S = wid == 10 ? q.s1 : q.s0;
+        const long long w0 = wid == 9 ? i * i : 1, w1 = wid == 9 ? j * j : i, w2 = wid == 9 ? i * j : j;
+        const long long a0 = S & 0xffffff, a1 = (S >> 24) & 0xffffff, a2 = S >> 48;
+        long long(*L)[33] = red[wid - 8];
+        L[0][lane] += a0 * w0; L[1][lane] += a1 * w0; L[2][lane] += a2 * w0;
+        L[3][lane] += a0 * w1; L[4][lane] += a1 * w1; L[5][lane] += a2 * w1;
+        L[6][lane] += a0 * w2; L[7][lane] += a1 * w2; L[8][lane] += a2 * w2;
+        if (wid == 10) {
+          L[9][lane] += (long long)(q.s2l & 0xffffffffull);
+          L[10][lane] += (long long)(q.s2l >> 32) + q.s2h;
+        } else if (wid == 8) {
+          bacc += (double)q.bb;
+        }
+      }
     }
   }
-  // lane 0 of each warp holds the warp's totals: sum the 8 warps in order
-  if (lane == 0) {
-#pragma unroll
-    for (int t = 0; t < 11; ++t) wsum[wid][t] = v[t];
+  if (!ticket) return;
+  if (wid >= 8) {
+    __syncwarp();
+    if (lane < (wid == 10 ? 11 : 9)) {
+      long long x = 0;
+#pragma unroll 8
+      for (int l = 0; l < 32; ++l) x += red[wid - 8][lane][l];
+      const int m = lane / 3, v = wid == 8 ? m : (wid == 9 ? (m == 2 ? 7 : 4 + m) : (m == 0 ? 3 : (m == 3 ? 6 : 7 + m)));
+      if (x != 0) atomicAdd((unsigned long long *)(limbs + 3 * v + (lane - 3 * m)), (unsigned long long)x);
+    }
+    if (wid == 8) {
+      for (int o = 16; o > 0; o >>= 1) bacc += __shfl_down_sync(0xffffffffu, bacc, o);
+      if (lane == 0) parts[blockIdx.x] = bacc;
+    }
+    __threadfence();  // before the block's ticket
   }
   __syncthreads();
-  if (threadIdx.x == 0) {  // one writer: the last-block reduction below fences its stores
-#pragma unroll 1
-    for (int t = 0; t < 11; ++t) {
-      double a = 0.0;
-      for (int w = 0; w < 8; ++w) a += wsum[w][t];
-      parts[(size_t)blockIdx.x * 11 + t] = a;
-    }
+  if (threadIdx.x == 256) last_s = atomicAdd(ticket, 1u) == gridDim.x - 1u;
+  __syncthreads();
+  if (!last_s) return;
+  __threadfence();
+  if (wid < 4) {
+    double x = 0.0;
+#pragma unroll 4
+    for (int r = threadIdx.x; r < (int)gridDim.x; r += 128) x += __ldcg(parts + r);
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_down_sync(0xffffffffu, x, o);
+    if (lane == 0) bsum[wid] = x;
   }
-  // the moments and ||b||^2 from the block partials by the last block
-  if (ticket && grid_finish_sum<11>(parts, gridDim.x, ticket, mom) && threadIdx.x == 0) *bnorm2 = mom[10];
+  if (wid == 8) {
+    if (lane < 10) {
+      const long long l0 = __ldcg(limbs + 3 * lane), l1 = __ldcg(limbs + 3 * lane + 1), l2 = __ldcg(limbs + 3 * lane + 2);
+      const double msc = ldexp(1.0, E) * dx * dx * dx;  // mass of one quantum
+      const double s = lane == 0 ? 1.0 : (lane < 4 ? dx : dx * dx);
+      mom[lane] = limbs_to_double(l0, l1, l2, lane == 6 ? 32 : 24, 48) * msc * s;
+    }
+    __syncwarp();
+    if (lane < 30) limbs[lane] = 0;  // for the next call
+  }
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    mom[10] = (bsum[0] + bsum[1]) + (bsum[2] + bsum[3]);
+    *bnorm2 = mom[10];
+    *ticket = 0u;
+  }
+}
+
+// Columns a warp takes per batch: four where that leaves a batch for every SM,
+// else two or one (a small grid is bound by latency, and wants its columns spread).
+int gc_convert_cpw(int G) {
+  int cpw = 4;
+  while (cpw > 1 && (long long)G * G < 8LL * gc_sms() * cpw) cpw >>= 1;
+  return cpw;
 }
 
 int gc_max_fixed_point_bits(const gc_ctx *ctx) {
@@ -939,14 +1039,15 @@ int gc_max_fixed_point_bits(const gc_ctx *ctx) {
 
 int gc_convert_q(gc_ctx *ctx, const double *qexp, float *rho_out, float *b_out) {
   const long long cols = (long long)ctx->G * ctx->G;
-  unsigned nb = gc_blocks(cols, 8);
-  if (nb > gc_sms() * 3u) nb = gc_sms() * 3u;  // persistent: 3 CTAs per SM (80 registers)
+  const int cpw = gc_convert_cpw(ctx->G);
+  unsigned nb = gc_blocks(cols, 8 * cpw);
+  if (nb > gc_sms() * 3u) nb = gc_sms() * 3u;  // persistent: 3 CTAs per SM
   int s = gc_ensure_red(ctx, (size_t)nb * 11);
   if (s) return s;
   const double bfac = 4.0 * M_PI * ctx->grav * ctx->dx * ctx->dx;
-  gc_launch(ctx, GK_CONVERT_Q, k_convert_q, dim3(nb), dim3(256), 0, ctx->q, ctx->G, ctx->dx, qexp, rho_out, b_out,
-            bfac, ctx->red, reinterpret_cast<unsigned *>(ctx->dsmall + GC_S_TICKET), ctx->dmom,
-            ctx->dsmall + GC_S_BNORM2);
+  gc_launch(ctx, GK_CONVERT_Q, k_convert_q, dim3(nb), dim3(CQ_THREADS), 0, ctx->q, ctx->G, cpw, ctx->dx, qexp, rho_out, b_out,
+            bfac, ctx->red, reinterpret_cast<unsigned *>(ctx->dsmall + GC_S_TICKET),
+            reinterpret_cast<long long *>(ctx->dsmall + GC_S_LIMBS), ctx->dmom, ctx->dsmall + GC_S_BNORM2);
   GC_LAUNCH_CHECK(ctx, "convert q");
   return GC_OK;
 }
