@@ -17,6 +17,8 @@
 #define WS_WAIT_BUDGET 2000000000LL
 // Warps whose lane 0 issues tensor-core MMAs (each commits once per phase).
 #define WS_ISSUERS 4
+// Layers of the network.
+#define WS_NL 11
 
 // ------------------------------------------------------------------------------
 // single-tile GEMM check: D (128 x N, f32) = A (128 x K) * B (N x K)^T
@@ -608,379 +610,238 @@ __global__ void __launch_bounds__(MA_THREADS) k_conv_march(const __grid_constant
 // ------------------------------------------------------------------------------
 // weight gradient: dW[t][co][ci] = sum_v gy[v][co] x[v + off_t][ci]
 // ------------------------------------------------------------------------------
-// GEMM with M = co (padded to 128), N = ci, K = voxels. The input tile (with
-// halo) is staged exactly as in the forward pass; read MN-major (8 channels of
-// one voxel per 16-byte row), the B operand of tap t is again the tile shifted
-// by off_t rows. gy arrives in stages of 128 voxels, each voxel's 16-byte rows
-// (8 output channels) placed in 2 KB groups of 8 voxels so that every one of the
-// 128 M rows addresses shared memory of the stage (rows >= Cout are never read
-// back). Voxels outside the CTA's block are zero in gy. Taps are split into
-// passes so that a pass's accumulators (tpp x Cin columns) fit Tensor Memory, one
-// CTA row of the grid per pass; persistent CTAs accumulate over all their blocks and
-// write one partial per CTA, summed in a fixed order afterwards. This form takes lines
-// of any length (levels whose size is not a multiple of 8).
+// GEMM with M = co (64 or 128 rows), N = ci, K = voxels. The voxels are divided into
+// blocks of BZ planes x BY lines x R, and the blocks over `nparts` partial sums (block b
+// to partial b mod nparts), which are added in their order afterwards. Within a partial
+// an accumulator takes its blocks one after another, 16 rows of the padded linear range
+// [L0, L1] at a time: that order is part of the result's bits and is kept whatever runs
+// beside what.
+// A CTA takes the taps of one dz (blockIdx.x = dz and a share of its nine taps; the
+// groups of a partial next to each other, so that the partials with a block more, which
+// come first, start first), so its x
+// tile is the block's BZ planes moved by dz, with the halo in y and x, staged as in the
+// forward pass and as one box; read MN-major (8 channels of one voxel per 16-byte row),
+// the B operand of a tap is again the tile shifted by some rows. gy arrives in stages of 128 rows, each row's 16-byte
+// pieces (8 output channels) placed in groups of 8 rows so that every one of the M rows
+// addresses shared memory of the stage (rows >= Cout are never read back). Rows outside
+// the CTA's block are zero in gy. A CTA (partial, tap group) has warps that fill the
+// ring of stages and at the end read the accumulators out, and warps that issue.
+// With one loop that loaded a stage, synchronised and issued from four threads, M always
+// 128, and the tap groups one after another, 16 -> 16 channels at R = 64 took 103 us and
+// 128 -> 64 at R = 8 145 us; so they take 44 and 7.7.
 struct ConvW {
-  const uint4 *x;    // layer input, Cin channels
-  const uint4 *gy;   // gradient of the pre-activation output, Cout channels
-  float *part;       // [gridDim.x][27][Cout][Cin]
+  CUtensorMap map;  // x: 8-channel rows of x, y, z, chunk; box one tile
+  int use_map;      // the tile's lines fit a box (R <= 126)
+  int sub;          // groups of a dz
+  const uint4 *x;   // layer input, Cin channels
+  const uint4 *gy;  // gradient of the pre-activation output, Cout channels
+  float *part;      // [nparts][27][Cout][Cin]
   unsigned *status;
   int R, Cin, Cout, BZ, BY;
-  int tpp;           // taps per pass
   int nblocks;
+  int tpg;   // taps of a group (dy3 = 0), or dx (dy3 = 1)
+  int dy3;   // N = the three dy taps of one channel chunk (24 columns) instead of Cin
+  int ns;    // stages
   uint32_t tmem_cols;
 };
 
-#define WG_STAGE_ROWS 128
-#define WG_STAGE_BYTES (16 * 2048)
+#define WG_ROWS 128  // rows of a stage
+#define WG_LOAD 8    // warps that load (and read out), then WS_ISSUERS that issue
+#define WG_THREADS (32 * (WG_LOAD + WS_ISSUERS))
+#define WG_MAX_STAGES 8
 
-__global__ void __launch_bounds__(256) k_conv_wgrad(ConvW a) {
+__global__ void __launch_bounds__(WG_THREADS) k_conv_wgrad(const __grid_constant__ ConvW a) {
   extern __shared__ __align__(1024) uint8_t sm[];
-  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const int R = a.R;
+  const int tid = threadIdx.x, lane = tid & 31;
+  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
+  const int R = a.R, ns = a.ns;
   int W2, P, V, L0, L1;
   conv_geom(R, a.BZ, a.BY, W2, P, V, L0, L1);
   const int kci = a.Cin >> 3, kco = a.Cout >> 3;
   const size_t R3 = (size_t)R * R * R;
   const int nby = R / a.BY;
-  const int nst = (L1 - L0 + WG_STAGE_ROWS) / WG_STAGE_ROWS;
-  const uint32_t tile_bytes = (uint32_t)(kci * V + 128) * 16u;
-  uint8_t *tile = sm;
-  uint8_t *stg = sm + ((tile_bytes + 1023u) & ~1023u);
-  uint64_t *bars = reinterpret_cast<uint64_t *>(stg + 2 * WG_STAGE_BYTES);
-  uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 2);
-  if (warp == 0) {
-    umma::tmem_alloc(tslot, a.tmem_cols);
-    umma::tmem_relinquish();
-  }
-  if (tid == 0) {  // one arrival per issuing warp
-    umma::mbar_init(&bars[0], WS_ISSUERS);
-    umma::mbar_init(&bars[1], WS_ISSUERS);
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  umma::tc_fence_before();
-  __syncthreads();
-  umma::tc_fence_after();
-  const uint32_t tmem = *tslot;
-  const uint32_t idesc = umma::idesc_bf16(128, a.Cin, 1, 1);
-  const uint32_t tile_u32 = umma::smem_u32(tile), stg_u32 = umma::smem_u32(stg);
-  uint32_t ph0 = 0u, ph1 = 0u;
-  bool pend0 = false, pend1 = false;
-  bool fail = false;
-  long long gs = 0;  // stages issued by this CTA
-  uint4 *trow = reinterpret_cast<uint4 *>(tile);
-  const int npass = (27 + a.tpp - 1) / a.tpp;
-  for (int pass = blockIdx.y; pass < npass && !fail; pass += gridDim.y) {
-    const int t0 = pass * a.tpp, t1 = min(27, t0 + a.tpp);
-    bool first = true;
-    for (int b = blockIdx.x; b < a.nblocks && !fail; b += gridDim.x) {
-      const int z0 = (b / nby) * a.BZ, y0 = (b % nby) * a.BY;
-      // every MMA reading the previous tile must be complete before it is overwritten
-      if (pend0) { fail |= !umma::mbar_wait(&bars[0], ph0, WS_WAIT_BUDGET); ph0 ^= 1u; pend0 = false; }
-      if (pend1) { fail |= !umma::mbar_wait(&bars[1], ph1, WS_WAIT_BUDGET); ph1 ^= 1u; pend1 = false; }
-      if (__syncthreads_or(fail)) { fail = true; break; }
-      {
-        const int nzy = (a.BZ + 2) * (a.BY + 2), nrows = kci * nzy, nwarps = blockDim.x >> 5;
-        for (int row = warp; row < nrows; row += nwarps) {
-          const int kc = row / nzy, rr = row - kc * nzy;
-          const int tz = rr / (a.BY + 2), ty = rr - tz * (a.BY + 2);
-          const int gz = z0 - 1 + tz, gy_ = y0 - 1 + ty;
-          const bool rowin = (unsigned)gz < (unsigned)R && (unsigned)gy_ < (unsigned)R;
-          const uint4 *src = a.x + (size_t)kc * R3 + ((size_t)(rowin ? gz : 0) * R + (rowin ? gy_ : 0)) * R;
-          uint4 *dst = trow + (size_t)kc * V + (size_t)rr * W2;
-          for (int tx = lane; tx < W2; tx += 32) {
-            const int gx = tx - 1;
-            const bool in = rowin && (unsigned)gx < (unsigned)R;
-            umma::cp_async16(dst + tx, in ? (const void *)(src + gx) : (const void *)a.x, in);
-          }
-        }
-      }
-      for (int i = tid; i < 128; i += blockDim.x) trow[kci * V + i] = make_uint4(0u, 0u, 0u, 0u);
-      for (int st = 0; st < nst; ++st, ++gs) {
-        const int s = (int)(gs & 1);
-        if (s ? pend1 : pend0) {
-          fail |= !umma::mbar_wait(&bars[s], s ? ph1 : ph0, WS_WAIT_BUDGET);
-          if (s) { ph1 ^= 1u; pend1 = false; } else { ph0 ^= 1u; pend0 = false; }
-        }
-        if (__syncthreads_or(fail)) { fail = true; break; }
-        const int Ls = L0 + WG_STAGE_ROWS * st;
-        uint8_t *sbuf = stg + s * WG_STAGE_BYTES;
-        for (int i = tid; i < WG_STAGE_ROWS * kco; i += blockDim.x) {
-          const int r = i % WG_STAGE_ROWS, c = i / WG_STAGE_ROWS;
-          const int L = Ls + r;
-          const int tz = L / P, rem = L - tz * P, ty = rem / W2, tx = rem - ty * W2;
-          const bool valid = L <= L1 && tz >= 1 && tz <= a.BZ && ty >= 1 && ty <= a.BY && tx >= 1 && tx <= R;
-          const uint4 *src =
-              valid ? a.gy + (size_t)c * R3 + ((size_t)(z0 + tz - 1) * R + (y0 + ty - 1)) * R + (tx - 1) : a.gy;
-          umma::cp_async16(sbuf + (r >> 3) * 2048 + c * 128 + (r & 7) * 16, src, valid);
-        }
-        umma::cp_async_wait_all();
-        umma::fence_async_smem();
-        __syncthreads();
-        if (lane == 0 && warp < WS_ISSUERS) {  // issuer w owns the taps t0 + w (mod WS_ISSUERS)
-          umma::tc_fence_after();
-          const uint64_t ad0 = umma::sdesc_mn(stg_u32 + (uint32_t)s * WG_STAGE_BYTES, 2048u, 128u);
-          const uint64_t bd0 = umma::sdesc_mn(tile_u32, 128u, (uint32_t)V * 16u);
-          for (int t = t0 + warp; t < t1; t += WS_ISSUERS) {
-            const int off = tap_offset(t, P, W2);
-            for (int ks = 0; ks < WG_STAGE_ROWS / 16; ++ks) {
-              umma::mma_bf16(tmem + (uint32_t)((t - t0) * a.Cin), ad0 + (uint32_t)ks * 256u,
-                             bd0 + (uint32_t)(Ls + 16 * ks + off), idesc, (first && ks == 0) ? 0u : 1u);
-            }
-          }
-          umma::mma_commit(&bars[s]);
-        }
-        if (s) pend1 = true; else pend0 = true;
-        first = false;
-      }
-    }
-    // pass complete: drain, then read the accumulators out
-    if (pend0) { fail |= !umma::mbar_wait(&bars[0], ph0, WS_WAIT_BUDGET); ph0 ^= 1u; pend0 = false; }
-    if (pend1) { fail |= !umma::mbar_wait(&bars[1], ph1, WS_WAIT_BUDGET); ph1 ^= 1u; pend1 = false; }
-    fail = __syncthreads_or(fail);
-    umma::tc_fence_after();
-    if (!fail) {
-      const int quad = warp & 3;
-      const int co = 32 * quad + lane;
-      for (int t = t0 + (warp >> 2); t < t1; t += (blockDim.x >> 7)) {
-        if (32 * quad >= a.Cout) continue;  // whole warp idle: rows beyond Cout
-        for (int c = 0; c < a.Cin; c += 16) {
-          uint32_t r[16];
-          umma::tmem_ld16(tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)((t - t0) * a.Cin + c), r);
-          umma::tmem_wait_ld();
-          if (co < a.Cout) {
-            float *dst = a.part + (((size_t)blockIdx.x * 27 + t) * a.Cout + co) * a.Cin + c;
-#pragma unroll
-            for (int j = 0; j < 16; ++j) dst[j] = first ? 0.0f : __uint_as_float(r[j]);
-          }
-        }
-      }
-    }
-    umma::tc_fence_before();
-    __syncthreads();
-  }
-  if (fail) {
-    if (pend0) umma::mbar_wait(&bars[0], ph0, WS_WAIT_BUDGET);
-    if (pend1) umma::mbar_wait(&bars[1], ph1, WS_WAIT_BUDGET);
-    if (tid == 0) atomicOr(a.status, 1u);
-  }
-  umma::tc_fence_before();
-  __syncthreads();
-  if (warp == 0) umma::tmem_dealloc(tmem, a.tmem_cols);
-}
-
-// ------------------------------------------------------------------------------
-// the same weight gradient with taps in the rows and columns of one product
-// ------------------------------------------------------------------------------
-// Both operands lie in shared memory as rows of 8 channels, so a group of 8 M (or N)
-// indices is named by an address and the next group by a constant distance. With x
-// stored [line][chunk][x], groups one line-and-chunk row apart run over (dy, chunk): one
-// MMA gives the three dy taps at once (N = 3 Cin). With gy of three planes stored
-// [line][plane][chunk][x], its groups run over (dz, chunk) (M = 3 Cout, where that is at
-// most 128 rows). The 27 taps are then 3 MMAs per 16 voxels, one per dx, instead of 27,
-// each with Cout of 128 rows in use. K runs over the voxels of the strip alone, so no
-// halo row is multiplied. Cases, by channels:
-//   mz = 3 (Cout <= 40): rows (dz, co), gy planes z - 1 .. z + 1 beside x plane z;
-//   mz = 1: rows co, one gy plane z - dz, dz by CTA group;
-//   ndx = 3 where 3 accumulators of 3 Cin columns fit Tensor Memory, else dx by CTA
-//   group; 3 Cin > 256 columns (Cin = 128): one MMA per dy.
-// A CTA (split, group) goes over its share of the units (strip, plane) with a ring of
-// stages, one box each of x and gy, and writes one partial. The bias gradient is summed
-// from the staged gy by the warps that read the accumulators out at the end.
-// An MMA of 64 x 48 x 16 takes 29 clk here, of 128 x 96 x 16 57, of 128 x 192 x 16 97.
-struct ConvWS {
-  CUtensorMap mx;  // x: rows of x, chunk, y, z
-  CUtensorMap mg;  // gy: rows of x, chunk, z, y
-  float *part;     // [gridDim.x][27 Cout Cin weights, Cout biases]
-  unsigned *status;
-  int R, Cin, Cout, BX, LN;
-  int mz, ndx;
-  int ns;    // stages
-  int units; // (R / BX) * (R / LN) * R
-  uint32_t tmem_cols;
-};
-
-#define WW_READ 4  // warps: readers (bias sums, accumulators out), issuers, loader
-#define WW_ISS 3
-#define WW_THREADS (32 * (WW_READ + WW_ISS + 1))
-#define WW_MAX_STAGES 4
-
-static __host__ __device__ inline uint32_t wgs_gy_bytes(int Cout, int BX, int LN, int mz) {
-  return ((uint32_t)(LN * mz * (Cout >> 3) * BX) * 16u + 127u) & ~127u;
-}
-static __host__ __device__ inline uint32_t wgs_x_bytes(int Cin, int BX, int LN) {
-  return ((uint32_t)((LN + 2) * (Cin >> 3) * (BX + 2)) * 16u + 127u) & ~127u;
-}
-
-__global__ void __launch_bounds__(WW_THREADS) k_wgrad_strip(const __grid_constant__ ConvWS a) {
-  extern __shared__ __align__(1024) uint8_t sm[];
-  const int tid = threadIdx.x, lane = tid & 31;
-  const int warp = __shfl_sync(0xffffffffu, tid >> 5, 0);
-  const int R = a.R, kci = a.Cin >> 3, kco = a.Cout >> 3, BX = a.BX, LN = a.LN, W2 = BX + 2, ns = a.ns;
-  const uint32_t gbytes = wgs_gy_bytes(a.Cout, BX, LN, a.mz), sbytes = gbytes + wgs_x_bytes(a.Cin, BX, LN);
-  uint64_t *full = reinterpret_cast<uint64_t *>(sm + (uint32_t)ns * sbytes);  // [ns] x and gy have arrived
-  uint64_t *empty = full + WW_MAX_STAGES;                                     // [ns] their readers are done
-  uint64_t *done = empty + WW_MAX_STAGES;                                     // the accumulators are complete
+  const int nst = (L1 - L0 + WG_ROWS) / WG_ROWS;
+  const int M = a.Cout <= 64 ? 64 : 128;
+  const uint32_t group_bytes = (uint32_t)M * 16u, stage_bytes = (WG_ROWS / 8) * group_bytes;
+  const int Vt = a.BZ * P;  // rows of a chunk of the tile: planes 1 + dz .. BZ + dz of the padded block
+  const uint32_t tile_bytes = ((uint32_t)(kci * Vt + 128) * 16u + 1023u) & ~1023u;
+  uint8_t *tile = sm, *stg = sm + tile_bytes;
+  uint64_t *full = reinterpret_cast<uint64_t *>(stg + (uint32_t)ns * stage_bytes);  // [ns] a stage is there
+  uint64_t *empty = full + WG_MAX_STAGES;                                           // [ns] its MMAs are done
+  uint64_t *tfull = empty + WG_MAX_STAGES;                                          // the x tile is there
+  uint64_t *tempty = tfull + 1;                                                     // its MMAs are done
+  uint64_t *done = tempty + 1;                                                      // every MMA is
   uint32_t *tslot = reinterpret_cast<uint32_t *>(done + 1);
-  float *red = reinterpret_cast<float *>(done + 2);  // [4 warps][4 chunks][8]
-  // this group's taps and accumulators
-  const int ngx = a.ndx == 3 ? 1 : 3;
-  const int gdz = blockIdx.y / ngx, gdx = blockIdx.y - gdz * ngx;  // dz (mz = 1) and dx (ndx = 1) of the group
-  const int ndy = 3 * a.Cin <= 256 ? 3 : 1;                        // dy taps in the columns of one MMA
-  const int nacc = a.ndx == 3 || ndy == 1 ? 3 : 1, N = ndy * a.Cin;
-  const int M = 8 * a.mz * kco <= 64 ? 64 : 128;
-  const bool bias = a.mz == 3 ? gdx == 0 : (gdz == 1 && gdx == 0);
+  // accumulators of this group: taps of a dz, or its dx of each chunk
+  const int all = a.dy3 ? 3 : 9, dzi = blockIdx.x / a.sub;
+  const int g0 = (blockIdx.x - dzi * a.sub) * a.tpg, g1 = min(all, g0 + a.tpg);
+  const int N = a.dy3 ? 24 : a.Cin, nacc = (g1 - g0) * (a.dy3 ? kci : 1);
   if (warp == 0) {
     umma::tmem_alloc(tslot, a.tmem_cols);
     umma::tmem_relinquish();
   }
   if (tid == 32) {
     for (int s = 0; s < ns; ++s) {
-      umma::mbar_init(&full[s], 1);
-      umma::mbar_init(&empty[s], nacc + (bias ? WW_READ : 0));
+      umma::mbar_init(&full[s], 32);
+      umma::mbar_init(&empty[s], WS_ISSUERS);
     }
-    umma::mbar_init(done, nacc);
+    umma::mbar_init(tfull, a.use_map ? 1 : 32 * WG_LOAD);
+    umma::mbar_init(tempty, WS_ISSUERS);
+    umma::mbar_init(done, WS_ISSUERS);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
+  // zero margin behind the tile, read by the last rows' shifts
+  uint4 *trow = reinterpret_cast<uint4 *>(tile);
+  for (int i = tid; i < 128; i += WG_THREADS) trow[kci * Vt + i] = make_uint4(0u, 0u, 0u, 0u);
+  umma::fence_async_smem();
   umma::tc_fence_before();
   __syncthreads();
   umma::tc_fence_after();
   const uint32_t tmem = *tslot;
-  const int nbx = R / BX;
-  const int u0 = (int)((long long)a.units * blockIdx.x / gridDim.x);
-  const int u1 = (int)((long long)a.units * (blockIdx.x + 1) / gridDim.x);
   bool ok = true;
+  int nb = 0;  // blocks done: parity of the tile's barriers
 
-  if (warp < WW_READ) {
-    float *part = a.part + (size_t)blockIdx.x * (27 * a.Cin + 1) * a.Cout;
-    if (bias) {
-      // ---- channel sums of plane z: warp w takes the (line, chunk) rows w, w + 4, ..
-      float acc[4][8] = {};
-      const int nch = kco > WW_READ ? kco / WW_READ : 1;  // chunks of this warp
-      const int c0 = warp & (kco - 1), lstep = kco < WW_READ ? WW_READ / kco : 1, l0 = kco < WW_READ ? warp / kco : 0;
-      int s = 0;
-      uint32_t ph = 0u;
-      for (int u = u0; u < u1; ++u) {
-        ok = __all_sync(0xffffffffu, umma::mbar_wait(&full[s], ph, WS_WAIT_BUDGET));
+  if (warp < WG_LOAD) {
+    // ---- load: warp w fills every WG_LOAD-th stage
+    int f = 0, s = 0;
+    uint32_t ph = 1u;  // the first round finds the stages empty
+    // quotients by P and W2 as high products with ceil(2^32 / d), exact for rows and
+    // divisors below 2^16 (four divisions a lane, one after another, took 2.8k clk a stage)
+    const uint32_t mP = 0xffffffffu / (uint32_t)P + 1u, mW = 0xffffffffu / (uint32_t)W2 + 1u;
+    for (int b = blockIdx.y; b < a.nblocks && ok; b += gridDim.y, ++nb) {
+      const int z0 = (b / nby) * a.BZ, y0 = (b % nby) * a.BY;
+      if (!a.use_map || warp == 0) {  // the tile, when the last block's MMAs are done with it
+        if (nb) ok = __all_sync(0xffffffffu, umma::mbar_wait(tempty, (nb - 1) & 1, WS_WAIT_BUDGET));
         if (!ok) break;
-        const uint4 *g = reinterpret_cast<const uint4 *>(sm + (uint32_t)s * sbytes) + (size_t)(a.mz >> 1) * kco * BX;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          if (j >= nch) continue;
-          const uint4 *gc = g + (size_t)(c0 + WW_READ * j) * BX;
-          for (int l = l0; l < LN; l += lstep)
-            for (int x = lane; x < BX; x += 32) {
-              float f[8];
-              unpack8(gc[(size_t)l * a.mz * kco * BX + x], f);
-#pragma unroll
-              for (int k = 0; k < 8; ++k) acc[j][k] += f[k];
-            }
+      }
+      if (a.use_map) {
+        if (tid == 0) {
+          umma::mbar_arrive_expect_tx(tfull, (uint32_t)(kci * Vt) * 16u);
+          umma::tma_load_4d(tile, &a.map, -2, y0 - 1, z0 - 1 + dzi, 0, tfull);
         }
         __syncwarp();
-        if (lane == 0) umma::mbar_arrive(&empty[s]);
+      } else {
+        const int nzy = a.BZ * (a.BY + 2), nrows = kci * nzy;
+        for (int row = warp; row < nrows; row += WG_LOAD) {
+          const int kc = row / nzy, rr = row - kc * nzy;
+          const int tz = rr / (a.BY + 2), ty = rr - tz * (a.BY + 2);
+          const int gz = z0 - 1 + dzi + tz, gy_ = y0 - 1 + ty;
+          const bool rowin = (unsigned)gz < (unsigned)R && (unsigned)gy_ < (unsigned)R;
+          const uint4 *src = a.x + (size_t)kc * R3 + ((size_t)(rowin ? gz : 0) * R + (rowin ? gy_ : 0)) * R;
+          uint4 *dst = trow + (size_t)kc * Vt + (size_t)rr * W2;
+          for (int tx = lane; tx < W2; tx += 32) {
+            const int gx = tx - 1;
+            const bool in = rowin && (unsigned)gx < (unsigned)R;
+            umma::cp_async16(dst + tx, in ? (const void *)(src + gx) : (const void *)a.x, in);
+          }
+        }
+        umma::cp_async_wait_all();
+        umma::fence_async_smem();
+        umma::mbar_arrive(tfull);
+      }
+      for (int st = 0; st < nst; ++st, ++f) {
+        // every warp waits for every stage in turn (a wait by parity must not fall a phase behind)
+        ok = __all_sync(0xffffffffu, umma::mbar_wait(&empty[s], ph, WS_WAIT_BUDGET));
+        if (!ok) break;
+        if (f % WG_LOAD == warp) {
+          uint8_t *sbuf = stg + (uint32_t)s * stage_bytes;
+#pragma unroll
+          for (int r = lane; r < WG_ROWS; r += 32) {
+            const int L = L0 + WG_ROWS * st + r;
+            const int tz = (int)__umulhi((uint32_t)L, mP), rem = L - tz * P;
+            const int ty = (int)__umulhi((uint32_t)rem, mW), tx = rem - ty * W2;
+            const bool valid = L <= L1 && ty >= 1 && ty <= a.BY && tx >= 1 && tx <= R;
+            const uint4 *src = valid ? a.gy + ((size_t)(z0 + tz - 1) * R + (y0 + ty - 1)) * R + (tx - 1) : a.gy;
+            uint8_t *d = sbuf + (uint32_t)(r >> 3) * group_bytes + (r & 7) * 16;
+            for (int c = 0; c < kco; ++c) umma::cp_async16(d + c * 128, valid ? src + (size_t)c * R3 : a.gy, valid);
+          }
+          umma::cp_async_wait_all();
+          umma::fence_async_smem();
+          umma::mbar_arrive(&full[s]);
+        }
         if (++s == ns) { s = 0; ph ^= 1u; }
       }
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-#pragma unroll
-        for (int k = 0; k < 8; ++k) {
-          float v = acc[j][k];
-#pragma unroll
-          for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-          if (lane == 0) red[(warp * 4 + j) * 8 + k] = v;
-        }
-      asm volatile("bar.sync 1, 128;" ::: "memory");
-      if (tid < a.Cout && ok) {
-        const int c = tid >> 3, k = tid & 7;
-        float v;
-        if (kco >= WW_READ) {
-          v = red[((c & 3) * 4 + (c >> 2)) * 8 + k];
-        } else {
-          v = 0.0f;
-          for (int w = c; w < WW_READ; w += kco) v += red[w * 32 + k];
-        }
-        part[(size_t)27 * a.Cout * a.Cin + tid] = v;
-      }
     }
-    // ---- accumulators out: row (dz, co) of column (dx or dy, .., ci)
+    // ---- every MMA complete: accumulators out
     ok = __all_sync(0xffffffffu, ok && umma::mbar_wait(done, 0, WS_WAIT_BUDGET));
     umma::tc_fence_after();
     if (ok) {
-      const int row = M == 64 ? 16 * warp + lane : 32 * warp + lane;
-      const int m = row / a.Cout, co = row - m * a.Cout;
-      const bool valid = m < a.mz && (M == 128 || lane < 16);
-      const int dz = a.mz == 3 ? 2 - m : gdz;  // gy plane z - 1 + m meets x plane z: dz = 1 - m
-      for (int q = 0; q < nacc; ++q)
-        for (int c = 0; c < N; c += 16) {
-          uint32_t r[16];
-          umma::tmem_ld16(tmem + ((uint32_t)(32 * warp) << 16) + (uint32_t)(q * N + c), r);
-          umma::tmem_wait_ld();
-          const int dyc = c / a.Cin, ci = c - dyc * a.Cin;
-          const int dy = ndy == 3 ? dyc : q, dx = a.ndx == 3 ? q : gdx;
-          if (valid) {
-            float4 *dst = reinterpret_cast<float4 *>(part + ((size_t)(9 * dz + 3 * dy + dx) * a.Cout + co) * a.Cin + ci);
+      const int quad = warp & 3, co = M == 64 ? 16 * quad + lane : 32 * quad + lane;
+      const bool mine = co < a.Cout && (M == 128 || lane < 16);
+      const int ncol8 = nacc * (N / 8);  // columns in pieces of 8
+      float *base = a.part + (size_t)blockIdx.y * 27 * a.Cout * a.Cin + (size_t)co * a.Cin;
+      for (int q = 2 * (warp >> 2); q < ncol8; q += 4) {
+        uint32_t r[16];
+        umma::tmem_ld16(tmem + ((uint32_t)(32 * quad) << 16) + (uint32_t)(8 * q), r);
+        umma::tmem_wait_ld();
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-              dst[j] = make_float4(__uint_as_float(r[4 * j]), __uint_as_float(r[4 * j + 1]),
-                                   __uint_as_float(r[4 * j + 2]), __uint_as_float(r[4 * j + 3]));
+        for (int h = 0; h < 2; ++h) {
+          const int c8 = q + h;
+          if (!mine || c8 >= ncol8) continue;
+          int t, ci;
+          if (a.dy3) {
+            const int u = c8 / 3, dy = c8 - 3 * u;
+            t = 9 * dzi + 3 * dy + g0 + u / kci;
+            ci = 8 * (u % kci);
+          } else {
+            t = 9 * dzi + g0 + c8 / kci;
+            ci = 8 * (c8 % kci);
           }
+          float4 *dst = reinterpret_cast<float4 *>(base + (size_t)t * a.Cout * a.Cin + ci);
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            dst[j] = make_float4(__uint_as_float(r[8 * h + 4 * j]), __uint_as_float(r[8 * h + 4 * j + 1]),
+                                 __uint_as_float(r[8 * h + 4 * j + 2]), __uint_as_float(r[8 * h + 4 * j + 3]));
         }
+      }
     }
-  } else if (warp < WW_READ + WW_ISS) {
-    // ---- issue: warp q feeds accumulator q
-    const int q = warp - WW_READ;
-    if (q < nacc) {
-      const uint32_t lead = umma::elect_one();
-      const uint32_t idesc = umma::idesc_bf16(M, N, 1, 1);
-      const uint32_t gl = (uint32_t)(a.mz * kco * BX), xl = (uint32_t)(kci * W2);  // rows of a line
-      const bool pair = BX < 16;  // 16 voxels of K: along x, or 8 of two lines
-      const uint64_t ad0 = umma::sdesc_mn(umma::smem_u32(sm), pair ? gl * 16u : 128u, (uint32_t)BX * 16u);
-      const uint64_t bd0 = umma::sdesc_mn(umma::smem_u32(sm) + gbytes, pair ? xl * 16u : 128u, (uint32_t)W2 * 16u) +
-                           (uint32_t)(a.ndx == 3 ? q : gdx) + (ndy == 1 ? (uint32_t)q * xl : 0u);
-      const uint32_t td = tmem + (uint32_t)(q * N);
-      const int lines = pair ? LN / 2 : LN, nxb = pair ? 1 : BX / 16;
-      const uint32_t glp = pair ? 2 * gl : gl, xlp = pair ? 2 * xl : xl;
-      uint32_t accum = 0u;
-      int s = 0;
-      uint32_t ph = 0u;
-      for (int u = u0; u < u1; ++u) {
+  } else {
+    // ---- issue: warp w feeds the accumulators w, w + WS_ISSUERS, ..
+    const int w = warp - WG_LOAD;
+    const uint32_t lead = umma::elect_one();
+    const uint32_t idesc = umma::idesc_bf16(M, N, 1, 1);
+    const uint64_t ad0 = umma::sdesc_mn(umma::smem_u32(stg), group_bytes, 128u);
+    const uint64_t bd0 = umma::sdesc_mn(umma::smem_u32(tile), 128u, a.dy3 ? (uint32_t)W2 * 16u : (uint32_t)Vt * 16u);
+    const uint32_t kstep = (2u * group_bytes) >> 4;
+    int s = 0;
+    uint32_t ph = 0u, accum = 0u;
+    for (int b = blockIdx.y; b < a.nblocks && ok; b += gridDim.y, ++nb) {
+      ok = __all_sync(0xffffffffu, umma::mbar_wait(tfull, nb & 1, WS_WAIT_BUDGET));
+      for (int st = 0; st < nst && ok; ++st) {
         ok = __all_sync(0xffffffffu, umma::mbar_wait(&full[s], ph, WS_WAIT_BUDGET));
         if (!ok) break;
         umma::tc_fence_after();
-        uint64_t al = ad0 + (((uint32_t)s * sbytes) >> 4), bl = bd0 + (((uint32_t)s * sbytes) >> 4);
-        for (int l = 0; l < lines; ++l, al += glp, bl += xlp) {
-#pragma unroll 4
-          for (int xb = 0; xb < nxb; ++xb) {
-            umma::mma_bf16_if(lead, td, al + 16u * xb, bl + 16u * xb, idesc, accum);
-            accum = 1u;
-          }
+        const uint64_t ad = ad0 + (((uint32_t)s * stage_bytes) >> 4);
+        const uint64_t bs = bd0 + (uint32_t)(L0 - P + WG_ROWS * st);
+        for (int q = w; q < nacc; q += WS_ISSUERS) {
+          int off;  // dy W2 + dx; dy = -1 is the first of the three column groups
+          if (a.dy3)
+            off = (g0 + q / kci - 1) - W2 + (q % kci) * Vt;
+          else
+            off = ((g0 + q) / 3 - 1) * W2 + (g0 + q) % 3 - 1;
+          const uint64_t bd = bs + (uint64_t)(int64_t)off;
+          const uint32_t td = tmem + (uint32_t)(q * N);
+          umma::mma_bf16_if(lead, td, ad, bd, idesc, accum);
+#pragma unroll
+          for (int ks = 1; ks < WG_ROWS / 16; ++ks)
+            umma::mma_bf16_if(lead, td, ad + ks * kstep, bd + 16u * ks, idesc, 1u);
         }
-        if (lead) umma::mma_commit(&empty[s]);
+        accum = 1u;
+        if (lead) {
+          umma::mma_commit(&empty[s]);
+          if (st == nst - 1) umma::mma_commit(tempty);
+        }
         __syncwarp();
         if (++s == ns) { s = 0; ph ^= 1u; }
       }
-      if (lead) umma::mma_commit(done);
     }
-  } else if (lane == 0) {
-    // ---- load: a box of x and one of gy per unit
-    const uint32_t bytes = (uint32_t)(LN * a.mz * kco * BX + (LN + 2) * kci * W2) * 16u;
-    int s = 0;
-    uint32_t ph = 1u;  // the first round finds the stages empty
-    for (int u = u0; u < u1; ++u) {
-      const int strip = u / R, z = u - strip * R, sy = strip / nbx, x0 = (strip - sy * nbx) * BX, y0 = sy * LN;
-      ok = umma::mbar_wait(&empty[s], ph, WS_WAIT_BUDGET);
-      if (!ok) break;
-      uint8_t *st = sm + (uint32_t)s * sbytes;
-      umma::mbar_arrive_expect_tx(&full[s], bytes);
-      umma::tma_load_4d(st, &a.mg, 2 * x0, 0, a.mz == 3 ? z - 1 : z + 1 - gdz, y0, &full[s]);
-      umma::tma_load_4d(st + gbytes, &a.mx, 2 * (x0 - 1), 0, y0 - 1, z, &full[s]);
-      if (++s == ns) { s = 0; ph ^= 1u; }
-    }
-    if (!ok) {  // after a timeout: let the copies in flight land before the CTA ends
-      for (int i = 0; i < ns; ++i) umma::mbar_wait(&full[i], i < s ? ph ^ 1u : ph, WS_WAIT_BUDGET);
-    }
+    if (lead) umma::mma_commit(done);
   }
   if (!ok && lane == 0) atomicOr(a.status, 1u);
-  if (warp == 0 && !umma::mbar_wait(done, 0, WS_WAIT_BUDGET) && lane == 0) atomicOr(a.status, 1u);
+  if (warp == 0) {  // after a timeout too, MMAs and copies in flight end first
+    if (!umma::mbar_wait(done, 0, WS_WAIT_BUDGET) && lane == 0) atomicOr(a.status, 1u);
+    if (!ok && a.use_map) umma::mbar_wait(tfull, nb & 1, WS_WAIT_BUDGET);
+  }
   umma::tc_fence_before();
   __syncthreads();
   if (warp == 0) umma::tmem_dealloc(tmem, a.tmem_cols);
@@ -988,10 +849,9 @@ __global__ void __launch_bounds__(WW_THREADS) k_wgrad_strip(const __grid_constan
 
 // out[e] = sum over c of part[c*nelem + e] for few elements and many partials:
 // one block per element, a fixed strided split and a fixed tree (deterministic).
-__global__ void __launch_bounds__(256) k_reduce_cols(const float *__restrict__ part, int nparts, int nelem,
-                                                     float *__restrict__ out) {
+__device__ __forceinline__ void reduce_col(const float *__restrict__ part, int nparts, int nelem, int e,
+                                           float *__restrict__ out) {
   __shared__ float red[256];
-  const int e = blockIdx.x;
   float s = 0.0f;
   for (int c = threadIdx.x; c < nparts; c += 256) s += part[(size_t)c * nelem + e];
   red[threadIdx.x] = s;
@@ -1002,31 +862,41 @@ __global__ void __launch_bounds__(256) k_reduce_cols(const float *__restrict__ p
   }
   if (threadIdx.x == 0) out[e] = red[0];
 }
+__global__ void __launch_bounds__(256) k_reduce_cols(const float *__restrict__ part, int nparts, int nelem,
+                                                     float *__restrict__ out) {
+  reduce_col(part, nparts, nelem, blockIdx.x, out);
+}
 
-// out[e] = sum over partials p of part[p][e], e < nelem (a multiple of 4): thread (x, y)
-// adds the partials y, y + 8, .. of four elements, then the eight sums are added in
-// order. One thread per element over all partials took as long as the product at 16
-// channels: 27 blocks of it, each a chain of 152 loads.
-__global__ void __launch_bounds__(256) k_wgrad_reduce(const float *__restrict__ part, int nparts, int nelem,
-                                                      float *__restrict__ out) {
-  __shared__ float4 red[8][32];
-  const int x = threadIdx.x & 31, y = threadIdx.x >> 5, e = blockIdx.x * 32 + x, n4 = nelem >> 2;
-  float4 s = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-  if (e < n4) {
-#pragma unroll 4
-    for (int p = y; p < nparts; p += 8) {
-      const float4 v = __ldg(reinterpret_cast<const float4 *>(part) + (size_t)p * n4 + e);
-      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-    }
+// dW[e] = sum over partials in their order, for several layers (blockIdx.y): one chain of
+// additions per element, U partials' loads of it in flight. A launch per layer took 4.6
+// us each at R = 64, all eleven in one 29.
+struct WgReduce {
+  struct Layer {
+    const float *part;
+    float *out;
+    int nparts, nelem;
+  } l[WS_NL];
+};
+template <int U>
+__device__ __forceinline__ void reduce_run(const float *__restrict__ p, size_t stride, int n, int &c, float &s) {
+  for (; c + U <= n; c += U) {
+    float v[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) v[u] = __ldcg(p + (size_t)u * stride);
+    p += (size_t)U * stride;
+#pragma unroll
+    for (int u = 0; u < U; ++u) s += v[u];
   }
-  red[y][x] = s;
-  __syncthreads();
-  if (y == 0 && e < n4) {
-    for (int k = 1; k < 8; ++k) {
-      const float4 v = red[k][x];
-      s.x += v.x; s.y += v.y; s.z += v.z; s.w += v.w;
-    }
-    reinterpret_cast<float4 *>(out)[e] = s;
+}
+__global__ void __launch_bounds__(64) k_wgrad_reduce(const __grid_constant__ WgReduce d) {
+  const WgReduce::Layer &L = d.l[blockIdx.y];
+  for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < L.nelem; e += gridDim.x * blockDim.x) {
+    float s = 0.0f;
+    int c = 0;
+    reduce_run<32>(L.part + e, L.nelem, L.nparts, c, s);
+    reduce_run<8>(L.part + (size_t)c * L.nelem + e, L.nelem, L.nparts, c, s);
+    reduce_run<1>(L.part + (size_t)c * L.nelem + e, L.nelem, L.nparts, c, s);
+    L.out[e] = s;
   }
 }
 
@@ -1113,36 +983,50 @@ __global__ void __launch_bounds__(64) k_pool_adj_add_mask(const uint4 *__restric
   out[i] = pack8<0>(p);
 }
 
-// Per-block partial channel sums of g (C = 8*kc channels): part[block][C].
-__global__ void __launch_bounds__(256) k_chan_sum(const uint4 *__restrict__ g, int kc, size_t R3,
-                                                  float *__restrict__ part) {
+// Bias gradients of all layers: per-block partial channel sums of g (C = 8*kc channels),
+// part[block][C], nb blocks for each chunk of each layer; then the sums
+// of the partials. Two launches where a pair per layer took 2 us a launch.
+struct WsBias {
+  struct Layer {
+    const uint4 *g;
+    float *part, *out;
+    size_t R3;
+    int kc, nb, first;  // chunks, blocks of each, first block of the layer in the grid
+  } l[WS_NL];
+};
+__global__ void __launch_bounds__(256) k_chan_sum(const __grid_constant__ WsBias d) {
   __shared__ float red[8][8];  // [warp][channel of the chunk]
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
-  for (int c = 0; c < kc; ++c) {
-    float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
-    for (size_t v = blockIdx.x * (size_t)blockDim.x + tid; v < R3; v += (size_t)gridDim.x * blockDim.x) {
-      float f[8];
-      unpack8(__ldg(g + (size_t)c * R3 + v), f);
+  int layer = 0;
+  while (layer + 1 < WS_NL && (int)blockIdx.x >= d.l[layer + 1].first) ++layer;
+  const WsBias::Layer &L = d.l[layer];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, kc = L.kc;
+  const int c = ((int)blockIdx.x - L.first) / L.nb, blk = (int)blockIdx.x - L.first - c * L.nb;
+  float acc[8] = {0, 0, 0, 0, 0, 0, 0, 0};
+  for (size_t v = blk * (size_t)blockDim.x + tid; v < L.R3; v += (size_t)L.nb * blockDim.x) {
+    float f[8];
+    unpack8(__ldg(L.g + (size_t)c * L.R3 + v), f);
 #pragma unroll
-      for (int j = 0; j < 8; ++j) acc[j] += f[j];
-    }
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
-    }
-    if (lane == 0) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) red[warp][j] = acc[j];
-    }
-    __syncthreads();
-    if (tid < 8) {
-      float s = 0.0f;
-      for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w][tid];
-      part[(size_t)blockIdx.x * (8 * kc) + 8 * c + tid] = s;
-    }
-    __syncthreads();
+    for (int j = 0; j < 8; ++j) acc[j] += f[j];
   }
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+  }
+  if (lane == 0) {
+#pragma unroll
+    for (int j = 0; j < 8; ++j) red[warp][j] = acc[j];
+  }
+  __syncthreads();
+  if (tid < 8) {
+    float s = 0.0f;
+    for (int w = 0; w < (int)(blockDim.x >> 5); ++w) s += red[w][tid];
+    L.part[(size_t)blk * (8 * kc) + 8 * c + tid] = s;
+  }
+}
+__global__ void __launch_bounds__(256) k_chan_finish(const __grid_constant__ WsBias d) {
+  const WsBias::Layer &L = d.l[blockIdx.y];
+  if ((int)blockIdx.x < 8 * L.kc) reduce_col(L.part, L.nb, 8 * L.kc, blockIdx.x, L.out);
 }
 
 // Network input: channels 0..3 from f16 planar features [4][R^3]; channels 4..15 zero.
@@ -1182,29 +1066,47 @@ __global__ void __launch_bounds__(256) k_mse(const float *__restrict__ y, const 
 // ------------------------------------------------------------------------------
 // parameters: Adam and the bf16 packing of the weights
 // ------------------------------------------------------------------------------
+// Where a layer's parameters and packed weights lie.
+struct WsPack {
+  struct Layer {
+    uint16_t *wf, *wb;
+    int off, Cin, Cout;  // W (f32 [27][Cout][Cin]) at params[off], the bias behind it
+  } l[WS_NL];
+};
+
+// W -> forward operand [27][Cin/8][Cout][8] and data-gradient operand
+// [27][Cout/8][Cin][8] with the tap mirrored (t' = 26 - t).
+__device__ __forceinline__ void pack_weight(const WsPack::Layer &L, int i, float v) {
+  const int t = i / (L.Cout * L.Cin), rem = i - t * L.Cout * L.Cin, co = rem / L.Cin, ci = rem - co * L.Cin;
+  const uint16_t u = (uint16_t)(bf_pack(v, 0.0f) & 0xffffu);
+  L.wf[(((size_t)t * (L.Cin >> 3) + (ci >> 3)) * L.Cout + co) * 8 + (ci & 7)] = u;
+  L.wb[(((size_t)(26 - t) * (L.Cout >> 3) + (co >> 3)) * L.Cin + ci) * 8 + (co & 7)] = u;
+}
+
+// All layers' weights in one launch (blockIdx.y is the layer).
+__global__ void __launch_bounds__(256) k_pack_weights(const float *__restrict__ p, const __grid_constant__ WsPack d) {
+  const WsPack::Layer &L = d.l[blockIdx.y];
+  const int n = 27 * L.Cout * L.Cin;
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) pack_weight(L, i, p[L.off + i]);
+}
+
+// One Adam step and the packing of the new weights. Every parameter is read, updated and
+// packed in one pass: Adam (7.7 us) and eleven packing launches of 1.9 us took 28, this 12.
 __global__ void __launch_bounds__(256) k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
-                                              float *__restrict__ v, size_t n, float lr, float b1, float b2, float eps,
-                                              float bc1, float bc2) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
+                                              float *__restrict__ v, const __grid_constant__ WsPack d, float lr, float b1,
+                                              float b2, float eps, float bc1, float bc2) {
+  const WsPack::Layer &L = d.l[blockIdx.y];
+  const int nw = 27 * L.Cout * L.Cin, n = nw + L.Cout;
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
+    const int i = L.off + j;
     const float gi = g[i];
     const float mi = b1 * m[i] + (1.0f - b1) * gi;
     const float vi = b2 * v[i] + (1.0f - b2) * gi * gi;
     m[i] = mi;
     v[i] = vi;
-    p[i] -= lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
-  }
-}
-
-// W (f32 [27][Cout][Cin]) -> forward operand [27][Cin/8][Cout][8] and data-gradient
-// operand [27][Cout/8][Cin][8] with the tap mirrored (t' = 26 - t).
-__global__ void __launch_bounds__(256) k_pack_weights(const float *__restrict__ W, int Cin, int Cout,
-                                                      uint16_t *__restrict__ wf, uint16_t *__restrict__ wb) {
-  const int n = 27 * Cout * Cin;
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-    const int t = i / (Cout * Cin), rem = i - t * Cout * Cin, co = rem / Cin, ci = rem - co * Cin;
-    const uint32_t u = bf_pack(W[i], 0.0f) & 0xffffu;
-    wf[(((size_t)t * (Cin >> 3) + (ci >> 3)) * Cout + co) * 8 + (ci & 7)] = (uint16_t)u;
-    wb[(((size_t)(26 - t) * (Cout >> 3) + (co >> 3)) * Cin + ci) * 8 + (co & 7)] = (uint16_t)u;
+    const float pi = p[i] - lr * (mi / bc1) / (sqrtf(vi / bc2) + eps);
+    p[i] = pi;
+    if (j < nw) pack_weight(L, j, pi);
   }
 }
 
@@ -1220,7 +1122,6 @@ __global__ void __launch_bounds__(256) k_pack_weights(const float *__restrict__ 
 //   y  = K f0 (channel 0)
 // every capital a 3x3x3 convolution with bias (zero padding), pool a 2x2x2 mean,
 // up a nearest-neighbour doubling. x0 has 16 channels, 3 in use.
-#define WS_NL 11
 static const int kWsLayer[WS_NL][4] = {  // cin, cout, level, relu
     {16, 16, 0, 1}, {16, 32, 1, 1}, {32, 64, 2, 1}, {64, 128, 3, 1}, {128, 64, 3, 0}, {64, 64, 2, 1},
     {64, 32, 2, 0}, {32, 32, 1, 1}, {32, 16, 1, 0}, {16, 16, 0, 1}, {16, 16, 0, 0}};
@@ -1234,9 +1135,10 @@ struct FwdPlan {
   size_t smem;
 };
 struct WgPlan {
-  int BX;  // 0: blocks of whole lines (k_conv_wgrad); else strips of BX voxels (k_wgrad_strip)
-  int BZ, BY, tpp, nblocks, grid;
-  int mz, ndx, ns, groups;
+  int BZ, BY, nblocks;
+  int grid;         // partial sums
+  int groups, sub, tpg;  // tap groups beside each other, of a dz, and taps (or dx) in each
+  int dy3, ns;
   uint32_t cols;
   size_t smem;
 };
@@ -1257,8 +1159,10 @@ struct gc_ws {
   uint4 *p2, *e2, *u1, *d2, *f2, *g_u1, *g_f2, *g_d2, *g_p2, *g_e2;
   uint4 *p3, *e3, *u2, *g_u2, *g_e3, *g_p3;
   float *y;
-  float *part;
-  size_t part_cap;
+  float *part;          // weight-gradient partials ..
+  size_t pofs[WS_NL];   // .. each layer's behind the other
+  WgReduce pend;        // layers whose partials wait for their sums
+  int npend;
   float *cpart;
   float *lpart;
   float *loss;
@@ -1388,53 +1292,16 @@ static bool plan_fwd(int R, int Cin, int Cout, int sm_count, FwdPlan &best) {
   return true;
 }
 
-// Weight gradient: strips wherever the lines come in multiples of 8 voxels, and only
-// where they do not, blocks of whole lines. Strips are enumerated by (BX, lines,
-// splits) with an estimate in clocks: loads at 40 bytes a clock and SM, MMAs at their
-// measured clocks, the partials written and read again at 6000 bytes a clock of the chip.
-// Strips against blocks: 16 -> 16 channels R = 128 48 / 721 us, R = 64 11.8 / 103;
-// 64 -> 64 R = 32 25 / 129, R = 16 11.2 / 94; 128 -> 64 R = 8 11.0 / 145.
+// Blocks of the weight gradient and how they run. (BZ, BY) and the number of partials
+// belong to the result's bits and follow a score of useful rows, filled SMs and tile
+// reuse; how many taps a CTA takes, and how deep its ring is, do not. The taps are divided
+// by an estimate in clocks: a CTA's fixed 5000 (measured: set-up, first tile and stage)
+// and its products or its stages of gy at 900 each, whichever is more, over the waves
+// that shared memory and Tensor Memory make of them. At 16 channels a product takes the
+// three dy taps of a channel chunk: 24 columns and 18 products per 16 rows where 27 of 16
+// columns need 1.5 times as long.
 static std::vector<WgPlan> enum_wgrad(int R, int Cin, int Cout, int sm_count, std::vector<double> *scores) {
   std::vector<WgPlan> out;
-  const int lns[] = {16, 8, 4, 2};
-  const int bxs[] = {64, 32, 16, 8};
-  const int mz = 3 * Cout <= 128 ? 3 : 1, ndx = 9 * Cin <= 512 ? 3 : 1;
-  const int groups = (mz == 3 ? 1 : 3) * (ndx == 3 ? 1 : 3);
-  const int N = 3 * Cin <= 256 ? 3 * Cin : Cin, nacc = ndx == 3 || N == Cin ? 3 : 1;
-  const int M = mz * Cout <= 64 ? 64 : 128;
-  const double mma = std::max(0.5 * N, M == 64 ? 29.0 : 32.0 + 0.25 * N);
-  for (int BX : bxs) {
-    if (R % BX) continue;
-    for (int LN : lns) {
-      if (R % LN) continue;
-      const size_t gb = wgs_gy_bytes(Cout, BX, LN, mz), xb = wgs_x_bytes(Cin, BX, LN);
-      // the M groups beyond mz * Cout / 8 read on into the x box of the stage
-      if ((size_t)(M / 8 - mz * Cout / 8) * BX * 16 > xb) continue;
-      const size_t fixed = (2 * WW_MAX_STAGES + 2) * 8 + 512;
-      if (fixed + 2 * (gb + xb) > WS_SMEM_MAX) continue;
-      const int units = (R / BX) * (R / LN) * R;
-      int last = 0;
-      for (int div = 1; div <= 8; div *= 2) {
-        WgPlan p = {};
-        p.BX = BX; p.BZ = 1; p.BY = LN; p.tpp = 27 / groups; p.nblocks = units;
-        p.mz = mz; p.ndx = ndx; p.groups = groups;
-        p.ns = (int)std::min<size_t>(WW_MAX_STAGES, (WS_SMEM_MAX - fixed) / (gb + xb));
-        p.cols = pow2_cols(nacc * N);
-        p.smem = smem_for_residency(fixed + p.ns * (gb + xb), 1);
-        p.grid = std::min(units, std::max(1, sm_count / groups / div));
-        if (p.grid == last) continue;
-        last = p.grid;
-        out.push_back(p);
-        if (scores) {
-          const int per = (units + p.grid - 1) / p.grid;
-          const double load = (double)(gb + xb) / 40.0, prod = LN * BX / 16.0 * nacc * mma;
-          const double parts = (double)p.grid * 27 * Cin * Cout * 4 * 2 / 6000.0;
-          scores->push_back(-(4000.0 + load + per * std::max(load, prod + 100.0) + 60.0 * nacc * N / 16 + parts));
-        }
-      }
-    }
-  }
-  if (!out.empty()) return out;
   const int bys[] = {32, 16, 8, 4, 2, 1};
   const int bzs[] = {1, 2, 4};
   for (int BY : bys) {
@@ -1444,20 +1311,40 @@ static std::vector<WgPlan> enum_wgrad(int R, int Cin, int Cout, int sm_count, st
       int W2, P, V, L0, L1;
       conv_geom(R, BZ, BY, W2, P, V, L0, L1);
       const size_t tile = (((size_t)(Cin / 8) * V + 128) * 16 + 1023) & ~(size_t)1023;
-      const size_t smem = tile + 2 * WG_STAGE_BYTES + 64;
-      if (smem > WS_SMEM_MAX) continue;
-      const int nst = (L1 - L0 + WG_STAGE_ROWS) / WG_STAGE_ROWS;
-      // few blocks: fewer taps a pass, more passes beside each other (64 -> 128 channels
-      // at R = 4: 2 CTAs with 4 passes each took 169 us, 54 CTAs of one tap 17)
-      int tpp = std::min(27, 512 / Cin);
-      while (tpp > 1 && (R / BZ) * (R / BY) * ((27 + tpp - 1) / tpp) * 2 < sm_count) tpp = (tpp + 1) / 2;
-      const uint32_t cols = pow2_cols(tpp * Cin);
+      // partials: as many as CTAs of one tile and two stages of 32 KB that hold 512 / Cin
+      // taps fit the chip
+      const size_t ref = tile + 2 * 32768 + 64;
+      if (ref > WS_SMEM_MAX) continue;
+      const int nst = (L1 - L0 + WG_ROWS) / WG_ROWS;
+      const size_t ref_res = smem_for_residency(ref, (int)(512 / pow2_cols(std::min(27, 512 / Cin) * Cin)));
       WgPlan p = {};
-      p.BZ = BZ; p.BY = BY; p.tpp = tpp; p.nblocks = (R / BZ) * (R / BY); p.cols = cols;
-      p.groups = (27 + tpp - 1) / tpp;
-      p.smem = smem_for_residency(smem, (int)(512 / cols));
-      const int per_sm = std::max(1, (int)(233472 / (p.smem + 1024)));
-      p.grid = std::min(p.nblocks, sm_count * per_sm);
+      p.BZ = BZ; p.BY = BY; p.nblocks = (R / BZ) * (R / BY);
+      p.grid = std::min(p.nblocks, sm_count * std::max(1, (int)(233472 / (ref_res + 1024))));
+      p.dy3 = Cin == 16 && Cout <= 64;
+      const int all = p.dy3 ? 3 : 9, acc = p.dy3 ? 24 * (Cin / 8) : Cin;  // columns of one of them
+      const size_t stage = (size_t)WG_ROWS * 2 * (Cout <= 64 ? 64 : 128), bars = (2 * WG_MAX_STAGES + 5) * 8;
+      const size_t dtile = (((size_t)(Cin / 8) * BZ * P + 128) * 16 + 1023) & ~(size_t)1023;  // one dz
+      const int most = (p.nblocks + p.grid - 1) / p.grid;  // blocks of a partial
+      const int N = p.dy3 ? 24 : Cin;
+      const double clk = std::max(0.5 * N, Cout <= 64 ? 24.0 : 32.0 + 0.25 * N);
+      double best = 0.0;
+      for (int sub = 1; sub <= all; ++sub) {
+        const int tpg = (all + sub - 1) / sub;
+        if (tpg * acc > 512 || (sub > 1 && tpg == (all + sub - 2) / (sub - 1))) continue;
+        const uint32_t cols = pow2_cols(tpg * acc);
+        int ns = (int)std::min<size_t>(std::min(WG_MAX_STAGES, most * nst), (WS_SMEM_MAX - dtile - bars) / stage);
+        if (ns > 4) ns = 4;
+        const size_t smem = smem_for_residency(dtile + ns * stage + bars, (int)(512 / cols));
+        const int res = std::max(1, std::min(4, (int)(233472 / (smem + 1024))));
+        const double prod = (double)most * nst * (WG_ROWS / 16) * tpg * (p.dy3 ? Cin / 8 : 1) * clk;
+        const double waves = std::ceil(3.0 * p.grid * sub / ((double)sm_count * res));
+        const double cost = waves * std::max(5000.0 + std::max(prod, 900.0 * most * nst), res * prod);
+        if (best == 0.0 || cost < best) {
+          best = cost;
+          p.sub = sub; p.tpg = tpg; p.groups = 3 * sub; p.cols = cols; p.ns = ns; p.smem = smem;
+        }
+      }
+      if (best == 0.0) continue;
       out.push_back(p);
       if (scores) {
         const double useful = (double)BZ * BY * R / (128.0 * nst);
@@ -1554,36 +1441,46 @@ static int ws_conv(gc_ws *ws, const FwdPlan &p, int R, int Cin, int Cout, const 
 static int ws_wgrad(gc_ws *ws, int l, const uint4 *x, const uint4 *gy) {
   const int Cin = kWsLayer[l][0], Cout = kWsLayer[l][1], R = ws->R >> kWsLayer[l][2];
   const WgPlan &p = ws->pw[l];
-  const int nelem = 27 * Cout * Cin;
-  if (p.BX) {
-    ConvWS a = {};
-    int st;
-    if ((st = ws_tmap(ws, &a.mx, x, R, Cin / 8, {WS_C, WS_Y, WS_Z}, p.BX + 2, Cin / 8, p.BY + 2, 1))) return st;
-    if ((st = ws_tmap(ws, &a.mg, gy, R, Cout / 8, {WS_C, WS_Z, WS_Y}, p.BX, Cout / 8, p.mz, p.BY))) return st;
-    a.part = ws->part; a.status = ws->status;
-    a.R = R; a.Cin = Cin; a.Cout = Cout; a.BX = p.BX; a.LN = p.BY; a.mz = p.mz; a.ndx = p.ndx; a.ns = p.ns;
-    a.units = p.nblocks; a.tmem_cols = p.cols;
-    k_wgrad_strip<<<dim3(p.grid, p.groups), WW_THREADS, p.smem, ws->stream>>>(a);
-    WS_CUDA(ws, cudaGetLastError());
-    // the biases follow the weights in the partials and in the gradient vector
-    const int n = nelem + Cout;
-    k_wgrad_reduce<<<(n / 4 + 31) / 32, 256, 0, ws->stream>>>(ws->part, p.grid, n, ws->grads + ws->w_off[l]);
-    WS_CUDA(ws, cudaGetLastError());
-    return GC_OK;
+  ConvW a = {};
+  a.use_map = R <= 126;
+  if (a.use_map) {
+    const int st = ws_tmap(ws, &a.map, x, R, Cin / 8, {WS_Y, WS_Z, WS_C}, R + 2, p.BY + 2, p.BZ, Cin / 8);
+    if (st) return st;
   }
-  ConvW a;
-  a.x = x; a.gy = gy; a.part = ws->part; a.status = ws->status;
-  a.R = R; a.Cin = Cin; a.Cout = Cout; a.BZ = p.BZ; a.BY = p.BY; a.tpp = p.tpp; a.nblocks = p.nblocks;
-  a.tmem_cols = p.cols;
-  k_conv_wgrad<<<dim3(p.grid, p.groups), 256, p.smem, ws->stream>>>(a);
+  a.x = x; a.gy = gy; a.part = ws->part + ws->pofs[l]; a.status = ws->status;
+  a.R = R; a.Cin = Cin; a.Cout = Cout; a.BZ = p.BZ; a.BY = p.BY; a.nblocks = p.nblocks;
+  a.tpg = p.tpg; a.sub = p.sub; a.dy3 = p.dy3; a.ns = p.ns; a.tmem_cols = p.cols;
+  k_conv_wgrad<<<dim3(p.groups, p.grid), WG_THREADS, p.smem, ws->stream>>>(a);
   WS_CUDA(ws, cudaGetLastError());
-  k_wgrad_reduce<<<(nelem / 4 + 31) / 32, 256, 0, ws->stream>>>(ws->part, p.grid, nelem, ws->grads + ws->w_off[l]);
+  ws->pend.l[ws->npend++] = {a.part, ws->grads + ws->w_off[l], p.grid, 27 * Cout * Cin};
+  return GC_OK;
+}
+
+// The sums of the layers that wait for them.
+static int ws_wgrad_finish(gc_ws *ws) {
+  int most = 0;
+  for (int i = 0; i < ws->npend; ++i) most = std::max(most, ws->pend.l[i].nelem);
+  const unsigned nb = std::min<unsigned>((unsigned)(most + 63) / 64, (unsigned)ws->sm_count * 8u);
+  if (ws->npend) k_wgrad_reduce<<<dim3(nb, ws->npend), 64, 0, ws->stream>>>(ws->pend);
+  ws->npend = 0;
   WS_CUDA(ws, cudaGetLastError());
-  // bias gradient: channel sums of gy
-  const size_t R3 = (size_t)R * R * R;
-  const unsigned nb = std::min<unsigned>(ew_blocks(R3, ws->sm_count), 1024u);
-  k_chan_sum<<<nb, 256, 0, ws->stream>>>(gy, Cout / 8, R3, ws->cpart);
-  k_reduce_cols<<<Cout, 256, 0, ws->stream>>>(ws->cpart, (int)nb, Cout, ws->grads + ws->b_off[l]);
+  return GC_OK;
+}
+
+// Bias gradients of every layer, from the output gradients of a whole backward pass.
+static int ws_bias_grads(gc_ws *ws) {
+  const uint4 *g[WS_NL] = {ws->g_e0, ws->g_e1, ws->g_e2, ws->g_e3, ws->g_u2, ws->g_f2, ws->g_u1, ws->g_f1, ws->g_u0,
+                           ws->g_f0, ws->gy};
+  WsBias d;
+  int blocks = 0;
+  for (int l = 0; l < WS_NL; ++l) {
+    const size_t R = (size_t)(ws->R >> kWsLayer[l][2]), R3 = R * R * R;
+    const int nb = (int)std::min<unsigned>(ew_blocks(R3, ws->sm_count), 1024u), kc = kWsLayer[l][1] / 8;
+    d.l[l] = {g[l], ws->cpart + (size_t)l * 1024 * 128, ws->grads + ws->b_off[l], R3, kc, nb, blocks};
+    blocks += nb * kc;
+  }
+  k_chan_sum<<<blocks, 256, 0, ws->stream>>>(d);
+  k_chan_finish<<<dim3(128, WS_NL), 256, 0, ws->stream>>>(d);
   WS_CUDA(ws, cudaGetLastError());
   return GC_OK;
 }
@@ -1690,19 +1587,21 @@ extern "C" int gc_ws_create(gc_ws **out, int R) {
       rc = GC_ERR_ARG;
     }
   }
-  size_t part = 0;  // weight-gradient partials: the largest grid any candidate plan may use
+  size_t part = 0;  // weight-gradient partials: the most any candidate plan of a layer may use
   for (int l = 0; l < WS_NL && rc == GC_OK; ++l) {
     const int Rl = R >> kWsLayer[l][2];
+    size_t most = 0;
     for (const WgPlan &c : enum_wgrad(Rl, kWsLayer[l][0], kWsLayer[l][1], ws->sm_count, nullptr))
-      part = std::max(part, (size_t)c.grid * (27 * kWsLayer[l][0] + 1) * kWsLayer[l][1]);
+      most = std::max(most, (size_t)c.grid * 27 * kWsLayer[l][0] * kWsLayer[l][1]);
+    ws->pofs[l] = part;
+    part += (most + 63) & ~(size_t)63;
   }
-  ws->part_cap = part;
-  if (rc == GC_OK && cudaMalloc(&ws->part, part * sizeof(float) + (size_t)(1024 * 128 + 1024 + 16) * sizeof(float) +
+  if (rc == GC_OK && cudaMalloc(&ws->part, part * sizeof(float) + (size_t)(WS_NL * 1024 * 128 + 1024 + 16) * sizeof(float) +
                                                64) != cudaSuccess)
     fail("partials");
   if (rc == GC_OK) {
     ws->cpart = ws->part + part;
-    ws->lpart = ws->cpart + 1024 * 128;
+    ws->lpart = ws->cpart + WS_NL * 1024 * 128;
     ws->loss = ws->lpart + 1024;
     ws->status = (unsigned *)(ws->loss + 8);
     cudaMemset(ws->status, 0, sizeof(unsigned));
@@ -1711,8 +1610,6 @@ extern "C" int gc_ws_create(gc_ws **out, int R) {
     if (cudaFuncSetAttribute(k_conv_march, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM_MAX) !=
             cudaSuccess ||
         cudaFuncSetAttribute(k_conv_fwd, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM_MAX) != cudaSuccess ||
-        cudaFuncSetAttribute(k_wgrad_strip, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM_MAX) !=
-            cudaSuccess ||
         cudaFuncSetAttribute(k_conv_wgrad, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)WS_SMEM_MAX) !=
             cudaSuccess)
       fail("shared memory attribute");
@@ -1752,12 +1649,14 @@ extern "C" int gc_ws_num_params(const gc_ws *ws, int64_t *n) {
   return GC_OK;
 }
 
+static WsPack ws_pack_desc(const gc_ws *ws) {
+  WsPack d;
+  for (int l = 0; l < WS_NL; ++l) d.l[l] = {ws->wf[l], ws->wb[l], (int)ws->w_off[l], kWsLayer[l][0], kWsLayer[l][1]};
+  return d;
+}
+
 static int ws_repack(gc_ws *ws) {
-  for (int l = 0; l < WS_NL; ++l) {
-    const int n = 27 * kWsLayer[l][0] * kWsLayer[l][1];
-    k_pack_weights<<<(n + 255) / 256, 256, 0, ws->stream>>>(ws->params + ws->w_off[l], kWsLayer[l][0], kWsLayer[l][1],
-                                                            ws->wf[l], ws->wb[l]);
-  }
+  k_pack_weights<<<dim3(512, WS_NL), 256, 0, ws->stream>>>(ws->params, ws_pack_desc(ws));
   WS_CUDA(ws, cudaGetLastError());
   return GC_OK;
 }
@@ -1831,6 +1730,7 @@ extern "C" int gc_ws_backward(gc_ws *ws, const void *target, float *loss_out) {
   const int sm = ws->sm_count;
   int s;
   const unsigned nl = std::min<unsigned>(ew_blocks(R3, sm), 1024u);
+  ws->npend = 0;
   k_mse<<<nl, 256, 0, ws->stream>>>(ws->y, (const __half *)target, R3, ws->gy, ws->lpart);
   k_reduce_cols<<<1, 256, 0, ws->stream>>>(ws->lpart, (int)nl, 1, ws->loss);
   WS_CUDA(ws, cudaGetLastError());
@@ -1868,6 +1768,7 @@ extern "C" int gc_ws_backward(gc_ws *ws, const void *target, float *loss_out) {
   k_pool_adj_add_mask<<<line_grid(R, 2, 64), 64, 0, ws->stream>>>(ws->g_d0, ws->g_p1, ws->e0, ws->g_e0, R);
   // A
   if ((s = ws_wgrad(ws, 0, ws->x0, ws->g_e0))) return s;
+  if ((s = ws_wgrad_finish(ws)) || (s = ws_bias_grads(ws))) return s;
   WS_CUDA(ws, cudaGetLastError());
   if (loss_out) WS_CUDA(ws, cudaMemcpyAsync(loss_out, ws->loss, sizeof(float), cudaMemcpyDeviceToDevice, ws->stream));
   return GC_OK;
@@ -1923,9 +1824,10 @@ extern "C" int gc_ws_autotune(gc_ws *ws, int iters, float *ms_out) {
         WgPlan keep = ws->pw[l];
         for (const WgPlan &p : c) {
           ws->pw[l] = p;
-          if ((rc = ws_wgrad(ws, l, b.in, b.mask))) break;
+          if ((rc = ws_wgrad(ws, l, b.in, b.mask)) || (rc = ws_wgrad_finish(ws))) break;
           cudaEventRecord(ev0, ws->stream);
-          for (int i = 0; i < iters && rc == GC_OK; ++i) rc = ws_wgrad(ws, l, b.in, b.mask);
+          for (int i = 0; i < iters && rc == GC_OK; ++i)
+            if (!(rc = ws_wgrad(ws, l, b.in, b.mask))) rc = ws_wgrad_finish(ws);
           cudaEventRecord(ev1, ws->stream);
           cudaEventSynchronize(ev1);
           float ms = 0.0f;
@@ -1973,7 +1875,7 @@ extern "C" int gc_ws_plan_info(const gc_ws *ws, int layer, int kind, int *out) {
   if (!ws || !out || layer < 0 || layer >= WS_NL || kind < 0 || kind > 2) return GC_ERR_ARG;
   if (kind == 2) {
     const WgPlan &p = ws->pw[layer];
-    out[0] = p.BZ; out[1] = p.BY; out[2] = p.tpp; out[3] = p.grid * p.groups; out[4] = 0;
+    out[0] = p.BZ; out[1] = p.BY; out[2] = p.dy3 ? 3 * p.tpg : p.tpg; out[3] = p.grid * p.groups; out[4] = 0;
   } else {
     const FwdPlan &p = kind == 0 ? ws->pf[layer] : ws->pb[layer];
     out[0] = p.BZ; out[1] = p.BY; out[2] = p.tpg; out[3] = p.grid * ws_cout(layer, kind) / p.Cn; out[4] = p.n_mt;
@@ -2003,10 +1905,10 @@ extern "C" int gc_ws_set_plan(gc_ws *ws, int layer, int kind, int index, int *co
 extern "C" int gc_ws_adam(gc_ws *ws, float lr, float beta1, float beta2, float eps, int step) {
   if (!ws || step < 1 || !(lr >= 0.0f)) return GC_ERR_ARG;
   const float bc1 = 1.0f - powf(beta1, (float)step), bc2 = 1.0f - powf(beta2, (float)step);
-  k_adam<<<ew_blocks(ws->nparams, ws->sm_count), 256, 0, ws->stream>>>(ws->params, ws->grads, ws->adam_m, ws->adam_v,
-                                                                       ws->nparams, lr, beta1, beta2, eps, bc1, bc2);
+  k_adam<<<dim3(512, WS_NL), 256, 0, ws->stream>>>(ws->params, ws->grads, ws->adam_m, ws->adam_v, ws_pack_desc(ws), lr,
+                                                  beta1, beta2, eps, bc1, bc2);
   WS_CUDA(ws, cudaGetLastError());
-  return ws_repack(ws);
+  return GC_OK;
 }
 
 // ------------------------------------------------------------------------------

@@ -1,11 +1,11 @@
 """The warm-start network's weight gradient under every plan, and against the oracle.
 
-Plans change the strip width (8, where a product's 16 voxels are two lines, to 64), the
-lines, the ring depth and the split of the voxels over CTAs; channel counts select 1 or 3
-planes in the rows and 1 or 3 shifts of x per CTA. All of them add the same products in
-FP32, in another order: over n voxels the sums differ by about 2^-24 sqrt(n) of their
-size, and 2^-21 sqrt(n) in the 2-norm of a layer is allowed. Levels whose size is not a
-multiple of 8 (24 -> 12, 6, 3 and 40 -> 20, 10, 5) take blocks of whole lines."""
+Plans change the blocks of voxels, how many partial sums they are dealt to, and with them
+how the taps are divided, the ring's depth and how often a CTA meets another block. All
+of them add the same products in FP32, in another order: over n voxels the sums differ by
+about 2^-24 sqrt(n) of their size, and 2^-21 sqrt(n) in the 2-norm of a layer is
+allowed. 24 and 40 have levels of 12, 6, 3 and 20, 10, 5 voxels.
+"""
 
 from __future__ import annotations
 
