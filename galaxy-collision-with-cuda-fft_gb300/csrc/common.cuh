@@ -129,6 +129,8 @@ struct gc_ctx {
   unsigned *hist_aux;   // scan auxiliaries
   size_t pcap;          // capacity of the particle scratch (elements)
   size_t hist_cap;
+  void *bin;            // the binned deposit's counters, items and particle copies
+  size_t bin_cap;
 
   double mass_sum_cache; // sum of masses for the engine's fixed-point quantum
   int last_step_valid;
@@ -438,7 +440,7 @@ int gc_fixed_point_setup(gc_ctx *ctx, const float *m, int64_t n, int bits, int m
 // particle order; runs of equal cells (cell-sorted input) are summed in registers.
 // `bits` is the fixed-point resolution *qexp was set up with (it only picks the pass).
 int gc_deposit_q(gc_ctx *ctx, const float *x, const float *y, const float *z, const float *m, int64_t n, int bits,
-                 const double *qexp);
+                 const double *qexp, bool any_order = false);
 // Read ctx->q, write rho (may be NULL) and b = f32(q 2^E 4 pi G h^2) (may be NULL),
 // zero q, and reduce the ten moments into ctx->dmom and ||b||^2 into dsmall[GC_S_BNORM2].
 int gc_convert_q(gc_ctx *ctx, const double *qexp, float *rho_out, float *b_out);

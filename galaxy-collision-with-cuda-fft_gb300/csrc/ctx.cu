@@ -210,6 +210,7 @@ extern "C" int gc_ctx_destroy(gc_ctx *ctx) {
   gc_mg_free(ctx);
   cudaFree(ctx->q);
   cudaFree(ctx->g4);
+  cudaFree(ctx->bin);
   cudaFree(ctx->ws_buf);
   cudaFree(ctx->red);
   cudaFree(ctx->dmom);
