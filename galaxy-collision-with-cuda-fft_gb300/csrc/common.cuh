@@ -44,6 +44,7 @@ enum {
   GC_S_MAXREL2 = 16, // ... and the largest (||r|| / ||b||)^2 they ended with
   GC_S_TICKET = 17,  // block ticket of the last-block grid reductions (an unsigned, 0 between them)
   GC_S_LIMBS = 64,   // [64, 94): integer limbs of the moments of k_convert_q (0 between calls)
+  GC_S_SCATTERED = 94, // whether a gather's particles come in no order (an int)
   GC_S_FIN_TMP = 128, // [128, 256): chunk partials of gc_finalize
   GC_S_NSLOTS = 256
 };
