@@ -218,6 +218,7 @@ __device__ __forceinline__ void mg_decide(const MgDecide &d, double *__restrict_
 __global__ void __launch_bounds__(256)
     k_fin_one(const double *__restrict__ parts, int nparts, double *__restrict__ dst, double *__restrict__ small,
               const __grid_constant__ MgDecide d) {
+  gc_after();
   __shared__ double sh[8];
   const int tid = threadIdx.x;
   double x[4] = {0.0, 0.0, 0.0, 0.0};
@@ -242,6 +243,7 @@ __global__ void __launch_bounds__(256)
 
 __global__ void __launch_bounds__(256)
     k_fin_chunks(const double *__restrict__ parts, int nparts, double *__restrict__ out) {
+  gc_after();
   __shared__ double sh[8];
   const int per = (nparts + gridDim.x - 1) / gridDim.x;
   const int i0 = blockIdx.x * per, i1 = min(nparts, i0 + per);
@@ -432,6 +434,7 @@ __device__ __forceinline__ void restrict_node(const float *__restrict__ rf, cons
 
 __global__ void __launch_bounds__(256)
     k_restrict(const float *__restrict__ rf, LevelGeom f, float *__restrict__ bc, LevelGeom cg) {
+  gc_after();
   const int K = blockIdx.x * 32 + threadIdx.x + 1;
   const int Jj = blockIdx.y * 8 + threadIdx.y + 1;
   const int I = blockIdx.z + 1;
@@ -620,6 +623,7 @@ template <bool PLAIN, bool SPLIT>
 __global__ void __launch_bounds__(256)
     k_resid0(const float *__restrict__ hi, const float *__restrict__ lo, const float *__restrict__ b,
              float *__restrict__ rout, float *__restrict__ e_first, double *__restrict__ parts, Split0 d) {
+  gc_after();
   const int G = d.G;
   const int k = blockIdx.x * 32 + threadIdx.x + 1;
   const int j = blockIdx.y * 8 + threadIdx.y + 1;
@@ -705,6 +709,7 @@ __device__ __forceinline__ void f4set(float4 &v, int q, float x) {
 template <bool FIRST>
 __global__ void __launch_bounds__(256)
     k_rb0x2(float *__restrict__ e, const float *__restrict__ r, Split0 d, int color) {
+  gc_after();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int i = blockIdx.z + 1;
@@ -742,6 +747,7 @@ template <bool PLAIN>
 __global__ void __launch_bounds__(256)
     k_rb0_lastx4(const float *__restrict__ e, const float *__restrict__ r, float *__restrict__ hi,
                  float *__restrict__ lo, Split0 d) {
+  gc_after();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int i = blockIdx.z + 1;
@@ -788,6 +794,7 @@ template <bool PLAIN, bool SPLIT>
 __global__ void __launch_bounds__(256)
     k_resid0x4(const float *__restrict__ hi, const float *__restrict__ lo, const float *__restrict__ b,
                float *__restrict__ rout, float *__restrict__ e_first, double *__restrict__ parts, Split0 d) {
+  gc_after();
   const int G = d.G;
   const int t = blockIdx.x * 32 + threadIdx.x;
   const int j = blockIdx.y * 8 + threadIdx.y + 1;
@@ -846,6 +853,7 @@ __global__ void __launch_bounds__(256)
 // Residual of the correction equation on four consecutive nodes, natural output.
 __global__ void __launch_bounds__(256)
     k_resid0ex4(const float *__restrict__ e, const float *__restrict__ r, float *__restrict__ rc, Split0 d) {
+  gc_after();
   const int G = d.G;
   const int t = blockIdx.x * 32 + threadIdx.x;
   const int j = blockIdx.y * 8 + threadIdx.y + 1;
@@ -882,6 +890,7 @@ __global__ void __launch_bounds__(256)
 // nodes share their i and j weights).
 __global__ void __launch_bounds__(256)
     k_prolong0bx2(const float *__restrict__ ec, LevelGeom cg, float *__restrict__ e, LevelGeom f, Split0 d) {
+  gc_after();
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   const int j = blockIdx.y * blockDim.y + threadIdx.y + 1;
   const int i = blockIdx.z + 1;
@@ -1183,6 +1192,7 @@ struct FlDown {
 __global__ void __launch_bounds__(FL_THREADS, 1)
     k_fine_down(const float *__restrict__ r, float *__restrict__ eb, float *__restrict__ bc, Split0 d, int m, int Jm,
                 int per) {
+  gc_after();
   using L = FL;
   extern __shared__ __align__(16) float fs[];
   for (int i = threadIdx.x; i < (int)(L::smem_down / sizeof(float)); i += FL_THREADS) fs[i] = 0.0f;
@@ -1376,6 +1386,7 @@ template <bool PLAIN>
 __global__ void __launch_bounds__(FL_THREADS, 1)
     k_fine_up(const float *__restrict__ ec, int m, const float *__restrict__ eb, const float *__restrict__ r, float *hi,
               float *lo, Split0 d, int per) {
+  gc_after();
   using L = FL;
   extern __shared__ __align__(16) float fs[];
   for (int i = threadIdx.x; i < (int)(L::smem_up / sizeof(float)); i += FL_THREADS) fs[i] = 0.0f;
@@ -1556,6 +1567,7 @@ __device__ __forceinline__ float blk_restrict(const float *p, int SI, const floa
 template <int NS, int CI>
 __global__ void __launch_bounds__(32 * BlkD<NS>::LJ, 1)
     k_block_down(float *__restrict__ e, const float *__restrict__ b, LevelGeom g, float *__restrict__ bc, LevelGeom cg) {
+  gc_after();
   using B = BlkD<NS>;
   constexpr int H = B::H, LJ = B::LJ, LI = 2 * CI + 3 + 2 * H;
   using Col = BlkCol<LI, LJ>;
@@ -1641,6 +1653,7 @@ template <int NS, int TI, int PHI>
 __global__ void __launch_bounds__(32 * BlkU<NS>::LJ, 1)
     k_block_up(const float *__restrict__ ec, LevelGeom cg, const float *__restrict__ e, const float *__restrict__ b,
                LevelGeom g, float *__restrict__ e_out, float *__restrict__ hi, float *__restrict__ lo) {
+  gc_after();
   using B = BlkU<NS>;
   constexpr int H = B::H, LJ = B::LJ, LI = TI + 2 * H;
   using Col = BlkCol<LI, LJ>;
@@ -1956,6 +1969,7 @@ __device__ __forceinline__ int t_node(int u, int n, int &sm) {
 }
 
 __global__ void __launch_bounds__(1024) k_tail(const float *__restrict__ b_in, float *__restrict__ e_out, TailDesc d) {
+  gc_after();
   extern __shared__ float tsm[];
   float *EA = tsm, *BA = EA + TL<4>::words, *RA = BA + TL<4>::words;
   float *EB = RA + TL<4>::words, *BB = EB + TL<3>::words, *RB = BB + TL<3>::words;
@@ -2283,7 +2297,7 @@ static int launch_tail(gc_ctx *ctx, const gc_mg_params *p) {
     GC_CUDA(ctx, cudaFuncSetAttribute(k_tail, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)TAIL_SMEM));
     ctx->tail_smem_set = 1;
   }
-  gc_launch(ctx, GK_TAIL, k_tail, dim3(1), dim3(1024), TAIL_SMEM, ctx->b[ctx->tail], ctx->e[ctx->tail], d);
+  gc_launch_after(ctx, GK_TAIL, k_tail, dim3(1), dim3(1024), TAIL_SMEM, ctx->b[ctx->tail], ctx->e[ctx->tail], d);
   GC_LAUNCH_CHECK(ctx, "tail");
   return GC_OK;
 }
@@ -2336,7 +2350,7 @@ static int blk_down(gc_ctx *ctx, int kid, float *e, const float *b, const LevelG
   const size_t smem = blk_down_smem<NS, CI>();
   if (smem > 48 * 1024)
     GC_CUDA(ctx, cudaFuncSetAttribute(k_block_down<NS, CI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  gc_launch(ctx, kid, k_block_down<NS, CI>, grid, dim3(32 * B::LJ), smem, e, b, g, bc, cg);
+  gc_launch_after(ctx, kid, k_block_down<NS, CI>, grid, dim3(32 * B::LJ), smem, e, b, g, bc, cg);
   GC_LAUNCH_CHECK(ctx, "block down");
   return GC_OK;
 }
@@ -2356,7 +2370,7 @@ static int blk_up(gc_ctx *ctx, int kid, const float *ec, const LevelGeom &cg, co
   if (smem > 48 * 1024)
     GC_CUDA(ctx,
             cudaFuncSetAttribute(k_block_up<NS, TI, PHI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-  gc_launch(ctx, kid, k_block_up<NS, TI, PHI>, grid, dim3(32 * B::LJ), smem, ec, cg, e, b, g, e_out, ctx->hi, ctx->lo);
+  gc_launch_after(ctx, kid, k_block_up<NS, TI, PHI>, grid, dim3(32 * B::LJ), smem, ec, cg, e, b, g, e_out, ctx->hi, ctx->lo);
   GC_LAUNCH_CHECK(ctx, "block up");
   return GC_OK;
 }
@@ -2398,7 +2412,7 @@ static int fine_down(gc_ctx *ctx) {
   const unsigned parts = gc_sms() > strips ? gc_sms() / strips : 1;
   const int per = (int)gc_blocks(cg.J, (int)parts);
   GC_CUDA(ctx, cudaFuncSetAttribute(k_fine_down, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::smem_down));
-  gc_launch(ctx, GK_SMOOTH0, k_fine_down, dim3(strips, gc_blocks(cg.J, per)), dim3(FL_THREADS), L::smem_down,
+  gc_launch_after(ctx, GK_SMOOTH0, k_fine_down, dim3(strips, gc_blocks(cg.J, per)), dim3(FL_THREADS), L::smem_down,
             ctx->r0s, ctx->e0s + ctx->half0, ctx->b[1], split0(ctx), cg.n, cg.J, per);
   GC_LAUNCH_CHECK(ctx, "fine down");
   return GC_OK;
@@ -2411,7 +2425,7 @@ static int fine_up(gc_ctx *ctx) {
   const unsigned parts = gc_sms() > strips ? gc_sms() / strips : 1;
   const int per = ((int)gc_blocks(g0.J, (int)parts) + 1) & ~1;  // even: a stretch starts on an odd plane
   GC_CUDA(ctx, cudaFuncSetAttribute(k_fine_up<PLAIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)L::smem_up));
-  gc_launch(ctx, GK_UPDATE0, k_fine_up<PLAIN>, dim3(strips, gc_blocks(g0.J, per)), dim3(FL_THREADS), L::smem_up,
+  gc_launch_after(ctx, GK_UPDATE0, k_fine_up<PLAIN>, dim3(strips, gc_blocks(g0.J, per)), dim3(FL_THREADS), L::smem_up,
             ctx->e[1], cg.n, ctx->e0s + ctx->half0, ctx->r0s, ctx->hi, ctx->lo, split0(ctx), per);
   GC_LAUNCH_CHECK(ctx, "fine up");
   return GC_OK;
@@ -2440,7 +2454,7 @@ static int coarse_levels(gc_ctx *ctx, const gc_mg_params *p) {
     GC_CUDA(ctx, cudaMemsetAsync(ctx->e[l], 0, n3 * sizeof(float), ctx->stream));
     if ((st = launch_smooth(ctx, l, pre))) return st;
     gc_launch(ctx, GK_RESID, k_resid, dim3(node_grid(g)), dim3(dim3(32, 8)), 0, ctx->e[l], ctx->b[l], ctx->rc, g);
-    gc_launch(ctx, GK_RESTRICT, k_restrict, dim3(node_grid(ctx->lev[l + 1])), dim3(dim3(32, 8)), 0, ctx->rc, g,
+    gc_launch_after(ctx, GK_RESTRICT, k_restrict, dim3(node_grid(ctx->lev[l + 1])), dim3(dim3(32, 8)), 0, ctx->rc, g,
               ctx->b[l + 1], ctx->lev[l + 1]);
     GC_LAUNCH_CHECK(ctx, "resid/restrict");
   }
@@ -2477,7 +2491,7 @@ static int residual0(gc_ctx *ctx, const gc_mg_params *p, const MgDecide *dec) {
     if ((st = gc_ensure_red(ctx, nq))) return st;
     auto k = natural ? (plain ? k_resid0x4<true, false> : k_resid0x4<false, false>)
                      : (plain ? k_resid0x4<true, true> : k_resid0x4<false, true>);
-    gc_launch(ctx, GK_RESID0, k, qg, dim3(32, 8), 0, ctx->hi, ctx->lo, ctx->b0, r, ef, ctx->red, d);
+    gc_launch_after(ctx, GK_RESID0, k, qg, dim3(32, 8), 0, ctx->hi, ctx->lo, ctx->b0, r, ef, ctx->red, d);
     GC_LAUNCH_CHECK(ctx, "resid0");
     // (a last-block sum of the 16k block partials in this kernel was slower: the
     // blocks' tickets serialise on one counter)
@@ -2485,7 +2499,7 @@ static int residual0(gc_ctx *ctx, const gc_mg_params *p, const MgDecide *dec) {
   }
   auto k = natural ? (plain ? k_resid0<true, false> : k_resid0<false, false>)
                    : (plain ? k_resid0<true, true> : k_resid0<false, true>);
-  gc_launch(ctx, GK_RESID0, k, grid, dim3(32, 8), 0, ctx->hi, ctx->lo, ctx->b0, r, ef, ctx->red, d);
+  gc_launch_after(ctx, GK_RESID0, k, grid, dim3(32, 8), 0, ctx->hi, ctx->lo, ctx->b0, r, ef, ctx->red, d);
   GC_LAUNCH_CHECK(ctx, "resid0");
   return finalize_to(ctx, (int)nb, GC_S_RNORM2, dec);
 }
@@ -2511,7 +2525,7 @@ static int vcycle(gc_ctx *ctx, const gc_mg_params *p, const MgDecide *dec) {
       gc_launch(ctx, GK_SMOOTH0, k_smooth, rb_grid(g0), dim3(RB_TX, RB_TY), 0, ctx->e0n, ctx->r0n, g0, h & 1);
     if (L > 1) {
       gc_launch(ctx, GK_RESIDE, k_resid, node_grid(g0), dim3(32, 8), 0, ctx->e0n, ctx->r0n, ctx->r0, g0);
-      gc_launch(ctx, GK_RESTRICT, k_restrict, node_grid(ctx->lev[1]), dim3(32, 8), 0, ctx->r0, g0, ctx->b[1],
+      gc_launch_after(ctx, GK_RESTRICT, k_restrict, node_grid(ctx->lev[1]), dim3(32, 8), 0, ctx->r0, g0, ctx->b[1],
                 ctx->lev[1]);
       GC_LAUNCH_CHECK(ctx, "natural resid/restrict");
       if ((st = coarse_levels(ctx, p))) return st;
@@ -2545,7 +2559,7 @@ static int vcycle(gc_ctx *ctx, const gc_mg_params *p, const MgDecide *dec) {
   const bool v4 = vec4(ctx);
   auto half_sweep = [&](int color) {
     if (v4)
-      gc_launch(ctx, GK_SMOOTH0, k_rb0x2<false>, sg2, SPLIT_BLOCK, 0, ctx->e0s, (const float *)ctx->r0s, d, color);
+      gc_launch_after(ctx, GK_SMOOTH0, k_rb0x2<false>, sg2, SPLIT_BLOCK, 0, ctx->e0s, (const float *)ctx->r0s, d, color);
     else
       gc_launch(ctx, GK_SMOOTH0, k_rb0<false>, sg, SPLIT_BLOCK, 0, ctx->e0s, (const float *)ctx->r0s, d, color);
   };
@@ -2554,17 +2568,17 @@ static int vcycle(gc_ctx *ctx, const gc_mg_params *p, const MgDecide *dec) {
   for (int h = 1; h < 2 * pre; ++h) half_sweep(h & 1);
   if (L > 1) {
     if (v4)
-      gc_launch(ctx, GK_RESIDE, k_resid0ex4, qg, dim3(32, 8), 0, (const float *)ctx->e0s, (const float *)ctx->r0s,
+      gc_launch_after(ctx, GK_RESIDE, k_resid0ex4, qg, dim3(32, 8), 0, (const float *)ctx->e0s, (const float *)ctx->r0s,
                 ctx->r0, d);
     else
       gc_launch(ctx, GK_RESIDE, k_resid0e, node_grid(g0), dim3(32, 8), 0, (const float *)ctx->e0s,
                 (const float *)ctx->r0s, ctx->r0, d);
-    gc_launch(ctx, GK_RESTRICT, k_restrict, node_grid(ctx->lev[1]), dim3(32, 8), 0, ctx->r0, g0, ctx->b[1],
+    gc_launch_after(ctx, GK_RESTRICT, k_restrict, node_grid(ctx->lev[1]), dim3(32, 8), 0, ctx->r0, g0, ctx->b[1],
               ctx->lev[1]);
     GC_LAUNCH_CHECK(ctx, "resid0e/restrict");
     if ((st = coarse_levels(ctx, p))) return st;
     if (v4 && post >= 1)
-      gc_launch(ctx, GK_PROLONG0, k_prolong0bx2, sg2, SPLIT_BLOCK, 0, (const float *)ctx->e[1], ctx->lev[1], ctx->e0s,
+      gc_launch_after(ctx, GK_PROLONG0, k_prolong0bx2, sg2, SPLIT_BLOCK, 0, (const float *)ctx->e[1], ctx->lev[1], ctx->e0s,
                 g0, d);
     else
       gc_launch(ctx, GK_PROLONG0, k_prolong0s, sg, SPLIT_BLOCK, 0, (const float *)ctx->e[1], ctx->lev[1], ctx->e0s,
@@ -2573,10 +2587,10 @@ static int vcycle(gc_ctx *ctx, const gc_mg_params *p, const MgDecide *dec) {
   }
   if (post >= 1 && v4) {  // last half-sweep (black) and phi += e in one pass
     if (plain)
-      gc_launch(ctx, GK_UPDATE0, k_rb0_lastx4<true>, sg2, SPLIT_BLOCK, 0, (const float *)ctx->e0s,
+      gc_launch_after(ctx, GK_UPDATE0, k_rb0_lastx4<true>, sg2, SPLIT_BLOCK, 0, (const float *)ctx->e0s,
                 (const float *)ctx->r0s, ctx->hi, ctx->lo, d);
     else
-      gc_launch(ctx, GK_UPDATE0, k_rb0_lastx4<false>, sg2, SPLIT_BLOCK, 0, (const float *)ctx->e0s,
+      gc_launch_after(ctx, GK_UPDATE0, k_rb0_lastx4<false>, sg2, SPLIT_BLOCK, 0, (const float *)ctx->e0s,
                 (const float *)ctx->r0s, ctx->hi, ctx->lo, d);
   } else if (post >= 1) {  // last half-sweep (black) and phi += e in one pass
     if (plain)
@@ -2603,11 +2617,11 @@ static int finalize_one(gc_ctx *ctx, const double *parts, int nparts, double *ds
   if (dec) d = *dec;
   if (nparts > 32 * GC_FIN_CHUNKS) {
     double *tmp = ctx->dsmall + GC_S_FIN_TMP;
-    gc_launch(ctx, GK_REDUCE, k_fin_chunks, dim3(GC_FIN_CHUNKS), dim3(256), 0, parts, nparts, tmp);
+    gc_launch_after(ctx, GK_REDUCE, k_fin_chunks, dim3(GC_FIN_CHUNKS), dim3(256), 0, parts, nparts, tmp);
     parts = tmp;
     nparts = GC_FIN_CHUNKS;
   }
-  gc_launch(ctx, GK_REDUCE, k_fin_one, dim3(1), dim3(256), 0, parts, nparts, dst, ctx->dsmall, d);
+  gc_launch_after(ctx, GK_REDUCE, k_fin_one, dim3(1), dim3(256), 0, parts, nparts, dst, ctx->dsmall, d);
   GC_LAUNCH_CHECK(ctx, "finalize");
   return GC_OK;
 }
