@@ -178,12 +178,14 @@ static inline void gc_launch(gc_ctx *ctx, int kid, void (*k)(KArgs...), dim3 gri
   if (slot >= 0) cudaEventRecord(ctx->prof.ev[2 * slot + 1], ctx->stream);
 }
 
-// The same for kernels that begin with gc_after(): the grid may be scheduled while the
-// kernel before it in the stream still runs, and waits in gc_after() until that kernel has
-// completed and its writes are visible, so a chain of short kernels does not pay a launch
-// each (the 14 of a V-cycle at 64^3: a step of 2.2 cycles 221 -> 210 us; six cycles at 97^3
-// 728 -> 708). Only for grids of at most 2048 blocks: with the thousands of blocks of the
-// 256^3 passes too, eight cycles took 3523 us, 3393 with none, 3350 so.
+// The same for kernels that begin with gc_after(): the grid is scheduled as the last blocks
+// of the kernel before it in the stream end, and waits in gc_after() until that kernel has
+// completed and its writes are visible, so a chain of short kernels does not pay a whole
+// launch each: a step of 131k particles at 64^3 221 -> 211 us, a training step of the
+// warm-start network at R = 64 695 -> 575, its forward pass at R = 128 455 -> 413, a chain
+// step of 250k particles 450 -> 422. No kernel lets the next one in earlier
+// (griddepcontrol.launch_dependents): read-only loads would then overlap the writes they
+// depend on, and eight cycles at 256^3 took 3523 us instead of 3388.
 template <typename... KArgs, typename... Args>
 static inline void gc_launch_after(gc_ctx *ctx, int kid, void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem,
                                    Args &&...args) {
@@ -197,18 +199,17 @@ static inline void gc_launch_after(gc_ctx *ctx, int kid, void (*k)(KArgs...), di
   cfg.stream = ctx->stream;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = (size_t)grid.x * grid.y * grid.z <= 2048;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
   cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(std::forward<Args>(args))...);
   if (slot >= 0) cudaEventRecord(ctx->prof.ev[2 * slot + 1], ctx->stream);
 }
 
-// First statement of a kernel launched with gc_launch_after: the kernel before it is
-// complete; then the kernel after it may be scheduled.
+// First statement of a kernel launched with gc_launch_after (behind set-up that touches
+// nothing of other kernels): the kernel before it is complete.
 __device__ __forceinline__ void gc_after() {
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
 
 // Kernel launches counted on ctx so far (all ids).

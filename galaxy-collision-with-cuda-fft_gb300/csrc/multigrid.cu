@@ -2068,6 +2068,7 @@ __global__ void __launch_bounds__(1024) k_tail(const float *__restrict__ b_in, f
 __global__ void __launch_bounds__(256)
     k_faces(float *__restrict__ hi, float *__restrict__ lo, int G,
             double dx, double grav, const double *__restrict__ mom) {
+  gc_after();
   // centre of mass and second moments about it, once per block (FP64 runs at a
   // small fraction of the f32 rate: each face node keeps only its own terms)
   __shared__ double sm[11];
@@ -2148,6 +2149,7 @@ __global__ void __launch_bounds__(256, 2)
     k_rhs_moments(const float *__restrict__ rho, float *__restrict__ b0, int G, double dx, float fpg, float h2,
                   double *__restrict__ parts, unsigned *__restrict__ ticket, double *__restrict__ mom,
                   double *__restrict__ bnorm2, unsigned *__restrict__ status) {
+  gc_after();
   __shared__ double wsum[8 * MOM_COLS][11];
   __shared__ double bsum[1];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -2647,7 +2649,7 @@ static int read_small(gc_ctx *ctx, int slot, int count) {
 
 int gc_faces_from_moments(gc_ctx *ctx) {
   const long long tot = 6LL * ctx->G * ctx->G;
-  gc_launch(ctx, GK_FACES, k_faces, dim3(gc_blocks(tot, 256)), dim3(256), 0, ctx->hi, ctx->lo, ctx->G, ctx->dx, ctx->grav, ctx->dmom);
+  gc_launch_after(ctx, GK_FACES, k_faces, dim3(gc_blocks(tot, 256)), dim3(256), 0, ctx->hi, ctx->lo, ctx->G, ctx->dx, ctx->grav, ctx->dmom);
   GC_LAUNCH_CHECK(ctx, "faces");
   return GC_OK;
 }
@@ -2870,7 +2872,7 @@ static int rhs_moments_async(gc_ctx *ctx, const float *rho, float *b0) {
   int s = gc_ensure_red(ctx, (size_t)nb * 11);
   if (s) return s;
   // b0 = h^2 * 4 pi G rho (multigrid.py:463)
-  gc_launch(ctx, b0 ? GK_RHS : GK_MOMENTS, k_rhs_moments, dim3(nb), dim3(256), 0, rho, b0, ctx->G, ctx->dx,
+  gc_launch_after(ctx, b0 ? GK_RHS : GK_MOMENTS, k_rhs_moments, dim3(nb), dim3(256), 0, rho, b0, ctx->G, ctx->dx,
             (float)(4.0 * M_PI * ctx->grav), (float)(ctx->dx * ctx->dx), ctx->red,
             reinterpret_cast<unsigned *>(ctx->dsmall + GC_S_TICKET), ctx->dmom, ctx->dsmall + GC_S_BNORM2,
             ctx->dstatus);

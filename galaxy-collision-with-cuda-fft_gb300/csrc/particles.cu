@@ -27,6 +27,7 @@
 // all n terms stays below 2^62, and the integers are summed exactly.
 __global__ void __launch_bounds__(256) k_mass_max(const float *__restrict__ m, long long n, float inv_vol,
                                                   unsigned *__restrict__ maxbits) {
+  gc_after();
   unsigned best = 0;
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
     const float mm = __fmul_rn(m[p], inv_vol);
@@ -44,6 +45,7 @@ __device__ __forceinline__ int mass_shift(unsigned maxbits, int log2n) {
 __global__ void __launch_bounds__(256) k_mass_isum(const float *__restrict__ m, long long n, float inv_vol,
                                                    const unsigned *__restrict__ maxbits, int log2n,
                                                    unsigned long long *__restrict__ isum) {
+  gc_after();
   const int s = mass_shift(*maxbits, log2n);
   unsigned long long acc = 0;
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
@@ -64,6 +66,7 @@ __global__ void __launch_bounds__(256) k_mass_isum(const float *__restrict__ m, 
 // E = exponent(S) - bits so that the whole mass is at most 2^bits quanta.
 __global__ void k_qexp(const unsigned *__restrict__ maxbits, const unsigned long long *__restrict__ isum, int log2n,
                        double *__restrict__ small, int mass_slot, int exp_slot, int bits) {
+  gc_after();
   if (threadIdx.x != 0) return;
   double S = 0.0;
   if (*maxbits) S = ldexp((double)(*isum), -mass_shift(*maxbits, log2n));
@@ -94,9 +97,9 @@ int gc_fixed_point_setup(gc_ctx *ctx, const float *m, int64_t n, int bits, int m
   unsigned nb = gc_blocks(n, 256);
   if (nb > gc_sms() * 8u) nb = gc_sms() * 8u;
   const int L = ceil_log2((long long)n);
-  gc_launch(ctx, GK_MASS, k_mass_max, dim3(nb), dim3(256), 0, m, (long long)n, inv_vol, maxbits);
-  gc_launch(ctx, GK_MASS, k_mass_isum, dim3(nb), dim3(256), 0, m, (long long)n, inv_vol, maxbits, L, isum);
-  gc_launch(ctx, GK_MASS, k_qexp, dim3(1), dim3(32), 0, maxbits, isum, L, ctx->dsmall, mass_slot, exp_slot, bits);
+  gc_launch_after(ctx, GK_MASS, k_mass_max, dim3(nb), dim3(256), 0, m, (long long)n, inv_vol, maxbits);
+  gc_launch_after(ctx, GK_MASS, k_mass_isum, dim3(nb), dim3(256), 0, m, (long long)n, inv_vol, maxbits, L, isum);
+  gc_launch_after(ctx, GK_MASS, k_qexp, dim3(1), dim3(32), 0, maxbits, isum, L, ctx->dsmall, mass_slot, exp_slot, bits);
   GC_LAUNCH_CHECK(ctx, "fixed-point set-up");
   return GC_OK;
 }
@@ -691,6 +694,7 @@ __global__ void __launch_bounds__(32 * WARPS, (WIDE ? 3 : 4) * (8 / WARPS))
                      const float *__restrict__ m, long long n, DepCtx d, float inv_dx,
                      const double *__restrict__ qexp, long long *__restrict__ qg, unsigned *__restrict__ status,
                      const int *__restrict__ skip) {
+  gc_after();
   __shared__ int dep_box[WARPS * DepW<WIDE>::words];
   if (skip && *skip) return;  // scattered particles: the binned passes take them
   const float qscale = ldexpf(1.0f, -(int)(*qexp));
@@ -862,6 +866,7 @@ __device__ __forceinline__ int bin_of(float px, float py, float pz, const DepCtx
 __global__ void __launch_bounds__(1024)
     k_bin_probe(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z, long long n,
                 float dx, int G, int box, int *__restrict__ scattered) {
+  gc_after();
   __shared__ int fit[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int fits = 0;
@@ -905,6 +910,7 @@ __global__ void __launch_bounds__(512)
     k_bin_count(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z, long long n,
                 DepCtx d, float inv_dx, int per, BinScratch *__restrict__ sc, int2 *__restrict__ items,
                 unsigned *__restrict__ status) {
+  gc_after();
   __shared__ int hist[BIN_MAX];
   __shared__ int wsum[2][16];
   __shared__ bool last_s;
@@ -989,6 +995,7 @@ __global__ void __launch_bounds__(512, 2)
     k_bin_scatter(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
                   const float *__restrict__ m, long long n, DepCtx d, float inv_dx, const double *__restrict__ qexp,
                   BinScratch *__restrict__ sc, float4 *__restrict__ out, int *__restrict__ rare) {
+  gc_after();
   __shared__ int hist[BIN_MAX];
   if (!sc->scattered) return;
   const float qscale = ldexpf(1.0f, -(int)(*qexp));
@@ -1038,6 +1045,7 @@ __global__ void __launch_bounds__(512, 2)
 __global__ void __launch_bounds__(256)
     k_bin_deposit(const float4 *__restrict__ part, int G, int per, const BinScratch *__restrict__ sc,
                   const int2 *__restrict__ items, long long *__restrict__ qg) {
+  gc_after();
   __shared__ int lo[BIN_NODES], hi[BIN_NODES];
   __shared__ int4 cur;  // the item: first and last particle, tile
   if (!sc->scattered) return;
@@ -1101,6 +1109,7 @@ __global__ void __launch_bounds__(256)
     k_bin_rare(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
                const float *__restrict__ m, DepCtx d, float inv_dx, const double *__restrict__ qexp,
                const BinScratch *__restrict__ sc, const int *__restrict__ rare, long long *__restrict__ qg) {
+  gc_after();
   if (!sc->scattered) return;
   const float qscale = ldexpf(1.0f, -(int)(*qexp));
   const int n = sc->nrare;
@@ -1180,9 +1189,9 @@ int gc_deposit_q(gc_ctx *ctx, const float *x, const float *y, const float *z, co
                     bin_scratch(ctx, n);
   BinScratch *sc = bins ? (BinScratch *)ctx->bin : nullptr;
   if (bins)
-    gc_launch(ctx, GK_DEPOSIT_RUNS, k_bin_probe, dim3(1), dim3(1024), 0, x, y, z, (long long)n, d.dx, ctx->G,
+    gc_launch_after(ctx, GK_DEPOSIT_RUNS, k_bin_probe, dim3(1), dim3(1024), 0, x, y, z, (long long)n, d.dx, ctx->G,
               wide ? (int)DepW<true>::box : (int)DepW<false>::box, &sc->scattered);
-  gc_launch(ctx, GK_DEPOSIT_RUNS, k, dim3(nb), dim3(32 * warps), 0, x, y, z, m, (long long)n, d, inv_dx, qexp, ctx->q,
+  gc_launch_after(ctx, GK_DEPOSIT_RUNS, k, dim3(nb), dim3(32 * warps), 0, x, y, z, m, (long long)n, d, inv_dx, qexp, ctx->q,
             ctx->dstatus, bins ? (const int *)&sc->scattered : (const int *)nullptr);
   if (bins) {
     const size_t head = (sizeof(BinScratch) + 255) & ~(size_t)255;
@@ -1194,14 +1203,14 @@ int gc_deposit_q(gc_ctx *ctx, const float *x, const float *y, const float *z, co
     const unsigned sms = (unsigned)gc_sms();
     auto k1 = pow2 ? k_bin_count<true> : k_bin_count<false>;
     auto k2 = pow2 ? k_bin_scatter<true> : k_bin_scatter<false>;
-    gc_launch(ctx, GK_DEPOSIT_RUNS, k1, dim3(std::min(gc_blocks(n, 2048), sms * 3u)), dim3(512), 0, x, y, z, (long long)n,
+    gc_launch_after(ctx, GK_DEPOSIT_RUNS, k1, dim3(std::min(gc_blocks(n, 2048), sms * 3u)), dim3(512), 0, x, y, z, (long long)n,
               d, inv_dx, per, sc, items, ctx->dstatus);
-    gc_launch(ctx, GK_DEPOSIT_RUNS, k2, dim3(std::min(gc_blocks(n, 2048), sms * 2u)), dim3(512), 0, x, y, z, m,
+    gc_launch_after(ctx, GK_DEPOSIT_RUNS, k2, dim3(std::min(gc_blocks(n, 2048), sms * 2u)), dim3(512), 0, x, y, z, m,
               (long long)n, d, inv_dx, qexp, sc, copy, rare);
-    gc_launch(ctx, GK_DEPOSIT_RUNS, k_bin_deposit, dim3(sms * 5u), dim3(256), 0, (const float4 *)copy, ctx->G, per,
+    gc_launch_after(ctx, GK_DEPOSIT_RUNS, k_bin_deposit, dim3(sms * 5u), dim3(256), 0, (const float4 *)copy, ctx->G, per,
               (const BinScratch *)sc, (const int2 *)items, ctx->q);
     auto k4 = pow2 ? k_bin_rare<true> : k_bin_rare<false>;
-    gc_launch(ctx, GK_DEPOSIT_RUNS, k4, dim3(sms), dim3(256), 0, x, y, z, m, d, inv_dx, qexp, (const BinScratch *)sc,
+    gc_launch_after(ctx, GK_DEPOSIT_RUNS, k4, dim3(sms), dim3(256), 0, x, y, z, m, d, inv_dx, qexp, (const BinScratch *)sc,
               (const int *)rare, ctx->q);
   }
   GC_LAUNCH_CHECK(ctx, "deposit");
@@ -1255,6 +1264,7 @@ __global__ void __launch_bounds__(CQ_THREADS, 3)
                 float *__restrict__ rho, float *__restrict__ b, double bfac, double *__restrict__ parts,
                 unsigned *__restrict__ ticket, long long *__restrict__ limbs, double *__restrict__ mom,
                 double *__restrict__ bnorm2) {
+  gc_after();
   __shared__ CqCol cols[2][32];
   __shared__ long long red[3][12][33];
   __shared__ double bsum[4];
@@ -1424,7 +1434,7 @@ int gc_convert_q(gc_ctx *ctx, const double *qexp, float *rho_out, float *b_out) 
   int s = gc_ensure_red(ctx, (size_t)nb * 11);
   if (s) return s;
   const double bfac = 4.0 * M_PI * ctx->grav * ctx->dx * ctx->dx;
-  gc_launch(ctx, GK_CONVERT_Q, k_convert_q, dim3(nb), dim3(CQ_THREADS), 0, ctx->q, ctx->G, cpw, ctx->dx, qexp, rho_out, b_out,
+  gc_launch_after(ctx, GK_CONVERT_Q, k_convert_q, dim3(nb), dim3(CQ_THREADS), 0, ctx->q, ctx->G, cpw, ctx->dx, qexp, rho_out, b_out,
             bfac, ctx->red, reinterpret_cast<unsigned *>(ctx->dsmall + GC_S_TICKET),
             reinterpret_cast<long long *>(ctx->dsmall + GC_S_LIMBS), ctx->dmom, ctx->dsmall + GC_S_BNORM2);
   GC_LAUNCH_CHECK(ctx, "convert q");
@@ -1474,6 +1484,7 @@ __host__ static GradCtx make_grad(const gc_ctx *ctx) {
 __global__ void __launch_bounds__(256)
     k_grad(const float *__restrict__ phi, float *__restrict__ ax, float *__restrict__ ay, float *__restrict__ az,
            GradCtx g) {
+  gc_after();
   const int k = blockIdx.x * 32 + threadIdx.x;
   const int j = blockIdx.y * 8 + threadIdx.y;
   const int i = blockIdx.z;
@@ -1489,7 +1500,7 @@ extern "C" int gc_potential_to_accel(gc_ctx *ctx, const float *phi, float *ax, f
   if (!ctx) return GC_ERR_ARG;
   GC_REQUIRE(ctx, phi && ax && ay && az, "gc_potential_to_accel: NULL pointer");
   const GradCtx g = make_grad(ctx);
-  gc_launch(ctx, GK_GRAD, k_grad, dim3(dim3(gc_blocks(g.G, 32), gc_blocks(g.G, 8), g.G)), dim3(dim3(32, 8)), 0, phi, ax, ay, az, g);
+  gc_launch_after(ctx, GK_GRAD, k_grad, dim3(dim3(gc_blocks(g.G, 32), gc_blocks(g.G, 8), g.G)), dim3(dim3(32, 8)), 0, phi, ax, ay, az, g);
   GC_LAUNCH_CHECK(ctx, "grad");
   return GC_OK;
 }
@@ -1503,6 +1514,7 @@ __global__ void __launch_bounds__(256)
              const float *__restrict__ axg, const float *__restrict__ ayg, const float *__restrict__ azg,
              float *__restrict__ ax, float *__restrict__ ay, float *__restrict__ az, float dx, int G,
              const int *__restrict__ skip) {
+  gc_after();
   if (skip && *skip) return;
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
@@ -1539,6 +1551,7 @@ __global__ void __launch_bounds__(256)
 __global__ void __launch_bounds__(256)
     k_pack_fields(const float *__restrict__ axg, const float *__restrict__ ayg, const float *__restrict__ azg, size_t n,
                   const int *__restrict__ scattered, float4 *__restrict__ g4) {
+  gc_after();
   if (!*scattered) return;
   for (size_t i = blockIdx.x * (size_t)256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256)
     g4[i] = make_float4(axg[i], ayg[i], azg[i], 0.0f);
@@ -1555,6 +1568,7 @@ __global__ void __launch_bounds__(256)
     k_gather_packed(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z, long long n,
                     const int *__restrict__ scattered, const float4 *__restrict__ g4, float *__restrict__ ax,
                     float *__restrict__ ay, float *__restrict__ az, float dx, int G) {
+  gc_after();
   if (!*scattered) return;
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
@@ -1615,16 +1629,16 @@ extern "C" int gc_gather_accel(gc_ctx *ctx, const float *x, const float *y, cons
     const size_t g3 = (size_t)ctx->G * ctx->G * ctx->G;
     float4 *g4 = (float4 *)ctx->g4;
     int *scattered = reinterpret_cast<int *>(ctx->dsmall + GC_S_SCATTERED);
-    gc_launch(ctx, GK_GATHER, k_bin_probe, dim3(1), dim3(1024), 0, x, y, z, (long long)n, (float)ctx->dx, ctx->G,
+    gc_launch_after(ctx, GK_GATHER, k_bin_probe, dim3(1), dim3(1024), 0, x, y, z, (long long)n, (float)ctx->dx, ctx->G,
               (int)DepW<false>::box, scattered);
-    gc_launch(ctx, GK_GATHER, k_pack_fields, dim3(gc_sms() * 16u), dim3(256), 0, ax_g, ay_g, az_g, g3,
+    gc_launch_after(ctx, GK_GATHER, k_pack_fields, dim3(gc_sms() * 16u), dim3(256), 0, ax_g, ay_g, az_g, g3,
               (const int *)scattered, g4);
-    gc_launch(ctx, GK_GATHER, k_gather, dim3(nb), dim3(256), 0, x, y, z, (long long)n, ax_g, ay_g, az_g, acc_x, acc_y,
+    gc_launch_after(ctx, GK_GATHER, k_gather, dim3(nb), dim3(256), 0, x, y, z, (long long)n, ax_g, ay_g, az_g, acc_x, acc_y,
               acc_z, (float)ctx->dx, ctx->G, (const int *)scattered);
-    gc_launch(ctx, GK_GATHER, k_gather_packed, dim3(std::min(nb, gc_sms() * 16u)), dim3(256), 0, x, y, z, (long long)n,
+    gc_launch_after(ctx, GK_GATHER, k_gather_packed, dim3(std::min(nb, gc_sms() * 16u)), dim3(256), 0, x, y, z, (long long)n,
               (const int *)scattered, (const float4 *)g4, acc_x, acc_y, acc_z, (float)ctx->dx, ctx->G);
   } else {
-    gc_launch(ctx, GK_GATHER, k_gather, dim3(nb), dim3(256), 0, x, y, z, (long long)n, ax_g, ay_g, az_g, acc_x, acc_y,
+    gc_launch_after(ctx, GK_GATHER, k_gather, dim3(nb), dim3(256), 0, x, y, z, (long long)n, ax_g, ay_g, az_g, acc_x, acc_y,
               acc_z, (float)ctx->dx, ctx->G, (const int *)nullptr);
   }
   GC_LAUNCH_CHECK(ctx, "gather");
@@ -1637,6 +1651,7 @@ extern "C" int gc_gather_accel(gc_ctx *ctx, const float *x, const float *y, cons
 __global__ void __launch_bounds__(256) k_axpy3(float *__restrict__ u, float *__restrict__ v, float *__restrict__ w,
                                                const float *__restrict__ a, const float *__restrict__ b,
                                                const float *__restrict__ c, long long n, float dt) {
+  gc_after();
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
     u[p] = __fadd_rn(u[p], __fmul_rn(a[p], dt));
     v[p] = __fadd_rn(v[p], __fmul_rn(b[p], dt));
@@ -1650,6 +1665,7 @@ __global__ void __launch_bounds__(256) k_axpy3(float *__restrict__ u, float *__r
 __global__ void __launch_bounds__(256)
     k_axpy3x4(float4 *__restrict__ u, float4 *__restrict__ v, float4 *__restrict__ w, const float4 *__restrict__ a,
               const float4 *__restrict__ b, const float4 *__restrict__ c, long long n, float dt) {
+  gc_after();
   const long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x;
   if (4 * p + 3 < n) {
     float4 U = u[p], V = v[p], W = w[p];
@@ -1680,13 +1696,13 @@ static int axpy3(gc_ctx *ctx, float *u, float *v, float *w, const float *a, cons
   GC_REQUIRE(ctx, u && v && w && a && b && c, "%s: NULL pointer", what);
   const uintptr_t all = (uintptr_t)u | (uintptr_t)v | (uintptr_t)w | (uintptr_t)a | (uintptr_t)b | (uintptr_t)c;
   if ((all & 15) == 0) {
-    gc_launch(ctx, GK_AXPY, k_axpy3x4, dim3(gc_blocks((n + 3) / 4, 256)), dim3(256), 0, reinterpret_cast<float4 *>(u),
+    gc_launch_after(ctx, GK_AXPY, k_axpy3x4, dim3(gc_blocks((n + 3) / 4, 256)), dim3(256), 0, reinterpret_cast<float4 *>(u),
               reinterpret_cast<float4 *>(v), reinterpret_cast<float4 *>(w), reinterpret_cast<const float4 *>(a),
               reinterpret_cast<const float4 *>(b), reinterpret_cast<const float4 *>(c), (long long)n, dt);
   } else {
     unsigned nb = gc_blocks(n, 256);
     if (nb > gc_sms() * 32u) nb = gc_sms() * 32u;
-    gc_launch(ctx, GK_AXPY, k_axpy3, dim3(nb), dim3(256), 0, u, v, w, a, b, c, (long long)n, dt);
+    gc_launch_after(ctx, GK_AXPY, k_axpy3, dim3(nb), dim3(256), 0, u, v, w, a, b, c, (long long)n, dt);
   }
   GC_LAUNCH_CHECK(ctx, what);
   return GC_OK;
@@ -1866,6 +1882,7 @@ __global__ void __launch_bounds__(256)
 // one pass over phi writes it (k_grad4), then each particle reads its 8 corner
 // nodes with one 16-byte load each. Same arithmetic as gather_grad.
 __global__ void __launch_bounds__(256) k_grad4(const float *__restrict__ phi, float4 *__restrict__ g4, GradCtx g) {
+  gc_after();
   const int k = blockIdx.x * 32 + threadIdx.x;
   const int j = blockIdx.y * 8 + threadIdx.y;
   const int i = blockIdx.z;
@@ -2132,6 +2149,7 @@ __global__ void __launch_bounds__(256)
                   float *__restrict__ vy, float *__restrict__ vz, const float *__restrict__ m, long long n,
                   const float4 *__restrict__ g4, FusedCtx f, DepCtx d, float inv_dx, const double *__restrict__ qexp,
                   long long *__restrict__ qg, unsigned *__restrict__ status) {
+  gc_after();
   using namespace umma;
   constexpr int NA = DEP ? 7 : 6;
   extern __shared__ __align__(128) float gt_smem[];
@@ -2246,7 +2264,7 @@ int gc_gather_kick_drift(gc_ctx *ctx, const gc_particles *p, float dt, int mode,
     const size_t g3 = (size_t)ctx->G * ctx->G * ctx->G;
     if (!ctx->g4) GC_CUDA(ctx, cudaMalloc(&ctx->g4, g3 * sizeof(float4)));
     const GradCtx g = make_grad(ctx);
-    gc_launch(ctx, GK_GRAD, k_grad4, dim3(gc_blocks(g.G, 32), gc_blocks(g.G, 8), g.G), dim3(32, 8), 0, ctx->hi,
+    gc_launch_after(ctx, GK_GRAD, k_grad4, dim3(gc_blocks(g.G, 32), gc_blocks(g.G, 8), g.G), dim3(32, 8), 0, ctx->hi,
               (float4 *)ctx->g4, g);
     int fe = 0;
     const bool pow2 = std::frexp(f.dx, &fe) == 0.5f;  // then inv_dx is exact
@@ -2272,7 +2290,7 @@ int gc_gather_kick_drift(gc_ctx *ctx, const gc_particles *p, float dt, int mode,
       const float inv_dx_dep = pow2 ? std::ldexp(1.0f, 1 - fe) : 0.0f;
       auto k = dep ? (pow2 ? k_gather4_tma<true, true> : k_gather4_tma<false, true>)
                    : (pow2 ? k_gather4_tma<true, false> : k_gather4_tma<false, false>);
-      gc_launch(ctx, GK_GATHER_KD, k, dim3(nbt), dim3(256), GT_SMEM(dep), p->x, p->y, p->z, p->vx, p->vy, p->vz, p->m,
+      gc_launch_after(ctx, GK_GATHER_KD, k, dim3(nbt), dim3(256), GT_SMEM(dep), p->x, p->y, p->z, p->vx, p->vy, p->vz, p->m,
                 (long long)p->n, (const float4 *)ctx->g4, f, d, inv_dx_dep, (const double *)(ctx->dsmall + GC_S_QEXP_PM),
                 ctx->q, ctx->dstatus);
       if (dep && deposited) *deposited = 1;

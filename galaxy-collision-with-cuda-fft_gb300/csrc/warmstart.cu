@@ -261,7 +261,6 @@ __global__ void __launch_bounds__(256) k_conv_fwd(const __grid_constant__ ConvFw
   uint64_t *bars = reinterpret_cast<uint64_t *>(ring + 2u * slot_bytes);
   uint32_t *tslot = reinterpret_cast<uint32_t *>(bars + 3);
   float *bias = reinterpret_cast<float *>(bars + 8);
-  if (tid < Cn) bias[tid] = a.bias ? a.bias[c0 + tid] : 0.0f;
   const int ngroups = (27 + a.tpg - 1) / a.tpg;
 
   if (warp == 0) {
@@ -273,12 +272,15 @@ __global__ void __launch_bounds__(256) k_conv_fwd(const __grid_constant__ ConvFw
     umma::mbar_init(&bars[1], WS_ISSUERS);
     umma::mbar_init(&bars[2], 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    if (a.use_map) {
-      umma::fence_async_smem();
-      umma::mbar_arrive_expect_tx(&bars[2], (uint32_t)(kci * V) * 16u);
-      umma::tma_load_4d(sm, &a.map, -2, y0 - 1, z0 - 1, 0, &bars[2]);
-    }
   }
+  __syncthreads();
+  gc_after();  // (behind the allocation: a grid behind this one must not get Tensor Memory first)
+  if (tid == 0 && a.use_map) {
+    umma::fence_async_smem();
+    umma::mbar_arrive_expect_tx(&bars[2], (uint32_t)(kci * V) * 16u);
+    umma::tma_load_4d(sm, &a.map, -2, y0 - 1, z0 - 1, 0, &bars[2]);
+  }
+  if (tid < Cn) bias[tid] = a.bias ? a.bias[c0 + tid] : 0.0f;
   // input tile, zero outside the grid, plus a zero margin read by the last M tile: one
   // box of the tensor map (1.2k clk for 23 KB), or one warp per padded line with lanes
   // along x (10k clk) where a line is longer than a box may be
@@ -449,7 +451,6 @@ __global__ void __launch_bounds__(MA_THREADS) k_conv_march(const __grid_constant
   uint64_t *done = wbar + 1;                                     // every MMA of the CTA is complete
   uint32_t *tslot = reinterpret_cast<uint32_t *>(done + 1);
   float *bias = reinterpret_cast<float *>(full + 2 * MA_MAX_SLOTS + 8);
-  if (tid < Cn) bias[tid] = a.bias ? a.bias[c0 + tid] : 0.0f;
   if (warp == 0) {
     umma::tmem_alloc(tslot, a.tmem_cols);
     umma::tmem_relinquish();
@@ -471,6 +472,9 @@ __global__ void __launch_bounds__(MA_THREADS) k_conv_march(const __grid_constant
   __syncthreads();
   umma::tc_fence_after();
   const uint32_t tmem = *tslot;
+  gc_after();  // (behind the allocation: a grid behind this one must not get Tensor Memory first)
+  // read after the weights have arrived, which these threads announce
+  if (tid < Cn) bias[tid] = a.bias ? a.bias[c0 + tid] : 0.0f;
   const int nbx = R / a.BX;
   const int u0 = (int)((long long)a.units * blockIdx.x / gridDim.x);
   const int u1 = (int)((long long)a.units * (blockIdx.x + 1) / gridDim.x);
@@ -698,6 +702,7 @@ __global__ void __launch_bounds__(WG_THREADS) k_conv_wgrad(const __grid_constant
   __syncthreads();
   umma::tc_fence_after();
   const uint32_t tmem = *tslot;
+  gc_after();  // (behind the allocation: a grid behind this one must not get Tensor Memory first)
   bool ok = true;
   int nb = 0;  // blocks done: parity of the tile's barriers
 
@@ -864,6 +869,7 @@ __device__ __forceinline__ void reduce_col(const float *__restrict__ part, int n
 }
 __global__ void __launch_bounds__(256) k_reduce_cols(const float *__restrict__ part, int nparts, int nelem,
                                                      float *__restrict__ out) {
+  gc_after();
   reduce_col(part, nparts, nelem, blockIdx.x, out);
 }
 
@@ -889,6 +895,7 @@ __device__ __forceinline__ void reduce_run(const float *__restrict__ p, size_t s
   }
 }
 __global__ void __launch_bounds__(64) k_wgrad_reduce(const __grid_constant__ WgReduce d) {
+  gc_after();
   const WgReduce::Layer &L = d.l[blockIdx.y];
   for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < L.nelem; e += gridDim.x * blockDim.x) {
     float s = 0.0f;
@@ -914,6 +921,7 @@ static dim3 line_grid(int Rl, int kc, int tpb) { return dim3((Rl + tpb - 1) / tp
 
 // out (R/2) = mean of the 8 children of in (R)
 __global__ void __launch_bounds__(64) k_pool2(const uint4 *__restrict__ in, uint4 *__restrict__ out, int R) {
+  gc_after();
   const int Rc = R >> 1;
   const int K = blockIdx.x * blockDim.x + threadIdx.x, J = blockIdx.y, c = blockIdx.z / Rc, I = blockIdx.z - c * Rc;
   if (K >= Rc) return;
@@ -934,6 +942,7 @@ __global__ void __launch_bounds__(64) k_pool2(const uint4 *__restrict__ in, uint
 // out (R) = relu(u[parent] + skip)
 __global__ void __launch_bounds__(64) k_up_add_relu(const uint4 *__restrict__ u, const uint4 *__restrict__ skip,
                                                     uint4 *__restrict__ out, int R) {
+  gc_after();
   const int Rc = R >> 1;
   const int z = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, c = blockIdx.z / R, x = blockIdx.z - c * R;
   if (z >= R) return;
@@ -949,6 +958,7 @@ __global__ void __launch_bounds__(64) k_up_add_relu(const uint4 *__restrict__ u,
 
 // out (R/2) = sum of the 8 children of g (R): adjoint of the nearest-neighbour upsample
 __global__ void __launch_bounds__(64) k_up_adjoint(const uint4 *__restrict__ g, uint4 *__restrict__ out, int R) {
+  gc_after();
   const int Rc = R >> 1;
   const int K = blockIdx.x * blockDim.x + threadIdx.x, J = blockIdx.y, c = blockIdx.z / Rc, I = blockIdx.z - c * Rc;
   if (K >= Rc) return;
@@ -969,6 +979,7 @@ __global__ void __launch_bounds__(64) k_up_adjoint(const uint4 *__restrict__ g, 
 __global__ void __launch_bounds__(64) k_pool_adj_add_mask(const uint4 *__restrict__ skipgrad,
                                                           const uint4 *__restrict__ gp, const uint4 *__restrict__ act,
                                                           uint4 *__restrict__ out, int R) {
+  gc_after();
   const int Rc = R >> 1;
   const int z = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, c = blockIdx.z / R, x = blockIdx.z - c * R;
   if (z >= R) return;
@@ -995,6 +1006,7 @@ struct WsBias {
   } l[WS_NL];
 };
 __global__ void __launch_bounds__(256) k_chan_sum(const __grid_constant__ WsBias d) {
+  gc_after();
   __shared__ float red[8][8];  // [warp][channel of the chunk]
   int layer = 0;
   while (layer + 1 < WS_NL && (int)blockIdx.x >= d.l[layer + 1].first) ++layer;
@@ -1025,12 +1037,14 @@ __global__ void __launch_bounds__(256) k_chan_sum(const __grid_constant__ WsBias
   }
 }
 __global__ void __launch_bounds__(256) k_chan_finish(const __grid_constant__ WsBias d) {
+  gc_after();
   const WsBias::Layer &L = d.l[blockIdx.y];
   if ((int)blockIdx.x < 8 * L.kc) reduce_col(L.part, L.nb, 8 * L.kc, blockIdx.x, L.out);
 }
 
 // Network input: channels 0..3 from f16 planar features [4][R^3]; channels 4..15 zero.
 __global__ void __launch_bounds__(256) k_pack_input(const __half *__restrict__ feat, uint4 *__restrict__ x0, size_t R3) {
+  gc_after();
   for (size_t v = blockIdx.x * (size_t)blockDim.x + threadIdx.x; v < R3; v += (size_t)gridDim.x * blockDim.x) {
     float f[8] = {__half2float(feat[v]), __half2float(feat[R3 + v]), __half2float(feat[2 * R3 + v]),
                   __half2float(feat[3 * R3 + v]), 0, 0, 0, 0};
@@ -1043,6 +1057,7 @@ __global__ void __launch_bounds__(256) k_pack_input(const __half *__restrict__ f
 // 16-channel bf16 tensor, other channels zero). Per-block partial loss sums.
 __global__ void __launch_bounds__(256) k_mse(const float *__restrict__ y, const __half *__restrict__ t, size_t R3,
                                              uint4 *__restrict__ gy, float *__restrict__ part) {
+  gc_after();
   __shared__ float red[8];
   const float inv_n = 1.0f / (float)R3;
   float acc = 0.0f;
@@ -1085,6 +1100,7 @@ __device__ __forceinline__ void pack_weight(const WsPack::Layer &L, int i, float
 
 // All layers' weights in one launch (blockIdx.y is the layer).
 __global__ void __launch_bounds__(256) k_pack_weights(const float *__restrict__ p, const __grid_constant__ WsPack d) {
+  gc_after();
   const WsPack::Layer &L = d.l[blockIdx.y];
   const int n = 27 * L.Cout * L.Cin;
   for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) pack_weight(L, i, p[L.off + i]);
@@ -1095,6 +1111,7 @@ __global__ void __launch_bounds__(256) k_pack_weights(const float *__restrict__ 
 __global__ void __launch_bounds__(256) k_adam(float *__restrict__ p, const float *__restrict__ g, float *__restrict__ m,
                                               float *__restrict__ v, const __grid_constant__ WsPack d, float lr, float b1,
                                               float b2, float eps, float bc1, float bc2) {
+  gc_after();
   const WsPack::Layer &L = d.l[blockIdx.y];
   const int nw = 27 * L.Cout * L.Cin, n = nw + L.Cout;
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
@@ -1184,6 +1201,22 @@ static int ws_fail(gc_ws *ws, int code, const char *fmt, ...) {
     if (e_ != cudaSuccess) return ws_fail(ws, GC_ERR_CUDA, "%s: %s", #call, cudaGetErrorString(e_)); \
   } while (0)
 
+// Launch on the object's stream; every kernel of the network begins with gc_after() (see
+// gc_launch_after).
+template <typename... KArgs, typename... Args>
+static void ws_launch(gc_ws *ws, void (*k)(KArgs...), dim3 grid, int block, size_t smem, Args &&...args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(block);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = ws->stream;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  cudaLaunchKernelEx(&cfg, k, static_cast<KArgs>(std::forward<Args>(args))...);
+}
 static uint32_t pow2_cols(int c) {
   uint32_t n = 32;
   while ((int)n < c) n <<= 1;
@@ -1419,7 +1452,7 @@ static int ws_conv(gc_ws *ws, const FwdPlan &p, int R, int Cin, int Cout, const 
     m.R = R; m.Cin = Cin; m.Cout = Cout; m.BX = p.BX; m.Cn = p.Cn; m.relu = relu; m.ns = p.ns;
     m.units = (R / p.BX) * (R / MA_LINES) * R;
     m.tmem_cols = p.cols;
-    k_conv_march<<<dim3(p.grid, Cout / p.Cn), MA_THREADS, p.smem, ws->stream>>>(m);
+    ws_launch(ws, k_conv_march, dim3(p.grid, Cout / p.Cn), MA_THREADS, p.smem, m);
     WS_CUDA(ws, cudaGetLastError());
     return GC_OK;
   }
@@ -1433,7 +1466,7 @@ static int ws_conv(gc_ws *ws, const FwdPlan &p, int R, int Cin, int Cout, const 
   a.out = out; a.out_f32 = out_f32; a.status = ws->status;
   a.R = R; a.Cin = Cin; a.Cout = Cout; a.BZ = p.BZ; a.BY = p.BY; a.Cn = p.Cn; a.relu = relu; a.tpg = p.tpg; a.n_mt = p.n_mt;
   a.tmem_cols = p.cols;
-  k_conv_fwd<<<dim3(p.grid, Cout / p.Cn), 256, p.smem, ws->stream>>>(a);
+  ws_launch(ws, k_conv_fwd, dim3(p.grid, Cout / p.Cn), 256, p.smem, a);
   WS_CUDA(ws, cudaGetLastError());
   return GC_OK;
 }
@@ -1450,7 +1483,7 @@ static int ws_wgrad(gc_ws *ws, int l, const uint4 *x, const uint4 *gy) {
   a.x = x; a.gy = gy; a.part = ws->part + ws->pofs[l]; a.status = ws->status;
   a.R = R; a.Cin = Cin; a.Cout = Cout; a.BZ = p.BZ; a.BY = p.BY; a.nblocks = p.nblocks;
   a.tpg = p.tpg; a.sub = p.sub; a.dy3 = p.dy3; a.ns = p.ns; a.tmem_cols = p.cols;
-  k_conv_wgrad<<<dim3(p.groups, p.grid), WG_THREADS, p.smem, ws->stream>>>(a);
+  ws_launch(ws, k_conv_wgrad, dim3(p.groups, p.grid), WG_THREADS, p.smem, a);
   WS_CUDA(ws, cudaGetLastError());
   ws->pend.l[ws->npend++] = {a.part, ws->grads + ws->w_off[l], p.grid, 27 * Cout * Cin};
   return GC_OK;
@@ -1461,7 +1494,7 @@ static int ws_wgrad_finish(gc_ws *ws) {
   int most = 0;
   for (int i = 0; i < ws->npend; ++i) most = std::max(most, ws->pend.l[i].nelem);
   const unsigned nb = std::min<unsigned>((unsigned)(most + 63) / 64, (unsigned)ws->sm_count * 8u);
-  if (ws->npend) k_wgrad_reduce<<<dim3(nb, ws->npend), 64, 0, ws->stream>>>(ws->pend);
+  if (ws->npend) ws_launch(ws, k_wgrad_reduce, dim3(nb, ws->npend), 64, 0, ws->pend);
   ws->npend = 0;
   WS_CUDA(ws, cudaGetLastError());
   return GC_OK;
@@ -1479,8 +1512,8 @@ static int ws_bias_grads(gc_ws *ws) {
     d.l[l] = {g[l], ws->cpart + (size_t)l * 1024 * 128, ws->grads + ws->b_off[l], R3, kc, nb, blocks};
     blocks += nb * kc;
   }
-  k_chan_sum<<<blocks, 256, 0, ws->stream>>>(d);
-  k_chan_finish<<<dim3(128, WS_NL), 256, 0, ws->stream>>>(d);
+  ws_launch(ws, k_chan_sum, dim3(blocks), 256, 0, d);
+  ws_launch(ws, k_chan_finish, dim3(128, WS_NL), 256, 0, d);
   WS_CUDA(ws, cudaGetLastError());
   return GC_OK;
 }
@@ -1656,7 +1689,7 @@ static WsPack ws_pack_desc(const gc_ws *ws) {
 }
 
 static int ws_repack(gc_ws *ws) {
-  k_pack_weights<<<dim3(512, WS_NL), 256, 0, ws->stream>>>(ws->params, ws_pack_desc(ws));
+  ws_launch(ws, k_pack_weights, dim3(512, WS_NL), 256, 0, ws->params, ws_pack_desc(ws));
   WS_CUDA(ws, cudaGetLastError());
   return GC_OK;
 }
@@ -1692,20 +1725,20 @@ static int ws_forward_packed(gc_ws *ws, float *y_out) {
   const int R = ws->R;
   int s;
   if ((s = ws_fwd_layer(ws, 0, ws->x0, nullptr, ws->e0, nullptr))) return s;
-  k_pool2<<<line_grid(R / 2, 2, 64), 64, 0, ws->stream>>>(ws->e0, ws->p1, R);
+  ws_launch(ws, k_pool2, dim3(line_grid(R / 2, 2, 64)), 64, 0, ws->e0, ws->p1, R);
   if ((s = ws_fwd_layer(ws, 1, ws->p1, nullptr, ws->e1, nullptr))) return s;
-  k_pool2<<<line_grid(R / 4, 4, 64), 64, 0, ws->stream>>>(ws->e1, ws->p2, R / 2);
+  ws_launch(ws, k_pool2, dim3(line_grid(R / 4, 4, 64)), 64, 0, ws->e1, ws->p2, R / 2);
   if ((s = ws_fwd_layer(ws, 2, ws->p2, nullptr, ws->e2, nullptr))) return s;
-  k_pool2<<<line_grid(R / 8, 8, 64), 64, 0, ws->stream>>>(ws->e2, ws->p3, R / 4);
+  ws_launch(ws, k_pool2, dim3(line_grid(R / 8, 8, 64)), 64, 0, ws->e2, ws->p3, R / 4);
   if ((s = ws_fwd_layer(ws, 3, ws->p3, nullptr, ws->e3, nullptr))) return s;
   if ((s = ws_fwd_layer(ws, 4, ws->e3, nullptr, ws->u2, nullptr))) return s;
-  k_up_add_relu<<<line_grid(R / 4, 8, 64), 64, 0, ws->stream>>>(ws->u2, ws->e2, ws->d2, R / 4);
+  ws_launch(ws, k_up_add_relu, dim3(line_grid(R / 4, 8, 64)), 64, 0, ws->u2, ws->e2, ws->d2, R / 4);
   if ((s = ws_fwd_layer(ws, 5, ws->d2, nullptr, ws->f2, nullptr))) return s;
   if ((s = ws_fwd_layer(ws, 6, ws->f2, nullptr, ws->u1, nullptr))) return s;
-  k_up_add_relu<<<line_grid(R / 2, 4, 64), 64, 0, ws->stream>>>(ws->u1, ws->e1, ws->d1, R / 2);
+  ws_launch(ws, k_up_add_relu, dim3(line_grid(R / 2, 4, 64)), 64, 0, ws->u1, ws->e1, ws->d1, R / 2);
   if ((s = ws_fwd_layer(ws, 7, ws->d1, nullptr, ws->f1, nullptr))) return s;
   if ((s = ws_fwd_layer(ws, 8, ws->f1, nullptr, ws->u0, nullptr))) return s;
-  k_up_add_relu<<<line_grid(R, 2, 64), 64, 0, ws->stream>>>(ws->u0, ws->e0, ws->d0, R);
+  ws_launch(ws, k_up_add_relu, dim3(line_grid(R, 2, 64)), 64, 0, ws->u0, ws->e0, ws->d0, R);
   if ((s = ws_fwd_layer(ws, 9, ws->d0, nullptr, ws->f0, nullptr))) return s;
   if ((s = ws_fwd_layer(ws, 10, ws->f0, nullptr, nullptr, y_out ? y_out : ws->y))) return s;
   WS_CUDA(ws, cudaGetLastError());
@@ -1715,7 +1748,7 @@ static int ws_forward_packed(gc_ws *ws, float *y_out) {
 extern "C" int gc_ws_forward(gc_ws *ws, const void *feat, float *y_out) {
   if (!ws || !feat) return GC_ERR_ARG;
   const size_t R3 = (size_t)ws->R * ws->R * ws->R;
-  k_pack_input<<<ew_blocks(R3, ws->sm_count), 256, 0, ws->stream>>>((const __half *)feat, ws->x0, R3);
+  ws_launch(ws, k_pack_input, dim3(ew_blocks(R3, ws->sm_count)), 256, 0, (const __half *)feat, ws->x0, R3);
   WS_CUDA(ws, cudaGetLastError());
   int s = ws_forward_packed(ws, ws->y);
   if (s) return s;
@@ -1731,41 +1764,41 @@ extern "C" int gc_ws_backward(gc_ws *ws, const void *target, float *loss_out) {
   int s;
   const unsigned nl = std::min<unsigned>(ew_blocks(R3, sm), 1024u);
   ws->npend = 0;
-  k_mse<<<nl, 256, 0, ws->stream>>>(ws->y, (const __half *)target, R3, ws->gy, ws->lpart);
-  k_reduce_cols<<<1, 256, 0, ws->stream>>>(ws->lpart, (int)nl, 1, ws->loss);
+  ws_launch(ws, k_mse, dim3(nl), 256, 0, ws->y, (const __half *)target, R3, ws->gy, ws->lpart);
+  ws_launch(ws, k_reduce_cols, dim3(1), 256, 0, ws->lpart, (int)nl, 1, ws->loss);
   WS_CUDA(ws, cudaGetLastError());
   // K, J
   if ((s = ws_wgrad(ws, 10, ws->f0, ws->gy))) return s;
   if ((s = ws_dgrad(ws, 10, ws->gy, ws->f0, ws->g_f0))) return s;
   if ((s = ws_wgrad(ws, 9, ws->d0, ws->g_f0))) return s;
   if ((s = ws_dgrad(ws, 9, ws->g_f0, ws->d0, ws->g_d0))) return s;
-  k_up_adjoint<<<line_grid(R / 2, 2, 64), 64, 0, ws->stream>>>(ws->g_d0, ws->g_u0, R);
+  ws_launch(ws, k_up_adjoint, dim3(line_grid(R / 2, 2, 64)), 64, 0, ws->g_d0, ws->g_u0, R);
   // I, H
   if ((s = ws_wgrad(ws, 8, ws->f1, ws->g_u0))) return s;
   if ((s = ws_dgrad(ws, 8, ws->g_u0, ws->f1, ws->g_f1))) return s;
   if ((s = ws_wgrad(ws, 7, ws->d1, ws->g_f1))) return s;
   if ((s = ws_dgrad(ws, 7, ws->g_f1, ws->d1, ws->g_d1))) return s;
-  k_up_adjoint<<<line_grid(R / 4, 4, 64), 64, 0, ws->stream>>>(ws->g_d1, ws->g_u1, R / 2);
+  ws_launch(ws, k_up_adjoint, dim3(line_grid(R / 4, 4, 64)), 64, 0, ws->g_d1, ws->g_u1, R / 2);
   // G, F
   if ((s = ws_wgrad(ws, 6, ws->f2, ws->g_u1))) return s;
   if ((s = ws_dgrad(ws, 6, ws->g_u1, ws->f2, ws->g_f2))) return s;
   if ((s = ws_wgrad(ws, 5, ws->d2, ws->g_f2))) return s;
   if ((s = ws_dgrad(ws, 5, ws->g_f2, ws->d2, ws->g_d2))) return s;
-  k_up_adjoint<<<line_grid(R / 8, 8, 64), 64, 0, ws->stream>>>(ws->g_d2, ws->g_u2, R / 4);
+  ws_launch(ws, k_up_adjoint, dim3(line_grid(R / 8, 8, 64)), 64, 0, ws->g_d2, ws->g_u2, R / 4);
   // E, D
   if ((s = ws_wgrad(ws, 4, ws->e3, ws->g_u2))) return s;
   if ((s = ws_dgrad(ws, 4, ws->g_u2, ws->e3, ws->g_e3))) return s;
   if ((s = ws_wgrad(ws, 3, ws->p3, ws->g_e3))) return s;
   if ((s = ws_dgrad(ws, 3, ws->g_e3, nullptr, ws->g_p3))) return s;
-  k_pool_adj_add_mask<<<line_grid(R / 4, 8, 64), 64, 0, ws->stream>>>(ws->g_d2, ws->g_p3, ws->e2, ws->g_e2, R / 4);
+  ws_launch(ws, k_pool_adj_add_mask, dim3(line_grid(R / 4, 8, 64)), 64, 0, ws->g_d2, ws->g_p3, ws->e2, ws->g_e2, R / 4);
   // C
   if ((s = ws_wgrad(ws, 2, ws->p2, ws->g_e2))) return s;
   if ((s = ws_dgrad(ws, 2, ws->g_e2, nullptr, ws->g_p2))) return s;
-  k_pool_adj_add_mask<<<line_grid(R / 2, 4, 64), 64, 0, ws->stream>>>(ws->g_d1, ws->g_p2, ws->e1, ws->g_e1, R / 2);
+  ws_launch(ws, k_pool_adj_add_mask, dim3(line_grid(R / 2, 4, 64)), 64, 0, ws->g_d1, ws->g_p2, ws->e1, ws->g_e1, R / 2);
   // B
   if ((s = ws_wgrad(ws, 1, ws->p1, ws->g_e1))) return s;
   if ((s = ws_dgrad(ws, 1, ws->g_e1, nullptr, ws->g_p1))) return s;
-  k_pool_adj_add_mask<<<line_grid(R, 2, 64), 64, 0, ws->stream>>>(ws->g_d0, ws->g_p1, ws->e0, ws->g_e0, R);
+  ws_launch(ws, k_pool_adj_add_mask, dim3(line_grid(R, 2, 64)), 64, 0, ws->g_d0, ws->g_p1, ws->e0, ws->g_e0, R);
   // A
   if ((s = ws_wgrad(ws, 0, ws->x0, ws->g_e0))) return s;
   if ((s = ws_wgrad_finish(ws)) || (s = ws_bias_grads(ws))) return s;
@@ -1905,7 +1938,7 @@ extern "C" int gc_ws_set_plan(gc_ws *ws, int layer, int kind, int index, int *co
 extern "C" int gc_ws_adam(gc_ws *ws, float lr, float beta1, float beta2, float eps, int step) {
   if (!ws || step < 1 || !(lr >= 0.0f)) return GC_ERR_ARG;
   const float bc1 = 1.0f - powf(beta1, (float)step), bc2 = 1.0f - powf(beta2, (float)step);
-  k_adam<<<dim3(512, WS_NL), 256, 0, ws->stream>>>(ws->params, ws->grads, ws->adam_m, ws->adam_v, ws_pack_desc(ws), lr,
+  ws_launch(ws, k_adam, dim3(512, WS_NL), 256, 0, ws->params, ws->grads, ws->adam_m, ws->adam_v, ws_pack_desc(ws), lr,
                                                   beta1, beta2, eps, bc1, bc2);
   WS_CUDA(ws, cudaGetLastError());
   return GC_OK;
@@ -1926,6 +1959,7 @@ extern "C" int gc_ws_adam(gc_ws *ws, float lr, float beta1, float beta2, float e
 // n (f16 [4][R^3]): log(1 + rho_c / mean rho_c), phi_c / rms, d_c / rms(d_c),
 // dd_c / rms(dd_c); training target dd_c(n) / rms(dd_c(n-1)).
 __global__ void __launch_bounds__(64) k_ws_coarsen(const float *__restrict__ f, int G, float *__restrict__ out) {
+  gc_after();
   const int R = G >> 1;
   const int K = blockIdx.x * blockDim.x + threadIdx.x, J = blockIdx.y, I = blockIdx.z;
   if (K >= R) return;
@@ -1939,6 +1973,7 @@ __global__ void __launch_bounds__(64) k_ws_coarsen(const float *__restrict__ f, 
 __global__ void __launch_bounds__(256) k_ws_stats(const float *__restrict__ rho, const float *__restrict__ phi,
                                                   const float *__restrict__ dlt, const float *__restrict__ ddl,
                                                   size_t n, float *__restrict__ part) {
+  gc_after();
   __shared__ float red[4][8];
   float a = 0.0f, b = 0.0f, c = 0.0f, e = 0.0f;
   for (size_t v = blockIdx.x * (size_t)blockDim.x + threadIdx.x; v < n; v += (size_t)gridDim.x * blockDim.x) {
@@ -1967,6 +2002,7 @@ __global__ void __launch_bounds__(256) k_ws_stats(const float *__restrict__ rho,
 // One block of 256 threads; fixed strided split and tree over the partials.
 __global__ void __launch_bounds__(256) k_ws_scales(const float *__restrict__ part, int nb, size_t n, int hist,
                                                    float *__restrict__ scal) {
+  gc_after();
   __shared__ double red[4][256];
   const int t = threadIdx.x;
   double ta = 0.0, tb = 0.0, tc = 0.0, te = 0.0;
@@ -1998,6 +2034,7 @@ __global__ void __launch_bounds__(256) k_ws_features(const float *__restrict__ r
                                                      const float *__restrict__ dlt, const float *__restrict__ ddl,
                                                      const float *__restrict__ scal, int hist, size_t n,
                                                      __half *__restrict__ feat, __half *__restrict__ rec) {
+  gc_after();
   const float ir = 1.0f / scal[0], ip = 1.0f / scal[1], id = 1.0f / scal[2], idd = 1.0f / scal[4];
   const bool has_p = hist >= 1, has_d = scal[3] != 0.0f, has_dd = scal[5] != 0.0f;
   for (size_t v = blockIdx.x * (size_t)blockDim.x + threadIdx.x; v < n; v += (size_t)gridDim.x * blockDim.x) {
@@ -2016,6 +2053,7 @@ __global__ void __launch_bounds__(256) k_ws_features(const float *__restrict__ r
 __global__ void __launch_bounds__(128) k_ws_apply(const float *__restrict__ yc, const float *__restrict__ scal,
                                                   int use_d, int G, float *__restrict__ hi, float *__restrict__ lo,
                                                   float *__restrict__ prev) {
+  gc_after();
   const int k = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y, i = blockIdx.z;
   if (k >= G) return;
   // the face nodes are the multipole faces' (computed beside this pass)
@@ -2062,6 +2100,7 @@ __global__ void __launch_bounds__(128) k_ws_apply(const float *__restrict__ yc, 
 __global__ void __launch_bounds__(64) k_ws_post(const float *__restrict__ hi, int G, float *__restrict__ phi,
                                                 float *__restrict__ dlt, float *__restrict__ ddl,
                                                 const float *__restrict__ scal, int hist, __half *__restrict__ rec) {
+  gc_after();
   const int R = G >> 1;
   const int K = blockIdx.x * blockDim.x + threadIdx.x, J = blockIdx.y, I = blockIdx.z;
   if (K >= R) return;
@@ -2135,13 +2174,13 @@ int gc_ws_pre_solve(gc_ctx *ctx, int warm, int mode) {
   // recording, or when tracking was asked for (the extrapolation needs neither)
   const bool coarse = ctx->ws_coarse || ctx->ws_record;
   if (coarse) {
-  gc_launch(ctx, GK_WARMSTART, k_ws_coarsen, dim3((R + 63) / 64, R, R), dim3(64), 0, (const float *)ctx->b0, ctx->G,
+  gc_launch_after(ctx, GK_WARMSTART, k_ws_coarsen, dim3((R + 63) / 64, R, R), dim3(64), 0, (const float *)ctx->b0, ctx->G,
             w.rho);
-  gc_launch(ctx, GK_WARMSTART, k_ws_stats, dim3(nb), dim3(256), 0, (const float *)w.rho, (const float *)w.phi,
+  gc_launch_after(ctx, GK_WARMSTART, k_ws_stats, dim3(nb), dim3(256), 0, (const float *)w.rho, (const float *)w.phi,
             (const float *)w.dlt, (const float *)w.ddl, R3, w.part);
-  gc_launch(ctx, GK_WARMSTART, k_ws_scales, dim3(1), dim3(256), 0, (const float *)w.part, (int)nb, R3, ctx->ws_hist,
+  gc_launch_after(ctx, GK_WARMSTART, k_ws_scales, dim3(1), dim3(256), 0, (const float *)w.part, (int)nb, R3, ctx->ws_hist,
             w.scal);
-  gc_launch(ctx, GK_WARMSTART, k_ws_features, dim3(nb), dim3(256), 0, (const float *)w.rho, (const float *)w.phi,
+  gc_launch_after(ctx, GK_WARMSTART, k_ws_features, dim3(nb), dim3(256), 0, (const float *)w.rho, (const float *)w.phi,
             (const float *)w.dlt, (const float *)w.ddl, (const float *)w.scal, ctx->ws_hist, R3, w.feat,
             (__half *)ctx->ws_record);
   GC_LAUNCH_CHECK(ctx, "warm-start features");
@@ -2168,7 +2207,7 @@ int gc_ws_pre_solve(gc_ctx *ctx, int warm, int mode) {
     yc = w.y;
   }
   const int use_d = ctx->ws_mode != GC_WS_PLAIN && ctx->ws_hist >= 2;
-  gc_launch(ctx, GK_WARMSTART, k_ws_apply, dim3((ctx->G + 127) / 128, ctx->G, ctx->G), dim3(128), 0, yc,
+  gc_launch_after(ctx, GK_WARMSTART, k_ws_apply, dim3((ctx->G + 127) / 128, ctx->G, ctx->G), dim3(128), 0, yc,
             (const float *)w.scal, use_d, ctx->G, ctx->hi, ctx->lo, w.prev);
   GC_LAUNCH_CHECK(ctx, "warm-start apply");
   return GC_OK;
@@ -2183,7 +2222,7 @@ int gc_ws_post_solve(gc_ctx *ctx) {
   }
   const WsViews w = ws_views(ctx);
   const int R = ctx->G / 2;
-  gc_launch(ctx, GK_WARMSTART, k_ws_post, dim3((R + 63) / 64, R, R), dim3(64), 0, (const float *)ctx->hi, ctx->G,
+  gc_launch_after(ctx, GK_WARMSTART, k_ws_post, dim3((R + 63) / 64, R, R), dim3(64), 0, (const float *)ctx->hi, ctx->G,
             w.phi, w.dlt, w.ddl, (const float *)w.scal, ctx->ws_hist, (__half *)ctx->ws_record);
   GC_LAUNCH_CHECK(ctx, "warm-start history");
   ctx->ws_hist = ctx->ws_hist < 3 ? ctx->ws_hist + 1 : 3;
