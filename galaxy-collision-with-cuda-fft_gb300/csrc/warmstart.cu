@@ -622,11 +622,11 @@ __global__ void __launch_bounds__(MA_THREADS) k_conv_march(const __grid_constant
 // beside what.
 // A CTA takes the taps of one dz (blockIdx.x = dz and a share of its nine taps; the
 // groups of a partial next to each other, so that the partials with a block more, which
-// come first, start first), so its x
-// tile is the block's BZ planes moved by dz, with the halo in y and x, staged as in the
-// forward pass and as one box; read MN-major (8 channels of one voxel per 16-byte row),
-// the B operand of a tap is again the tile shifted by some rows. gy arrives in stages of 128 rows, each row's 16-byte
-// pieces (8 output channels) placed in groups of 8 rows so that every one of the M rows
+// come first, start first), so its x tile is the block's BZ planes moved by dz, with the
+// halo in y and x, staged as in the forward pass and as one box; read MN-major
+// (8 channels of one voxel per 16-byte row), the B operand of a tap is again the tile
+// shifted by some rows. gy arrives in stages of 128 rows, each row's 16-byte pieces
+// (8 output channels) placed in groups of 8 rows so that every one of the M rows
 // addresses shared memory of the stage (rows >= Cout are never read back). Rows outside
 // the CTA's block are zero in gy. A CTA (partial, tap group) has warps that fill the
 // ring of stages and at the end read the accumulators out, and warps that issue.
