@@ -912,12 +912,13 @@ __global__ void __launch_bounds__(64) k_wgrad_reduce(const __grid_constant__ WgR
 // ------------------------------------------------------------------------------
 // Coarse voxel (I,J,K) of an R/2 grid covers fine voxels (2I..2I+1, 2J.., 2K..).
 // The elementwise kernels run one thread per voxel of a line: blockIdx.z = chunk *
-// R_line + z, blockIdx.y = y, x from blockIdx.x (no index division).
+// planes + plane, blockIdx.y = line, the voxel from blockIdx.x.
 __device__ __forceinline__ size_t child_index(int R, int I, int J, int K, int c) {
   return ((size_t)(2 * I + (c >> 2)) * R + (2 * J + ((c >> 1) & 1))) * R + (2 * K + (c & 1));
 }
 
 static dim3 line_grid(int Rl, int kc, int tpb) { return dim3((Rl + tpb - 1) / tpb, Rl, Rl * kc); }
+static dim3 quad_grid(int R, int kc, int tpb) { return dim3((R + tpb - 1) / tpb, R / 2, R / 2 * kc); }
 
 // out (R/2) = mean of the 8 children of in (R)
 __global__ void __launch_bounds__(64) k_pool2(const uint4 *__restrict__ in, uint4 *__restrict__ out, int R) {
@@ -939,21 +940,37 @@ __global__ void __launch_bounds__(64) k_pool2(const uint4 *__restrict__ in, uint
   out[c * Rc3 + ((size_t)I * Rc + J) * Rc + K] = pack8<0>(acc);
 }
 
+// Two passes over a level's fine grid that add a parent's value to its eight children:
+// a thread takes the four children of a parent at its x (blockIdx.z = chunk * R/2 + X,
+// blockIdx.y = Y: two lines of two planes), so that each load of the warp is one
+// stretch, four (eight) are on their way at once and the parent is read once a line.
+// With a voxel per thread (65536 blocks of 64 threads at R = 128, which the chip is slow
+// to hand out) the upsampling took 50.7 us on its three levels at R = 128; so 30.4.
+__device__ __forceinline__ size_t quad_index(int R, int X, int Y, int q, int z) {
+  return ((size_t)(2 * X + (q >> 1)) * R + (2 * Y + (q & 1))) * R + z;
+}
+
 // out (R) = relu(u[parent] + skip)
 __global__ void __launch_bounds__(64) k_up_add_relu(const uint4 *__restrict__ u, const uint4 *__restrict__ skip,
                                                     uint4 *__restrict__ out, int R) {
   gc_after();
   const int Rc = R >> 1;
-  const int z = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, c = blockIdx.z / R, x = blockIdx.z - c * R;
+  const int z = blockIdx.x * blockDim.x + threadIdx.x, Y = blockIdx.y, c = blockIdx.z / Rc, X = blockIdx.z - c * Rc;
   if (z >= R) return;
   const size_t R3 = (size_t)R * R * R, Rc3 = (size_t)Rc * Rc * Rc;
-  const size_t i = c * R3 + ((size_t)x * R + y) * R + z;
-  float a[8], b[8];
-  unpack8(__ldg(u + c * Rc3 + ((size_t)(x >> 1) * Rc + (y >> 1)) * Rc + (z >> 1)), a);
-  unpack8(__ldg(skip + i), b);
+  uint4 v[4];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) a[j] = fmaxf(a[j] + b[j], 0.0f);
-  out[i] = pack8<0>(a);
+  for (int q = 0; q < 4; ++q) v[q] = __ldg(skip + c * R3 + quad_index(R, X, Y, q, z));
+  float a[8];
+  unpack8(__ldg(u + c * Rc3 + ((size_t)X * Rc + Y) * Rc + (z >> 1)), a);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    float b[8];
+    unpack8(v[q], b);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) b[j] = fmaxf(a[j] + b[j], 0.0f);
+    out[c * R3 + quad_index(R, X, Y, q, z)] = pack8<0>(b);
+  }
 }
 
 // out (R/2) = sum of the 8 children of g (R): adjoint of the nearest-neighbour upsample
@@ -981,17 +998,25 @@ __global__ void __launch_bounds__(64) k_pool_adj_add_mask(const uint4 *__restric
                                                           uint4 *__restrict__ out, int R) {
   gc_after();
   const int Rc = R >> 1;
-  const int z = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y, c = blockIdx.z / R, x = blockIdx.z - c * R;
+  const int z = blockIdx.x * blockDim.x + threadIdx.x, Y = blockIdx.y, c = blockIdx.z / Rc, X = blockIdx.z - c * Rc;
   if (z >= R) return;
   const size_t R3 = (size_t)R * R * R, Rc3 = (size_t)Rc * Rc * Rc;
-  const size_t i = c * R3 + ((size_t)x * R + y) * R + z;
-  float p[8], s[8], m[8];
-  unpack8(__ldg(gp + c * Rc3 + ((size_t)(x >> 1) * Rc + (y >> 1)) * Rc + (z >> 1)), p);
-  unpack8(__ldg(skipgrad + i), s);
-  unpack8(__ldg(act + i), m);
+  uint4 vs[4], vm[4];
 #pragma unroll
-  for (int j = 0; j < 8; ++j) p[j] = m[j] > 0.0f ? s[j] + 0.125f * p[j] : 0.0f;
-  out[i] = pack8<0>(p);
+  for (int q = 0; q < 4; ++q) vs[q] = __ldg(skipgrad + c * R3 + quad_index(R, X, Y, q, z));
+#pragma unroll
+  for (int q = 0; q < 4; ++q) vm[q] = __ldg(act + c * R3 + quad_index(R, X, Y, q, z));
+  float p[8];
+  unpack8(__ldg(gp + c * Rc3 + ((size_t)X * Rc + Y) * Rc + (z >> 1)), p);
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    float s[8], m[8];
+    unpack8(vs[q], s);
+    unpack8(vm[q], m);
+#pragma unroll
+    for (int j = 0; j < 8; ++j) s[j] = m[j] > 0.0f ? s[j] + 0.125f * p[j] : 0.0f;
+    out[c * R3 + quad_index(R, X, Y, q, z)] = pack8<0>(s);
+  }
 }
 
 // Bias gradients of all layers: per-block partial channel sums of g (C = 8*kc channels),
@@ -1732,13 +1757,13 @@ static int ws_forward_packed(gc_ws *ws, float *y_out) {
   ws_launch(ws, k_pool2, dim3(line_grid(R / 8, 8, 64)), 64, 0, ws->e2, ws->p3, R / 4);
   if ((s = ws_fwd_layer(ws, 3, ws->p3, nullptr, ws->e3, nullptr))) return s;
   if ((s = ws_fwd_layer(ws, 4, ws->e3, nullptr, ws->u2, nullptr))) return s;
-  ws_launch(ws, k_up_add_relu, dim3(line_grid(R / 4, 8, 64)), 64, 0, ws->u2, ws->e2, ws->d2, R / 4);
+  ws_launch(ws, k_up_add_relu, dim3(quad_grid(R / 4, 8, 64)), 64, 0, ws->u2, ws->e2, ws->d2, R / 4);
   if ((s = ws_fwd_layer(ws, 5, ws->d2, nullptr, ws->f2, nullptr))) return s;
   if ((s = ws_fwd_layer(ws, 6, ws->f2, nullptr, ws->u1, nullptr))) return s;
-  ws_launch(ws, k_up_add_relu, dim3(line_grid(R / 2, 4, 64)), 64, 0, ws->u1, ws->e1, ws->d1, R / 2);
+  ws_launch(ws, k_up_add_relu, dim3(quad_grid(R / 2, 4, 64)), 64, 0, ws->u1, ws->e1, ws->d1, R / 2);
   if ((s = ws_fwd_layer(ws, 7, ws->d1, nullptr, ws->f1, nullptr))) return s;
   if ((s = ws_fwd_layer(ws, 8, ws->f1, nullptr, ws->u0, nullptr))) return s;
-  ws_launch(ws, k_up_add_relu, dim3(line_grid(R, 2, 64)), 64, 0, ws->u0, ws->e0, ws->d0, R);
+  ws_launch(ws, k_up_add_relu, dim3(quad_grid(R, 2, 64)), 64, 0, ws->u0, ws->e0, ws->d0, R);
   if ((s = ws_fwd_layer(ws, 9, ws->d0, nullptr, ws->f0, nullptr))) return s;
   if ((s = ws_fwd_layer(ws, 10, ws->f0, nullptr, nullptr, y_out ? y_out : ws->y))) return s;
   WS_CUDA(ws, cudaGetLastError());
@@ -1790,15 +1815,15 @@ extern "C" int gc_ws_backward(gc_ws *ws, const void *target, float *loss_out) {
   if ((s = ws_dgrad(ws, 4, ws->g_u2, ws->e3, ws->g_e3))) return s;
   if ((s = ws_wgrad(ws, 3, ws->p3, ws->g_e3))) return s;
   if ((s = ws_dgrad(ws, 3, ws->g_e3, nullptr, ws->g_p3))) return s;
-  ws_launch(ws, k_pool_adj_add_mask, dim3(line_grid(R / 4, 8, 64)), 64, 0, ws->g_d2, ws->g_p3, ws->e2, ws->g_e2, R / 4);
+  ws_launch(ws, k_pool_adj_add_mask, dim3(quad_grid(R / 4, 8, 64)), 64, 0, ws->g_d2, ws->g_p3, ws->e2, ws->g_e2, R / 4);
   // C
   if ((s = ws_wgrad(ws, 2, ws->p2, ws->g_e2))) return s;
   if ((s = ws_dgrad(ws, 2, ws->g_e2, nullptr, ws->g_p2))) return s;
-  ws_launch(ws, k_pool_adj_add_mask, dim3(line_grid(R / 2, 4, 64)), 64, 0, ws->g_d1, ws->g_p2, ws->e1, ws->g_e1, R / 2);
+  ws_launch(ws, k_pool_adj_add_mask, dim3(quad_grid(R / 2, 4, 64)), 64, 0, ws->g_d1, ws->g_p2, ws->e1, ws->g_e1, R / 2);
   // B
   if ((s = ws_wgrad(ws, 1, ws->p1, ws->g_e1))) return s;
   if ((s = ws_dgrad(ws, 1, ws->g_e1, nullptr, ws->g_p1))) return s;
-  ws_launch(ws, k_pool_adj_add_mask, dim3(line_grid(R, 2, 64)), 64, 0, ws->g_d0, ws->g_p1, ws->e0, ws->g_e0, R);
+  ws_launch(ws, k_pool_adj_add_mask, dim3(quad_grid(R, 2, 64)), 64, 0, ws->g_d0, ws->g_p1, ws->e0, ws->g_e0, R);
   // A
   if ((s = ws_wgrad(ws, 0, ws->x0, ws->g_e0))) return s;
   if ((s = ws_wgrad_finish(ws)) || (s = ws_bias_grads(ws))) return s;
