@@ -44,7 +44,6 @@ enum {
   GC_S_MAXREL2 = 16, // ... and the largest (||r|| / ||b||)^2 they ended with
   GC_S_TICKET = 17,  // block ticket of the last-block grid reductions (an unsigned, 0 between them)
   GC_S_LIMBS = 64,   // [64, 94): integer limbs of the moments of k_convert_q (0 between calls)
-  GC_S_SCATTERED = 94, // whether a gather's particles come in no order (an int)
   GC_S_FIN_TMP = 128, // [128, 256): chunk partials of gc_finalize
   GC_S_NSLOTS = 256
 };
@@ -136,6 +135,7 @@ struct gc_ctx {
   double mass_sum_cache; // sum of masses for the engine's fixed-point quantum
   int last_step_valid;
   int q_next_ready;     // q holds the deposit of the current positions (made by the last particle pass)
+  int pool_user;        // the context has taken scratch from the device's pool (gc_scratch_get)
   int tail_smem_set;    // the tail kernel's dynamic shared-memory limit has been raised
   int gt_smem_set;      // the TMA particle-pass kernels' dynamic shared-memory limit has been raised
   const uint32_t *import_perm;  // gc_pm_import_order's permutation (in the sort scratch) ...
@@ -164,6 +164,13 @@ struct gc_ctx {
 
 int gc_ws_pre_solve(gc_ctx *ctx, int warm, int mode);
 int gc_ws_post_solve(gc_ctx *ctx);
+
+// Scratch of one call, in the order of ctx's stream: the context may be shared by callers
+// on several streams, so nothing that a call's kernels hand to each other lies in it.
+// False (and *p null) where there is none: no device memory, or a stream under capture,
+// whose replays would outlive the block. gc_scratch_put follows the last kernel that uses it.
+bool gc_scratch_get(gc_ctx *ctx, size_t bytes, void **p);
+void gc_scratch_put(gc_ctx *ctx, void *p);
 
 // Launch `k` on ctx's stream, counting it under `kid` and bracketing it with
 // CUDA events when profiling is enabled.

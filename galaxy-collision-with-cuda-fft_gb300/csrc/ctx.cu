@@ -3,6 +3,8 @@
 
 #include <stdlib.h>
 
+#include <mutex>
+
 static char g_create_err[512] = "";
 
 const char *const gc_kernel_names[GK_COUNT] = {
@@ -130,6 +132,69 @@ int gc_ensure_particle_scratch(gc_ctx *ctx, size_t n) {
   return GC_OK;
 }
 
+// ---- scratch of one call -------------------------------------------------------
+// One stream-ordered pool a device: two calls in flight at once, on two streams or from
+// two threads, get two blocks. It keeps what its largest calls needed (16 bytes a node for a
+// gather) while a context that used it lives and gives everything
+// back with the last one.
+struct ScratchPool {
+  cudaMemPool_t pool;
+  int users;
+};
+static ScratchPool g_scratch[64];
+static std::mutex g_scratch_lock;
+
+static void scratch_keep(cudaMemPool_t pool, unsigned long long bytes) {
+  cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &bytes);
+  if (bytes == 0) cudaMemPoolTrimTo(pool, 0);
+}
+
+static cudaMemPool_t scratch_pool(gc_ctx *ctx) {
+  if (ctx->device < 0 || ctx->device >= 64) return nullptr;
+  std::lock_guard<std::mutex> hold(g_scratch_lock);
+  ScratchPool &s = g_scratch[ctx->device];
+  if (!s.pool) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = ctx->device;
+    if (cudaMemPoolCreate(&s.pool, &props) != cudaSuccess) {
+      cudaGetLastError();
+      s.pool = nullptr;
+      return nullptr;
+    }
+  }
+  if (!ctx->pool_user) {
+    ctx->pool_user = 1;
+    if (s.users++ == 0) scratch_keep(s.pool, ~0ULL);
+  }
+  return s.pool;
+}
+
+bool gc_scratch_get(gc_ctx *ctx, size_t bytes, void **p) {
+  *p = nullptr;
+  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
+  const cudaError_t e = cudaStreamIsCapturing(ctx->stream, &cs);
+  if (e != cudaSuccess) cudaGetLastError();
+  if (e != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
+  const cudaMemPool_t pool = scratch_pool(ctx);
+  if (!pool) return false;
+  if (cudaMallocFromPoolAsync(p, bytes, pool, ctx->stream) != cudaSuccess) {
+    cudaGetLastError();
+    *p = nullptr;
+  }
+  return *p != nullptr;
+}
+
+void gc_scratch_put(gc_ctx *ctx, void *p) { cudaFreeAsync(p, ctx->stream); }
+
+static void scratch_leave(gc_ctx *ctx) {
+  if (!ctx->pool_user) return;
+  std::lock_guard<std::mutex> hold(g_scratch_lock);
+  ScratchPool &s = g_scratch[ctx->device];
+  if (--s.users == 0) scratch_keep(s.pool, 0);
+}
+
 extern "C" int gc_abi_version(void) { return GC_ABI_VERSION; }
 
 extern "C" const char *gc_last_error(const gc_ctx *ctx) { return ctx ? ctx->err : g_create_err; }
@@ -206,6 +271,7 @@ extern "C" int gc_ctx_create(gc_ctx **out, int grid_size, double dx, double grav
 extern "C" int gc_ctx_destroy(gc_ctx *ctx) {
   if (!ctx) return GC_OK;
   cudaStreamSynchronize(ctx->stream);
+  scratch_leave(ctx);
   gc_mg_loop_free(ctx);
   gc_mg_free(ctx);
   cudaFree(ctx->q);

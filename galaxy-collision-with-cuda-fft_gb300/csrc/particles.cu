@@ -1600,22 +1600,6 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// Whether a gather of n particles may pack the fields (not where the packed copy cannot be
-// had: device memory, a stream being captured).
-static bool gather_packed(gc_ctx *ctx, int64_t n) {
-  const size_t g3 = (size_t)ctx->G * ctx->G * ctx->G;
-  if (n < PACK_MIN || (size_t)n < g3 / 8) return false;
-  if (ctx->g4) return true;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
-  if (cudaMalloc(&ctx->g4, g3 * sizeof(float4)) != cudaSuccess) {
-    cudaGetLastError();
-    ctx->g4 = nullptr;
-    return false;
-  }
-  return true;
-}
-
 extern "C" int gc_gather_accel(gc_ctx *ctx, const float *x, const float *y, const float *z, int64_t n,
                                const float *ax_g, const float *ay_g, const float *az_g, float *acc_x, float *acc_y,
                                float *acc_z) {
@@ -1625,10 +1609,11 @@ extern "C" int gc_gather_accel(gc_ctx *ctx, const float *x, const float *y, cons
   GC_REQUIRE(ctx, x && y && z && ax_g && ay_g && az_g && acc_x && acc_y && acc_z, "gc_gather_accel: NULL pointer");
   unsigned nb = gc_blocks(n, 256);
   if (nb > gc_sms() * 32u) nb = gc_sms() * 32u;
-  if (gather_packed(ctx, n)) {
-    const size_t g3 = (size_t)ctx->G * ctx->G * ctx->G;
-    float4 *g4 = (float4 *)ctx->g4;
-    int *scattered = reinterpret_cast<int *>(ctx->dsmall + GC_S_SCATTERED);
+  const size_t g3 = (size_t)ctx->G * ctx->G * ctx->G;
+  void *own = nullptr;  // the call's packed fields and flag
+  if (n >= PACK_MIN && (size_t)n >= g3 / 8 && gc_scratch_get(ctx, g3 * sizeof(float4) + 16, &own)) {
+    float4 *g4 = (float4 *)own;
+    int *scattered = reinterpret_cast<int *>(g4 + g3);
     gc_launch_after(ctx, GK_GATHER, k_bin_probe, dim3(1), dim3(1024), 0, x, y, z, (long long)n, (float)ctx->dx, ctx->G,
               (int)DepW<false>::box, scattered);
     gc_launch_after(ctx, GK_GATHER, k_pack_fields, dim3(gc_sms() * 16u), dim3(256), 0, ax_g, ay_g, az_g, g3,
@@ -1637,6 +1622,7 @@ extern "C" int gc_gather_accel(gc_ctx *ctx, const float *x, const float *y, cons
               acc_z, (float)ctx->dx, ctx->G, (const int *)scattered);
     gc_launch_after(ctx, GK_GATHER, k_gather_packed, dim3(std::min(nb, gc_sms() * 16u)), dim3(256), 0, x, y, z, (long long)n,
               (const int *)scattered, (const float4 *)g4, acc_x, acc_y, acc_z, (float)ctx->dx, ctx->G);
+    gc_scratch_put(ctx, own);
   } else {
     gc_launch_after(ctx, GK_GATHER, k_gather, dim3(nb), dim3(256), 0, x, y, z, (long long)n, ax_g, ay_g, az_g, acc_x, acc_y,
               acc_z, (float)ctx->dx, ctx->G, (const int *)nullptr);
