@@ -1508,14 +1508,58 @@ extern "C" int gc_potential_to_accel(gc_ctx *ctx, const float *phi, float *ax, f
 // ------------------------------------------------------------------------------
 // gather (deposit.py:85-129)
 // ------------------------------------------------------------------------------
-// Returns at once where `skip` says so (the packed gather below takes the particles).
-__global__ void __launch_bounds__(256)
+#define PACK_MIN 4194304  // particles, and at least an eighth of the nodes
+#define PACK_LINES 16     // stretches of 32 particles that tell whether they come in order
+
+// Pairs of neighbours among 32 particles that lie in about the same column of cells.
+__device__ __forceinline__ int near_pairs(const float *__restrict__ x, const float *__restrict__ y,
+                                          const float *__restrict__ z, long long p0, float dx) {
+  const int lane = threadIdx.x & 31;
+  const float px = __ldg(x + p0 + lane), py = __ldg(y + p0 + lane), pz = __ldg(z + p0 + lane);
+  const float ex = px - __shfl_down_sync(0xffffffffu, px, 1), ey = py - __shfl_down_sync(0xffffffffu, py, 1),
+              ez = pz - __shfl_down_sync(0xffffffffu, pz, 1);
+  const bool near = lane < 31 && fabsf(ex) < dx && fabsf(ey) < dx && fabsf(ez) < 4.0f * dx;
+  return __popc(__ballot_sync(0xffffffffu, near));
+}
+
+// Particles whose corners are all nodes of the grid load the 24 values at once; bounds
+// checks and an address for each corner made this bound by instructions (8M particles on
+// 256^3 in the order of their cells, a Gaussian: 113 us, 87 so; 32 registers, eight CTAs an
+// SM: with six 92).
+//
+// With g4 (many particles) every block looks at the same PACK_LINES stretches, spread over
+// the array. Where few neighbours lie near each other the blocks set the three fields side
+// by side for k_gather_packed instead, and *scattered tells it so. Few: an eighth of the
+// pairs; half of them with more particles than nodes, whose packing then costs less than it
+// saves (particles one cell off their order: 4.2M on 256^3 117 us from the fields, 165
+// packed; 20M on 256^3 504 and 410, 8M on 128^3 206 and 146). A look costs 1 us, the
+// kernel that returns 3. g4 and scattered are the call's own.
+__global__ void __launch_bounds__(256, 8)
     k_gather(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z, long long n,
              const float *__restrict__ axg, const float *__restrict__ ayg, const float *__restrict__ azg,
              float *__restrict__ ax, float *__restrict__ ay, float *__restrict__ az, float dx, int G,
-             const int *__restrict__ skip) {
+             float4 *__restrict__ g4, int *__restrict__ scattered) {
   gc_after();
-  if (skip && *skip) return;
+  if (g4) {
+    __shared__ int near_s[8];
+    const int warp = threadIdx.x >> 5;
+    int c = 0;
+#pragma unroll
+    for (int s = 0; s < PACK_LINES / 8; ++s) c += near_pairs(x, y, z, (n - 32) * (warp + 8 * s) / (PACK_LINES - 1), dx);
+    if ((threadIdx.x & 31) == 0) near_s[warp] = c;
+    __syncthreads();
+    c = 0;
+#pragma unroll
+    for (int w = 0; w < 8; ++w) c += near_s[w];
+    const size_t nodes = (size_t)G * G * G;
+    const bool sc = c < PACK_LINES * 31 / ((size_t)n > nodes + nodes / 8 ? 2 : 8);
+    if (blockIdx.x == 0 && threadIdx.x == 0) *scattered = sc;
+    if (sc) {
+      for (size_t i = blockIdx.x * (size_t)256 + threadIdx.x; i < nodes; i += (size_t)gridDim.x * 256)
+        g4[i] = make_float4(axg[i], ayg[i], azg[i], 0.0f);
+      return;
+    }
+  }
   for (long long p = blockIdx.x * (long long)blockDim.x + threadIdx.x; p < n; p += (long long)gridDim.x * blockDim.x) {
     float sx = 0.0f, sy = 0.0f, sz = 0.0f;
     CellPos c;
@@ -1523,21 +1567,34 @@ __global__ void __launch_bounds__(256)
       const float wx[2] = {__fsub_rn(1.0f, c.fx), c.fx};
       const float wy[2] = {__fsub_rn(1.0f, c.fy), c.fy};
       const float wz[2] = {__fsub_rn(1.0f, c.fz), c.fz};
+      if (min(min(c.ix, c.iy), c.iz) >= 0 && max(max(c.ix, c.iy), c.iz) + 1 < G) {
+        const int at = (c.ix * G + c.iy) * G + c.iz;  // G^3 <= 2^30
+        float u[8], v[8], w[8];
 #pragma unroll
-      for (int cx = 0; cx < 2; ++cx)
+        for (int k = 0; k < 8; ++k) u[k] = __ldg(axg + at + ((k >> 2) * G + ((k >> 1) & 1)) * G + (k & 1));
 #pragma unroll
-        for (int cy = 0; cy < 2; ++cy)
+        for (int k = 0; k < 8; ++k) v[k] = __ldg(ayg + at + ((k >> 2) * G + ((k >> 1) & 1)) * G + (k & 1));
 #pragma unroll
-          for (int cz = 0; cz < 2; ++cz) {
-            const int jx = c.ix + cx, jy = c.iy + cy, jz = c.iz + cz;
-            if ((unsigned)jx < (unsigned)G && (unsigned)jy < (unsigned)G && (unsigned)jz < (unsigned)G) {
-              const float w = __fmul_rn(__fmul_rn(wx[cx], wy[cy]), wz[cz]);
-              const size_t idx = ((size_t)jx * G + jy) * G + jz;
-              sx = __fadd_rn(sx, __fmul_rn(w, axg[idx]));
-              sy = __fadd_rn(sy, __fmul_rn(w, ayg[idx]));
-              sz = __fadd_rn(sz, __fmul_rn(w, azg[idx]));
-            }
-          }
+        for (int k = 0; k < 8; ++k) w[k] = __ldg(azg + at + ((k >> 2) * G + ((k >> 1) & 1)) * G + (k & 1));
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const float f = __fmul_rn(__fmul_rn(wx[k >> 2], wy[(k >> 1) & 1]), wz[k & 1]);
+          sx = __fadd_rn(sx, __fmul_rn(f, u[k]));
+          sy = __fadd_rn(sy, __fmul_rn(f, v[k]));
+          sz = __fadd_rn(sz, __fmul_rn(f, w[k]));
+        }
+      } else {
+#pragma unroll
+        for (int k = 0; k < 8; ++k) {
+          const int jx = c.ix + (k >> 2), jy = c.iy + ((k >> 1) & 1), jz = c.iz + (k & 1);
+          if ((unsigned)jx >= (unsigned)G || (unsigned)jy >= (unsigned)G || (unsigned)jz >= (unsigned)G) continue;
+          const float f = __fmul_rn(__fmul_rn(wx[k >> 2], wy[(k >> 1) & 1]), wz[k & 1]);
+          const size_t idx = ((size_t)jx * G + jy) * G + jz;
+          sx = __fadd_rn(sx, __fmul_rn(f, axg[idx]));
+          sy = __fadd_rn(sy, __fmul_rn(f, ayg[idx]));
+          sz = __fadd_rn(sz, __fmul_rn(f, azg[idx]));
+        }
+      }
     }
     ax[p] = sx;
     ay[p] = sy;
@@ -1545,25 +1602,11 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-#define PACK_MIN 4194304  // particles, and at least an eighth of the nodes
-
-// The three fields side by side, for the gather below.
-__global__ void __launch_bounds__(256)
-    k_pack_fields(const float *__restrict__ axg, const float *__restrict__ ayg, const float *__restrict__ azg, size_t n,
-                  const int *__restrict__ scattered, float4 *__restrict__ g4) {
-  gc_after();
-  if (!*scattered) return;
-  for (size_t i = blockIdx.x * (size_t)256 + threadIdx.x; i < n; i += (size_t)gridDim.x * 256)
-    g4[i] = make_float4(axg[i], ayg[i], azg[i], 0.0f);
-}
-
-// k_gather for many scattered particles (k_bin_probe), from the packed fields: the same
-// sums in the same order, 8 loads of 16 bytes a particle where three fields take 24 of 4,
-// each of them another sector of the L2, which is what bounds it. 10M on 256^3 in a
-// Gaussian 784 us, 318 with 70 for packing, evenly spread 1437 and 691. Particles in the
-// order of their cells share sectors and keep the three fields (133; packed 188); the
-// probe and the kernels that return cost them 8 us, so it is asked from 4M particles on.
-// (One kernel for both kinds took 175 us for ordered particles: its registers.)
+// k_gather for many scattered particles, from the packed fields: the same sums in the
+// same order, 8 loads of 16 bytes a particle where three fields take 24 of 4, each of them
+// another sector of the L2, which is what bounds it. In no order, a Gaussian, with the packing: 8M on 256^3 633 us
+// from the fields, 273 so; 20M 1569 and 554; 4.2M on 64^3 222 and 96. (One kernel for
+// both kinds was slower for ordered particles: its registers.)
 __global__ void __launch_bounds__(256)
     k_gather_packed(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z, long long n,
                     const int *__restrict__ scattered, const float4 *__restrict__ g4, float *__restrict__ ax,
@@ -1609,23 +1652,17 @@ extern "C" int gc_gather_accel(gc_ctx *ctx, const float *x, const float *y, cons
   GC_REQUIRE(ctx, x && y && z && ax_g && ay_g && az_g && acc_x && acc_y && acc_z, "gc_gather_accel: NULL pointer");
   unsigned nb = gc_blocks(n, 256);
   if (nb > gc_sms() * 32u) nb = gc_sms() * 32u;
-  const size_t g3 = (size_t)ctx->G * ctx->G * ctx->G;
-  void *own = nullptr;  // the call's packed fields and flag
-  if (n >= PACK_MIN && (size_t)n >= g3 / 8 && gc_scratch_get(ctx, g3 * sizeof(float4) + 16, &own)) {
-    float4 *g4 = (float4 *)own;
-    int *scattered = reinterpret_cast<int *>(g4 + g3);
-    gc_launch_after(ctx, GK_GATHER, k_bin_probe, dim3(1), dim3(1024), 0, x, y, z, (long long)n, (float)ctx->dx, ctx->G,
-              (int)DepW<false>::box, scattered);
-    gc_launch_after(ctx, GK_GATHER, k_pack_fields, dim3(gc_sms() * 16u), dim3(256), 0, ax_g, ay_g, az_g, g3,
-              (const int *)scattered, g4);
-    gc_launch_after(ctx, GK_GATHER, k_gather, dim3(nb), dim3(256), 0, x, y, z, (long long)n, ax_g, ay_g, az_g, acc_x, acc_y,
-              acc_z, (float)ctx->dx, ctx->G, (const int *)scattered);
+  const size_t nodes = (size_t)ctx->G * ctx->G * ctx->G;
+  void *own = nullptr;
+  if (n >= PACK_MIN && (size_t)n >= nodes / 8) gc_scratch_get(ctx, nodes * sizeof(float4) + 16, &own);
+  float4 *g4 = (float4 *)own;
+  int *scattered = own ? reinterpret_cast<int *>(g4 + nodes) : nullptr;
+  gc_launch_after(ctx, GK_GATHER, k_gather, dim3(nb), dim3(256), 0, x, y, z, (long long)n, ax_g, ay_g, az_g, acc_x, acc_y,
+                  acc_z, (float)ctx->dx, ctx->G, g4, scattered);
+  if (own) {
     gc_launch_after(ctx, GK_GATHER, k_gather_packed, dim3(std::min(nb, gc_sms() * 16u)), dim3(256), 0, x, y, z, (long long)n,
-              (const int *)scattered, (const float4 *)g4, acc_x, acc_y, acc_z, (float)ctx->dx, ctx->G);
+                    (const int *)scattered, (const float4 *)g4, acc_x, acc_y, acc_z, (float)ctx->dx, ctx->G);
     gc_scratch_put(ctx, own);
-  } else {
-    gc_launch_after(ctx, GK_GATHER, k_gather, dim3(nb), dim3(256), 0, x, y, z, (long long)n, ax_g, ay_g, az_g, acc_x, acc_y,
-              acc_z, (float)ctx->dx, ctx->G, (const int *)nullptr);
   }
   GC_LAUNCH_CHECK(ctx, "gather");
   return GC_OK;
