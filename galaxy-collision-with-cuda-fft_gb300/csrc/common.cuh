@@ -165,6 +165,9 @@ struct gc_ctx {
 int gc_ws_pre_solve(gc_ctx *ctx, int warm, int mode);
 int gc_ws_post_solve(gc_ctx *ctx);
 
+// Whether ctx's stream is being captured (or may be: a query that fails).
+bool gc_stream_capturing(gc_ctx *ctx);
+
 // Scratch of one call, in the order of ctx's stream: the context may be shared by callers
 // on several streams, so nothing that a call's kernels hand to each other lies in it.
 // False (and *p null) where there is none: no device memory, or a stream under capture,

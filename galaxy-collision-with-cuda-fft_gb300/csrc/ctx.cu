@@ -171,12 +171,16 @@ static cudaMemPool_t scratch_pool(gc_ctx *ctx) {
   return s.pool;
 }
 
-bool gc_scratch_get(gc_ctx *ctx, size_t bytes, void **p) {
-  *p = nullptr;
+bool gc_stream_capturing(gc_ctx *ctx) {
   cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
   const cudaError_t e = cudaStreamIsCapturing(ctx->stream, &cs);
   if (e != cudaSuccess) cudaGetLastError();
-  if (e != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
+  return e != cudaSuccess || cs != cudaStreamCaptureStatusNone;
+}
+
+bool gc_scratch_get(gc_ctx *ctx, size_t bytes, void **p) {
+  *p = nullptr;
+  if (gc_stream_capturing(ctx)) return false;
   const cudaMemPool_t pool = scratch_pool(ctx);
   if (!pool) return false;
   if (cudaMallocFromPoolAsync(p, bytes, pool, ctx->stream) != cudaSuccess) {

@@ -1125,8 +1125,9 @@ __global__ void __launch_bounds__(256)
 }
 
 // The binned passes' scratch for n particles, grown as needed and kept by the context:
-// counters, items, copies, list. False where it cannot be had (device memory, a stream being
-// captured): the particles are then deposited one by one as before.
+// counters, items, copies, list. False where it cannot be had (device memory) and for a
+// stream under capture, whose recorded kernels would go on using a block that a larger
+// deposit has replaced: the particles are then deposited one by one.
 //
 // Particles per item: BIN_ITEM where that leaves two items for every SM, else BIN_SUB (250k
 // particles on 64^3: the tiles take 42 us with 8192, 14 with 2048).
@@ -1135,9 +1136,8 @@ static bool bin_scratch(gc_ctx *ctx, int64_t n) {
   const size_t items = (size_t)BIN_MAX + (size_t)(n / bin_item(n)) + 1;
   const size_t head = (sizeof(BinScratch) + 255) & ~(size_t)255, ib = (items * sizeof(int2) + 255) & ~(size_t)255;
   const size_t need = head + ib + (size_t)n * (sizeof(float4) + sizeof(int));
+  if (gc_stream_capturing(ctx)) return false;
   if (ctx->bin && ctx->bin_cap >= need) return true;
-  cudaStreamCaptureStatus cs = cudaStreamCaptureStatusNone;
-  if (cudaStreamIsCapturing(ctx->stream, &cs) != cudaSuccess || cs != cudaStreamCaptureStatusNone) return false;
   if (ctx->bin) cudaFree(ctx->bin);  // (waits for the work that uses it)
   ctx->bin = nullptr;
   ctx->bin_cap = 0;
