@@ -821,6 +821,7 @@ __global__ void __launch_bounds__(32 * WARPS, (WIDE ? 3 : 4) * (8 / WARPS))
 #define BIN_MIN 200000      // particles, and at least an eighth of the nodes
 #define BIN_MAX 4096        // tiles: grids up to 256^3
 #define BIN_MAX_GRID 256
+#define BIN_CHUNK (1 << 25) // particles that the passes take at a time: bounds their scratch (671 MB) and places
 #define BIN_ITEM 8192       // most particles per flush
 #define BIN_SUB 2048        // particles between carries: low halves of at most 2^19 each stay below 2^30
 #define BIN_NY (BIN_Y + 1)
@@ -1124,7 +1125,7 @@ __global__ void __launch_bounds__(256)
   }
 }
 
-// The binned passes' scratch for n particles, grown as needed and kept by the context:
+// The binned passes' scratch for n <= BIN_CHUNK particles, grown as needed and kept by the context:
 // counters, items, copies, list. False where it cannot be had (device memory) and for a
 // stream under capture, whose recorded kernels would go on using a block that a larger
 // deposit has replaced: the particles are then deposited one by one.
@@ -1186,7 +1187,7 @@ int gc_deposit_q(gc_ctx *ctx, const float *x, const float *y, const float *z, co
   // tile on: 2M in a Gaussian on 128^3 104 us one by one, 68 binned, on 256^3 114 and 102,
   // 10M 465 and 335; but 500k on 128^3 34 and 35, on 256^3 45 and 54.
   const bool bins = any_order && n >= BIN_MIN && n >= (int64_t)ctx->G * ctx->G * ctx->G / 8 && ctx->G <= BIN_MAX_GRID &&
-                    bin_scratch(ctx, n);
+                    bin_scratch(ctx, std::min<int64_t>(n, BIN_CHUNK));
   BinScratch *sc = bins ? (BinScratch *)ctx->bin : nullptr;
   if (bins)
     gc_launch_after(ctx, GK_DEPOSIT_RUNS, k_bin_probe, dim3(1), dim3(1024), 0, x, y, z, (long long)n, d.dx, ctx->G,
@@ -1194,24 +1195,29 @@ int gc_deposit_q(gc_ctx *ctx, const float *x, const float *y, const float *z, co
   gc_launch_after(ctx, GK_DEPOSIT_RUNS, k, dim3(nb), dim3(32 * warps), 0, x, y, z, m, (long long)n, d, inv_dx, qexp, ctx->q,
             ctx->dstatus, bins ? (const int *)&sc->scattered : (const int *)nullptr);
   if (bins) {
+    const int64_t most_c = std::min<int64_t>(n, BIN_CHUNK);
     const size_t head = (sizeof(BinScratch) + 255) & ~(size_t)255;
-    const int per = bin_item(n);
-    const size_t ib = (((size_t)BIN_MAX + (size_t)(n / per) + 1) * sizeof(int2) + 255) & ~(size_t)255;
+    const int per = bin_item(most_c);
+    const size_t ib = (((size_t)BIN_MAX + (size_t)(most_c / per) + 1) * sizeof(int2) + 255) & ~(size_t)255;
     int2 *items = (int2 *)((char *)ctx->bin + head);
     float4 *copy = (float4 *)((char *)ctx->bin + head + ib);
-    int *rare = (int *)(copy + n);
+    int *rare = (int *)(copy + most_c);
     const unsigned sms = (unsigned)gc_sms();
     auto k1 = pow2 ? k_bin_count<true> : k_bin_count<false>;
     auto k2 = pow2 ? k_bin_scatter<true> : k_bin_scatter<false>;
-    gc_launch_after(ctx, GK_DEPOSIT_RUNS, k1, dim3(std::min(gc_blocks(n, 2048), sms * 3u)), dim3(512), 0, x, y, z, (long long)n,
-              d, inv_dx, per, sc, items, ctx->dstatus);
-    gc_launch_after(ctx, GK_DEPOSIT_RUNS, k2, dim3(std::min(gc_blocks(n, 2048), sms * 2u)), dim3(512), 0, x, y, z, m,
-              (long long)n, d, inv_dx, qexp, sc, copy, rare);
-    gc_launch_after(ctx, GK_DEPOSIT_RUNS, k_bin_deposit, dim3(sms * 5u), dim3(256), 0, (const float4 *)copy, ctx->G, per,
-              (const BinScratch *)sc, (const int2 *)items, ctx->q);
     auto k4 = pow2 ? k_bin_rare<true> : k_bin_rare<false>;
-    gc_launch_after(ctx, GK_DEPOSIT_RUNS, k4, dim3(sms), dim3(256), 0, x, y, z, m, d, inv_dx, qexp, (const BinScratch *)sc,
-              (const int *)rare, ctx->q);
+    for (int64_t at = 0; at < n; at += BIN_CHUNK) {
+      const int64_t c = std::min<int64_t>(n - at, BIN_CHUNK);
+      const float *px = x + at, *py = y + at, *pz = z + at, *pm = m + at;
+      gc_launch_after(ctx, GK_DEPOSIT_RUNS, k1, dim3(std::min(gc_blocks(c, 2048), sms * 3u)), dim3(512), 0, px, py, pz,
+                (long long)c, d, inv_dx, per, sc, items, ctx->dstatus);
+      gc_launch_after(ctx, GK_DEPOSIT_RUNS, k2, dim3(std::min(gc_blocks(c, 2048), sms * 2u)), dim3(512), 0, px, py, pz, pm,
+                (long long)c, d, inv_dx, qexp, sc, copy, rare);
+      gc_launch_after(ctx, GK_DEPOSIT_RUNS, k_bin_deposit, dim3(sms * 5u), dim3(256), 0, (const float4 *)copy, ctx->G, per,
+                (const BinScratch *)sc, (const int2 *)items, ctx->q);
+      gc_launch_after(ctx, GK_DEPOSIT_RUNS, k4, dim3(sms), dim3(256), 0, px, py, pz, pm, d, inv_dx, qexp,
+                (const BinScratch *)sc, (const int *)rare, ctx->q);
+    }
   }
   GC_LAUNCH_CHECK(ctx, "deposit");
   return GC_OK;
