@@ -33,12 +33,12 @@ enum {
   GC_S_RNORM64 = 5,  // FP64 residual norm^2 (verification kernel)
   GC_S_GRIDPE = 6,   // Sum b0*phi (engine grid energy, h^2 4 pi G units)
   GC_S_MASS_PM = 7,  // engine: total density-mass of its particles
-  GC_S_QEXP_PM = 8,  // engine: quantum exponent
+  GC_S_QEXP_PM = 8,  // engine: quantum exponent; the slot behind it: see k_mass_heavy (an int)
   GC_S_CYCLES = 2,   // V-cycles of the last device-decided (graph-captured) solve
   GC_S_CONVERGED = 3,// 1 if that solve met its tolerance
   GC_S_MIRROR = 4,   // slots [0, 4) are copied to the pinned mirror by captured solves
-  GC_S_MASS = 12,    // total deposited density-mass used for the fixed-point quantum
-  GC_S_QEXP = 13,    // quantum exponent E: quantum = 2^E (density units)
+  GC_S_MASS = 10,    // total deposited density-mass used for the fixed-point quantum
+  GC_S_QEXP = 11,    // quantum exponent E: quantum = 2^E (density units); behind it as for the engine's
   GC_S_SOLVES = 14,  // device-decided solves since the counters were reset ...
   GC_S_CYC_TOTAL = 15, // ... their V-cycles ...
   GC_S_MAXREL2 = 16, // ... and the largest (||r|| / ||b||)^2 they ended with
@@ -479,11 +479,13 @@ int gc_faces_from_moments(gc_ctx *ctx);
 int gc_convert_cpw(int G);
 int gc_finalize(gc_ctx *ctx, const double *parts, int nparts, int nv, double *dst);
 // Sum of m/dx^3 (FP64, deterministic) into dsmall[mass_slot] and the fixed-point
-// exponent E (quantum 2^E, total <= 2^bits quanta) into dsmall[exp_slot].
+// exponent E (quantum 2^E, total <= 2^bits quanta) into dsmall[exp_slot]; behind it, as an
+// int, whether many particles reach 2^22 quanta, where gc_deposit_q asks for it.
 int gc_fixed_point_setup(gc_ctx *ctx, const float *m, int64_t n, int bits, int mass_slot, int exp_slot);
 // int64 fixed-point CIC deposit into ctx->q (which must be zero on entry). Any
 // particle order; runs of equal cells (cell-sorted input) are summed in registers.
-// `bits` is the fixed-point resolution *qexp was set up with (it only picks the pass).
+// `bits` is the fixed-point resolution *qexp was set up with (it only picks the pass), and
+// qexp the slot gc_fixed_point_setup wrote.
 int gc_deposit_q(gc_ctx *ctx, const float *x, const float *y, const float *z, const float *m, int64_t n, int bits,
                  const double *qexp, bool any_order = false);
 // Read ctx->q, write rho (may be NULL) and b = f32(q 2^E 4 pi G h^2) (may be NULL),

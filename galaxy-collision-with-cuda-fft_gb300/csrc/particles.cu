@@ -79,6 +79,26 @@ __global__ void k_qexp(const unsigned *__restrict__ maxbits, const unsigned long
   small[exp_slot] = (double)E;
 }
 
+// Quanta of the mean particle, 1 to 2 times this; where it lies between 2^20 and 2^22 and
+// the particles are many, their masses decide which pass of the deposit takes them (see
+// gc_deposit_q).
+#define HEAVY_MIN (1 << 20)
+static double mean_quanta(int bits, int64_t n) { return std::ldexp(1.0, bits - 1) / (double)n; }
+static bool quanta_undecided(int bits, int64_t n) {
+  const double q = mean_quanta(bits, n);
+  return n >= HEAVY_MIN && q >= 1048576.0 && q < 4194304.0;
+}
+
+// Whether at least 1/32 of 1024 masses, spread over the array, reach 2^22 quanta.
+__global__ void __launch_bounds__(1024)
+    k_mass_heavy(const float *__restrict__ m, long long n, float inv_vol, const double *__restrict__ qexp,
+                 int *__restrict__ heavy) {
+  gc_after();
+  const float mm = __fmul_rn(__ldg(m + (n - 1) * (long long)threadIdx.x / 1023), inv_vol);
+  const int c = __syncthreads_count(!(fabsf(__fmul_rn(mm, ldexpf(1.0f, -(int)*qexp))) < 4194304.0f));
+  if (threadIdx.x == 0) *heavy = c >= 32;
+}
+
 static int ceil_log2(long long n) {
   int L = 0;
   while ((1LL << L) < n) ++L;
@@ -100,6 +120,9 @@ int gc_fixed_point_setup(gc_ctx *ctx, const float *m, int64_t n, int bits, int m
   gc_launch_after(ctx, GK_MASS, k_mass_max, dim3(nb), dim3(256), 0, m, (long long)n, inv_vol, maxbits);
   gc_launch_after(ctx, GK_MASS, k_mass_isum, dim3(nb), dim3(256), 0, m, (long long)n, inv_vol, maxbits, L, isum);
   gc_launch_after(ctx, GK_MASS, k_qexp, dim3(1), dim3(32), 0, maxbits, isum, L, ctx->dsmall, mass_slot, exp_slot, bits);
+  if (quanta_undecided(bits, n))
+    gc_launch_after(ctx, GK_MASS, k_mass_heavy, dim3(1), dim3(1024), 0, m, (long long)n, inv_vol,
+                    (const double *)(ctx->dsmall + exp_slot), reinterpret_cast<int *>(ctx->dsmall + exp_slot + 1));
   GC_LAUNCH_CHECK(ctx, "fixed-point set-up");
   return GC_OK;
 }
@@ -693,10 +716,11 @@ __global__ void __launch_bounds__(32 * WARPS, (WIDE ? 3 : 4) * (8 / WARPS))
     k_deposit_sorted(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
                      const float *__restrict__ m, long long n, DepCtx d, float inv_dx,
                      const double *__restrict__ qexp, long long *__restrict__ qg, unsigned *__restrict__ status,
-                     const int *__restrict__ skip) {
+                     const int *__restrict__ skip, const int *__restrict__ heavy) {
   gc_after();
   __shared__ int dep_box[WARPS * DepW<WIDE>::words];
-  if (skip && *skip) return;  // scattered particles: the binned passes take them
+  if (heavy && (*heavy != 0) != WIDE) return;  // the other form takes the particles
+  if (skip && *skip) return;                   // scattered particles: the binned passes take them
   const float qscale = ldexpf(1.0f, -(int)(*qexp));
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   constexpr int tile = WARPS * DEP_WTILE;
@@ -1162,25 +1186,24 @@ int gc_deposit_q(gc_ctx *ctx, const float *x, const float *y, const float *z, co
   int fe = 0;
   const bool pow2 = std::frexp(d.dx, &fe) == 0.5f;
   const float inv_dx = pow2 ? std::ldexp(1.0f, 1 - fe) : 0.0f;
-  // The narrow pass takes particles below 2^22 quanta, the wide one below 2^41;
-  // both leave the rest to the out-of-line rounding, so the choice changes only
-  // speed. The mean particle has at least 2^(bits - 1) / n quanta: wide from 2^20
-  // on, where particles of a few times the mean leave the narrow range (1.5M sorted
-  // particles at 2^-52: 327 us narrow, 21 wide; where both fit, the narrow pass has
-  // half the sums: 10M sorted particles at 2^-44 take 64 us narrow, 105 wide).
-  const bool wide = std::ldexp(1.0, bits - 1) / (double)n >= 1048576.0;
+  // The narrow pass takes particles below 2^22 quanta, the wide one below 2^41; both
+  // leave the rest to the out-of-line rounding, so the choice changes only speed. Where
+  // the particles fit it, the narrow pass has half the sums (8M on 64^3 in the order of their
+  // cells at 2^-44 of the mass: a deposit 91 us narrow, 127 wide; drifted by a third of a
+  // cell 126 and 204); beyond 2^22 quanta its out-of-line particles take thirty times as long
+  // (1.5M at 2^-52: 327 us narrow, 21 wide). The mean particle has 1 to 2 times mean_quanta:
+  // narrow below 2^20, where particles of a few times the mean still fit, wide from 2^22 on.
+  // Between them both are launched and a sample of the masses (k_mass_heavy) tells the one
+  // whose particles they are not to return (4 us in all), from HEAVY_MIN particles on, below
+  // which the passes differ by less (600k on 32^3: 38 and 44 us).
+  const bool both = quanta_undecided(bits, n), wide = mean_quanta(bits, n) >= 1048576.0;
+  const int *heavy = both ? reinterpret_cast<const int *>(qexp + 1) : nullptr;
   // CTAs of eight warps; of two while eight would leave SMs without one (131072
   // particles: 20.4 us with eight, 18.5 with two)
   const bool few = n < (int64_t)gc_sms() * 8 * DEP_WTILE;
-  auto k = few ? (wide ? (pow2 ? k_deposit_sorted<true, true, 2> : k_deposit_sorted<false, true, 2>)
-                       : (pow2 ? k_deposit_sorted<true, false, 2> : k_deposit_sorted<false, false, 2>))
-               : (wide ? (pow2 ? k_deposit_sorted<true, true, 8> : k_deposit_sorted<false, true, 8>)
-                       : (pow2 ? k_deposit_sorted<true, false, 8> : k_deposit_sorted<false, false, 8>));
   const int warps = few ? 2 : 8;
   const long long tile = (long long)warps * DEP_WTILE;
   const long long ntiles = (n + tile - 1) / tile;
-  const long long most = (long long)gc_sms() * (wide ? 3 : 4) * (8 / warps);  // resident CTAs: persistent
-  const unsigned nb = (unsigned)(ntiles < most ? ntiles : most);
   // Callers that cannot say how their particles are ordered: a probe on the device
   // chooses between this kernel and the binned passes, and the one not chosen returns at
   // once (10 us of launches for sorted particles). The passes win from some 500 particles a
@@ -1192,8 +1215,17 @@ int gc_deposit_q(gc_ctx *ctx, const float *x, const float *y, const float *z, co
   if (bins)
     gc_launch_after(ctx, GK_DEPOSIT_RUNS, k_bin_probe, dim3(1), dim3(1024), 0, x, y, z, (long long)n, d.dx, ctx->G,
               wide ? (int)DepW<true>::box : (int)DepW<false>::box, &sc->scattered);
-  gc_launch_after(ctx, GK_DEPOSIT_RUNS, k, dim3(nb), dim3(32 * warps), 0, x, y, z, m, (long long)n, d, inv_dx, qexp, ctx->q,
-            ctx->dstatus, bins ? (const int *)&sc->scattered : (const int *)nullptr);
+  for (int w = 0; w < 2; ++w) {
+    if (!both && (w != 0) != wide) continue;
+    auto k = few ? (w ? (pow2 ? k_deposit_sorted<true, true, 2> : k_deposit_sorted<false, true, 2>)
+                      : (pow2 ? k_deposit_sorted<true, false, 2> : k_deposit_sorted<false, false, 2>))
+                 : (w ? (pow2 ? k_deposit_sorted<true, true, 8> : k_deposit_sorted<false, true, 8>)
+                      : (pow2 ? k_deposit_sorted<true, false, 8> : k_deposit_sorted<false, false, 8>));
+    const long long most = (long long)gc_sms() * (w ? 3 : 4) * (8 / warps);  // resident CTAs: persistent
+    const unsigned nb = (unsigned)(ntiles < most ? ntiles : most);
+    gc_launch_after(ctx, GK_DEPOSIT_RUNS, k, dim3(nb), dim3(32 * warps), 0, x, y, z, m, (long long)n, d, inv_dx, qexp, ctx->q,
+              ctx->dstatus, bins ? (const int *)&sc->scattered : (const int *)nullptr, heavy);
+  }
   if (bins) {
     const int64_t most_c = std::min<int64_t>(n, BIN_CHUNK);
     const size_t head = (sizeof(BinScratch) + 255) & ~(size_t)255;
