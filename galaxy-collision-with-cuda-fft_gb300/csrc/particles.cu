@@ -886,45 +886,61 @@ __device__ __forceinline__ int bin_of(float px, float py, float pz, const DepCtx
   return ((ix / BIN_X) * b.ny + iy / BIN_Y) * b.nz + iz / BIN_Z;
 }
 
+// Pairs of neighbours among 32 particles that lie in about the same column of cells.
+__device__ __forceinline__ int near_pairs(float px, float py, float pz, float dx) {
+  const float ex = px - __shfl_down_sync(0xffffffffu, px, 1), ey = py - __shfl_down_sync(0xffffffffu, py, 1),
+              ez = pz - __shfl_down_sync(0xffffffffu, pz, 1);
+  const bool near = (threadIdx.x & 31) < 31 && fabsf(ex) < dx && fabsf(ey) < dx && fabsf(ez) < 4.0f * dx;
+  return __popc(__ballot_sync(0xffffffffu, near));
+}
+
 // Whether the particles come scattered: of 32 stretches of DEP_WTILE, spread over the
-// array, most span more cells than a warp's box of k_deposit_sorted.
+// array, most span more cells than a warp's box of k_deposit_sorted, and fewer than half
+// of their neighbours lie near each other. (Few particles in the order of their cells do the
+// first, and yet their corners share sectors of the grid: 4.3M on 256^3 172 us one by one,
+// 305 binned; drifted by a third of a cell 211 and 278, by a whole one 264 and 272, 8M so
+// 409 and 341.)
 __global__ void __launch_bounds__(1024)
     k_bin_probe(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z, long long n,
                 float dx, int G, int box, int *__restrict__ scattered) {
   gc_after();
-  __shared__ int fit[32];
+  __shared__ int fit[32], near[32];
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  int fits = 0;
-  {
-    const long long p0 = (n - DEP_WTILE) * warp / 31;
-    float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
+  const long long p0 = (n - DEP_WTILE) * warp / 31;
+  float lo[3] = {3.0e38f, 3.0e38f, 3.0e38f}, hi[3] = {-3.0e38f, -3.0e38f, -3.0e38f};
+  int pairs = 0;
 #pragma unroll
-    for (int j = 0; j < DEP_WTILE / 32; ++j) {
-      const long long p = p0 + 32 * j + lane;
-      const float c[3] = {x[p], y[p], z[p]};
+  for (int j = 0; j < DEP_WTILE / 32; ++j) {
+    const long long p = p0 + 32 * j + lane;
+    const float c[3] = {x[p], y[p], z[p]};
+    pairs += near_pairs(c[0], c[1], c[2], dx);
 #pragma unroll
-      for (int a = 0; a < 3; ++a) { lo[a] = fminf(lo[a], c[a]); hi[a] = fmaxf(hi[a], c[a]); }
-    }
-    float vol = 1.0f;
-#pragma unroll
-    for (int a = 0; a < 3; ++a) {
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) {
-        lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
-        hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
-      }
-      const float l = fminf(fmaxf(floorf(lo[a] / dx), -1.0f), (float)G - 1.0f);
-      const float h = fminf(fmaxf(floorf(hi[a] / dx), -1.0f), (float)G - 1.0f);
-      vol *= fmaxf(h - l + 2.0f, 2.0f);
-    }
-    fits += vol <= (float)box;
+    for (int a = 0; a < 3; ++a) { lo[a] = fminf(lo[a], c[a]); hi[a] = fmaxf(hi[a], c[a]); }
   }
-  if (lane == 0) fit[warp] = fits;
+  float vol = 1.0f;
+#pragma unroll
+  for (int a = 0; a < 3; ++a) {
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      lo[a] = fminf(lo[a], __shfl_xor_sync(0xffffffffu, lo[a], o));
+      hi[a] = fmaxf(hi[a], __shfl_xor_sync(0xffffffffu, hi[a], o));
+    }
+    const float l = fminf(fmaxf(floorf(lo[a] / dx), -1.0f), (float)G - 1.0f);
+    const float h = fminf(fmaxf(floorf(hi[a] / dx), -1.0f), (float)G - 1.0f);
+    vol *= fmaxf(h - l + 2.0f, 2.0f);
+  }
+  if (lane == 0) {
+    fit[warp] = vol <= (float)box;
+    near[warp] = pairs;
+  }
   __syncthreads();
   if (threadIdx.x == 0) {
-    int t = 0;
-    for (int w = 0; w < 32; ++w) t += fit[w];
-    *scattered = t < 16;
+    int t = 0, q = 0;
+    for (int w = 0; w < 32; ++w) {
+      t += fit[w];
+      q += near[w];
+    }
+    *scattered = t < 16 && q < 32 * (DEP_WTILE / 32) * 31 / 2;
   }
 }
 
@@ -1549,17 +1565,6 @@ extern "C" int gc_potential_to_accel(gc_ctx *ctx, const float *phi, float *ax, f
 #define PACK_MIN 4194304  // particles, and at least an eighth of the nodes
 #define PACK_LINES 16     // stretches of 32 particles that tell whether they come in order
 
-// Pairs of neighbours among 32 particles that lie in about the same column of cells.
-__device__ __forceinline__ int near_pairs(const float *__restrict__ x, const float *__restrict__ y,
-                                          const float *__restrict__ z, long long p0, float dx) {
-  const int lane = threadIdx.x & 31;
-  const float px = __ldg(x + p0 + lane), py = __ldg(y + p0 + lane), pz = __ldg(z + p0 + lane);
-  const float ex = px - __shfl_down_sync(0xffffffffu, px, 1), ey = py - __shfl_down_sync(0xffffffffu, py, 1),
-              ez = pz - __shfl_down_sync(0xffffffffu, pz, 1);
-  const bool near = lane < 31 && fabsf(ex) < dx && fabsf(ey) < dx && fabsf(ez) < 4.0f * dx;
-  return __popc(__ballot_sync(0xffffffffu, near));
-}
-
 // Particles whose corners are all nodes of the grid load the 24 values at once; bounds
 // checks and an address for each corner made this bound by instructions (8M particles on
 // 256^3 in the order of their cells, a Gaussian: 113 us, 87 so; 32 registers, eight CTAs an
@@ -1583,7 +1588,10 @@ __global__ void __launch_bounds__(256, 8)
     const int warp = threadIdx.x >> 5;
     int c = 0;
 #pragma unroll
-    for (int s = 0; s < PACK_LINES / 8; ++s) c += near_pairs(x, y, z, (n - 32) * (warp + 8 * s) / (PACK_LINES - 1), dx);
+    for (int s = 0; s < PACK_LINES / 8; ++s) {
+      const long long p = (n - 32) * (warp + 8 * s) / (PACK_LINES - 1) + (threadIdx.x & 31);
+      c += near_pairs(__ldg(x + p), __ldg(y + p), __ldg(z + p), dx);
+    }
     if ((threadIdx.x & 31) == 0) near_s[warp] = c;
     __syncthreads();
     c = 0;
