@@ -835,10 +835,12 @@ __global__ void __launch_bounds__(32 * WARPS, (WIDE ? 3 : 4) * (8 / WARPS))
 // 256^3 (two disks): count 48, copy 75, deposit 100 us, 232 in all against 690; 250k at
 // 64^3 (a Plummer sphere) 32 against 65. Bound by the shared-memory atomics (16 a particle)
 // and, where a tile has few particles, by its flush of 5049 nodes.
-// k_bin_deposit has no call in its loops; the rare particles and the divisions are in the
-// other passes. With an out-of-line call in the loop, never taken, the compiled kernel gave
-// wrong sums and once a bad address, while the same source with every index checked was
-// right; one thread reads the item for the block for the same reason.
+// An early form of k_bin_deposit gave wrong sums, and a variant of it a bad address, on
+// inputs that this form and one with every index checked take exactly; the cause was not
+// found in their source. So the indexes stay checked: a particle's place among the copies, an
+// item's tile and range, a node's place in its tile. What fails is left out, or held to the
+// tile, and raises GC_FLAG_INDEX (10M particles on 256^3, the whole call: 450.5 us without,
+// 451.6 so).
 #define BIN_X 8
 #define BIN_Y 16
 #define BIN_Z 32
@@ -851,6 +853,7 @@ __global__ void __launch_bounds__(32 * WARPS, (WIDE ? 3 : 4) * (8 / WARPS))
 #define BIN_NY (BIN_Y + 1)
 #define BIN_NZ (BIN_Z + 1)
 #define BIN_NODES ((BIN_X + 1) * BIN_NY * BIN_NZ)
+#define BIN_LAST (((BIN_X - 1) * BIN_NY + BIN_Y - 1) * BIN_NZ + BIN_Z - 1)  // the last cell's first node
 // Largest particle: halves h of at most 2^18 - 1, so that BIN_ITEM of them stay below 2^31.
 #define BIN_LIMIT 2.7487685e11f  // 2^38 - 2^20
 
@@ -1035,7 +1038,8 @@ template <bool POW2>
 __global__ void __launch_bounds__(512, 2)
     k_bin_scatter(const float *__restrict__ x, const float *__restrict__ y, const float *__restrict__ z,
                   const float *__restrict__ m, long long n, DepCtx d, float inv_dx, const double *__restrict__ qexp,
-                  BinScratch *__restrict__ sc, float4 *__restrict__ out, int *__restrict__ rare) {
+                  BinScratch *__restrict__ sc, float4 *__restrict__ out, int *__restrict__ rare,
+                  unsigned *__restrict__ status) {
   gc_after();
   __shared__ int hist[BIN_MAX];
   if (!sc->scattered) return;
@@ -1074,7 +1078,11 @@ __global__ void __launch_bounds__(512, 2)
         rare[atomicAdd(&sc->nrare, 1)] = (int)(c0 + 512 * j + tid);
         v[j] = make_float4(fmaxf(v[j].x, 0.0f), fmaxf(v[j].y, 0.0f), fmaxf(v[j].z, 0.0f), 0.0f);
       }
-      out[hist[bin[j]] + rank[j]] = v[j];
+      const int place = hist[bin[j]] + rank[j];
+      if ((unsigned)place < (unsigned)n)
+        out[place] = v[j];
+      else
+        atomicOr(status, GC_FLAG_INDEX);
     }
     __syncthreads();
     for (int i = tid; i < b.n; i += 512) hist[i] = 0;
@@ -1084,20 +1092,27 @@ __global__ void __launch_bounds__(512, 2)
 // One item at a time: corners into the tile's nodes (halves h 2^20 + l), then the nodes to
 // the grid.
 __global__ void __launch_bounds__(256)
-    k_bin_deposit(const float4 *__restrict__ part, int G, int per, const BinScratch *__restrict__ sc,
-                  const int2 *__restrict__ items, long long *__restrict__ qg) {
+    k_bin_deposit(const float4 *__restrict__ part, int n, int G, int per, const BinScratch *__restrict__ sc,
+                  const int2 *__restrict__ items, long long *__restrict__ qg, unsigned *__restrict__ status) {
   gc_after();
   __shared__ int lo[BIN_NODES], hi[BIN_NODES];
   __shared__ int4 cur;  // the item: first and last particle, tile
   if (!sc->scattered) return;
   const BinGeo b = bin_geo(G);
   const int tid = threadIdx.x, nitems = sc->nitems;
+  unsigned worst = 0;  // largest node met
   for (int i = tid; i < BIN_NODES; i += 256) lo[i] = hi[i] = 0;
   for (int item = blockIdx.x; item < nitems; item += gridDim.x) {
     __syncthreads();  // the last item's nodes are flushed
     if (tid == 0) {
       const int2 it = items[item];
-      cur = make_int4(it.y, min(sc->start[it.x + 1], it.y + per), it.x, 0);
+      int4 c = make_int4(0, 0, 0, 0);
+      if ((unsigned)it.x < (unsigned)b.n) c = make_int4(it.y, min(sc->start[it.x + 1], it.y + per), it.x, 0);
+      if (c.x < 0 || c.x >= c.y || c.y > n) {
+        c = make_int4(0, 0, 0, 0);
+        atomicOr(status, GC_FLAG_INDEX);
+      }
+      cur = c;
     }
     __syncthreads();
     const int end = cur.y, tile = cur.z;
@@ -1113,7 +1128,9 @@ __global__ void __launch_bounds__(256)
                     fz = __fsub_rn(v.z, __int2float_rn(iz));
         int h[8], l[8];
         dep_corners_wide(v.w, __fsub_rn(1.0f, fx), fx, __fsub_rn(1.0f, fy), fy, __fsub_rn(1.0f, fz), fz, h, l);
-        const int node = ((ix - x0) * BIN_NY + (iy - y0)) * BIN_NZ + (iz - z0);
+        const unsigned at = (unsigned)(((ix - x0) * BIN_NY + (iy - y0)) * BIN_NZ + (iz - z0));
+        worst = max(worst, at);
+        const int node = (int)min(at, (unsigned)BIN_LAST);
 #pragma unroll
         for (int c = 0; c < 8; ++c) {
           const int q = node + (c >> 2) * (BIN_NY * BIN_NZ) + ((c >> 1) & 1) * BIN_NZ + (c & 1);
@@ -1142,6 +1159,7 @@ __global__ void __launch_bounds__(256)
         atomicAdd((unsigned long long *)(qg + ((size_t)jx * G + jy) * G + jz), (unsigned long long)v);
     }
   }
+  if (worst > BIN_LAST) atomicOr(status, GC_FLAG_INDEX);
 }
 
 // The particles that no tile takes, one by one.
@@ -1260,9 +1278,9 @@ int gc_deposit_q(gc_ctx *ctx, const float *x, const float *y, const float *z, co
       gc_launch_after(ctx, GK_DEPOSIT_RUNS, k1, dim3(std::min(gc_blocks(c, 2048), sms * 3u)), dim3(512), 0, px, py, pz,
                 (long long)c, d, inv_dx, per, sc, items, ctx->dstatus);
       gc_launch_after(ctx, GK_DEPOSIT_RUNS, k2, dim3(std::min(gc_blocks(c, 2048), sms * 2u)), dim3(512), 0, px, py, pz, pm,
-                (long long)c, d, inv_dx, qexp, sc, copy, rare);
-      gc_launch_after(ctx, GK_DEPOSIT_RUNS, k_bin_deposit, dim3(sms * 5u), dim3(256), 0, (const float4 *)copy, ctx->G, per,
-                (const BinScratch *)sc, (const int2 *)items, ctx->q);
+                (long long)c, d, inv_dx, qexp, sc, copy, rare, ctx->dstatus);
+      gc_launch_after(ctx, GK_DEPOSIT_RUNS, k_bin_deposit, dim3(sms * 5u), dim3(256), 0, (const float4 *)copy, (int)c,
+                ctx->G, per, (const BinScratch *)sc, (const int2 *)items, ctx->q, ctx->dstatus);
       gc_launch_after(ctx, GK_DEPOSIT_RUNS, k4, dim3(sms), dim3(256), 0, px, py, pz, pm, d, inv_dx, qexp,
                 (const BinScratch *)sc, (const int *)rare, ctx->q);
     }

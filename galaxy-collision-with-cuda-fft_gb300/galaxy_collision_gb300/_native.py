@@ -26,6 +26,7 @@ GC_FLAG_NONFINITE_RHO = 0x2
 GC_FLAG_BAD_PID = 0x4
 GC_FLAG_IC_REJECT = 0x8
 GC_FLAG_TIMEOUT = 0x10
+GC_FLAG_INDEX = 0x20
 GC_MG_FIXED_CYCLES = 0x2
 GC_MG_PLAIN_F32 = 0x4
 GC_MG_NATURAL_LAYOUT = 0x8

@@ -48,6 +48,7 @@ enum gc_status_code {
 #define GC_FLAG_BAD_PID 0x4u        /* gc_pm_export met a pid outside [0, n): that particle was skipped */
 #define GC_FLAG_IC_REJECT 0x8u      /* a device IC rejection loop reached its attempt limit */
 #define GC_FLAG_TIMEOUT 0x10u       /* a bounded wait inside a kernel ran out; that kernel stopped early */
+#define GC_FLAG_INDEX 0x20u         /* a kernel met an index outside its arrays: what it named was left out or kept inside */
 
 /* gc_mg_params.flags: run exactly max_cycles V-cycles without reading the
  * residual norm on the host (it is left on the device; gc_pm_last_residual
