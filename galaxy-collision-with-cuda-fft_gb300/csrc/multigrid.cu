@@ -2126,7 +2126,9 @@ __global__ void __launch_bounds__(256)
 // b0 = h^2 * f32(f32(4 pi G) * rho) with ||b0||^2, in one pass. A warp takes
 // eight neighbouring columns (i, j .. j+7) at a time, persistent over those
 // units: Kahan-compensated FP32 sums of rho, rho k and rho k^2 along k (the
-// reference's column scheme, multigrid.py:192-221), finished in FP64.
+// reference's column scheme, multigrid.py:192-221), finished in FP64. The squares of b0 are
+// added eight to a tree and those as pairs: a chain of single sums (220 squares a thread at
+// 256^3) was 2.3e-8 off in ||b0||, the 32 squares of a thread before that 2.7e-9, this 1.4e-10.
 //
 // Bound by HBM (read rho, write b0) once FP64 is kept out of the way: an FP64
 // warp instruction, conversions included, takes 16 clocks of the SM on this part.
@@ -2151,14 +2153,13 @@ __global__ void __launch_bounds__(256, 2)
                   double *__restrict__ bnorm2, unsigned *__restrict__ status) {
   gc_after();
   __shared__ double wsum[8 * MOM_COLS][11];
-  __shared__ double bsum[1];
   const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
   const int upr = (G + MOM_COLS - 1) / MOM_COLS;  // units per i
   const long long nunits = (long long)G * upr;
   // a row of sums per (warp, column): kept in shared memory, only its lane touches it
   for (int t = threadIdx.x; t < 8 * MOM_COLS * 11; t += 256) (&wsum[0][0])[t] = 0.0;
   __syncthreads();
-  float acc = 0.0f;
+  float acc = 0.0f, accl = 0.0f;  // ||b0||^2 of the thread, as a pair
   bool bad = false;
   // the column of the unit whose sums this lane ends up with (bits 4, 3, 2 of the lane)
   const int mine = lane >> 2;
@@ -2184,24 +2185,28 @@ __global__ void __launch_bounds__(256, 2)
 #pragma unroll
       for (int t = 0; t < MOM_COLS; ++t) rn[t] = t < nc && k + 32 < G ? src[(size_t)t * G] : 0.0f;
       if (b0) {
+        float bv[MOM_COLS];
 #pragma unroll
         for (int t = 0; t < MOM_COLS; ++t) {
-          const float bv = __fmul_rn(__fmul_rn(fpg, r[t]), h2);
-          if (t < nc) b0[at + (size_t)t * G + k] = bv;
-          acc += bv * bv;
+          bv[t] = __fmul_rn(__fmul_rn(fpg, r[t]), h2);
+          if (t < nc) b0[at + (size_t)t * G + k] = bv[t];
         }
+        const float q0 = __fmaf_rn(bv[1], bv[1], __fmul_rn(bv[0], bv[0])), q1 = __fmaf_rn(bv[3], bv[3], __fmul_rn(bv[2], bv[2])),
+                    q2 = __fmaf_rn(bv[5], bv[5], __fmul_rn(bv[4], bv[4])), q3 = __fmaf_rn(bv[7], bv[7], __fmul_rn(bv[6], bv[6]));
+        float e;
+        df_two_sum(acc, __fadd_rn(__fadd_rn(q0, q1), __fadd_rn(q2, q3)), acc, e);
+        accl = __fadd_rn(accl, e);
       }
 #pragma unroll
       for (int t = 0; t < MOM_COLS; ++t) {
         const bool fin = fabsf(r[t]) <= 3.402823466e38f;
         bad |= !fin;
-        float x = fin ? r[t] : 0.0f;
+        const float x = fin ? r[t] : 0.0f, x1 = __fmul_rn(x, fk);
 #pragma unroll
         for (int q = 0; q < 3; ++q) {
-          const float y = __fsub_rn(x, c[q][t]), z = __fadd_rn(s[q][t], y);
+          const float y = q == 2 ? __fmaf_rn(x1, fk, -c[q][t]) : __fsub_rn(q ? x1 : x, c[q][t]), z = __fadd_rn(s[q][t], y);
           c[q][t] = __fsub_rn(__fsub_rn(z, s[q][t]), y);
           s[q][t] = z;
-          x = __fmul_rn(x, fk);
         }
       }
     }
@@ -2239,20 +2244,32 @@ __global__ void __launch_bounds__(256, 2)
     }
   }
   if (bad) atomicOr(status, GC_FLAG_NONFINITE_RHO);
-  block_sum_f32(acc, bsum);  // (its barrier also orders wsum)
+  // the lanes' pairs of ||b0||^2 (an overflow stays an infinity: its error terms are NaN)
+  accl = fabsf(acc) <= 3.402823466e38f ? accl : 0.0f;
+#pragma unroll
+  for (int o = 16; o >= 1; o >>= 1) {
+    const float gh = __shfl_xor_sync(0xffffffffu, acc, o), gl = __shfl_xor_sync(0xffffffffu, accl, o);
+    const float h = __fadd_rn(acc, gh);
+    if (fabsf(h) <= 3.402823466e38f) {
+      pair_add(acc, accl, gh, gl, acc, accl);
+    } else {
+      acc = h;
+      accl = 0.0f;
+    }
+  }
+  if (lane == 0) wsum[wid * MOM_COLS][10] = (double)acc + (double)accl;
   __syncthreads();
-  if (threadIdx.x < 10) {
+  if (threadIdx.x < 11) {
     const int q = threadIdx.x;
     const double vol = dx * dx * dx;
-    const double sc = q == 0 ? vol : q <= 3 ? vol * dx : vol * dx * dx;
+    const double sc = q == 10 ? 1.0 : q == 0 ? vol : q <= 3 ? vol * dx : vol * dx * dx;
     double a = 0.0;
     for (int r = 0; r < 8 * MOM_COLS; ++r) a += wsum[r][q];
     wsum[0][q] = a * sc;
   }
   __syncthreads();
   if (threadIdx.x == 0) {  // one writer: the last-block reduction fences its stores
-    for (int q = 0; q < 10; ++q) parts[(size_t)blockIdx.x * 11 + q] = wsum[0][q];
-    parts[(size_t)blockIdx.x * 11 + 10] = bsum[0];
+    for (int q = 0; q < 11; ++q) parts[(size_t)blockIdx.x * 11 + q] = wsum[0][q];
   }
   if (grid_finish_sum<11>(parts, gridDim.x, ticket, mom) && threadIdx.x == 0 && b0) *bnorm2 = mom[10];
 }
