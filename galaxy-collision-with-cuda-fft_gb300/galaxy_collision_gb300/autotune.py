@@ -95,8 +95,17 @@ def time_candidate(make_engine, state, dt: float, settings: dict, steps: int = 2
 def tune(grid: int, n: int, make_engine, state, dt: float, *, device: str, candidates=CANDIDATES, steps: int = 20,
          measure=None, path: Path | None = None) -> dict:
     """Time every candidate and cache the fastest. `measure(settings) -> ms`
-    replaces the GPU timing (tests)."""
-    measure = measure or (lambda c: time_candidate(make_engine, state, dt, c, steps=steps))
+    replaces the GPU timing (tests). Candidates that differ in ``phase_launches``
+    alone are the same program: they are timed once, and the first listed is picked."""
+    if measure is None:
+        timed = {}
+
+        def measure(c):
+            k = _label({q: v for q, v in c.items() if q != "phase_launches"})
+            if k not in timed:
+                timed[k] = time_candidate(make_engine, state, dt, c, steps=steps)
+            return timed[k]
+
     timings = {}
     by_label = {}
     for c in candidates:
