@@ -1,7 +1,10 @@
-"""Shared device contexts for the stateless operators (deposit, grad, gather, kick, drift).
+"""Shared device contexts for the operators without state of their own (deposit, grad, gather, kick, drift).
 
 One ``gc_ctx`` per (device, grid size, dx) is cached; the solver and the fused
-engine own their own contexts because they keep state between calls.
+engine own their own contexts because they keep state between calls. Gradients,
+gathers, kicks and drifts may run on several streams at once; a deposit uses its
+context's mass grid and scratch, so deposits of one (device, grid size, dx) on
+different streams are to be ordered by their caller.
 """
 
 from __future__ import annotations

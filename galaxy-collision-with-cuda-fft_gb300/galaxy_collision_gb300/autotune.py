@@ -4,7 +4,7 @@ Some of the engine's choices change its speed and nothing else (the states are
 bit-identical, or every solve still meets the same tolerance): the cell-sort
 period (``sort_every``, with the look-ahead at half the period), and
 ``phase_launches``, which no longer changes anything and stays so that older
-cache files keep their meaning. ``tune`` times every candidate on a short run of a given
+cache files keep their meaning. ``tune`` times every program on a short run of a given
 state (CUDA events around whole-step graph replays) and caches the fastest
 under the key ``<device>/G<grid>/N2^<k>`` (k = floor(log2 particle count)) in
 a JSON file: ``$GC_AUTOTUNE_CACHE`` or ``~/.cache/galaxy_collision_gb300/

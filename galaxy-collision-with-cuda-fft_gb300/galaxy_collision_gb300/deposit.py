@@ -2,8 +2,8 @@
 
 Drop-in for the reference module src/galaxy_collision/deposit.py: same function
 names, arguments and node-centred convention (node (i,j,k) at (i,j,k)*dx;
-out-of-box weight dropped, never wrapped). Each call is one launch of a
-hand-written sm_103a kernel through ``libgcpm.so``:
+out-of-box weight dropped, never wrapped). Each call runs a few hand-written
+sm_103a kernels of ``libgcpm.so`` on the current stream, without a host wait:
 
 * :func:`deposit_density` -- CIC deposit (deposit.py:47-82, 177-182). The
   reference's per-corner f32 contributions are summed in int64 fixed point, so

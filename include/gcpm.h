@@ -182,6 +182,9 @@ int gc_level_info(const gc_ctx *ctx, int level, int *n_nodes, int *last_interior
  * weight. Accumulates in int64 fixed point (quantum 2^-fixed_point_bits of the
  * total), so rho is bit-identical run to run whatever the particle order.
  * fixed_point_bits must be in [24, 62 - ceil(log2 G)] (GC_ERR_ARG otherwise).
+ * Many particles in no order are binned by tiles first, with scratch of at most
+ * 671 MB that the context keeps (not under stream capture). Uses the context's
+ * mass grid: deposits on one context are ordered by the caller.
  * Replaces _deposit_cic / deposit_density (deposit.py:47-82, 177-182). */
 int gc_deposit_cic(gc_ctx *ctx, const float *x, const float *y, const float *z, const float *m,
                    int64_t n, int fixed_point_bits, float *rho);
@@ -212,7 +215,10 @@ int gc_deposit_cic_noalloc(const float *x, const float *y, const float *z, const
 int gc_potential_to_accel(gc_ctx *ctx, const float *phi, float *ax, float *ay, float *az);
 
 /* Trilinear gather of the node acceleration field to particles; out-of-box
- * nodes contribute zero. Replaces _gather_accel / gather_acceleration
+ * nodes contribute zero. Touches nothing of the context: gathers on one context
+ * may run on several streams at once (4M particles or more in no order take 16
+ * bytes a node of the device's scratch pool, where they can be had).
+ * Replaces _gather_accel / gather_acceleration
  * (deposit.py:85-129, 185-201). */
 int gc_gather_accel(gc_ctx *ctx, const float *x, const float *y, const float *z, int64_t n,
                     const float *ax_g, const float *ay_g, const float *az_g,
