@@ -899,7 +899,7 @@ __device__ __forceinline__ int near_pairs(float px, float py, float pz, float dx
 
 // Whether the particles come scattered: of 32 stretches of DEP_WTILE, spread over the
 // array, most span more cells than a warp's box of k_deposit_sorted, and fewer than half
-// of their neighbours lie near each other. (Few particles in the order of their cells do the
+// of the neighbours among the first 64 of each lie near each other. (Few particles in the order of their cells do the
 // first, and yet their corners share sectors of the grid: 4.3M on 256^3 172 us one by one,
 // 305 binned; drifted by a third of a cell 211 and 278, by a whole one 264 and 272, 8M so
 // 409 and 341.)
@@ -916,7 +916,7 @@ __global__ void __launch_bounds__(1024)
   for (int j = 0; j < DEP_WTILE / 32; ++j) {
     const long long p = p0 + 32 * j + lane;
     const float c[3] = {x[p], y[p], z[p]};
-    pairs += near_pairs(c[0], c[1], c[2], dx);
+    if (j < 2) pairs += near_pairs(c[0], c[1], c[2], dx);
 #pragma unroll
     for (int a = 0; a < 3; ++a) { lo[a] = fminf(lo[a], c[a]); hi[a] = fmaxf(hi[a], c[a]); }
   }
@@ -943,7 +943,7 @@ __global__ void __launch_bounds__(1024)
       t += fit[w];
       q += near[w];
     }
-    *scattered = t < 16 && q < 32 * (DEP_WTILE / 32) * 31 / 2;
+    *scattered = t < 16 && q < 32 * 2 * 31 / 2;
   }
 }
 
