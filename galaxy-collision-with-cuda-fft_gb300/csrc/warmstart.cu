@@ -314,8 +314,7 @@ __global__ void __launch_bounds__(256) k_conv_fwd(const __grid_constant__ ConvFw
   const uint32_t tile_u32 = umma::smem_u32(tile), ring_u32 = umma::smem_u32(ring);
   uint32_t ph0 = 0u, ph1 = 0u;  // next completion parity of each slot's barrier
   int last = 0;                  // slot of the last commit
-  // (the whole warp's: a warp that gave up on the tile issues nothing, but commits)
-  bool fail = !__all_sync(0xffffffffu, !a.use_map || umma::mbar_wait(&bars[2], 0, WS_WAIT_BUDGET));
+  bool fail = a.use_map && !umma::mbar_wait(&bars[2], 0, WS_WAIT_BUDGET);  // (then nothing is stored)
   for (int g = 0; g < ngroups; ++g) {
     const int s = g & 1;
     if (warp < WS_ISSUERS) {  // issuer w owns the M tiles mt = w (mod WS_ISSUERS)
@@ -331,7 +330,7 @@ __global__ void __launch_bounds__(256) k_conv_fwd(const __grid_constant__ ConvFw
       // (16 -> 16 channels, R = 128), so 40: the operand rows are 32 clk to read.
       const uint32_t kstep_a = (2u * a_lbo) >> 4, kstep_b = (2u * b_lbo) >> 4;
       const int nks = kci / 2;
-      for (int t = fail ? t1 : t0; t < t1; ++t) {
+      for (int t = t0; t < t1; ++t) {
         const uint64_t bd = bd0 + (((uint32_t)s * slot_bytes + (uint32_t)(t - t0) * tap_bytes) >> 4);
         uint64_t ad = ad0 + (uint32_t)(L0 + 128 * warp + tap_offset(t, P, W2));
         uint32_t td = tmem + (uint32_t)(warp * Cn);
@@ -348,7 +347,7 @@ __global__ void __launch_bounds__(256) k_conv_fwd(const __grid_constant__ ConvFw
     if (g + 1 < ngroups) {
       const int s1 = (g + 1) & 1;
       if (g >= 1) {
-        fail |= !umma::mbar_wait(&bars[s1], s1 ? ph1 : ph0, WS_WAIT_BUDGET);
+        fail = !umma::mbar_wait(&bars[s1], s1 ? ph1 : ph0, WS_WAIT_BUDGET);
         if (s1) ph1 ^= 1u; else ph0 ^= 1u;
       }
       if (__syncthreads_or(fail)) { fail = true; break; }
